@@ -1318,6 +1318,8 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     }
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_root[1], err, 4, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = image_shape(pool, map, nodes, st.voxel, scal, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&st.unshaped, scal, 4, cudaMemcpyDeviceToHost, s);
     if (x) {
         x->dots_of_id.resize(nodes);
         if (e == cudaSuccess && x->order)

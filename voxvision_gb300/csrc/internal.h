@@ -44,7 +44,13 @@ struct ImageStats {
     uint64_t nodes, units, inner, leaf, dense, dots, depth;
     float bbox[6];
     float voxel[3];
+    uint32_t unshaped;   // SHAPE_* bits the image does not have (image_shape)
 };
+
+/* The SHAPE_* bits (traverse.cuh) an image on the device does not have, into
+ * the device word `word`; enqueued on s (voxtrees_cuda.cu). */
+cudaError_t image_shape(const uint4 *pool, const uint32_t *rec_of_id, uint64_t nodes, const float voxel[3],
+                        uint32_t *word, cudaStream_t s);
 
 /* Makes t serve a device image built in place: `pool` (st.units 16-byte
  * units) and `map` (st.nodes pre-order id -> record entries), both

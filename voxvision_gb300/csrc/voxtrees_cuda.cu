@@ -417,6 +417,35 @@ __global__ void SQUARES_BOUNDS render_squares_kernel(DevTree t, vox_cuda_camera 
     if (overflow) atomicOr(status, 1u);
 }
 
+// What the searches may rely on in the image (SHAPE_* of traverse.cuh),
+// checked record by record: *bad gets the bits that do not hold.
+__global__ void __launch_bounds__(256) image_shape_kernel(const uint4 *__restrict__ pool,
+                                                          const uint32_t *__restrict__ rec_of_id, uint32_t n_nodes,
+                                                          float vx, float vy, float vz, uint32_t *__restrict__ bad)
+{
+    using vox::ubf;
+    auto fine = [](float v) { return fabsf(v) <= vox::SHAPE_LIMIT; };   // false for NaN
+    bool ok = fine(vx) && fine(vy) && fine(vz) && vx > 0.0f && vy > 0.0f && vz > 0.0f;
+    const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id < n_nodes) {
+        const uint32_t rec = rec_of_id[id];
+        const uint4 a = pool[rec], b = pool[rec + 1], c = pool[rec + 2];
+        ok = ok && fine(ubf(a.x)) && fine(ubf(a.y)) && fine(ubf(a.z)) && fine(ubf(a.w)) && fine(ubf(b.x)) &&
+             fine(ubf(b.y)) && ubf(a.x) <= ubf(a.w) && ubf(a.y) <= ubf(b.x) && ubf(a.z) <= ubf(b.y);
+        const uint32_t kind = b.z & 3u;
+        if (kind == VOXP_KIND_INNER) {
+            ok = ok && fine(ubf(c.x)) && fine(ubf(c.y)) && fine(ubf(c.z));
+        } else if (kind == VOXP_KIND_LEAF) {
+            const uint32_t n = b.z >> 2;
+            for (uint32_t i = 0; i < n && ok; i++) {
+                const uint4 v = pool[b.w + i];
+                ok = fine(ubf(v.x)) && fine(ubf(v.y)) && fine(ubf(v.z));
+            }
+        }
+    }
+    if (__any_sync(0xFFFFFFFFu, !ok) && (threadIdx.x & 31) == 0) atomicOr(bad, vox::SHAPE_ORDERED);
+}
+
 // ---------------------------------------------------------------- launchers
 
 // Batches of at least this many rays are traced in coherent order (raysort.cu).
@@ -905,6 +934,19 @@ EXPORT int vox_cuda_build_checked(void) { return vox::CHECKED ? 1 : 0; }
 
 EXPORT uint64_t vox_cuda_launch_count(void) { return g_launches.load(); }
 
+// The SHAPE_* bits of an image on the device, enqueued on s: `word` (device)
+// holds the bits that do not hold once s has run.
+cudaError_t image_shape(const uint4 *pool, const uint32_t *rec_of_id, uint64_t nodes, const float voxel[3],
+                        uint32_t *word, cudaStream_t s)
+{
+    cudaError_t e = cudaMemsetAsync(word, 0, 4, s);
+    if (e != cudaSuccess || nodes == 0) return e;
+    image_shape_kernel<<<(unsigned)((nodes + 255) / 256), 256, 0, s>>>(pool, rec_of_id, (uint32_t)nodes, voxel[0],
+                                                                       voxel[1], voxel[2], word);
+    count_launch();
+    return cudaGetLastError();
+}
+
 // Flattens `root` into t (host maps) and copies the image to the device,
 // reusing t's device buffers when they are large enough.  On failure t keeps
 // its previous contents when `keep` is set (a refresh), else is left empty.
@@ -942,10 +984,15 @@ static int load_tree(vox_cuda_tree *t, const struct vox_node *root, int layout =
         if (new_map) cudaFree(map);
         return VOX_CUDA_ENOMEM;
     }
-    cudaError_t e = cudaMemset(t->d_status, 0, 4);
-    if (e == cudaSuccess && flat.units.size())
+    uint32_t unshaped = 0;
+    cudaError_t e = cudaSuccess;
+    if (flat.units.size())
         e = cudaMemcpy(pool, flat.units.data(), flat.units.size() * 16, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && nodes) e = cudaMemcpy(map, flat.rec_of_id.data(), nodes * 4, cudaMemcpyHostToDevice);
+    // (the status word is the check's output first, then cleared)
+    if (e == cudaSuccess) e = image_shape(pool, map, nodes, flat.voxel, t->d_status, cudaStreamLegacy);
+    if (e == cudaSuccess) e = cudaMemcpy(&unshaped, t->d_status, 4, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemset(t->d_status, 0, 4);
     // A copy from pageable memory may still be in flight when cudaMemcpy
     // returns; the pool must be complete before any kernel on any stream
     // reads it (the frame kernel reads it ahead of its stream dependency).
@@ -983,6 +1030,7 @@ static int load_tree(vox_cuda_tree *t, const struct vox_node *root, int layout =
     uint64_t steps = (uint64_t)nodes + flat.n_dots + 2;
     t->dev.max_steps = steps > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)steps;
     t->dev.n_units = (uint32_t)units;
+    t->dev.shape = vox::SHAPE_ORDERED & ~unshaped;
     t->dev.fault = t->d_status;
     t->n_nodes = nodes;
     t->n_units = flat.units.size();
@@ -1037,6 +1085,7 @@ int adopt_image(vox_cuda_tree *t, uint4 *pool, size_t pool_bytes, uint32_t *map,
     uint64_t steps = st.nodes + st.dots + 2;
     t->dev.max_steps = steps > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)steps;
     t->dev.n_units = (uint32_t)(empty ? VOXP_REC_UNITS : st.units);
+    t->dev.shape = vox::SHAPE_ORDERED & ~st.unshaped;
     t->dev.fault = t->d_status;
     t->n_nodes = st.nodes;
     t->n_units = empty ? 0 : st.units;
