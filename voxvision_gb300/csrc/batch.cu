@@ -141,14 +141,12 @@ __device__ __forceinline__ void run_clear(const BatchJobDev &J, uint32_t c, uint
     }
 }
 
-// Register bound of the persistent kernels: 8 resident blocks of 128 threads
-// per SM (at most 64 registers; the 8x4 batch kernel now fits in 62 with
-// nothing spilled).  On the 120-frame 1080p orbit this drew 12% faster than
-// the unbounded build (68 registers, 7 blocks); 10 and 12 blocks (48 and 40
-// registers) spill more and draw slower.
-#ifndef BATCH_MIN_BLOCKS
-#define BATCH_MIN_BLOCKS 8
-#endif
+// Register bounds of the persistent kernels, in resident blocks of 128 threads
+// per SM.  32 frames of the 1080p orbit in the batch kernel take 1,298 us with
+// 7 blocks (72 registers), 1,310 with 8 (64) and 1,360 with 6; 24 host frames
+// in the frames kernel take 1,188 us with 6 blocks (its item count keeps more
+// values live), 1,200 with 7 and 1,270 with 8.
+constexpr int BATCH_MIN_BLOCKS = 7, FRAMES_MIN_BLOCKS = 6;
 
 // Queue index -> frame: the last job whose tile (or clearing) base is <=
 // item (frames with no item of that kind share their base with the next
@@ -203,7 +201,7 @@ __global__ void __launch_bounds__(128, BATCH_MIN_BLOCKS) batch_kernel(const Batc
 // count then finds the item's stores long complete instead of waiting for
 // them (the 120-frame 1080p orbit call 7.41 against 7.43 ms).
 template <int CAP, int TW, int TH>
-__global__ void __launch_bounds__(128, BATCH_MIN_BLOCKS) frames_kernel(const BatchHead *__restrict__ head, uint32_t grab,
+__global__ void __launch_bounds__(128, FRAMES_MIN_BLOCKS) frames_kernel(const BatchHead *__restrict__ head, uint32_t grab,
                                                      uint32_t *__restrict__ counter, uint32_t *__restrict__ done,
                                                      uint32_t *flags, uint32_t epoch)
 {

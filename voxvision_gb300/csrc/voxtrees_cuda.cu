@@ -62,8 +62,13 @@ __device__ __forceinline__ void add_counts(unsigned long long *counts, const Cou
     }
 }
 
+// Threads of a ray block: a block holds its place on the SM until its slowest
+// ray is done, so smaller blocks leave less of it idle (4M incoherent rays:
+// 533 us in blocks of 128, 564 in blocks of 256; 64 are no better).
+constexpr int RAY_THREADS = 128;
+
 template <int CAP, bool COUNT>
-__global__ void __launch_bounds__(256) ray_kernel(DevTree t, const float *__restrict__ o,
+__global__ void __launch_bounds__(RAY_THREADS) ray_kernel(DevTree t, const float *__restrict__ o,
                                                   const float *__restrict__ d,
                                                   const uint32_t *__restrict__ roots, size_t n,
                                                   uint32_t *__restrict__ leaf, uint8_t *__restrict__ slot,
@@ -171,8 +176,15 @@ __device__ __forceinline__ void clear_outside(const FramePlan &p, uint32_t w, ui
     }
 }
 
-template <int CAP, bool COUNT, int MINB, bool LIT>
-__global__ void __launch_bounds__(128, MINB) render_kernel(DevTree t, vox_cuda_camera cam, uint32_t w, uint32_t h,
+// Resident blocks per SM of the frame kernel: 8, the registers its warps want
+// (at most 64, nothing spilled).  A build of 12 blocks (40 registers) for
+// frames enqueued back to back is no faster with the mirrored search (a 1080p
+// orbit frame 59.6 us against 60.2, a 256x256 frame 4.9 against 4.0), and alone
+// its frames take 98 us against 88.
+constexpr int RENDER_MIN_BLOCKS = 8;
+
+template <int CAP, bool COUNT, bool LIT>
+__global__ void __launch_bounds__(128, RENDER_MIN_BLOCKS) render_kernel(DevTree t, vox_cuda_camera cam, uint32_t w, uint32_t h,
                                                      FramePlan p, const uint8_t *__restrict__ tex,
                                                      uint32_t *__restrict__ argb,
                                                      unsigned long long *__restrict__ counts,
@@ -237,15 +249,11 @@ __device__ __forceinline__ void pixel_dir(const vox_cuda_camera &cam, const floa
     }
 }
 
-// Register bound of render_squares_kernel: none by default (72 registers, 7
-// blocks of 128 threads per SM).  Bounds of 8 and 9 blocks (64 and 56
-// registers, with spills) drew the 1080p orbit's FAST and ADAPTIVE frames 1-3%
-// slower.
-#ifdef SQUARES_MIN_BLOCKS
-#define SQUARES_BOUNDS __launch_bounds__(128, SQUARES_MIN_BLOCKS)
-#else
-#define SQUARES_BOUNDS __launch_bounds__(128)
-#endif
+// Register bound of render_squares_kernel: 7 blocks of 128 threads per SM (72
+// registers).  Unbounded it takes 80 (6 blocks): the 1080p orbit's ADAPTIVE
+// frames take 77.6 us with the bound and 79.2 without, the near 4K FAST frame
+// 1,040 and 1,070 us; 8 blocks give 78.5 and 1,033 us.
+constexpr int SQUARES_MIN_BLOCKS = 7;
 
 // FAST and ADAPTIVE frames, and with a ray buffer frames of every quality,
 // in one launch.  In renderer.c a pixel's leaf is either the previous
@@ -266,7 +274,8 @@ __device__ __forceinline__ void pixel_dir(const vox_cuda_camera &cam, const floa
 // same rays, the same choices between them; searches made for pixels the
 // walk then reaches another way are dropped.
 template <int CAP, bool RAYS>
-__global__ void SQUARES_BOUNDS render_squares_kernel(DevTree t, vox_cuda_camera cam, uint32_t w, uint32_t h,
+__global__ void __launch_bounds__(128, SQUARES_MIN_BLOCKS)
+render_squares_kernel(DevTree t, vox_cuda_camera cam, uint32_t w, uint32_t h,
                                                      FramePlan fp, unsigned int quality,
                                                      const uint8_t *__restrict__ tex, uint32_t *__restrict__ argb,
                                                      uint32_t *__restrict__ status, vox::DevLights lights,
@@ -468,7 +477,7 @@ cudaError_t launch_rays(const vox_cuda_tree *t, const float *o, const float *d, 
             return e;
         }
     }
-    dim3 block(256), grid((unsigned)((n + 255) / 256));
+    dim3 block(RAY_THREADS), grid((unsigned)((n + RAY_THREADS - 1) / RAY_THREADS));
     switch (t->cap_class) {
     case 0: ray_kernel<CAP0, COUNT><<<grid, block, 0, s>>>(t->dev, o, d, roots, n, leaf, slot, pts, counts, t->d_status, order); break;
     case 1: ray_kernel<CAP1, COUNT><<<grid, block, 0, s>>>(t->dev, o, d, roots, n, leaf, slot, pts, counts, t->d_status, order); break;
@@ -514,19 +523,10 @@ cudaError_t launch_balls(const vox_cuda_tree *t, const float *c, const float *r,
 // Process-wide settings of the BEST frame kernel (vox_cuda_render_set_config).
 std::atomic<uint32_t> g_render_cull{1}, g_render_overlap{1};
 
-// Two builds of the frame kernel draw the same frame.  A frame that is
-// waited for on its own (the host-buffer calls) is bound by its slowest
-// warps, which run fastest with the registers they want (8 blocks per SM).
-// Frames enqueued back to back (the device calls) overlap one another, and
-// there more warps per SM hide more latency: 12 blocks per SM, at the cost of
-// a few spilled registers.
-constexpr int MINB_ALONE = 8, MINB_PIPELINED = 12;
-
 template <bool COUNT>
 cudaError_t launch_render(const vox_cuda_tree *t, const vox_cuda_camera &cam, uint32_t w, uint32_t h,
                           const uint8_t *tex, uint32_t *argb, unsigned long long *counts, cudaStream_t s,
-                          bool pipelined = false, const vox::DevLights *lights = nullptr,
-                          vox::FrameMemo *memo = nullptr)
+                          const vox::DevLights *lights = nullptr, vox::FrameMemo *memo = nullptr)
 {
     // the counting kernel counts the reference's work: every pixel traced
     FramePlan p;
@@ -538,22 +538,12 @@ cudaError_t launch_render(const vox_cuda_tree *t, const vox_cuda_camera &cam, ui
     if (lights) L = *lights;
     const bool lit = !COUNT && L.on;
     const int cap = t->cap_class;
-    if (lit) {
-        if (pipelined) kern = cap == 0 ? render_kernel<CAP0, COUNT, MINB_PIPELINED, true>
-                            : cap == 1 ? render_kernel<CAP1, COUNT, MINB_PIPELINED, true>
-                                       : render_kernel<CAP2, COUNT, MINB_PIPELINED, true>;
-        else kern = cap == 0 ? render_kernel<CAP0, COUNT, MINB_ALONE, true>
-                  : cap == 1 ? render_kernel<CAP1, COUNT, MINB_ALONE, true>
-                             : render_kernel<CAP2, COUNT, MINB_ALONE, true>;
-    } else if (pipelined && !COUNT) {
-        kern = cap == 0 ? render_kernel<CAP0, COUNT, MINB_PIPELINED, false>
-             : cap == 1 ? render_kernel<CAP1, COUNT, MINB_PIPELINED, false>
-                        : render_kernel<CAP2, COUNT, MINB_PIPELINED, false>;
-    } else {
-        kern = cap == 0 ? render_kernel<CAP0, COUNT, MINB_ALONE, false>
-             : cap == 1 ? render_kernel<CAP1, COUNT, MINB_ALONE, false>
-                        : render_kernel<CAP2, COUNT, MINB_ALONE, false>;
-    }
+    if (lit)
+        kern = cap == 0 ? render_kernel<CAP0, COUNT, true>
+             : cap == 1 ? render_kernel<CAP1, COUNT, true> : render_kernel<CAP2, COUNT, true>;
+    else
+        kern = cap == 0 ? render_kernel<CAP0, COUNT, false>
+             : cap == 1 ? render_kernel<CAP1, COUNT, false> : render_kernel<CAP2, COUNT, false>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.ntiles + p.nclear);
     cfg.blockDim = dim3(128);
@@ -1392,7 +1382,7 @@ EXPORT int vox_cuda_render_device(const vox_cuda_tree *t, const vox_cuda_camera 
 try {
     int rc = check_render_args(t, cam, w, h, tex, argb);
     if (rc) return rc;
-    return status_of(launch_render<false>(t, *cam, w, h, tex, argb, nullptr, as_stream(stream), true));
+    return status_of(launch_render<false>(t, *cam, w, h, tex, argb, nullptr, as_stream(stream)));
 } VOX_ABI_FAIL_INT
 
 // Per host thread and device: what the synchronous host-buffer frame calls
@@ -1773,7 +1763,7 @@ try {
     if (!d_argb) return VOX_CUDA_ENOMEM;
     FrameMemo m{false, 0, 0, 0, 0};
     cudaError_t e = host_call_texture(hc, tex, s);
-    if (e == cudaSuccess) e = launch_render<false>(t, *cam, w, h, hc->d_tex, d_argb, nullptr, s, false, nullptr, &m);
+    if (e == cudaSuccess) e = launch_render<false>(t, *cam, w, h, hc->d_tex, d_argb, nullptr, s, nullptr, &m);
     if (e == cudaSuccess) e = host_frame_out(hc, argb, d_argb, w, h, m, s);
     return host_call_finish(hc, t, s, e);
 } VOX_ABI_FAIL_INT
@@ -1962,7 +1952,7 @@ int render_frame_memo(const vox_cuda_tree *t, const vox_cuda_camera *cam, const 
     if (!valid_quality(quality)) return VOX_CUDA_EINVAL;
     const vox::DevLights *L = lights ? &lights->dev : nullptr;
     if (!dirs && (quality & VOX_CUDA_QUALITY_MODE_MASK) == VOX_CUDA_QUALITY_BEST)
-        return status_of(launch_render<false>(t, *cam, w, h, tex, argb, nullptr, s, true, L, memo));
+        return status_of(launch_render<false>(t, *cam, w, h, tex, argb, nullptr, s, L, memo));
     return status_of(launch_render_squares(t, *cam, w, h, quality, tex, argb, s, L, dirs, memo));
 }
 
