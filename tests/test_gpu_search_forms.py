@@ -103,3 +103,50 @@ def test_both_forms_of_the_search_match_the_oracle(kind, voxel, shift):
     finally:
         vg.set_voxel_size((1, 1, 1))
         orc.set_voxel((1, 1, 1))
+
+
+def _balls(kind, seed, box, voxel):
+    r = np.random.RandomState(seed)
+    lo, hi = box
+    n = 4096
+    c = (lo - 3 + (hi - lo + 6) * r.random_sample((n, 3))).astype(np.float32)
+    rad = (4 * np.abs(voxel).max() * r.random_sample(n)).astype(np.float32)
+    if kind == "touching":   # the radius is the float distance to a cell face, or one step to either side
+        face = np.rint(c[np.arange(n), r.randint(0, 3, n)]).astype(np.float32)
+        rad = np.abs(face - c[np.arange(n), r.randint(0, 3, n)]).astype(np.float32)
+        rad = np.nextafter(rad, np.array([-1e9, 1e9], np.float32)[r.randint(0, 2, n)]).astype(np.float32)
+        c[::2] = np.rint(c[::2] / voxel) * voxel
+        rad[::2] = (np.rint(rad[::2]) * np.abs(voxel[0])).astype(np.float32)
+    elif kind == "odd numbers":
+        odd = np.array([np.nan, np.inf, -np.inf, 3e38, -3e38, 1e-40, -0.0, 1e25], np.float32)
+        rad[::3] = odd[r.randint(0, 8, len(rad[::3]))]
+        c[np.arange(1, n, 3), r.randint(0, 3, len(c[1::3]))] = odd[r.randint(0, 8, len(c[1::3]))]
+        rad[2::6] = -rad[2::6]
+    return np.ascontiguousarray(c), np.ascontiguousarray(rad)
+
+
+@pytest.mark.parametrize("voxel,shift", [((1, 1, 1), (0, 0, 0)), ((0.5, 1, 2), (3, -5, 40)), ((1, -1, 1), (0, 0, 0))])
+@pytest.mark.parametrize("kind", ["plain", "touching", "odd numbers"])
+@pytest.mark.parametrize("off_grid", [False, True])
+def test_both_forms_of_the_ball_search_match_the_oracle(kind, voxel, shift, off_grid):
+    import voxvision_gb300 as vg
+    try:
+        vg.set_voxel_size(voxel)   # a negative size gives unordered boxes: the general form
+        orc.set_voxel(voxel)
+        vox = _voxels(5, voxel, shift)
+        if off_grid:               # voxels that reach past the dividing planes
+            vox += np.random.RandomState(3).uniform(-0.4, 0.4, vox.shape).astype(np.float32)
+        ht = vg.HostTree.from_voxels(vox)
+        box = vox.min(0).astype(np.float64), vox.max(0).astype(np.float64) + np.abs(voxel)
+        c, rad = _balls(kind, 11, box, np.asarray(voxel, np.float64))
+        want, _ = orc.ball_batch(ht.ptr, c, rad)
+        if kind == "plain" and voxel[1] > 0:
+            assert 0.1 < want.mean() < 0.95
+        for dt in (vg.DeviceTree(ht.ptr), vg.DeviceTree.build(vox)):
+            assert np.array_equal(dt.balls(c, rad), want)
+        # one voxel, whose record is the root
+        one = vg.HostTree.from_voxels(vox[:1])
+        assert np.array_equal(vg.DeviceTree(one.ptr).balls(c, rad), orc.ball_batch(one.ptr, c, rad)[0])
+    finally:
+        vg.set_voxel_size((1, 1, 1))
+        orc.set_voxel((1, 1, 1))

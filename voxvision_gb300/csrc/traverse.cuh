@@ -46,7 +46,11 @@ struct DevTree {
 // SHAPE_LIMIT in magnitude, and min <= max on every axis (the voxel size
 // positive).  Trees that vox_make_tree or the GPU build make from ordinary
 // voxels have it; a caller's own tree need not.
-constexpr uint32_t SHAPE_ORDERED = 1u;
+//
+// SHAPE_NESTED: every child's box and every leaf's voxel lie inside their
+// node's box, and a child on the lower side of a dividing plane reaches at
+// most one voxel past it, one on the upper side not below it.
+constexpr uint32_t SHAPE_ORDERED = 1u, SHAPE_NESTED = 2u;
 constexpr float SHAPE_LIMIT = 1.152921504606847e18f;   // 2^60
 
 struct Counts {
@@ -769,6 +773,98 @@ __device__ __forceinline__ bool trace_ball(const DevTree &t, float cx, float cy,
         if (sp == 0) return false;
         cur = stack[--sp];
     }
+}
+
+/* The same answer in a tree of ordered, nested boxes, where it depends on no
+ * order: a ball hits when any voxel's or dense leaf's own test passes.
+ *
+ * In round-to-nearest arithmetic the test is monotone -- a box inside
+ * another is no nearer on any axis, nor, squared and summed in the same
+ * order, in all -- so the tests of the nodes above a voxel that passes pass
+ * too, and pruning by them (search.c:160) changes nothing.  By the same
+ * monotony a child needs no test when on one axis the ball stays its radius
+ * away from all that lies on the child's side of the dividing plane: the
+ * child's own distance there is at least the radius, its square at least the
+ * radius's square (ball_side).
+ *
+ * What bounds the search is instruction issue at few active lanes.  A ball
+ * small beside the upper nodes can meet one or two of their eight children,
+ * so leaving the others out takes a search from 45 box tests to 13 on
+ * average (balls of radius 0.5-8 in the 256^3 tree), and the child where the
+ * centre lies goes first, where a voxel is likeliest.  One record a step
+ * keeps the lanes of a warp alike; testing all of a node's children in one
+ * step, handing idle lanes new balls, and accepting nodes of which the ball
+ * holds a whole face were each slower (see launch_balls). */
+// The octants (a bit each, as in a child mask) a ball can meet on one axis:
+// none below the dividing plane when it stays r above the highest face a
+// voxel there can have, none above when it stays r below the plane.  `low` is
+// the axis's octants below the plane (geom.c:44-51: their bit is set).
+__device__ __forceinline__ uint32_t ball_side(float c, float plane, float v, float r, uint32_t low)
+{
+    uint32_t m = 0xFFu;
+    if (__fsub_rn(c, __fadd_rn(plane, v)) >= r) m = ~low;
+    if (__fsub_rn(plane, c) >= r) m = low;
+    return m;
+}
+
+template <int CAP>
+__device__ __forceinline__ bool trace_ball_nested(const DevTree &t, float cx, float cy, float cz, float r, bool &overflow)
+{
+    if (t.root == VOXP_EMPTY || !(cx == cx && cy == cy && cz == cz && r == r)) return false;   // NaN is near nothing
+    const uint4 *pool = t.pool;
+    const float rr = __fmul_rn(r, r);
+    r = fabsf(r);
+    uint32_t stack[CAP];
+    int sp = 0;
+    uint32_t cur = t.root;
+    for (uint32_t steps = 0; steps < t.max_steps; steps++) {
+        if (!in_range(cur, VOXP_REC_UNITS, t.n_units, t.fault)) break;
+        const uint4 a = ld16(pool + cur), b = ld16(pool + cur + 1), c = ld16(pool + cur + 2);
+        const float ex = fmaxf(fmaxf(__fsub_rn(ubf(a.x), cx), __fsub_rn(cx, ubf(a.w))), 0.0f),
+                    ey = fmaxf(fmaxf(__fsub_rn(ubf(a.y), cy), __fsub_rn(cy, ubf(b.x))), 0.0f),
+                    ez = fmaxf(fmaxf(__fsub_rn(ubf(a.z), cz), __fsub_rn(cz, ubf(b.y))), 0.0f);
+        const float s = __fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez));
+        bool pop = true;
+        if (s < rr) {
+            const uint32_t kind = b.z & 3u, link = b.w;
+            if (kind == VOXP_KIND_DENSE) return true;
+            if (kind == VOXP_KIND_LEAF) {
+                const uint32_t n = b.z >> 2;
+                if (!in_range(link, n, t.n_units, t.fault)) break;
+                for (uint32_t j = 0; j < n; j++) {
+                    const uint4 v = ld16(pool + link + j);
+                    const float vx = ubf(v.x), vy = ubf(v.y), vz = ubf(v.z);
+                    if (ball_box(vx, vy, vz, __fadd_rn(vx, t.vx), __fadd_rn(vy, t.vy), __fadd_rn(vz, t.vz), cx, cy, cz, rr))
+                        return true;
+                }
+            } else {
+                const uint32_t mask = (b.z >> 8) & 0xFFu;
+                uint32_t left = mask & ball_side(cx, ubf(c.x), t.vx, r, 0xAAu) & ball_side(cy, ubf(c.y), t.vy, r, 0xCCu) &
+                                ball_side(cz, ubf(c.z), t.vz, r, 0xF0u);
+                if (left) {
+                    // the octant of the centre first, else the first one
+                    const uint32_t home = 1u << ((uint32_t)(ubf(c.x) > cx) | ((uint32_t)(ubf(c.y) > cy) << 1) |
+                                                 ((uint32_t)(ubf(c.z) > cz) << 2));
+                    const uint32_t first = left & home ? home : left & (0u - left);
+                    left ^= first;
+                    cur = link + VOXP_REC_UNITS * (uint32_t)__popc(mask & (first - 1u));
+                    pop = false;
+                    if (sp + __popc(left) > CAP) break;
+                    while (left) {
+                        const uint32_t low = left & (0u - left);
+                        left ^= low;
+                        stack[sp++] = link + VOXP_REC_UNITS * (uint32_t)__popc(mask & (low - 1u));
+                    }
+                }
+            }
+        }
+        if (pop) {
+            if (sp == 0) return false;
+            cur = stack[--sp];
+        }
+    }
+    overflow = true;   // damaged pool
+    return false;
 }
 
 /* simple-camera.c:21-31 (+ vect-ops.c:7-15, :28-36) and doom-camera.c:24-57. */
