@@ -214,7 +214,7 @@ int vox_cuda_tree_node_id(const vox_cuda_tree *tree, const struct vox_node *node
  * (n x 3, written only on a hit, like `res`).  roots: NULL to start every
  * ray at the tree's root, else n pre-order indices of the node each search
  * starts from (vox_ray_tree_intersection accepts any node as its root;
- * renderer.c:297).  slot and points may be NULL.  Batches of 65,536 rays or
+ * renderer.c:297).  slot and points may be NULL.  Batches of 393,216 rays or
  * more are traced grouped by direction and origin (results are the same for
  * any order), with a stream-ordered scratch allocation (cudaMallocAsync) of
  * about 6 bytes per ray for that order.

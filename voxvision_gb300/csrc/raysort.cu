@@ -7,11 +7,10 @@
  * unrelated searches in every warp.  Tracing them grouped by the octant of
  * their direction, then by the cell of the point where they enter the tree's
  * box on an 8x8x8 grid over it (Morton order), makes the searches of a warp
- * start at the same part of the tree and walk it the same way: 16M random
- * rays over the 256^3 tree take 2.8 ms, sorting included, against 5.4 ms in
- * the given order.  Ball batches of 262,144 or more are grouped the same way
- * by the cell of their centre on a 16x16x16 grid over the tree's box: 1M
- * random balls take 0.40 ms, sorting included, against 0.47 ms.
+ * start at the same part of the tree and walk it the same way: 1M random
+ * rays over the 256^3 tree take 163 us, sorting included, against 223 in the
+ * given order.  Ball batches can be grouped the same way by the cell of their
+ * centre on a 16x16x16 grid over the tree's box (launch_balls says when).
  *
  * The order is a counting sort on those 12-bit keys: per block of up to
  * 65,536 items (fewer for smaller batches, so that every SM gets blocks) a
@@ -37,13 +36,13 @@ constexpr int KEY_BITS = 12;
 constexpr uint32_t NKEYS = 1u << KEY_BITS;
 constexpr int SORT_THREADS = 1024;
 
-// Items one block keys and places: 65,536 for large batches (256 blocks for
-// 16M rays), fewer for smaller ones so that a batch of a million still
-// spreads over the SMs (8,192 at least, which keeps the per-block
-// histograms small beside the items).
+// Items one block keys and places: 65,536 for large batches, for smaller ones
+// as many as give two blocks to each of 152 SMs (4M rays: 528 us searched and
+// all, 531 in 256 blocks, 535 in 152), 8,192 at least, which keeps the
+// per-block histograms small beside the items.
 size_t items_per_block(size_t n)
 {
-    size_t per = (n + 255) / 256;
+    size_t per = (n + 303) / 304;
     per = per < 8192 ? 8192 : (per > 65536 ? 65536 : per);
     return per;
 }
@@ -79,7 +78,7 @@ __device__ __forceinline__ uint32_t ray_key(const float *o, const float *d, size
     uint32_t oct = (d[3 * i] < 0.0f) | ((d[3 * i + 1] < 0.0f) << 1) | ((d[3 * i + 2] < 0.0f) << 2);
     float t0 = 0.0f, t1 = 3.0e38f;
     for (int a = 0; a < 3; a++) {
-        const float inv = 1.0f / d[3 * i + a];
+                const float inv = 1.0f / d[3 * i + a];
         float ta = (f.blo[a] - o[3 * i + a]) * inv, tb = (f.bhi[a] - o[3 * i + a]) * inv;
         if (ta > tb) { float x = ta; ta = tb; tb = x; }
         t0 = fmaxf(t0, ta);      // NaN (a zero direction inside the slab) keeps the bound
@@ -94,8 +93,9 @@ __device__ __forceinline__ uint32_t ray_key(const float *o, const float *d, size
 // Keys of a block's items and the block's histogram (block-major): rays
 // (d given) by ray_key, balls (d NULL) by the cell of their centre on a
 // 16^3 grid over the tree's box.
-__global__ void __launch_bounds__(SORT_THREADS) k_keys(const float *o, const float *d, size_t n, size_t per,
-                                                        KeyFrame f, uint16_t *keys, uint32_t *hist)
+__global__ void __launch_bounds__(SORT_THREADS) k_keys(const float *__restrict__ o, const float *__restrict__ d, size_t n,
+                                                        size_t per, KeyFrame f, uint16_t *__restrict__ keys,
+                                                        uint32_t *__restrict__ hist)
 {
     __shared__ uint32_t h[NKEYS];
     for (uint32_t k = threadIdx.x; k < NKEYS; k += SORT_THREADS) h[k] = 0;
@@ -110,52 +110,62 @@ __global__ void __launch_bounds__(SORT_THREADS) k_keys(const float *o, const flo
     for (uint32_t k = threadIdx.x; k < NKEYS; k += SORT_THREADS) hist[(size_t)blockIdx.x * NKEYS + k] = h[k];
 }
 
-// For every key: its count before each block (in place) and its total.
-__global__ void k_key_blocks(uint32_t *hist, uint32_t nblocks, uint32_t *total)
+// For every key: its count before each block (in place) and its total; a warp
+// a key, 32 blocks at a time.
+__global__ void __launch_bounds__(256) k_key_blocks(uint32_t *hist, uint32_t nblocks, uint32_t *total)
 {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= NKEYS) return;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t k = blockIdx.x * 8 + (threadIdx.x >> 5);
     uint32_t run = 0;
-    for (uint32_t b = 0; b < nblocks; b++) {
-        uint32_t c = hist[(size_t)b * NKEYS + k];
-        hist[(size_t)b * NKEYS + k] = run;
-        run += c;
+    for (uint32_t b0 = 0; b0 < nblocks; b0 += 32) {
+        const uint32_t b = b0 + lane;
+        const uint32_t c = b < nblocks ? hist[(size_t)b * NKEYS + k] : 0u;
+        uint32_t x = c;
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+            if (lane >= (uint32_t)off) x += y;
+        }
+        if (b < nblocks) hist[(size_t)b * NKEYS + k] = run + x - c;
+        run += __shfl_sync(0xFFFFFFFFu, x, 31);
     }
-    total[k] = run;
+    if (lane == 0) total[k] = run;
 }
 
-// Exclusive scan of the NKEYS totals in place (one block).
-__global__ void __launch_bounds__(1024) k_key_starts(uint32_t *total)
-{
-    __shared__ uint32_t part[1024];
-    constexpr uint32_t PER = NKEYS / 1024;
-    uint32_t v[PER], s = 0;
-    for (uint32_t j = 0; j < PER; j++) {
-        v[j] = total[threadIdx.x * PER + j];
-        s += v[j];
-    }
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (uint32_t off = 1; off < 1024; off <<= 1) {   // inclusive scan of the parts
-        uint32_t x = threadIdx.x >= off ? part[threadIdx.x - off] : 0u;
-        __syncthreads();
-        part[threadIdx.x] += x;
-        __syncthreads();
-    }
-    uint32_t run = part[threadIdx.x] - s;
-    for (uint32_t j = 0; j < PER; j++) {
-        total[threadIdx.x * PER + j] = run;
-        run += v[j];
-    }
-}
-
-// Each ray's slot in the traced order.
-__global__ void __launch_bounds__(SORT_THREADS) k_place(const uint16_t *keys, size_t n, size_t per,
-                                                         const uint32_t *hist, const uint32_t *start, uint32_t *order)
+// Each item's slot in the traced order: the keys' starts (an exclusive scan of
+// the totals, made by every block for itself), the counts of the blocks
+// before, then a place each.
+__global__ void __launch_bounds__(SORT_THREADS) k_place(const uint16_t *__restrict__ keys, size_t n, size_t per,
+                                                         const uint32_t *__restrict__ hist,
+                                                         const uint32_t *__restrict__ total, uint32_t *__restrict__ order)
 {
     __shared__ uint32_t base[NKEYS];
-    for (uint32_t k = threadIdx.x; k < NKEYS; k += SORT_THREADS)
-        base[k] = start[k] + hist[(size_t)blockIdx.x * NKEYS + k];
+    __shared__ uint32_t part[32];
+    constexpr uint32_t PER = NKEYS / SORT_THREADS;
+    static_assert(PER == 4, "a thread scans one 16-byte piece of the totals");
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint4 v = reinterpret_cast<const uint4 *>(total)[threadIdx.x];
+    const uint4 h = reinterpret_cast<const uint4 *>(hist + (size_t)blockIdx.x * NKEYS)[threadIdx.x];
+    const uint32_t sum = v.x + v.y + v.z + v.w;
+    uint32_t x = sum;
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+        if (lane >= (uint32_t)off) x += y;
+    }
+    if (lane == 31) part[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t p = part[lane];
+        uint32_t q = p;
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, q, off);
+            if (lane >= (uint32_t)off) q += y;
+        }
+        part[lane] = q - p;
+    }
+    __syncthreads();
+    const uint32_t first = part[warp] + x - sum;
+    reinterpret_cast<uint4 *>(base)[threadIdx.x] =
+        make_uint4(first + h.x, first + v.x + h.y, first + v.x + v.y + h.z, first + v.x + v.y + v.z + h.w);
     __syncthreads();
     size_t b0 = (size_t)blockIdx.x * per, b1 = b0 + per < n ? b0 + per : n;
     for (size_t i = b0 + threadIdx.x; i < b1; i += SORT_THREADS) order[atomicAdd(&base[keys[i]], 1u)] = (uint32_t)i;
@@ -194,10 +204,9 @@ static cudaError_t sort_order(const vox_cuda_tree *t, const float *o, const floa
         f.inv[a] = cells / fmaxf(t->bbox[3 + a] - t->bbox[a], 1e-30f);
     }
     k_keys<<<(unsigned)nb, SORT_THREADS, 0, s>>>(o, d, n, per, f, keys, hist);
-    k_key_blocks<<<NKEYS / 256, 256, 0, s>>>(hist, (uint32_t)nb, total);
-    k_key_starts<<<1, 1024, 0, s>>>(total);
+    k_key_blocks<<<NKEYS / 8, 256, 0, s>>>(hist, (uint32_t)nb, total);
     k_place<<<(unsigned)nb, SORT_THREADS, 0, s>>>(keys, n, per, hist, total, *order);
-    for (int i = 0; i < 4; i++) count_launch();
+    for (int i = 0; i < 3; i++) count_launch();
     return cudaGetLastError();
 }
 

@@ -492,7 +492,11 @@ __global__ void __launch_bounds__(256) image_shape_kernel(const uint4 *__restric
 // ---------------------------------------------------------------- launchers
 
 // Batches of at least this many rays are traced in coherent order (raysort.cu).
-constexpr size_t RAY_SORT_MIN = 1 << 16;
+// Below, the order costs more than it saves: 262,144 rays over the 64^3 /
+// 256^3 / 512^3 trees take 52 / 74 / 86 us as given and 69 / 85 / 103 sorted,
+// 393,216 take 65 / 101 / 125 and 77 / 101 / 126, 524,288 84 / 123 / 144 and
+// 83 / 110 / 136.
+constexpr size_t RAY_SORT_MIN = 3 << 17;
 
 template <bool COUNT>
 cudaError_t launch_rays(const vox_cuda_tree *t, const float *o, const float *d, const uint32_t *roots,
@@ -524,7 +528,11 @@ cudaError_t launch_rays(const vox_cuda_tree *t, const float *o, const float *d, 
 }
 
 // Batches of at least this many balls are searched grouped by centre cell.
-constexpr size_t BALL_SORT_MIN = 1 << 18;
+// The nested search walks so little of a tree that this pays only where the
+// image is too large for L2 to hold beside the queries: 1M / 4M balls of radius
+// 0.5-8 over the 512^3 tree (300 MB) take 242 / 783 us as given and 239 / 716
+// sorted, over the 256^3 tree (37 MB) 185 / 612 and 204 / 646.
+constexpr size_t BALL_SORT_MIN = 1 << 18, NESTED_SORT_MIN = 1 << 20, NESTED_SORT_BYTES = 64 << 20;
 
 template <bool COUNT>
 cudaError_t launch_balls(const vox_cuda_tree *t, const float *c, const float *r, size_t n, uint8_t *hit,
@@ -533,7 +541,10 @@ cudaError_t launch_balls(const vox_cuda_tree *t, const float *c, const float *r,
     if (n == 0) return cudaSuccess;
     void *scratch = nullptr;
     uint32_t *order = nullptr;
-    if (!COUNT && n >= BALL_SORT_MIN && n <= 0xFFFFFFFFull) {
+    constexpr uint32_t SHAPE = vox::SHAPE_ORDERED | vox::SHAPE_NESTED;
+    const bool nested = !COUNT && (t->dev.shape & SHAPE) == SHAPE;
+    const bool sorted = nested ? n >= NESTED_SORT_MIN && t->n_units * 16 > NESTED_SORT_BYTES : n >= BALL_SORT_MIN;
+    if (!COUNT && sorted && n <= 0xFFFFFFFFull) {
         cudaError_t e = cudaMallocAsync(&scratch, ray_order_bytes(n), s);
         if (e != cudaSuccess) return e;
         e = ball_order(t, c, n, scratch, &order, s);
@@ -543,11 +554,9 @@ cudaError_t launch_balls(const vox_cuda_tree *t, const float *c, const float *r,
         }
     }
     // A tree of ordered, nested boxes: the search that may choose its own order
-    // (1M balls of radius 0.5-8 over the 256^3 tree, sort included: 204 us
-    // against 341).  Counting calls count the reference's work, and other
+    // (1M balls of radius 0.5-8 over the 256^3 tree: 185 us against 341).  Counting calls count the reference's work, and other
     // trees (image_shape) take its own order.
-    constexpr uint32_t SHAPE = vox::SHAPE_ORDERED | vox::SHAPE_NESTED;
-    if (!COUNT && (t->dev.shape & SHAPE) == SHAPE) {
+    if (nested) {
         const dim3 block(BALL_THREADS), grid((unsigned)((n + BALL_THREADS - 1) / BALL_THREADS));
         switch (t->cap_class) {
         case 0: nested_ball_kernel<4 * CAP0><<<grid, block, 0, s>>>(t->dev, c, r, n, hit, t->d_status, order); break;
