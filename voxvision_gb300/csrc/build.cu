@@ -75,6 +75,7 @@ constexpr int SCAN_ITEMS = 8;
 constexpr uint32_t SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 constexpr uint32_t BIG = 4096;       // nodes with more voxels sum their coordinates by chunks
 constexpr uint32_t SMALL = 512;      // nodes with at most this many voxels are split by one warp
+constexpr uint32_t MID = 8192;       // nodes with at most this many by one block, larger ones tile by tile
 constexpr uint32_t TINY = 32;        // nodes with at most this many voxels get their box from one thread
 constexpr uint32_t CHUNK = 1024;     // voxels per chunk
 constexpr int CHUNK_THREADS = 128;   // 8 consecutive voxels per thread
@@ -579,10 +580,29 @@ __device__ __forceinline__ float centre_of(float acc, uint32_t nk, float mn, flo
     return __fmul_rn(ceilf(__fdiv_rn(mean, v)), v);
 }
 
+// The nodes of a level that are split by a block each (above SMALL voxels) and
+// tile by tile (above MID), in no particular order: a tiled node's slot and
+// its first tile come from one counter, so that first tiles ascend with slots.
+struct SplitLists {
+    uint32_t *mid, *nmid, *tiled, *first_tile;
+    unsigned long long *ntiled;   // slots in the upper half, tiles in the lower
+    uint32_t tile;                // positions per tile
+    __device__ void add(uint32_t k, uint32_t n) const
+    {
+        if (n > MID) {
+            const unsigned long long at = atomicAdd(ntiled, (1ull << 32) | ((n + tile - 1) / tile));
+            tiled[at >> 32] = k;
+            first_tile[at >> 32] = (uint32_t)at;
+        } else if (n > SMALL) {
+            mid[atomicAdd(nmid, 1u)] = k;
+        }
+    }
+};
+
 // Node kinds and, for nodes of at most BIG voxels, subdivision centres
 // (tree.c:249-275, find_center tree.c:125-136, density test geom.c:157-167);
 // a warp per node.
-__global__ void k_classify(const float *P, Level L, float vx, float vy, float vz)
+__global__ void k_classify(const float *P, Level L, float vx, float vy, float vz, SplitLists lists)
 {
     uint32_t k = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     int lane = threadIdx.x & 31;
@@ -594,7 +614,10 @@ __global__ void k_classify(const float *P, Level L, float vx, float vy, float vz
     float vv = __fmul_rn(__fmul_rn(vx, vy), vz);
     uint8_t kind = fabsf(__fsub_rn(__fmul_rn(__uint2float_rn(nk), vv), bbv)) < vv ? K_DENSE
                  : (nk <= VOX_MAX_DOTS ? K_LEAF : K_INNER);
-    if (lane == 0) L.kind[k] = kind;
+    if (lane == 0) {
+        L.kind[k] = kind;
+        if (kind == K_INNER) lists.add(k, nk);
+    }
     if (kind != K_INNER || nk > BIG) return;
     float v[3] = {vx, vy, vz};
     uint64_t s = L.start[k];
@@ -752,148 +775,318 @@ __global__ void k_oct_init(const float *P, Level L, const uint32_t *seg_of, uint
     oct[t] = (uint8_t)((c[0] > p[0]) | ((c[1] > p[1]) << 1) | ((c[2] > p[2]) << 2));
 }
 
-// ---- one swapping pass (sort_set, tree.c:166-183) over every node above SMALL
+// ---- the swapping passes of nodes above SMALL
 //
-// Four kernels a pass: claimed counts per tile of SCAN_TILE positions (and,
-// for every range starting in a tile, the count before its start), a scan of
-// the tile counts, the claimed voxels to the front (with each position's
-// claimed count since its range start and the unclaimed positions listed),
-// then the walk back for the rest of each range.
+// A pass needs, at any position, whether its voxel is claimed, how many
+// claimed ones stand before it and where the last unclaimed one before it
+// stands: a bit per position, and per 32-bit word of them the count and that
+// position so far (Marks).  Claimed voxels leave for good, straight to their
+// place in the next level's order; only the others move on to the next pass.
 
-struct Pass {
-    const uint32_t *seg_of, *start, *n, *cnt;
-    const uint8_t *kind;
-    uint32_t o;
-    // The node of position t and where its pass range starts; false when t
-    // is outside every pass range (voxels of other octants already claimed,
-    // nodes not split here, voxels already in leaves).
-    __device__ __forceinline__ bool range(uint64_t t, uint32_t &k, uint32_t &from) const
-    {
-        k = seg_of[t];
-        if (k == NONE || kind[k] != K_INNER || n[k] <= SMALL) return false;
-        uint32_t f = start[k];
-        for (uint32_t q = 0; q < o; q++) f += cnt[8 * k + q];
-        from = f;
-        return t >= f;
-    }
-};
+constexpr uint32_t NO_POS = 0xFFFFFFFFu;
 
-// Block-wide exclusive scan of one flag per thread; *total gets the block's sum.
-__device__ __forceinline__ uint32_t block_excl(uint32_t x, uint32_t *ws, uint32_t &total)
+// The source of position t (local to the node) in a pass whose range starts
+// at `from`: the walk back described at the top of the file.  claimed(s, c, u)
+// says whether position s is claimed and gives the claimed count before it
+// and the last unclaimed position before it.
+template <class F>
+__device__ __forceinline__ uint32_t walk_back(uint32_t t, uint32_t from, uint32_t limit, F claimed, uint32_t *err)
 {
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t incl = warp_incl_scan(x);
-    if (lane == 31) ws[warp] = incl;
-    __syncthreads();
-    uint32_t before = 0, tot = 0;
-    for (int q = 0; q < SCAN_THREADS / 32; q++) {
-        uint32_t t = ws[q];
-        before += q < warp ? t : 0u;
-        tot += t;
-    }
-    __syncthreads();
-    total = tot;
-    return before + incl - x;
-}
-
-// Claimed count of each tile, and for every range starting in the tile the
-// count before its start within the tile.
-__device__ __forceinline__ void tile_count(const Pass &p, uint64_t t, bool cl, bool head, uint32_t k,
-                                           uint32_t &run, uint32_t *ws, uint32_t *head_before)
-{
-    uint32_t tot;
-    uint32_t ex = block_excl(cl ? 1u : 0u, ws, tot);
-    if (head) head_before[k] = run + ex;
-    run += tot;
-}
-
-__global__ void __launch_bounds__(SCAN_THREADS) k_pass_count(Pass p, const uint8_t *oct, uint64_t N,
-                                                             uint32_t *tile, uint32_t *head_before)
-{
-    __shared__ uint32_t ws[SCAN_THREADS / 32];
-    uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
-    uint32_t run = 0;
-    for (int j = 0; j < SCAN_ITEMS; j++) {
-        uint64_t t = base + (uint64_t)j * SCAN_THREADS + threadIdx.x;
-        uint32_t k = 0, from = 0;
-        bool in = t < N && p.range(t, k, from);
-        tile_count(p, t, in && oct[t] == p.o, in && t == from, k, run, ws, head_before);
-    }
-    if (threadIdx.x == 0) tile[blockIdx.x] = run;
-}
-
-// Claimed voxels to the front of their range, in order; each position's
-// claimed count since its range start (C); unclaimed positions listed; each
-// node's claimed count.  Positions outside the ranges are carried over.
-__global__ void __launch_bounds__(SCAN_THREADS) k_pass_front(Pass p, uint64_t N, const uint32_t *tile,
-                                                             const uint32_t *head_before, const uint8_t *in_oct,
-                                                             const uint32_t *in_idx, uint8_t *out_oct,
-                                                             uint32_t *out_idx, uint32_t *C, uint32_t *upos,
-                                                             uint32_t *cnt)
-{
-    __shared__ uint32_t ws[SCAN_THREADS / 32];
-    uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
-    uint32_t run = tile[blockIdx.x];   // claimed positions before this tile
-    for (int j = 0; j < SCAN_ITEMS; j++) {
-        uint64_t t = base + (uint64_t)j * SCAN_THREADS + threadIdx.x;
-        uint32_t k = 0, from = 0;
-        bool in = t < N && p.range(t, k, from);
-        uint8_t q = t < N ? in_oct[t] : (uint8_t)0xFF;
-        bool cl = in && q == p.o;
-        uint32_t tot;
-        uint32_t ex = block_excl(cl ? 1u : 0u, ws, tot);
-        if (t < N) {
-            if (!in) {
-                out_idx[t] = in_idx[t];
-                out_oct[t] = q;
-            } else {
-                uint32_t cf = tile[from / SCAN_TILE] + head_before[k];   // claimed positions before the range
-                uint32_t crel = run + ex - cf;
-                C[t] = crel;
-                if (cl) {
-                    out_idx[from + crel] = in_idx[t];
-                    out_oct[from + crel] = q;
-                } else {
-                    upos[from + ((uint32_t)t - from) - crel] = (uint32_t)t;
-                }
-                if (t + 1 == (uint64_t)p.start[k] + p.n[k]) cnt[8 * k + p.o] = crel + (cl ? 1u : 0u);
-            }
-        }
-        run += tot;
-    }
-}
-
-// The rest of each range: the walk back described at the top of the file.
-__global__ void k_pass_back(Pass p, uint64_t N, const uint32_t *C, const uint32_t *upos, const uint8_t *in_oct,
-                            const uint32_t *in_idx, uint8_t *out_oct, uint32_t *out_idx, uint32_t *err)
-{
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= N) return;
-    uint32_t k, from;
-    if (!p.range(t, k, from) || (uint32_t)t - from < p.cnt[8 * k + p.o]) return;
-    uint32_t s = (uint32_t)t;
-    for (uint32_t steps = 0; in_oct[s] == p.o; steps++) {
-        uint32_t u = (s - from) - C[s];           // unclaimed positions before s
-        if (u == 0 || steps > (1u << 22)) {        // impossible for a consistent pass
+    uint32_t s = t, c, last;
+    for (uint32_t steps = 0; claimed(s, c, last); steps++) {
+        const uint32_t u = (s - from) - c;                 // unclaimed positions before s
+        if (u == 0 || last == NO_POS || steps > limit) {   // impossible for a consistent pass
             atomicOr(err, ERR_WALK);
-            break;
+            return t;
         }
-        uint32_t a = upos[from + u - 1] + 1;      // start of the claimed run holding s
-        uint32_t back = ((s - a) / u + 1) * u;
+        const uint32_t a = last + 1;                       // start of the claimed run holding s
+        const uint32_t back = ((s - a) / u + 1) * u;
         if (a > s || back > s - from) {
             atomicOr(err, ERR_WALK);
-            break;
+            return t;
         }
         s -= back;
     }
-    out_idx[t] = in_idx[s];
-    out_oct[t] = in_oct[s];
+    return s;
 }
 
-__global__ void k_gather(uint64_t N, const uint32_t *idx, const float *P, float *Pn)
+// Scan of up to 32 * PER words' claimed counts and last unclaimed positions
+// by one warp, in place: before[w] and last[w] become those of the words
+// before w (from `run` and `prev` on, which advance).
+template <int PER>
+__device__ __forceinline__ void scan_words(uint32_t *before, uint32_t *last, uint32_t nw, uint32_t &run, uint32_t &prev)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t c[PER], l[PER], sum = 0, top = 0;   // top: last position + 1, 0 for none
+    for (int j = 0; j < PER; j++) {
+        const uint32_t w = lane * PER + j;
+        c[j] = w < nw ? before[w] : 0u;
+        l[j] = w < nw ? last[w] + 1u : 0u;
+        sum += c[j];
+        top = max(top, l[j]);
+    }
+    uint32_t ps = sum, pt = top;
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t a = __shfl_up_sync(0xffffffffu, ps, off), b = __shfl_up_sync(0xffffffffu, pt, off);
+        if (lane >= (uint32_t)off) { ps += a; pt = max(pt, b); }
+    }
+    const uint32_t all = __shfl_sync(0xffffffffu, ps, 31), high = __shfl_sync(0xffffffffu, pt, 31);
+    uint32_t r = run + ps - sum, t = __shfl_up_sync(0xffffffffu, pt, 1);
+    t = max(lane ? t : 0u, prev + 1u);
+    for (int j = 0; j < PER; j++) {
+        const uint32_t w = lane * PER + j;
+        if (w < nw) { before[w] = r; last[w] = t - 1u; }
+        r += c[j];
+        t = max(t, l[j]);
+    }
+    run += all;
+    prev = max(prev + 1u, high) - 1u;
+}
+
+__device__ __forceinline__ uint32_t lanes_below(uint32_t i) { return (1u << i) - 1u; }
+
+// The last unclaimed position before bit i of word w, whose claimed bits are
+// m; positions before `from` are none.  NO_POS when the word has none.
+__device__ __forceinline__ uint32_t last_in_word(uint32_t w, uint32_t i, uint32_t m, uint32_t from)
+{
+    uint32_t u = ~m & lanes_below(i);
+    if (w == from >> 5) u &= ~lanes_below(from & 31);
+    return u ? (w << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
+}
+
+// The gathered voxels of a claimed position's place in the next order.
+__device__ __forceinline__ void place(const float *P, float *Pn, uint64_t to, uint64_t i)
+{
+    Pn[3 * to] = P[3 * i];
+    Pn[3 * to + 1] = P[3 * i + 1];
+    Pn[3 * to + 2] = P[3 * i + 2];
+}
+
+// Nodes of SMALL+1..MID voxels: a block each, all eight passes in shared
+// memory, a voxel in 16 bits {octant, place in the node}.
+constexpr int MID_THREADS = 512;
+__global__ void __launch_bounds__(MID_THREADS) k_partition_block(Level L, SplitLists lists, const uint8_t *oct,
+                                                                 const float *P, float *Pn, uint32_t *err)
+{
+    static_assert(MID == 8192 && MID / 32 == 256, "13 bits of place; 8 words a lane in scan_words");
+    __shared__ uint16_t buf[2][MID];
+    __shared__ uint32_t mask[MID / 32], before[MID / 32], last[MID / 32], total;
+    if (blockIdx.x >= *lists.nmid) return;
+    const uint32_t k = lists.mid[blockIdx.x], n = L.n[k], s0 = L.start[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint32_t i = threadIdx.x; i < n; i += MID_THREADS) buf[0][i] = (uint16_t)(((uint32_t)oct[s0 + i] << 13) | i);
+    const uint32_t nw = (n + 31) / 32;
+    uint32_t from = 0;
+    for (uint32_t o = 0; o < 8; o++) {
+        const uint16_t *in = buf[o & 1];
+        uint16_t *out = buf[(o & 1) ^ 1];
+        __syncthreads();
+        for (uint32_t w = (from >> 5) + warp; w < nw; w += MID_THREADS / 32) {
+            const uint32_t t = (w << 5) + lane;
+            const bool range = t >= from && t < n;
+            const bool cl = range && (in[t] >> 13) == o;
+            const uint32_t m = __ballot_sync(0xffffffffu, cl), u = __ballot_sync(0xffffffffu, range && !cl);
+            if (lane == 0) {
+                mask[w] = m;
+                before[w] = (uint32_t)__popc(m);
+                last[w] = u ? (w << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
+            }
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t w0 = from >> 5;
+            uint32_t run = 0, prev = NO_POS;
+            scan_words<MID / 32 / 32>(before + w0, last + w0, nw - w0, run, prev);
+            if (lane == 0) {
+                total = run;
+                L.cnt[8 * k + o] = run;
+            }
+        }
+        __syncthreads();
+        const uint32_t rest = from + total;
+        auto claimed = [&](uint32_t s, uint32_t &c, uint32_t &l) {
+            const uint32_t w = s >> 5, i = s & 31, m = mask[w];
+            c = before[w] + (uint32_t)__popc(m & lanes_below(i));
+            l = last_in_word(w, i, m, from);
+            if (l == NO_POS) l = last[w];
+            return ((m >> i) & 1u) != 0u;
+        };
+        for (uint32_t t = from + threadIdx.x; t < n; t += MID_THREADS) {
+            uint32_t c, l;
+            if (claimed(t, c, l)) place(P, Pn, (uint64_t)s0 + from + c, (uint64_t)s0 + (in[t] & 8191u));
+            if (t >= rest) out[t] = in[walk_back(t, from, MID, claimed, err)];
+        }
+        from = rest;
+        if (from >= n) break;
+    }
+}
+
+// Larger nodes, tile by tile: a launch a pass, a block a tile of one node.
+// The marks of a pass are made by the launch before it (the first ones by
+// k_tile_marks): per word as above, counted from the tile's start, and per
+// tile the claimed count and the last unclaimed position.  Every block scans
+// its node's tiles for itself (at most MAX_TILES).
+//
+// What bounds a pass is the chain of dependent loads of each word's walk, so
+// a warp has few words to go through: the 256^3 set's raw build takes 4,790 us
+// with 4 words a warp (256 threads on 1,024 positions, or 512 on 2,048), 5,190
+// with 16, and 4,930 with 2 in blocks of 1,024 threads.  With the four kernels
+// a pass (count, scan, place, walk) over every position of the level that
+// this replaces it took 6,080.
+constexpr int PASS_THREADS = 256;
+constexpr uint32_t SUB = 1024;          // positions marked at a time; a tile is a multiple of it
+constexpr uint32_t MAX_TILES = 2048;    // tiles of one node
+
+struct Marks {
+    uint32_t *mask, *before, *last;     // per word of a tile
+    uint32_t *count, *tail;             // per tile
+};
+
+// Marks of one SUB of positions from their claimed flags, word by word.
+struct SubMarks {
+    uint32_t before[SUB / 32], last[SUB / 32];
+    __device__ void flush(const Marks &m, uint64_t word0, uint32_t nw, uint32_t &run, uint32_t &prev)
+    {
+        __syncthreads();
+        if (threadIdx.x < 32) scan_words<SUB / 32 / 32>(before, last, nw, run, prev);
+        __syncthreads();
+        for (uint32_t w = threadIdx.x; w < nw; w += PASS_THREADS) {
+            m.before[word0 + w] = before[w];
+            m.last[word0 + w] = last[w];
+        }
+        __syncthreads();
+    }
+};
+
+// The node of this block's tile: its slot, or NO_POS for a block without one.
+__device__ __forceinline__ uint32_t tile_slot(const SplitLists &lists, uint32_t tile)
+{
+    const unsigned long long n = *lists.ntiled;
+    if (tile >= (uint32_t)n) return NO_POS;
+    uint32_t lo = 0, hi = (uint32_t)(n >> 32);
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (lists.first_tile[mid] <= tile) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// Marks of octant 0 over the given order.
+__global__ void __launch_bounds__(PASS_THREADS) k_tile_marks(Level L, SplitLists lists, const uint8_t *oct, Marks out)
+{
+    __shared__ SubMarks sub;
+    const uint32_t slot = tile_slot(lists, blockIdx.x);
+    if (slot == NO_POS) return;
+    const uint32_t k = lists.tiled[slot], n = L.n[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t start = L.start[k];
+    const uint32_t b = (blockIdx.x - lists.first_tile[slot]) * lists.tile, e = min(n, b + lists.tile);
+    uint64_t word0 = (uint64_t)blockIdx.x * (lists.tile / 32);
+    uint32_t run = 0, prev = NO_POS;
+    for (uint32_t sb = b; sb < e; sb += SUB, word0 += SUB / 32) {
+        const uint32_t nw = (min(e - sb, SUB) + 31) / 32;
+        for (uint32_t w = warp; w < nw; w += PASS_THREADS / 32) {
+            const uint32_t t = sb + (w << 5) + lane;
+            const bool in = t < e, cl = in && oct[start + t] == 0;
+            const uint32_t m = __ballot_sync(0xffffffffu, cl), u = __ballot_sync(0xffffffffu, in && !cl);
+            if (lane == 0) {
+                out.mask[word0 + w] = m;
+                sub.before[w] = (uint32_t)__popc(m);
+                sub.last[w] = u ? sb + (w << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
+            }
+        }
+        sub.flush(out, word0, nw, run, prev);
+    }
+    if (threadIdx.x == 0) {
+        out.count[blockIdx.x] = run;
+        out.tail[blockIdx.x] = prev;
+    }
+}
+
+// Pass o over every tiled node.
+__global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, SplitLists lists, uint32_t o, Marks in, Marks out,
+                                                            const uint32_t *in_idx, const uint8_t *in_oct,
+                                                            uint32_t *out_idx, uint8_t *out_oct, const float *P,
+                                                            float *Pn, uint32_t *err)
+{
+    __shared__ SubMarks sub;
+    __shared__ uint32_t tbefore[MAX_TILES], tlast[MAX_TILES];
+    __shared__ uint32_t s_total;
+    const uint32_t slot = tile_slot(lists, blockIdx.x);
+    if (slot == NO_POS) return;
+    const uint32_t tile = lists.tile, ft = lists.first_tile[slot], ti = blockIdx.x - ft;
+    const uint32_t k = lists.tiled[slot], n = L.n[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t start = L.start[k];
+    uint32_t from = 0;
+    for (uint32_t q = 0; q < o; q++) from += L.cnt[8 * k + q];
+    const uint32_t b = ti * tile, e = min(n, b + tile);
+    if (e <= from) return;                     // all of it placed by earlier passes
+    const uint32_t t0 = from / tile, nt = (n + tile - 1) / tile - t0;   // the tiles still in play
+    for (uint32_t i = threadIdx.x; i < nt; i += PASS_THREADS) {
+        tbefore[i] = in.count[ft + t0 + i];
+        tlast[i] = in.tail[ft + t0 + i];
+    }
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t run = 0, prev = NO_POS;
+        for (uint32_t i = 0; i < nt; i += 128)
+            scan_words<4>(tbefore + i, tlast + i, min(nt - i, 128u), run, prev);
+        if (lane == 0) {
+            s_total = run;
+            if (e == n) L.cnt[8 * k + o] = run;   // read by later launches only
+        }
+    }
+    __syncthreads();
+    const uint32_t rest = from + s_total;
+    const uint64_t words = (uint64_t)ft * (tile / 32);   // the node's first word: tiles hold whole words
+    auto claimed = [&](uint32_t s, uint32_t &c, uint32_t &l) {
+        const uint32_t w = s >> 5, i = s & 31, m = in.mask[words + w], ts = s / tile - t0;
+        c = tbefore[ts] + in.before[words + w] + (uint32_t)__popc(m & lanes_below(i));
+        l = last_in_word(w, i, m, from);
+        if (l == NO_POS) l = in.last[words + w];
+        if (l == NO_POS) l = tlast[ts];
+        return ((m >> i) & 1u) != 0u;
+    };
+    uint32_t run = 0, prev = NO_POS;
+    for (uint32_t sb = b; sb < e; sb += SUB) {
+        const uint32_t nw = (min(e - sb, SUB) + 31) / 32;
+        for (uint32_t w = warp; w < nw; w += PASS_THREADS / 32) {
+            const uint32_t t = sb + (w << 5) + lane;
+            uint8_t q = 0xFF;
+            if (t >= from && t < e) {
+                uint32_t c, l;
+                if (claimed(t, c, l))
+                    place(P, Pn, start + from + c, o == 0 ? start + t : (uint64_t)in_idx[start + t]);
+                if (t >= rest) {
+                    const uint32_t s = walk_back(t, from, 1u << 22, claimed, err);
+                    q = in_oct[start + s];
+                    out_idx[start + t] = o == 0 ? (uint32_t)start + s : in_idx[start + s];
+                    out_oct[start + t] = q;
+                }
+            }
+            const bool left = t >= rest && t < e, cl = left && q == o + 1;
+            const uint32_t m = __ballot_sync(0xffffffffu, cl), u = __ballot_sync(0xffffffffu, left && !cl);
+            if (lane == 0) {
+                out.mask[words + (sb >> 5) + w] = m;
+                sub.before[w] = (uint32_t)__popc(m);
+                sub.last[w] = u ? sb + (w << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
+            }
+        }
+        sub.flush(out, words + (sb >> 5), nw, run, prev);
+    }
+    if (threadIdx.x == 0) {
+        out.count[blockIdx.x] = run;
+        out.tail[blockIdx.x] = prev;
+    }
+}
+
+// The next level's order outside the nodes above SMALL, whose passes place
+// their voxels themselves.
+__global__ void k_gather(uint64_t N, Level L, const uint32_t *seg_of, const uint32_t *idx, const float *P, float *Pn)
 {
     uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= N) return;
+    const uint32_t k = seg_of[t];
+    if (k != NONE && L.kind[k] == K_INNER && L.n[k] > SMALL) return;
     uint64_t i = idx[t];
     Pn[3 * t] = P[3 * i];
     Pn[3 * t + 1] = P[3 * i + 1];
@@ -1145,7 +1338,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     } level_free{levels, s};
 
     float *P[2];
-    uint32_t *idx[2], *C, *upos, *seg_of, *tile, *scal, *maps, *cidx, *big;
+    uint32_t *idx[2], *seg_of, *tile, *scal, *maps, *cidx, *big;
     uint8_t *oct[2], *nz;
     float *cv;
     unsigned long long *stats;
@@ -1158,14 +1351,11 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     TRY(d.get(&idx[1], N));
     TRY(d.get(&oct[0], N));
     TRY(d.get(&oct[1], N));
-    TRY(d.get(&C, N));
-    TRY(d.get(&upos, N));
     TRY(d.get(&seg_of, N));
     TRY(d.get(&tile, max_tiles));
-    uint32_t *hbefore;   // per node: claimed count before its range start within its tile
-    TRY(d.get(&hbefore, N));
-    // scal: 0 chunks, 1 claimed, 2 children, 3 big nodes, 4 largest child, 7 error bits
-    TRY(d.get(&scal, 8));
+    // scal: 0 chunks, 1 mid nodes, 2 children, 3 big nodes, 4 largest child, 6-7 tiled nodes and tiles,
+    // 8 error bits
+    TRY(d.get(&scal, 12));
     TRY(d.get(&big, max_big));
     if (N > BIG) {
         TRY(d.get(&cv, 6 * max_chunks));
@@ -1178,8 +1368,27 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         nz = nullptr;
     }
     TRY(d.get(&stats, 4 * MAX_LEVELS));
-    uint32_t *err = scal + 7;
-    TRY(cudaMemsetAsync(scal, 0, 8 * 4, s));
+    uint32_t *err = scal + 8;
+    TRY(cudaMemsetAsync(scal, 0, 12 * 4, s));
+    // nodes split by a block each and tile by tile, and the tiles' marks (two sets)
+    SplitLists lists{};
+    lists.nmid = scal + 1;
+    lists.ntiled = reinterpret_cast<unsigned long long *>(scal + 6);
+    lists.tile = SUB * (uint32_t)((N + (uint64_t)SUB * MAX_TILES - 1) / ((uint64_t)SUB * MAX_TILES));
+    const uint64_t max_mid = N / SMALL, max_tiled = N / MID, max_pass_tiles = N / lists.tile + max_tiled;
+    TRY(d.get(&lists.mid, max_mid + 1));
+    Marks marks[2] = {};
+    if (N > MID) {
+        TRY(d.get(&lists.tiled, max_tiled));
+        TRY(d.get(&lists.first_tile, max_tiled));
+        for (Marks &m : marks) {
+            TRY(d.get(&m.mask, max_pass_tiles * (lists.tile / 32)));
+            TRY(d.get(&m.before, max_pass_tiles * (lists.tile / 32)));
+            TRY(d.get(&m.last, max_pass_tiles * (lists.tile / 32)));
+            TRY(d.get(&m.count, max_pass_tiles));
+            TRY(d.get(&m.tail, max_pass_tiles));
+        }
+    }
     TRY(cudaMemsetAsync(stats, 0, 4 * MAX_LEVELS * sizeof(unsigned long long), s));
     TRY(cudaMemcpyAsync(P[0], d_set, 12 * N, cudaMemcpyDeviceToDevice, s));
 
@@ -1204,7 +1413,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         if (lv >= MAX_LEVELS) return VOX_CUDA_EDEPTH;
         Level L = levels[lv];
         uint32_t m = L.m;
-        TRY(cudaMemsetAsync(scal, 0, 5 * 4, s));
+        TRY(cudaMemsetAsync(scal, 0, 8 * 4, s));
         k_seg_of<<<grid_for(N, TB), TB, 0, s>>>(L.start, L.n, m, N, seg_of);
         count_launch();
         bool has_big = largest > BIG;
@@ -1223,7 +1432,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
             k_chunk_maps<<<(unsigned)max_chunks, CHUNK_THREADS, 0, s>>>(P[cur], L, scal + 0, maps, nz, max_chunks);
             count_launch();
         }
-        k_classify<<<grid_for((uint64_t)m * 32, TB), TB, 0, s>>>(P[cur], L, vx, vy, vz);
+        k_classify<<<grid_for((uint64_t)m * 32, TB), TB, 0, s>>>(P[cur], L, vx, vy, vz, lists);
         count_launch();
         if (has_big) {
             k_centre_big<<<grid_for(max_big * 3 * 32, CENTRE_WARPS * 32), CENTRE_WARPS * 32, 0, s>>>(
@@ -1232,23 +1441,22 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         }
         k_oct_init<<<grid_for(N, TB), TB, 0, s>>>(P[cur], L, seg_of, N, idx[0], oct[0]);
         count_launch();
-        if (largest > SMALL) {
-            // the eight swapping passes of nodes above SMALL; the result lands back in buffer 0
-            unsigned nt = (unsigned)((N + SCAN_TILE - 1) / SCAN_TILE);
+        if (largest > MID) {   // the eight swapping passes of the largest nodes
+            k_tile_marks<<<(unsigned)max_pass_tiles, PASS_THREADS, 0, s>>>(L, lists, oct[0], marks[0]);
             for (uint32_t o = 0; o < 8; o++) {
-                int in = o & 1, out = in ^ 1;
-                Pass p{seg_of, L.start, L.n, L.cnt, L.kind, o};
-                k_pass_count<<<nt, SCAN_THREADS, 0, s>>>(p, oct[in], N, tile, hbefore);
-                k_scan_tiles<<<1, 1024, 0, s>>>(tile, nt, scal + 1);
-                k_pass_front<<<nt, SCAN_THREADS, 0, s>>>(p, N, tile, hbefore, oct[in], idx[in], oct[out], idx[out], C,
-                                                         upos, L.cnt);
-                k_pass_back<<<grid_for(N, TB), TB, 0, s>>>(p, N, C, upos, oct[in], idx[in], oct[out], idx[out], err);
-                for (int i = 0; i < 4; i++) count_launch();
+                const int in = o & 1, out = in ^ 1;
+                k_tile_pass<<<(unsigned)max_pass_tiles, PASS_THREADS, 0, s>>>(
+                    L, lists, o, marks[in], marks[out], idx[in], oct[in], idx[out], oct[out], P[cur], P[cur ^ 1], err);
             }
+            for (int i = 0; i < 9; i++) count_launch();
+        }
+        if (largest > SMALL) {
+            k_partition_block<<<(unsigned)max_mid, MID_THREADS, 0, s>>>(L, lists, oct[0], P[cur], P[cur ^ 1], err);
+            count_launch();
         }
         k_partition_warp<<<grid_for((uint64_t)m * 32, PART_WARPS * 32), PART_WARPS * 32, 0, s>>>(L, idx[0], oct[0],
                                                                                               err);
-        k_gather<<<grid_for(N, TB), TB, 0, s>>>(N, idx[0], P[cur], P[cur ^ 1]);
+        k_gather<<<grid_for(N, TB), TB, 0, s>>>(N, L, seg_of, idx[0], P[cur], P[cur ^ 1]);
         cur ^= 1;
         k_finish<<<grid_for(m, TB), TB, 0, s>>>(L, stats + 4 * lv, scal + 4, err);
         count_launch();
