@@ -33,12 +33,16 @@
  *  and delta in {0, 1}, which depends on the fraction of d/2^e and, for an
  *  exact half (rounded to even), on the parity of A + q.  A run of additions
  *  is therefore a map from the parity of A to (increment, new parity): a
- *  two-state machine, and such maps compose associatively.  Chunks of 1024
- *  voxels get their map for each of 12 binades in parallel; one thread per
- *  node then walks its chunks, applying the map of the binade the sum is in,
- *  and adds a chunk voxel by voxel only where the sum leaves its binade
- *  inside the chunk (a dozen times per node) or lies below the precomputed
- *  binades.
+ *  two-state machine, and such maps compose associatively.  Most sums need
+ *  none of it: no addition rounds while the sum stays below 2^24 times a power
+ *  of two that divides every term, and then any order gives it (PlainSum).
+ *  For the others, chunks of 1024 voxels get their maps, in parallel, for the
+ *  two binades the sum is expected in there (from the chunks' plain sums); a
+ *  warp then scans 32 chunks' maps at a time, and adds a chunk voxel by voxel
+ *  only where the sum leaves its binade inside the chunk (a dozen times per
+ *  node) or no map was made for it.  The root of the 256^3 set: 423 us walking
+ *  its 1,332 chunks one by one, and 147 for maps of 16 binades, became 70 and
+ *  26 (raw volume with a first frame 4,790 -> 3,920 us).
  *
  * The rest (bounding boxes, the density test, leaf decisions, children) is
  * per node or per voxel.  The tree is built a level at a time.  Then subtree
@@ -269,6 +273,15 @@ struct ChunkCount {
     const uint32_t *n;
     __device__ uint32_t operator()(uint64_t k) const { return n[k] > BIG ? (n[k] + CHUNK - 1) / CHUNK : 0u; }
 };
+// First chunks, and the nodes that have chunks listed.
+struct StoreChunks {
+    uint32_t *out, *big, *nbig;
+    __device__ void operator()(uint64_t i, uint32_t excl, uint32_t chunks) const
+    {
+        out[i] = excl;
+        if (chunks) big[atomicAdd(nbig, 1u)] = (uint32_t)i;
+    }
+};
 struct StoreExcl {
     uint32_t *out;
     __device__ void operator()(uint64_t i, uint32_t excl, uint32_t) const { out[i] = excl; }
@@ -404,39 +417,99 @@ __global__ void k_box_thread(const float *P, Level L, float vx, float vy, float 
     write_box(L, k, mn, mx, v);
 }
 
-// The other nodes: a warp per node over its voxels, or over its chunks'
-// partial extremes for a big node (listed for the centre kernel).
-__global__ void k_box_warp(const float *P, Level L, const float *cv, const uint32_t *ci, float vx, float vy,
-                           float vz, uint32_t *big, uint32_t *nbig)
+// Nodes of TINY+1..BIG voxels: a warp per node over its voxels.
+__global__ void k_box_warp(const float *P, Level L, float vx, float vy, float vz)
 {
     uint32_t k = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     int lane = threadIdx.x & 31;
     if (k >= L.m) return;
     uint32_t nk = L.n[k];
-    if (nk <= TINY) return;
+    if (nk <= TINY || nk > BIG) return;
     Extremes x;
     x.init();
-    if (nk > BIG) {
-        uint32_t nch = (nk + CHUNK - 1) / CHUNK, c0 = L.chunk_base[k];
-        for (uint32_t j = lane; j < nch; j += 32) {
-            Extremes o;
-            uint32_t c = c0 + j;
-            for (int a = 0; a < 3; a++) {
-                o.mn[a] = cv[6 * c + a]; o.mni[a] = ci[6 * c + a];
-                o.mx[a] = cv[6 * c + 3 + a]; o.mxi[a] = ci[6 * c + 3 + a];
-            }
-            x.merge(o);
-        }
-    } else {
-        uint64_t s = L.start[k];
-        for (uint32_t j = lane; j < nk; j += 32) x.add(P + 3 * (s + j), (uint32_t)(s + j));
-    }
+    uint64_t s = L.start[k];
+    for (uint32_t j = lane; j < nk; j += 32) x.add(P + 3 * (s + j), (uint32_t)(s + j));
     x.warp_merge();
     if (lane) return;
     float v[3] = {vx, vy, vz};
     write_box(L, k, x.mn, x.mx, v);
-    if (nk > BIG) big[atomicAdd(nbig, 1u)] = k;
 }
+
+// Big nodes: a block per node over its chunks' partial extremes.
+constexpr int NODE_THREADS = 256;
+__global__ void __launch_bounds__(NODE_THREADS) k_box_big(Level L, const uint32_t *big, const uint32_t *nbig,
+                                                          const float *cv, const uint32_t *ci, float vx, float vy,
+                                                          float vz)
+{
+    __shared__ Extremes part[NODE_THREADS / 32];
+    if (blockIdx.x >= *nbig) return;
+    const uint32_t k = big[blockIdx.x], nch = (L.n[k] + CHUNK - 1) / CHUNK, c0 = L.chunk_base[k];
+    Extremes x;
+    x.init();
+    for (uint32_t j = threadIdx.x; j < nch; j += NODE_THREADS) {
+        Extremes o;
+        const uint32_t c = c0 + j;
+        for (int a = 0; a < 3; a++) {
+            o.mn[a] = cv[6 * c + a]; o.mni[a] = ci[6 * c + a];
+            o.mx[a] = cv[6 * c + 3 + a]; o.mxi[a] = ci[6 * c + 3 + a];
+        }
+        x.merge(o);
+    }
+    x.warp_merge();
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = x;
+    __syncthreads();
+    if (threadIdx.x) return;
+    for (int w = 1; w < NODE_THREADS / 32; w++) x.merge(part[w]);
+    float v[3] = {vx, vy, vz};
+    write_box(L, k, x.mn, x.mx, v);
+}
+
+// ---- sums that no addition rounds
+//
+// When every d of a node is a multiple of some power of two g and their sum is
+// below 2^24 g, each partial sum, in any order, is a multiple of g below 2^24 g:
+// a float, so no addition rounds and the serial sum is the sum.  (A sum made in
+// floats in another order that comes out below 2^24 g proves it: rounding is
+// monotone, so no partial sum can have reached 2^24 g.)  On unit voxels g is 1
+// and this covers all but the largest nodes.
+
+// The exponent of the largest power of two that divides d (d > 0).
+__device__ __forceinline__ int grid_exp(float d)
+{
+    const uint32_t b = __float_as_uint(d), e = max(b >> 23, 1u), m = (b & 0x7FFFFFu) | (b >> 23 ? 0x800000u : 0u);
+    return (int)e - 150 + __ffs((int)m) - 1;
+}
+
+struct PlainSum {
+    float sum[3];
+    int g[3];       // exponent of the common power of two
+    __device__ void init()
+    {
+        for (int a = 0; a < 3; a++) { sum[a] = 0.0f; g[a] = 1000; }
+    }
+    __device__ void add(int a, float d)
+    {
+        sum[a] = __fadd_rn(sum[a], d);
+        if (d > 0.0f) g[a] = min(g[a], grid_exp(d));
+    }
+    __device__ void merge(int a, float x, int e)
+    {
+        sum[a] = __fadd_rn(sum[a], x);
+        g[a] = min(g[a], e);
+    }
+    __device__ void warp_merge()
+    {
+        for (int off = 16; off; off >>= 1)
+            for (int a = 0; a < 3; a++)
+                merge(a, __shfl_xor_sync(0xffffffffu, sum[a], off), __shfl_xor_sync(0xffffffffu, g[a], off));
+    }
+    // sum[a] is the serial float sum
+    __device__ bool exact(int a) const
+    {
+        const int e = g[a] + 24;
+        return sum[a] == 0.0f || (e >= -126 && (e > 127 || sum[a] < __int_as_float((e + 127) << 23)));
+    }
+};
 
 // ---- the two-state machine of a float sum within one binade
 
@@ -479,42 +552,134 @@ __device__ __forceinline__ Tr tr_shfl_down(Tr t, int off)
     return {__shfl_down_sync(0xffffffffu, t.w0, off), __shfl_down_sync(0xffffffffu, t.w1, off)};
 }
 
-// Maps of one chunk of a big node, for the NBIN binades ending at the node's
-// top binade, per axis; and whether any of its d is non-zero.
-__device__ __forceinline__ size_t map_index(uint64_t maxc, int a, uint32_t c, int bi)
+// Sums and common powers of two of one chunk of a big node, per axis.
+__global__ void __launch_bounds__(CHUNK_THREADS) k_chunk_sums(const float *P, Level L, const uint32_t *total,
+                                                              float *csum, int *cgrid)
 {
-    return (((size_t)a * maxc + c) * NBIN + bi) * 2;
+    __shared__ PlainSum part[CHUNK_THREADS / 32];
+    const uint32_t c = blockIdx.x;
+    if (c >= *total) return;
+    const uint32_t k = chunk_node(L.chunk_base, L.m, c);
+    const uint64_t b = (uint64_t)L.start[k] + (uint64_t)(c - L.chunk_base[k]) * CHUNK;
+    const uint64_t e = min(b + CHUNK, (uint64_t)L.start[k] + L.n[k]);
+    PlainSum x;
+    x.init();
+    for (uint64_t t = b + threadIdx.x; t < e; t += CHUNK_THREADS)
+        for (int a = 0; a < 3; a++) x.add(a, __fsub_rn(P[3 * t + a], L.box[6 * k + a]));
+    x.warp_merge();
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < CHUNK_THREADS / 32; w++)
+            for (int a = 0; a < 3; a++) x.merge(a, part[w].sum[a], part[w].g[a]);
+        for (int a = 0; a < 3; a++) {
+            csum[3 * c + a] = x.sum[a];
+            cgrid[3 * c + a] = x.g[a];
+        }
+    }
 }
 
+__device__ __forceinline__ float centre_of(float acc, uint32_t nk, float mn, float v)
+{
+    float mean = __fadd_rn(__fdiv_rn(acc, __uint2float_rn(nk)), mn);
+    return __fmul_rn(ceilf(__fdiv_rn(mean, v)), v);
+}
+
+// Centres of the big nodes whose sums no addition rounds, a block per node;
+// for the other axes, where the first addition may round (the first chunk that
+// takes the sum to 2^24 of the common power of two, and the sum before it,
+// which is still a plain one), and the first of the binades (biased exponent) that each
+// chunk gets a map for: the one that 63/64 of the sum before the chunk lies in,
+// so that with the next one the sum's own binade is among them unless its
+// roundings added up to more than that.  0: the axis needs no maps.  With
+// window > 2 (sums so long that they do) the binades below the node's top.
+__global__ void __launch_bounds__(NODE_THREADS) k_centre_plain(Level L, const uint32_t *big, const uint32_t *nbig,
+                                                               const float *csum, const int *cgrid, uint8_t *cbase,
+                                                               int window, uint2 *starts, float vx, float vy, float vz)
+{
+    __shared__ PlainSum part[NODE_THREADS / 32];
+    __shared__ double wsum[NODE_THREADS / 32], carry;
+    if (blockIdx.x >= *nbig) return;
+    const uint32_t k = big[blockIdx.x], nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK, c0 = L.chunk_base[k];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    PlainSum x;
+    x.init();
+    for (uint32_t j = threadIdx.x; j < nch; j += NODE_THREADS)
+        for (int a = 0; a < 3; a++) x.merge(a, csum[3 * (c0 + j) + a], cgrid[3 * (c0 + j) + a]);
+    x.warp_merge();
+    if (lane == 0) part[warp] = x;
+    __syncthreads();
+    x = part[0];
+    for (int w = 1; w < NODE_THREADS / 32; w++)
+        for (int a = 0; a < 3; a++) x.merge(a, part[w].sum[a], part[w].g[a]);
+    const float v[3] = {vx, vy, vz};
+    for (int a = 0; a < 3; a++) {
+        if (x.exact(a)) {
+            if (threadIdx.x == 0) L.centre[3 * k + a] = centre_of(x.sum[a], nk, L.box[6 * k + a], v[a]);
+            for (uint32_t j = threadIdx.x; j < nch; j += NODE_THREADS) cbase[3 * (c0 + j) + a] = 0;
+            continue;
+        }
+        const int top = max(1, min(254, L.ehi[3 * k + a] + 150 - (window - 1)));
+        const double limit = ldexp(1.0, x.g[a] + 24);
+        if (threadIdx.x == 0) starts[3 * blockIdx.x + a] = make_uint2(0u, 0u);
+        __syncthreads();   // the axis before may still set it
+        if (threadIdx.x == 0) carry = 0.0;
+        for (uint32_t j0 = 0; j0 < nch; j0 += NODE_THREADS) {
+            const uint32_t j = j0 + threadIdx.x;
+            const double d = j < nch ? (double)csum[3 * (c0 + j) + a] : 0.0;
+            double s = d;
+            for (int off = 1; off < 32; off <<= 1) {
+                const double y = __shfl_up_sync(0xffffffffu, s, off);
+                if (lane >= (uint32_t)off) s += y;
+            }
+            if (lane == 31) wsum[warp] = s;
+            __syncthreads();
+            double before = carry + s - d;
+            for (uint32_t w = 0; w < warp; w++) before += wsum[w];
+            if (j < nch) {
+                const uint32_t e = __float_as_uint((float)(before * (63.0 / 64.0))) >> 23;
+                cbase[3 * (c0 + j) + a] = (uint8_t)(window > 2 ? (uint32_t)top : max(1u, min(e, 253u)));
+                if (before < limit && before + d >= limit)
+                    starts[3 * blockIdx.x + a] = make_uint2(j, __float_as_uint((float)before));
+            }
+            __syncthreads();
+            if (threadIdx.x == NODE_THREADS - 1) carry = before + d;
+        }
+    }
+}
+
+__device__ __forceinline__ size_t map_index(uint64_t maxc, int window, int a, uint32_t c, int bi)
+{
+    return ((size_t)a * maxc + c) * window + bi;
+}
+
+// Maps of one chunk of a big node for the `window` binades from its base on,
+// per axis that needs them.
 __global__ void __launch_bounds__(CHUNK_THREADS) k_chunk_maps(const float *P, Level L, const uint32_t *total,
-                                                             uint32_t *maps, uint8_t *nz, uint64_t maxc)
+                                                             const uint8_t *cbase, int window, uint2 *maps,
+                                                             uint64_t maxc)
 {
     __shared__ Tr part[NBIN][3][CHUNK_THREADS / 32];
-    __shared__ uint32_t any[3];
     uint32_t c = blockIdx.x;
     if (c >= *total) return;
-    if (threadIdx.x < 3) any[threadIdx.x] = 0;
+    const int base[3] = {cbase[3 * c], cbase[3 * c + 1], cbase[3 * c + 2]};
+    if (!(base[0] | base[1] | base[2])) return;
     uint32_t k = chunk_node(L.chunk_base, L.m, c);
     uint64_t b = (uint64_t)L.start[k] + (uint64_t)(c - L.chunk_base[k]) * CHUNK;
     uint64_t e = min(b + CHUNK, (uint64_t)L.start[k] + L.n[k]);
     uint64_t t0 = b + (uint64_t)threadIdx.x * 8;
     float d[8][3];
     uint32_t cnt = t0 < e ? (uint32_t)(e - t0 < 8 ? e - t0 : 8) : 0u;
-    uint32_t nzm = 0;
     for (int q = 0; q < 8; q++)
-        for (int a = 0; a < 3; a++) {
+        for (int a = 0; a < 3; a++)
             d[q][a] = (uint32_t)q < cnt ? __fsub_rn(P[3 * (t0 + q) + a], L.box[6 * k + a]) : 0.0f;
-            if (d[q][a] > 0.0f) nzm |= 1u << a;
-        }
-    __syncthreads();
-    for (int a = 0; a < 3; a++)
-        if (nzm & (1u << a)) atomicOr(&any[a], 1u);
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int bi = 0; bi < NBIN; bi++)
+    for (int bi = 0; bi < window; bi++)
         for (int a = 0; a < 3; a++) {
-            int ee = L.ehi[3 * k + a] - (NBIN - 1) + bi;
+            if (!base[a]) continue;
             Tr t = tr_id();
-            for (uint32_t q = 0; q < cnt; q++) t = tr_cat(t, tr_elem(d[q][a], ee));
+            for (int q = 0; q < 8; q++)
+                if ((uint32_t)q < cnt) t = tr_cat(t, tr_elem(d[q][a], base[a] + bi - 150));
             for (int off = 1; off < 32; off <<= 1) {
                 Tr u = tr_shfl_down(t, off);
                 if ((lane & (2 * off - 1)) == 0) t = tr_cat(t, u);
@@ -522,24 +687,23 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_chunk_maps(const float *P, Le
             if (lane == 0) part[bi][a][warp] = t;
         }
     __syncthreads();
-    if (threadIdx.x < NBIN * 3) {
+    if (threadIdx.x < (uint32_t)window * 3) {
         int bi = threadIdx.x / 3, a = threadIdx.x % 3;
+        if (!base[a]) return;
         Tr t = part[bi][a][0];
         for (int w = 1; w < CHUNK_THREADS / 32; w++) t = tr_cat(t, part[bi][a][w]);
-        size_t o = map_index(maxc, a, c, bi);
-        maps[o] = t.w0;
-        maps[o + 1] = t.w1;
+        maps[map_index(maxc, window, a, c, bi)] = make_uint2(t.w0, t.w1);
     }
-    if (threadIdx.x < 3) nz[3 * c + threadIdx.x] = (uint8_t)any[threadIdx.x];
 }
 
 // acc plus the d of positions [b, e) in order, by one warp (every lane returns
-// the same sum): 128 voxels a step, 4 consecutive ones per lane, added by the
-// composed map of the binade acc is in, or one at a time when acc is not a
-// normal float or the step would leave its binade.
+// the same sum): 128 voxels a step, 4 consecutive ones per lane.  A scan of the
+// lanes' maps of the binade acc is in adds all of them up to the first lane
+// in which the sum leaves it; that lane's four are added one at a time, and
+// the scan goes on behind it in the new binade.
 __device__ float warp_sum(const float *P, uint64_t b, uint64_t e, int a, float mn, float acc)
 {
-    int lane = threadIdx.x & 31;
+    const uint32_t lane = threadIdx.x & 31;
     float nx[4];
     for (int j = 0; j < 4; j++) {
         uint64_t t = b + 4 * (uint64_t)lane + j;
@@ -552,32 +716,34 @@ __device__ float warp_sum(const float *P, uint64_t b, uint64_t e, int a, float m
             uint64_t t = s + 128 + 4 * (uint64_t)lane + j;
             nx[j] = t < e ? P[3 * t + a] : mn;
         }
-        uint32_t bits = __float_as_uint(acc), E = bits >> 23;
-        if (E >= 1u && E < 255u) {
-            int ee = (int)E - 150;
-            Tr t = tr_cat(tr_cat(tr_elem(d[0], ee), tr_elem(d[1], ee)), tr_cat(tr_elem(d[2], ee), tr_elem(d[3], ee)));
-            for (int off = 1; off < 32; off <<= 1) {
-                Tr u = tr_shfl_down(t, off);
-                if ((lane & (2 * off - 1)) == 0) t = tr_cat(t, u);
+        for (uint32_t done = 0; done < 32;) {                      // lanes below `done` are added
+            uint32_t f = done;                                     // the next lane to add one at a time
+            const uint32_t bits = __float_as_uint(acc), E = bits >> 23, A = (bits & 0x7FFFFFu) | 0x800000u;
+            if (acc == 0.0f) {
+                const bool some = lane >= done && !(d[0] == 0.0f && d[1] == 0.0f && d[2] == 0.0f && d[3] == 0.0f);
+                const uint32_t any = __ballot_sync(0xffffffffu, some);
+                f = any ? (uint32_t)__ffs((int)any) - 1u : 32u;
+            } else if (E >= 1u && E < 255u) {
+                const int ee = (int)E - 150;
+                Tr t = tr_id();
+                if (lane >= done)
+                    t = tr_cat(tr_cat(tr_elem(d[0], ee), tr_elem(d[1], ee)), tr_cat(tr_elem(d[2], ee), tr_elem(d[3], ee)));
+                for (int off = 1; off < 32; off <<= 1) {
+                    const Tr u = {__shfl_up_sync(0xffffffffu, t.w0, off), __shfl_up_sync(0xffffffffu, t.w1, off)};
+                    if (lane >= (uint32_t)off) t = tr_cat(u, t);
+                }
+                const uint32_t An = A + (((A & 1u) ? t.w1 : t.w0) & 0x7FFFFFFFu);
+                const uint32_t leaves = __ballot_sync(0xffffffffu, An >= (1u << 24));
+                f = leaves ? (uint32_t)__ffs((int)leaves) - 1u : 32u;
+                const uint32_t Af = __shfl_sync(0xffffffffu, An, f ? f - 1u : 0u);
+                if (f) acc = __uint_as_float((E << 23) | (Af & 0x7FFFFFu));
             }
-            uint32_t A = (bits & 0x7FFFFFu) | 0x800000u;
-            uint32_t w = __shfl_sync(0xffffffffu, (A & 1u) ? t.w1 : t.w0, 0);
-            uint32_t An = A + (w & 0x7FFFFFFFu);
-            if (An < (1u << 24)) {
-                acc = __uint_as_float((E << 23) | (An & 0x7FFFFFu));
-                continue;
-            }
+            if (f < 32)
+                for (int j = 0; j < 4; j++) acc = __fadd_rn(__shfl_sync(0xffffffffu, d[j], f), acc);
+            done = f + 1;
         }
-        for (int l = 0; l < 32; l++)
-            for (int j = 0; j < 4; j++) acc = __fadd_rn(__shfl_sync(0xffffffffu, d[j], l), acc);
     }
     return acc;
-}
-
-__device__ __forceinline__ float centre_of(float acc, uint32_t nk, float mn, float v)
-{
-    float mean = __fadd_rn(__fdiv_rn(acc, __uint2float_rn(nk)), mn);
-    return __fmul_rn(ceilf(__fdiv_rn(mean, v)), v);
 }
 
 // The nodes of a level that are split by a block each (above SMALL voxels) and
@@ -621,55 +787,99 @@ __global__ void k_classify(const float *P, Level L, float vx, float vy, float vz
     if (kind != K_INNER || nk > BIG) return;
     float v[3] = {vx, vy, vz};
     uint64_t s = L.start[k];
+    PlainSum x;
+    x.init();
+    for (uint32_t j = lane; j < nk; j += 32)
+        for (int a = 0; a < 3; a++) x.add(a, __fsub_rn(P[3 * (s + j) + a], bx[a]));
+    x.warp_merge();
     for (int a = 0; a < 3; a++) {
-        float acc = warp_sum(P, s, s + nk, a, bx[a], 0.0f);
+        float acc = x.exact(a) ? x.sum[a] : warp_sum(P, s, s + nk, a, bx[a], 0.0f);
         if (lane == 0) L.centre[3 * k + a] = centre_of(acc, nk, bx[a], v[a]);
     }
 }
 
-// Centres of big nodes: a warp per (node, axis) walks the node's chunks,
-// taking each chunk's map of the binade the sum is in from shared memory.
+// Centres of the other big nodes: a warp per (node, axis) walks the node's
+// chunks from where additions may round, 32 at a time: a scan of their maps of
+// the binade the sum is in gives the sum after each, up to the first chunk in
+// which it leaves the binade (or which has no map of it); that chunk is added
+// by its voxels.  The next 32 chunks' bases and sums, and with two maps a
+// chunk the maps, are loaded meanwhile: the walk is one warp's chain.
 constexpr int CENTRE_WARPS = 4;
+
+struct ChunkMaps {
+    int base;
+    bool some;       // the chunk's sum is not zero
+    uint4 two;       // its maps (window 2)
+    __device__ __forceinline__ void load(const uint2 *maps, const uint8_t *cbase, const float *csum, int window,
+                                         uint64_t maxc, int a, uint32_t c, bool in)
+    {
+        base = 0;
+        some = false;
+        two = make_uint4(0u, 0u, 0u, 0u);
+        if (!in) return;
+        base = cbase[3 * c + a];
+        some = csum[3 * c + a] != 0.0f;
+        if (window == 2) two = *reinterpret_cast<const uint4 *>(maps + map_index(maxc, 2, a, c, 0));
+    }
+};
+
 __global__ void __launch_bounds__(CENTRE_WARPS * 32) k_centre_big(const float *P, Level L, const uint32_t *big,
-                                                                  const uint32_t *nbig, const uint32_t *maps,
-                                                                  const uint8_t *nz, uint64_t maxc, float vx,
-                                                                  float vy, float vz)
+                                                                  const uint32_t *nbig, const uint2 *maps,
+                                                                  const uint8_t *cbase, const float *csum, int window,
+                                                                  const uint2 *starts, uint64_t maxc, float vx, float vy,
+                                                                  float vz)
 {
-    __shared__ uint32_t sm[CENTRE_WARPS][32 * NBIN * 2];
-    __shared__ uint8_t snz[CENTRE_WARPS][32];
     uint32_t w = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31;
     uint32_t j = w / 3;
     int a = (int)(w % 3);
     if (j >= *nbig) return;
-    uint32_t k = big[j];
-    if (L.kind[k] != K_INNER) return;
-    uint32_t nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK, c0 = L.chunk_base[k];
+    uint32_t k = big[j], c0 = L.chunk_base[k];
+    if (L.kind[k] != K_INNER || !cbase[3 * c0 + a]) return;
+    uint32_t nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK;
     uint64_t s = L.start[k], end = s + nk;
-    float mn = L.box[6 * k + a], acc = 0.0f;
-    int elo = L.ehi[3 * k + a] - (NBIN - 1);
-    for (uint32_t g = 0; g < nch; g += 32) {
-        uint32_t cnt = min(32u, nch - g);
-        const uint32_t *src = maps + map_index(maxc, a, c0 + g, 0);
-        __syncwarp();
-        for (uint32_t i = lane; i < cnt * NBIN * 2; i += 32) sm[wb][i] = src[i];
-        if ((uint32_t)lane < cnt) snz[wb][lane] = nz[3 * (c0 + g + lane) + a];
-        __syncwarp();
-        for (uint32_t i = 0; i < cnt; i++) {
-            if (acc == 0.0f && !snz[wb][i]) continue;   // all of its d are zero
-            uint32_t bits = __float_as_uint(acc), E = bits >> 23;
-            int bi = (int)E - 150 - elo;
-            if (E >= 1u && E < 255u && bi >= 0 && bi < NBIN) {
-                uint32_t A = (bits & 0x7FFFFFu) | 0x800000u;
-                uint32_t An = A + (sm[wb][(i * NBIN + bi) * 2 + (A & 1u)] & 0x7FFFFFFFu);
-                if (An < (1u << 24)) {
-                    acc = __uint_as_float((E << 23) | (An & 0x7FFFFFu));
-                    continue;
+    const uint2 first = starts[3 * j + a];
+    float mn = L.box[6 * k + a], acc = __uint_as_float(first.y);
+    uint32_t g = first.x;
+    ChunkMaps now, next;
+    now.load(maps, cbase, csum, window, maxc, a, c0 + g + lane, g + lane < nch);
+    for (; g < nch; g += 32) {
+        next.load(maps, cbase, csum, window, maxc, a, c0 + g + 32 + lane, g + 32 + lane < nch);
+        const uint32_t cnt = min(32u, nch - g);
+        for (uint32_t done = 0; done < cnt;) {            // chunks before g + done are added
+            uint32_t f = done;                            // the next chunk to add by its voxels
+            const uint32_t bits = __float_as_uint(acc), E = bits >> 23, A = (bits & 0x7FFFFFu) | 0x800000u;
+            if (acc == 0.0f) {                            // chunks of zeros change nothing
+                const uint32_t some = __ballot_sync(0xffffffffu, lane >= done && now.some);
+                f = some ? (uint32_t)__ffs((int)some) - 1u : cnt;
+            } else if (E >= 1u && E < 255u) {
+                const int bi = (int)E - now.base;
+                Tr t = tr_id();
+                if (lane >= done && lane < cnt) {
+                    t = {SAT, SAT | 0x80000000u};
+                    if (bi >= 0 && bi < window) {
+                        uint2 m = bi ? make_uint2(now.two.z, now.two.w) : make_uint2(now.two.x, now.two.y);
+                        if (window != 2) m = maps[map_index(maxc, window, a, c0 + g + lane, bi)];
+                        t = {m.x, m.y};
+                    }
                 }
+                for (int off = 1; off < 32; off <<= 1) {
+                    const Tr u = {__shfl_up_sync(0xffffffffu, t.w0, off), __shfl_up_sync(0xffffffffu, t.w1, off)};
+                    if (lane >= (uint32_t)off) t = tr_cat(u, t);
+                }
+                const uint32_t An = A + (((A & 1u) ? t.w1 : t.w0) & 0x7FFFFFFFu);
+                const uint32_t leaves = __ballot_sync(0xffffffffu, An >= (1u << 24));
+                f = leaves ? (uint32_t)__ffs((int)leaves) - 1u : cnt;
+                const uint32_t Af = __shfl_sync(0xffffffffu, An, f ? f - 1u : 0u);
+                if (f) acc = __uint_as_float((E << 23) | (Af & 0x7FFFFFu));
             }
-            uint64_t b = s + (uint64_t)(g + i) * CHUNK;
-            acc = warp_sum(P, b, min(b + CHUNK, end), a, mn, acc);
+            if (f < cnt) {
+                const uint64_t b = s + (uint64_t)(g + f) * CHUNK;
+                acc = warp_sum(P, b, min(b + CHUNK, end), a, mn, acc);
+            }
+            done = f + 1;
         }
+        now = next;
     }
     float v[3] = {vx, vy, vz};
     if (lane == 0) L.centre[3 * k + a] = centre_of(acc, nk, mn, v[a]);
@@ -1338,9 +1548,11 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     } level_free{levels, s};
 
     float *P[2];
-    uint32_t *idx[2], *seg_of, *tile, *scal, *maps, *cidx, *big;
-    uint8_t *oct[2], *nz;
-    float *cv;
+    uint32_t *idx[2], *seg_of, *tile, *scal, *cidx, *big;
+    uint8_t *oct[2], *cbase;
+    float *cv, *csum;
+    int *cgrid;
+    uint2 *maps, *starts;
     unsigned long long *stats;
     uint64_t max_chunks = N / CHUNK + N / BIG + 2;
     uint64_t max_big = N / BIG + 1;
@@ -1357,15 +1569,22 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     // 8 error bits
     TRY(d.get(&scal, 12));
     TRY(d.get(&big, max_big));
+    // past 2^24 additions a sum's roundings can add up to a sizeable part of it
+    const int window = N > (1u << 24) ? NBIN : 2;
     if (N > BIG) {
         TRY(d.get(&cv, 6 * max_chunks));
         TRY(d.get(&cidx, 6 * max_chunks));
-        TRY(d.get(&maps, max_chunks * NBIN * 3 * 2));
-        TRY(d.get(&nz, 3 * max_chunks));
+        TRY(d.get(&maps, max_chunks * window * 3));
+        TRY(d.get(&starts, 3 * max_big));
+        TRY(d.get(&csum, 3 * max_chunks));
+        TRY(d.get(&cgrid, 3 * max_chunks));
+        TRY(d.get(&cbase, 3 * max_chunks));
     } else {
-        cv = nullptr;
-        cidx = maps = nullptr;
-        nz = nullptr;
+        cv = csum = nullptr;
+        cidx = nullptr;
+        maps = starts = nullptr;
+        cgrid = nullptr;
+        cbase = nullptr;
     }
     TRY(d.get(&stats, 4 * MAX_LEVELS));
     uint32_t *err = scal + 8;
@@ -1417,27 +1636,30 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         k_seg_of<<<grid_for(N, TB), TB, 0, s>>>(L.start, L.n, m, N, seg_of);
         count_launch();
         bool has_big = largest > BIG;
-        if (has_big) {   // chunk extremes of big nodes
-            scan(ChunkCount{L.n}, StoreExcl{L.chunk_base}, m, tile, scal + 0, s);
+        const unsigned nodes_big = (unsigned)max_big;
+        if (has_big) {   // boxes of big nodes from their chunks
+            scan(ChunkCount{L.n}, StoreChunks{L.chunk_base, big, scal + 3}, m, tile, scal + 0, s);
             k_chunk_box<<<(unsigned)max_chunks, CHUNK_THREADS, 0, s>>>(P[cur], L, scal + 0, cv, cidx);
+            k_box_big<<<nodes_big, NODE_THREADS, 0, s>>>(L, big, scal + 3, cv, cidx, vx, vy, vz);
+            count_launch();
             count_launch();
         }
         k_box_thread<<<grid_for(m, TB), TB, 0, s>>>(P[cur], L, vx, vy, vz);
         count_launch();
         if (largest > TINY) {
-            k_box_warp<<<grid_for((uint64_t)m * 32, TB), TB, 0, s>>>(P[cur], L, cv, cidx, vx, vy, vz, big, scal + 3);
-            count_launch();
-        }
-        if (has_big) {
-            k_chunk_maps<<<(unsigned)max_chunks, CHUNK_THREADS, 0, s>>>(P[cur], L, scal + 0, maps, nz, max_chunks);
+            k_box_warp<<<grid_for((uint64_t)m * 32, TB), TB, 0, s>>>(P[cur], L, vx, vy, vz);
             count_launch();
         }
         k_classify<<<grid_for((uint64_t)m * 32, TB), TB, 0, s>>>(P[cur], L, vx, vy, vz, lists);
         count_launch();
-        if (has_big) {
+        if (has_big) {   // their centres
+            k_chunk_sums<<<(unsigned)max_chunks, CHUNK_THREADS, 0, s>>>(P[cur], L, scal + 0, csum, cgrid);
+            k_centre_plain<<<nodes_big, NODE_THREADS, 0, s>>>(L, big, scal + 3, csum, cgrid, cbase, window, starts, vx, vy, vz);
+            k_chunk_maps<<<(unsigned)max_chunks, CHUNK_THREADS, 0, s>>>(P[cur], L, scal + 0, cbase, window, maps,
+                                                                       max_chunks);
             k_centre_big<<<grid_for(max_big * 3 * 32, CENTRE_WARPS * 32), CENTRE_WARPS * 32, 0, s>>>(
-                P[cur], L, big, scal + 3, maps, nz, max_chunks, vx, vy, vz);
-            count_launch();
+                P[cur], L, big, scal + 3, maps, cbase, csum, window, starts, max_chunks, vx, vy, vz);
+            for (int i = 0; i < 4; i++) count_launch();
         }
         k_oct_init<<<grid_for(N, TB), TB, 0, s>>>(P[cur], L, seg_of, N, idx[0], oct[0]);
         count_launch();
