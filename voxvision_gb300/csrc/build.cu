@@ -77,10 +77,8 @@ constexpr uint32_t NONE = 0xFFFFFFFFu;
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
 constexpr uint32_t SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
-constexpr uint32_t BIG = 4096;       // nodes with more voxels sum their coordinates by chunks
-constexpr uint32_t SMALL = 512;      // nodes with at most this many voxels are split by one warp
+constexpr uint32_t SMALL = 512;      // nodes with at most this many voxels are made by one warp
 constexpr uint32_t MID = 8192;       // nodes with at most this many by one block, larger ones tile by tile
-constexpr uint32_t TINY = 32;        // nodes with at most this many voxels get their box from one thread
 constexpr uint32_t CHUNK = 1024;     // voxels per chunk
 constexpr int CHUNK_THREADS = 128;   // 8 consecutive voxels per thread
 constexpr int NBIN = 16;             // binades with a precomputed map per chunk
@@ -89,6 +87,7 @@ constexpr int MAX_LEVELS = 90;       // deeper trees exceed the traversal stack 
 constexpr uint64_t MAX_VOXELS = 0x7FFFFFFFull;
 
 enum : uint8_t { K_INNER = 0, K_LEAF = 1, K_DENSE = 2, K_OVER = 3 };
+enum : int { S_INNER = 0, S_LEAF = 1, S_DENSE = 2, S_DOTS = 3, S_OVER = 4, NSTATS = 5 };   // a level's counts
 
 // error bits reported by kernels
 constexpr uint32_t ERR_WALK = 1u;       // a swapping-pass walk did not end as it must
@@ -183,30 +182,17 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_tile_apply(V v, W w, uint64_t 
     }
 }
 
-template <class V, class W>
-void scan(V v, W w, uint64_t m, uint32_t *tile, uint32_t *total, cudaStream_t s)
-{
-    uint32_t nt = (uint32_t)((m + SCAN_TILE - 1) / SCAN_TILE);
-    if (nt == 0) {
-        cudaMemsetAsync(total, 0, 4, s);
-        return;
-    }
-    k_tile_sums<<<nt, SCAN_THREADS, 0, s>>>(v, m, tile);
-    k_scan_tiles<<<1, 1024, 0, s>>>(tile, nt, total);
-    k_tile_apply<<<nt, SCAN_THREADS, 0, s>>>(v, w, m, tile);
-    count_launch();
-    count_launch();
-    count_launch();
-}
-
 // ------------------------------------------------------------ level arrays
 
-// The nodes of one level, in position order (children are made in parent
-// order, octant order, so their voxel ranges ascend).
+// The nodes of one level, in no particular order (the children of a node are
+// consecutive, in octant order).  The voxels of a level's leaves stay where
+// they are in the order of their level: the orders of successive levels
+// alternate between two buffers, and a later level writes only where its own
+// nodes lie.
 struct Level {
     uint32_t m = 0;
     void *mem = nullptr;
-    uint32_t *start, *n, *cnt, *first_child, *chunk_base, *sub_nodes, *id, *ustart, *rec;
+    uint32_t *start, *n, *cnt, *first_child, *sub_nodes, *id, *ustart, *rec;
     unsigned long long *sub_units;
     float *box, *centre;
     int *ehi;
@@ -226,7 +212,7 @@ cudaError_t level_alloc(Level &L, uint32_t m, cudaStream_t s)
     size_t mm = m ? m : 1;
     size_t bytes = 0;
     auto add = [&](size_t b) { bytes += (b + 255) & ~size_t(255); };
-    add(4 * mm); add(4 * mm); add(32 * mm); add(4 * mm); add(4 * mm); add(4 * mm); add(4 * mm); add(4 * mm);
+    add(4 * mm); add(4 * mm); add(32 * mm); add(4 * mm); add(4 * mm); add(4 * mm); add(4 * mm);
     add(4 * mm); add(8 * mm); add(24 * mm); add(12 * mm); add(12 * mm); add(mm); add(mm);
     cudaError_t e = cudaMallocAsync(&L.mem, bytes, s);
     if (e != cudaSuccess) { L.mem = nullptr; return e; }
@@ -236,7 +222,6 @@ cudaError_t level_alloc(Level &L, uint32_t m, cudaStream_t s)
     L.n = carve<uint32_t>(p, mm);
     L.cnt = carve<uint32_t>(p, 8 * mm);
     L.first_child = carve<uint32_t>(p, mm);
-    L.chunk_base = carve<uint32_t>(p, mm);
     L.sub_nodes = carve<uint32_t>(p, mm);
     L.id = carve<uint32_t>(p, mm);
     L.ustart = carve<uint32_t>(p, mm);
@@ -247,58 +232,71 @@ cudaError_t level_alloc(Level &L, uint32_t m, cudaStream_t s)
     L.ehi = carve<int>(p, 3 * mm);
     L.kind = carve<uint8_t>(p, mm);
     L.mask = carve<uint8_t>(p, mm);
-    return cudaMemsetAsync(L.cnt, 0, 32 * mm, s);
+    return cudaSuccess;
 }
 
 // -------------------------------------------------------- per-level kernels
 
-__global__ void k_seg_of(const uint32_t *start, const uint32_t *n, uint32_t m, uint64_t N, uint32_t *seg_of)
-{
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= N) return;
-    if (m == 0 || start[0] > t) {
-        seg_of[t] = NONE;
-        return;
-    }
-    uint32_t lo = 0, hi = m;   // the last node starting at or before t is in [lo, hi)
-    while (hi - lo > 1) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (start[mid] <= t) lo = mid;
-        else hi = mid;
-    }
-    seg_of[t] = t < (uint64_t)start[lo] + n[lo] ? lo : NONE;
-}
-
-struct ChunkCount {
-    const uint32_t *n;
-    __device__ uint32_t operator()(uint64_t k) const { return n[k] > BIG ? (n[k] + CHUNK - 1) / CHUNK : 0u; }
-};
-// First chunks, and the nodes that have chunks listed.
-struct StoreChunks {
-    uint32_t *out, *big, *nbig;
-    __device__ void operator()(uint64_t i, uint32_t excl, uint32_t chunks) const
+// The nodes of a level that take more than one thread, by size class, in no
+// particular order: above VOX_MAX_DOTS voxels a warp each, above SMALL a
+// block, above MID tile by tile.  A tiled node's slot and its first tile come
+// from one counter, so that first tiles ascend with slots.
+struct NodeLists {
+    uint32_t *small, *mid, *tiled, *first_tile;
+    uint32_t *nsmall, *nmid;
+    unsigned long long *ntiled;   // slots in the upper half, tiles in the lower
+    uint32_t tile;                // positions per tile
+    __device__ void add_large(uint32_t k, uint32_t n) const
     {
-        out[i] = excl;
-        if (chunks) big[atomicAdd(nbig, 1u)] = (uint32_t)i;
+        if (n > MID) {
+            const unsigned long long at = atomicAdd(ntiled, (1ull << 32) | ((n + tile - 1) / tile));
+            tiled[at >> 32] = k;
+            first_tile[at >> 32] = (uint32_t)at;
+        } else if (n > SMALL) {
+            mid[atomicAdd(nmid, 1u)] = k;
+        }
     }
 };
-struct StoreExcl {
-    uint32_t *out;
-    __device__ void operator()(uint64_t i, uint32_t excl, uint32_t) const { out[i] = excl; }
+
+// What a level counts: kinds (S_*), the next level's nodes and the largest.
+struct Tally {
+    unsigned long long *stats;
+    uint32_t *children, *largest, *err;
 };
 
-// The node of chunk c: the last node whose first chunk is at or before c
-// (nodes without chunks share their successor's base).
-__device__ __forceinline__ uint32_t chunk_node(const uint32_t *chunk_base, uint32_t m, uint32_t c)
+// The node of a tile: its slot, or NO_POS for a block without one.
+constexpr uint32_t NO_POS = 0xFFFFFFFFu;
+__device__ __forceinline__ uint32_t tile_slot(const NodeLists &lists, uint32_t tile)
 {
-    uint32_t lo = 0, hi = m;
+    const unsigned long long n = *lists.ntiled;
+    if (tile >= (uint32_t)n) return NO_POS;
+    uint32_t lo = 0, hi = (uint32_t)(n >> 32);
     while (hi - lo > 1) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (chunk_base[mid] <= c) lo = mid;
+        const uint32_t mid = (lo + hi) >> 1;
+        if (lists.first_tile[mid] <= tile) lo = mid;
         else hi = mid;
     }
     return lo;
 }
+
+// Tiled nodes are summed by chunks of CHUNK voxels, counted through the tiles
+// (a tile is a multiple of CHUNK): the range of chunk c; false for a chunk
+// past its node's end.
+struct ChunkRange {
+    uint32_t k;
+    uint64_t b, e;
+    __device__ bool find(const NodeLists &lists, const Level &L, uint32_t c)
+    {
+        const uint32_t per = lists.tile / CHUNK, slot = tile_slot(lists, c / per);
+        if (slot == NO_POS) return false;
+        k = lists.tiled[slot];
+        const uint32_t at = (c - lists.first_tile[slot] * per) * CHUNK, n = L.n[k];
+        if (at >= n) return false;
+        b = (uint64_t)L.start[k] + at;
+        e = min(b + CHUNK, (uint64_t)L.start[k] + n);
+        return true;
+    }
+};
 
 // First-occurrence extremes: the serial scan of tree.c:138-155 keeps the first
 // of equal values (which matters only for -0 against +0), so ties go to the
@@ -350,19 +348,17 @@ struct Extremes {
     }
 };
 
-// Partial extremes of one chunk of a big node.
-__global__ void __launch_bounds__(CHUNK_THREADS) k_chunk_box(const float *P, Level L, const uint32_t *total,
-                                                            float *cv, uint32_t *ci)
+// Partial extremes of one chunk of a tiled node.
+__global__ void __launch_bounds__(CHUNK_THREADS) k_chunk_box(const float *P, Level L, NodeLists lists, float *cv,
+                                                            uint32_t *ci)
 {
     __shared__ Extremes part[CHUNK_THREADS / 32];
-    uint32_t c = blockIdx.x;
-    if (c >= *total) return;
-    uint32_t k = chunk_node(L.chunk_base, L.m, c);
-    uint64_t b = (uint64_t)L.start[k] + (uint64_t)(c - L.chunk_base[k]) * CHUNK;
-    uint64_t e = min(b + CHUNK, (uint64_t)L.start[k] + L.n[k]);
+    const uint32_t c = blockIdx.x;
+    ChunkRange r;
+    if (!r.find(lists, L, c)) return;
     Extremes x;
     x.init();
-    for (uint64_t t = b + threadIdx.x; t < e; t += CHUNK_THREADS) x.add(P + 3 * t, (uint32_t)t);
+    for (uint64_t t = r.b + threadIdx.x; t < r.e; t += CHUNK_THREADS) x.add(P + 3 * t, (uint32_t)t);
     x.warp_merge();
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = x;
     __syncthreads();
@@ -375,80 +371,40 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_chunk_box(const float *P, Lev
     }
 }
 
-// The box of node k and the top binade its coordinate sums can reach.
-__device__ void write_box(const Level &L, uint32_t k, const float *mn, const float *mx, const float *v)
+// The box of node k (calc_bounding_box, tree.c:138-155) and what it is by its
+// density (geom.c:157-167) and size, before it is split (tree.c:249-275).
+__device__ uint8_t write_box(const Level &L, uint32_t k, uint32_t nk, const float *mn, const float *mx, const float *v)
 {
-    uint32_t nk = L.n[k];
+    float hi[3];
     for (int a = 0; a < 3; a++) {
-        L.box[6 * k + a] = mn[a];
-        float hi = __fadd_rn(mx[a], v[a]);
-        L.box[6 * k + 3 + a] = hi;
-        // The float sum of nk values in [0, extent] stays below 2 * nk * extent
-        // for any nk this builder accepts (each addition rounds up by at most
-        // 2^-24 relative); were it ever higher, its chunks would just be added
-        // one voxel at a time.
-        double bound = 2.0 * (double)nk * (double)__fsub_rn(hi, mn[a]);
-        int ehi = -100000;
-        if (bound > 0.0 && bound < 1e38) {
-            int ex;
-            frexp(bound, &ex);
-            ehi = ex - 24;           // bound in [2^(ex-1), 2^ex): its ulp exponent
-            if (ehi < -149) ehi = -149;
-        }
-        L.ehi[3 * k + a] = ehi;
+        hi[a] = __fadd_rn(mx[a], v[a]);
+        L.box[6 * (size_t)k + a] = mn[a];
+        L.box[6 * (size_t)k + 3 + a] = hi[a];
     }
+    const float bbv = __fmul_rn(__fmul_rn(__fsub_rn(hi[0], mn[0]), __fsub_rn(hi[1], mn[1])), __fsub_rn(hi[2], mn[2]));
+    const float vv = __fmul_rn(__fmul_rn(v[0], v[1]), v[2]);
+    const uint8_t kind = fabsf(__fsub_rn(__fmul_rn(__uint2float_rn(nk), vv), bbv)) < vv ? K_DENSE
+                       : (nk <= VOX_MAX_DOTS ? K_LEAF : K_INNER);
+    L.kind[k] = kind;
+    L.mask[k] = 0;
+    return kind;
 }
 
-// Bounding boxes (calc_bounding_box, tree.c:138-155) of nodes of at most TINY
-// voxels: the serial scan itself, one thread per node.
-__global__ void k_box_thread(const float *P, Level L, float vx, float vy, float vz)
-{
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= L.m || L.n[k] > TINY) return;
-    const float *p = P + 3 * (uint64_t)L.start[k];
-    float mn[3] = {p[0], p[1], p[2]}, mx[3] = {p[0], p[1], p[2]};
-    for (uint32_t i = 1; i < L.n[k]; i++)
-        for (int a = 0; a < 3; a++) {
-            float x = p[3 * i + a];
-            if (x < mn[a]) mn[a] = x;
-            else if (x > mx[a]) mx[a] = x;
-        }
-    float v[3] = {vx, vy, vz};
-    write_box(L, k, mn, mx, v);
-}
-
-// Nodes of TINY+1..BIG voxels: a warp per node over its voxels.
-__global__ void k_box_warp(const float *P, Level L, float vx, float vy, float vz)
-{
-    uint32_t k = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    int lane = threadIdx.x & 31;
-    if (k >= L.m) return;
-    uint32_t nk = L.n[k];
-    if (nk <= TINY || nk > BIG) return;
-    Extremes x;
-    x.init();
-    uint64_t s = L.start[k];
-    for (uint32_t j = lane; j < nk; j += 32) x.add(P + 3 * (s + j), (uint32_t)(s + j));
-    x.warp_merge();
-    if (lane) return;
-    float v[3] = {vx, vy, vz};
-    write_box(L, k, x.mn, x.mx, v);
-}
-
-// Big nodes: a block per node over its chunks' partial extremes.
+// Tiled nodes: a block per node over its chunks' partial extremes; and the top
+// binade its coordinate sums can reach.
 constexpr int NODE_THREADS = 256;
-__global__ void __launch_bounds__(NODE_THREADS) k_box_big(Level L, const uint32_t *big, const uint32_t *nbig,
-                                                          const float *cv, const uint32_t *ci, float vx, float vy,
-                                                          float vz)
+__global__ void __launch_bounds__(NODE_THREADS) k_box_tiled(Level L, NodeLists lists, const float *cv,
+                                                            const uint32_t *ci, float vx, float vy, float vz, Tally tally)
 {
     __shared__ Extremes part[NODE_THREADS / 32];
-    if (blockIdx.x >= *nbig) return;
-    const uint32_t k = big[blockIdx.x], nch = (L.n[k] + CHUNK - 1) / CHUNK, c0 = L.chunk_base[k];
+    if (blockIdx.x >= (uint32_t)(*lists.ntiled >> 32)) return;
+    const uint32_t k = lists.tiled[blockIdx.x], nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK,
+                   c0 = lists.first_tile[blockIdx.x] * (lists.tile / CHUNK);
     Extremes x;
     x.init();
     for (uint32_t j = threadIdx.x; j < nch; j += NODE_THREADS) {
         Extremes o;
-        const uint32_t c = c0 + j;
+        const size_t c = c0 + j;
         for (int a = 0; a < 3; a++) {
             o.mn[a] = cv[6 * c + a]; o.mni[a] = ci[6 * c + a];
             o.mx[a] = cv[6 * c + 3 + a]; o.mxi[a] = ci[6 * c + 3 + a];
@@ -460,8 +416,23 @@ __global__ void __launch_bounds__(NODE_THREADS) k_box_big(Level L, const uint32_
     __syncthreads();
     if (threadIdx.x) return;
     for (int w = 1; w < NODE_THREADS / 32; w++) x.merge(part[w]);
-    float v[3] = {vx, vy, vz};
-    write_box(L, k, x.mn, x.mx, v);
+    const float v[3] = {vx, vy, vz};
+    if (write_box(L, k, nk, x.mn, x.mx, v) == K_DENSE) atomicAdd(&tally.stats[S_DENSE], 1ull);
+    for (int a = 0; a < 3; a++) {
+        // The float sum of nk values in [0, extent] stays below 2 * nk * extent
+        // for any nk this builder accepts (each addition rounds up by at most
+        // 2^-24 relative); were it ever higher, its chunks would just be added
+        // one voxel at a time.
+        double bound = 2.0 * (double)nk * (double)__fsub_rn(L.box[6 * (size_t)k + 3 + a], x.mn[a]);
+        int ehi = -100000;
+        if (bound > 0.0 && bound < 1e38) {
+            int ex;
+            frexp(bound, &ex);
+            ehi = ex - 24;           // bound in [2^(ex-1), 2^ex): its ulp exponent
+            if (ehi < -149) ehi = -149;
+        }
+        L.ehi[3 * (size_t)k + a] = ehi;
+    }
 }
 
 // ---- sums that no addition rounds
@@ -552,20 +523,18 @@ __device__ __forceinline__ Tr tr_shfl_down(Tr t, int off)
     return {__shfl_down_sync(0xffffffffu, t.w0, off), __shfl_down_sync(0xffffffffu, t.w1, off)};
 }
 
-// Sums and common powers of two of one chunk of a big node, per axis.
-__global__ void __launch_bounds__(CHUNK_THREADS) k_chunk_sums(const float *P, Level L, const uint32_t *total,
-                                                              float *csum, int *cgrid)
+// Sums and common powers of two of one chunk of a tiled node, per axis.
+__global__ void __launch_bounds__(CHUNK_THREADS) k_chunk_sums(const float *P, Level L, NodeLists lists, float *csum,
+                                                              int *cgrid)
 {
     __shared__ PlainSum part[CHUNK_THREADS / 32];
     const uint32_t c = blockIdx.x;
-    if (c >= *total) return;
-    const uint32_t k = chunk_node(L.chunk_base, L.m, c);
-    const uint64_t b = (uint64_t)L.start[k] + (uint64_t)(c - L.chunk_base[k]) * CHUNK;
-    const uint64_t e = min(b + CHUNK, (uint64_t)L.start[k] + L.n[k]);
+    ChunkRange r;
+    if (!r.find(lists, L, c)) return;
     PlainSum x;
     x.init();
-    for (uint64_t t = b + threadIdx.x; t < e; t += CHUNK_THREADS)
-        for (int a = 0; a < 3; a++) x.add(a, __fsub_rn(P[3 * t + a], L.box[6 * k + a]));
+    for (uint64_t t = r.b + threadIdx.x; t < r.e; t += CHUNK_THREADS)
+        for (int a = 0; a < 3; a++) x.add(a, __fsub_rn(P[3 * t + a], L.box[6 * (size_t)r.k + a]));
     x.warp_merge();
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = x;
     __syncthreads();
@@ -593,14 +562,15 @@ __device__ __forceinline__ float centre_of(float acc, uint32_t nk, float mn, flo
 // so that with the next one the sum's own binade is among them unless its
 // roundings added up to more than that.  0: the axis needs no maps.  With
 // window > 2 (sums so long that they do) the binades below the node's top.
-__global__ void __launch_bounds__(NODE_THREADS) k_centre_plain(Level L, const uint32_t *big, const uint32_t *nbig,
-                                                               const float *csum, const int *cgrid, uint8_t *cbase,
+__global__ void __launch_bounds__(NODE_THREADS) k_centre_plain(Level L, NodeLists lists, const float *csum,
+                                                               const int *cgrid, uint8_t *cbase,
                                                                int window, uint2 *starts, float vx, float vy, float vz)
 {
     __shared__ PlainSum part[NODE_THREADS / 32];
     __shared__ double wsum[NODE_THREADS / 32], carry;
-    if (blockIdx.x >= *nbig) return;
-    const uint32_t k = big[blockIdx.x], nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK, c0 = L.chunk_base[k];
+    if (blockIdx.x >= (uint32_t)(*lists.ntiled >> 32)) return;
+    const uint32_t k = lists.tiled[blockIdx.x], nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK,
+                   c0 = lists.first_tile[blockIdx.x] * (lists.tile / CHUNK);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     PlainSum x;
     x.init();
@@ -655,24 +625,22 @@ __device__ __forceinline__ size_t map_index(uint64_t maxc, int window, int a, ui
 
 // Maps of one chunk of a big node for the `window` binades from its base on,
 // per axis that needs them.
-__global__ void __launch_bounds__(CHUNK_THREADS) k_chunk_maps(const float *P, Level L, const uint32_t *total,
+__global__ void __launch_bounds__(CHUNK_THREADS) k_chunk_maps(const float *P, Level L, NodeLists lists,
                                                              const uint8_t *cbase, int window, uint2 *maps,
                                                              uint64_t maxc)
 {
     __shared__ Tr part[NBIN][3][CHUNK_THREADS / 32];
-    uint32_t c = blockIdx.x;
-    if (c >= *total) return;
+    const uint32_t c = blockIdx.x;
+    ChunkRange r;
+    if (!r.find(lists, L, c)) return;
     const int base[3] = {cbase[3 * c], cbase[3 * c + 1], cbase[3 * c + 2]};
     if (!(base[0] | base[1] | base[2])) return;
-    uint32_t k = chunk_node(L.chunk_base, L.m, c);
-    uint64_t b = (uint64_t)L.start[k] + (uint64_t)(c - L.chunk_base[k]) * CHUNK;
-    uint64_t e = min(b + CHUNK, (uint64_t)L.start[k] + L.n[k]);
-    uint64_t t0 = b + (uint64_t)threadIdx.x * 8;
+    const uint64_t t0 = r.b + (uint64_t)threadIdx.x * 8, e = r.e;
     float d[8][3];
     uint32_t cnt = t0 < e ? (uint32_t)(e - t0 < 8 ? e - t0 : 8) : 0u;
     for (int q = 0; q < 8; q++)
         for (int a = 0; a < 3; a++)
-            d[q][a] = (uint32_t)q < cnt ? __fsub_rn(P[3 * (t0 + q) + a], L.box[6 * k + a]) : 0.0f;
+            d[q][a] = (uint32_t)q < cnt ? __fsub_rn(P[3 * (t0 + q) + a], L.box[6 * (size_t)r.k + a]) : 0.0f;
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int bi = 0; bi < window; bi++)
         for (int a = 0; a < 3; a++) {
@@ -746,58 +714,6 @@ __device__ float warp_sum(const float *P, uint64_t b, uint64_t e, int a, float m
     return acc;
 }
 
-// The nodes of a level that are split by a block each (above SMALL voxels) and
-// tile by tile (above MID), in no particular order: a tiled node's slot and
-// its first tile come from one counter, so that first tiles ascend with slots.
-struct SplitLists {
-    uint32_t *mid, *nmid, *tiled, *first_tile;
-    unsigned long long *ntiled;   // slots in the upper half, tiles in the lower
-    uint32_t tile;                // positions per tile
-    __device__ void add(uint32_t k, uint32_t n) const
-    {
-        if (n > MID) {
-            const unsigned long long at = atomicAdd(ntiled, (1ull << 32) | ((n + tile - 1) / tile));
-            tiled[at >> 32] = k;
-            first_tile[at >> 32] = (uint32_t)at;
-        } else if (n > SMALL) {
-            mid[atomicAdd(nmid, 1u)] = k;
-        }
-    }
-};
-
-// Node kinds and, for nodes of at most BIG voxels, subdivision centres
-// (tree.c:249-275, find_center tree.c:125-136, density test geom.c:157-167);
-// a warp per node.
-__global__ void k_classify(const float *P, Level L, float vx, float vy, float vz, SplitLists lists)
-{
-    uint32_t k = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    int lane = threadIdx.x & 31;
-    if (k >= L.m) return;
-    uint32_t nk = L.n[k];
-    const float *bx = L.box + 6 * k;
-    float s0 = __fsub_rn(bx[3], bx[0]), s1 = __fsub_rn(bx[4], bx[1]), s2 = __fsub_rn(bx[5], bx[2]);
-    float bbv = __fmul_rn(__fmul_rn(s0, s1), s2);
-    float vv = __fmul_rn(__fmul_rn(vx, vy), vz);
-    uint8_t kind = fabsf(__fsub_rn(__fmul_rn(__uint2float_rn(nk), vv), bbv)) < vv ? K_DENSE
-                 : (nk <= VOX_MAX_DOTS ? K_LEAF : K_INNER);
-    if (lane == 0) {
-        L.kind[k] = kind;
-        if (kind == K_INNER) lists.add(k, nk);
-    }
-    if (kind != K_INNER || nk > BIG) return;
-    float v[3] = {vx, vy, vz};
-    uint64_t s = L.start[k];
-    PlainSum x;
-    x.init();
-    for (uint32_t j = lane; j < nk; j += 32)
-        for (int a = 0; a < 3; a++) x.add(a, __fsub_rn(P[3 * (s + j) + a], bx[a]));
-    x.warp_merge();
-    for (int a = 0; a < 3; a++) {
-        float acc = x.exact(a) ? x.sum[a] : warp_sum(P, s, s + nk, a, bx[a], 0.0f);
-        if (lane == 0) L.centre[3 * k + a] = centre_of(acc, nk, bx[a], v[a]);
-    }
-}
-
 // Centres of the other big nodes: a warp per (node, axis) walks the node's
 // chunks from where additions may round, 32 at a time: a scan of their maps of
 // the binade the sum is in gives the sum after each, up to the first chunk in
@@ -823,8 +739,8 @@ struct ChunkMaps {
     }
 };
 
-__global__ void __launch_bounds__(CENTRE_WARPS * 32) k_centre_big(const float *P, Level L, const uint32_t *big,
-                                                                  const uint32_t *nbig, const uint2 *maps,
+__global__ void __launch_bounds__(CENTRE_WARPS * 32) k_centre_big(const float *P, Level L, NodeLists lists,
+                                                                  const uint2 *maps,
                                                                   const uint8_t *cbase, const float *csum, int window,
                                                                   const uint2 *starts, uint64_t maxc, float vx, float vy,
                                                                   float vz)
@@ -833,8 +749,8 @@ __global__ void __launch_bounds__(CENTRE_WARPS * 32) k_centre_big(const float *P
     const uint32_t lane = threadIdx.x & 31;
     uint32_t j = w / 3;
     int a = (int)(w % 3);
-    if (j >= *nbig) return;
-    uint32_t k = big[j], c0 = L.chunk_base[k];
+    if (j >= (uint32_t)(*lists.ntiled >> 32)) return;
+    uint32_t k = lists.tiled[j], c0 = lists.first_tile[j] * (lists.tile / CHUNK);
     if (L.kind[k] != K_INNER || !cbase[3 * c0 + a]) return;
     uint32_t nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK;
     uint64_t s = L.start[k], end = s + nk;
@@ -885,115 +801,13 @@ __global__ void __launch_bounds__(CENTRE_WARPS * 32) k_centre_big(const float *P
     if (lane == 0) L.centre[3 * k + a] = centre_of(acc, nk, mn, v[a]);
 }
 
-// The eight swapping passes (sort_set, tree.c:166-183) of nodes of at most
-// SMALL voxels: a warp per node in shared memory, each pass in the parallel
-// form of the file's header (ballot prefix counts, the walk back for the rest).
-constexpr int PART_WARPS = 4;
-__global__ void __launch_bounds__(PART_WARPS * 32) k_partition_warp(Level L, uint32_t *idx, uint8_t *oct,
-                                                                     uint32_t *err)
-{
-    __shared__ uint32_t sidx[PART_WARPS][2][SMALL];
-    __shared__ uint8_t soct[PART_WARPS][2][SMALL];
-    __shared__ uint16_t sc[PART_WARPS][SMALL], su[PART_WARPS][SMALL];
-    uint32_t k = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    uint32_t lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
-    if (k >= L.m) return;
-    uint32_t nk = L.n[k];
-    if (L.kind[k] != K_INNER || nk > SMALL) return;
-    uint32_t s0 = L.start[k];
-    for (uint32_t i = lane; i < nk; i += 32) {
-        sidx[wb][0][i] = idx[s0 + i];
-        soct[wb][0][i] = oct[s0 + i];
-    }
-    __syncwarp();
-    const uint32_t lt = (1u << lane) - 1u;
-    uint32_t from = 0;
-    int cur = 0;
-    for (uint32_t o = 0; o < 8; o++) {
-        const uint32_t *in_i = sidx[wb][cur];
-        const uint8_t *in_o = soct[wb][cur];
-        uint32_t *out_i = sidx[wb][cur ^ 1];
-        uint8_t *out_o = soct[wb][cur ^ 1];
-        for (uint32_t i = lane; i < from; i += 32) {   // claimed by earlier passes
-            out_i[i] = in_i[i];
-            out_o[i] = in_o[i];
-        }
-        uint32_t run = 0, urun = 0;
-        for (uint32_t base = from; base < nk; base += 32) {
-            uint32_t t = base + lane;
-            bool in = t < nk;
-            uint8_t q = in ? in_o[t] : (uint8_t)0xFF;
-            bool cl = in && q == o;
-            uint32_t bm = __ballot_sync(0xffffffffu, cl), um = __ballot_sync(0xffffffffu, in && !cl);
-            uint32_t crel = run + __popc(bm & lt), urel = urun + __popc(um & lt);
-            if (in) {
-                sc[wb][t] = (uint16_t)crel;
-                if (cl) {
-                    out_i[from + crel] = in_i[t];
-                    out_o[from + crel] = q;
-                } else {
-                    su[wb][from + urel] = (uint16_t)t;
-                }
-            }
-            run += __popc(bm);
-            urun += __popc(um);
-        }
-        __syncwarp();
-        for (uint32_t t = from + run + lane; t < nk; t += 32) {
-            uint32_t s = t;
-            for (uint32_t steps = 0; in_o[s] == o; steps++) {
-                uint32_t u = (s - from) - sc[wb][s];
-                if (u == 0 || steps > SMALL) {
-                    atomicOr(err, ERR_WALK);
-                    break;
-                }
-                uint32_t a = su[wb][from + u - 1] + 1u;
-                uint32_t back = ((s - a) / u + 1) * u;
-                if (a > s || back > s - from) {
-                    atomicOr(err, ERR_WALK);
-                    break;
-                }
-                s -= back;
-            }
-            out_i[t] = in_i[s];
-            out_o[t] = in_o[s];
-        }
-        if (lane == 0) L.cnt[8 * k + o] = run;
-        from += run;
-        cur ^= 1;
-        __syncwarp();
-    }
-    for (uint32_t i = lane; i < nk; i += 32) {   // eight passes: back in buffer 0
-        idx[s0 + i] = sidx[wb][0][i];
-        oct[s0 + i] = soct[wb][0][i];
-    }
-}
-
-// Identity permutation and octants (get_subspace_idx, geom.c:44-51) of the
-// voxels of nodes to split; 0xFF elsewhere.
-__global__ void k_oct_init(const float *P, Level L, const uint32_t *seg_of, uint64_t N, uint32_t *idx, uint8_t *oct)
-{
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= N) return;
-    idx[t] = (uint32_t)t;
-    uint32_t k = seg_of[t];
-    if (k == NONE || L.kind[k] != K_INNER) {
-        oct[t] = 0xFF;
-        return;
-    }
-    const float *c = L.centre + 3 * k, *p = P + 3 * t;
-    oct[t] = (uint8_t)((c[0] > p[0]) | ((c[1] > p[1]) << 1) | ((c[2] > p[2]) << 2));
-}
-
-// ---- the swapping passes of nodes above SMALL
+// ---- the swapping passes (sort_set, tree.c:166-183)
 //
 // A pass needs, at any position, whether its voxel is claimed, how many
 // claimed ones stand before it and where the last unclaimed one before it
 // stands: a bit per position, and per 32-bit word of them the count and that
 // position so far (Marks).  Claimed voxels leave for good, straight to their
 // place in the next level's order; only the others move on to the next pass.
-
-constexpr uint32_t NO_POS = 0xFFFFFFFFu;
 
 // The source of position t (local to the node) in a pass whose range starts
 // at `from`: the walk back described at the top of the file.  claimed(s, c, u)
@@ -1072,28 +886,326 @@ __device__ __forceinline__ void place(const float *P, float *Pn, uint64_t to, ui
     Pn[3 * to + 2] = P[3 * i + 2];
 }
 
-// Nodes of SMALL+1..MID voxels: a block each, all eight passes in shared
-// memory, a voxel in 16 bits {octant, place in the node}.
+// Octant of voxel p about centre c (get_subspace_idx, geom.c:44-51).
+__device__ __forceinline__ uint32_t octant(const float *c, const float *p)
+{
+    return (uint32_t)(c[0] > p[0]) | ((uint32_t)(c[1] > p[1]) << 1) | ((uint32_t)(c[2] > p[2]) << 2);
+}
+
+// What a warp has counted of the nodes it made, added to the level's tally
+// when it leaves.
+struct WarpTally {
+    uint32_t inner = 0, dense = 0, over = 0, top = 0;
+    unsigned long long over_dots = 0;
+    // One split node, from its octants' counts (lane o < 8 holds octant o's):
+    // an overflowed leaf when one octant took the whole set (tree.c:281-305).
+    // Returns its child mask.
+    __device__ uint32_t split(const Level &L, uint32_t k, uint32_t n, uint32_t cnt, uint32_t *err)
+    {
+        const uint32_t lane = threadIdx.x & 31;
+        if (lane < 8) L.cnt[8 * (size_t)k + lane] = cnt;
+        const uint32_t mask = __ballot_sync(0xffffffffu, lane < 8 && cnt), most = __reduce_max_sync(0xffffffffu, lane < 8 ? cnt : 0u);
+        if (most == n) {
+            over++;
+            over_dots += n;
+            if (lane == 0) {
+                L.kind[k] = K_OVER;
+                if (n >= (1u << 30)) atomicOr(err, ERR_BIG_LEAF);
+            }
+            return 0u;
+        }
+        inner++;
+        top = max(top, most);
+        if (lane == 0) L.mask[k] = (uint8_t)mask;
+        return mask;
+    }
+    __device__ void flush(const Tally &t) const
+    {
+        if (threadIdx.x & 31) return;
+        if (inner) {
+            atomicAdd(&t.stats[S_INNER], (unsigned long long)inner);
+            atomicMax(t.largest, top);
+        }
+        if (dense) atomicAdd(&t.stats[S_DENSE], (unsigned long long)dense);
+        if (over) {
+            atomicAdd(&t.stats[S_LEAF], (unsigned long long)over);
+            atomicAdd(&t.stats[S_OVER], (unsigned long long)over);
+            atomicAdd(&t.stats[S_DOTS], over_dots);
+        }
+    }
+};
+
+// A float's bits in an order that unsigned comparison follows, and back.
+__device__ __forceinline__ uint32_t ordered(float f)
+{
+    const uint32_t b = __float_as_uint(f);
+    return b ^ ((uint32_t)((int)b >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ float unordered(uint32_t u)
+{
+    return __uint_as_float(u ^ ((u >> 31) ? 0x80000000u : 0xFFFFFFFFu));
+}
+
+// Nodes of VOX_MAX_DOTS+1..32 voxels in the lanes of a warp, a voxel a lane:
+// box, density, centre, octants and all eight passes in registers.  Returns
+// the child mask.
+__device__ uint32_t node_in_lanes(const Level &L, uint32_t k, uint32_t n, const float *P, float *Pn, const float *v,
+                                  uint8_t *order, WarpTally &tally, uint32_t *err)
+{
+    constexpr uint32_t FULL = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t s0 = L.start[k];
+    const bool in = lane < n;
+    float p[3] = {0.0f, 0.0f, 0.0f}, mn[3], mx[3];
+    if (in)
+        for (int a = 0; a < 3; a++) p[a] = P[3 * (s0 + lane) + a];
+    for (int a = 0; a < 3; a++) {   // the first of equal extremes (-0 equals +0), NaN never one
+        const float lo = in && p[a] < INFINITY ? p[a] + 0.0f : INFINITY, hi = in && p[a] > -INFINITY ? p[a] + 0.0f : -INFINITY;
+        mn[a] = unordered(__reduce_min_sync(FULL, ordered(lo)));
+        mx[a] = unordered(__reduce_max_sync(FULL, ordered(hi)));
+        const uint32_t il = __ballot_sync(FULL, in && p[a] == mn[a]), ih = __ballot_sync(FULL, in && p[a] == mx[a]);
+        const float fl = __shfl_sync(FULL, p[a], il ? __ffs((int)il) - 1 : 0), fh = __shfl_sync(FULL, p[a], ih ? __ffs((int)ih) - 1 : 0);
+        if (il) mn[a] = fl;
+        if (ih) mx[a] = fh;
+    }
+    uint32_t kind = 0;
+    if (lane == 0) kind = write_box(L, k, n, mn, mx, v);
+    kind = __shfl_sync(FULL, kind, 0);
+    if (kind != K_INNER) {
+        tally.dense++;              // above VOX_MAX_DOTS voxels it is no leaf
+        return 0u;
+    }
+    float c[3];
+    PlainSum x;
+    x.init();
+    if (in)
+        for (int a = 0; a < 3; a++) x.add(a, __fsub_rn(p[a], mn[a]));
+    for (int a = 0; a < 3; a++) {
+        x.g[a] = __reduce_min_sync(FULL, x.g[a]);
+        for (int off = 16; off; off >>= 1) x.sum[a] = __fadd_rn(x.sum[a], __shfl_xor_sync(FULL, x.sum[a], off));
+    }
+    for (int a = 0; a < 3; a++) {
+        const float acc = x.exact(a) ? x.sum[a] : warp_sum(P, s0, s0 + n, a, mn[a], 0.0f);
+        c[a] = centre_of(acc, n, mn[a], v[a]);
+        if (lane == 0) L.centre[3 * (size_t)k + a] = c[a];
+    }
+    uint32_t q = in ? octant(c, p) : 8u, src = lane, cnt = 0, from = 0;   // the voxel now at this lane, and where it was
+    for (uint32_t o = 0; o < 8; o++) {
+        const uint32_t m = __ballot_sync(FULL, q == o && lane >= from);
+        if (lane == o) cnt = (uint32_t)__popc(m);
+        if (!m) continue;           // nothing claimed: nothing moves
+        const uint32_t rest = from + (uint32_t)__popc(m);
+        if ((m >> lane) & 1u) order[from + __popc(m & lanes_below(lane))] = (uint8_t)src;
+        uint32_t s = lane;
+        if (in && lane >= rest) {
+            auto claimed = [&](uint32_t i, uint32_t &before, uint32_t &last) {
+                before = (uint32_t)__popc(m & lanes_below(i));
+                last = last_in_word(0, i, m, from);
+                return ((m >> i) & 1u) != 0u;
+            };
+            s = walk_back(lane, from, 32u, claimed, err);
+        }
+        const uint32_t q2 = __shfl_sync(FULL, q, s), src2 = __shfl_sync(FULL, src, s);
+        if (in && lane >= rest) { q = q2; src = src2; }
+        from = rest;
+    }
+    __syncwarp();
+    const uint32_t at = in ? order[lane] : lane;
+    for (int a = 0; a < 3; a++) {
+        const float y = __shfl_sync(FULL, p[a], at);
+        if (in) Pn[3 * (s0 + lane) + a] = y;
+    }
+    __syncwarp();
+    return tally.split(L, k, n, cnt, err);
+}
+
+// Nodes of 33..SMALL voxels by a warp: the same in shared memory, a voxel in
+// 16 bits {octant, place in the node}.
+struct WarpNode {
+    uint16_t buf[2][SMALL], order[SMALL];
+    uint32_t mask[SMALL / 32], before[SMALL / 32], last[SMALL / 32];
+};
+
+__device__ uint32_t node_in_warp(const Level &L, uint32_t k, uint32_t n, const float *P, float *Pn, const float *v,
+                                 WarpNode &w, WarpTally &tally, uint32_t *err)
+{
+    constexpr uint32_t FULL = 0xffffffffu;
+    static_assert(SMALL == 512, "9 bits of place; one word a lane in scan_words");
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t s0 = L.start[k];
+    Extremes e;
+    e.init();
+    for (uint32_t j = lane; j < n; j += 32) e.add(P + 3 * (s0 + j), j);
+    e.warp_merge();
+    uint32_t kind = 0;
+    if (lane == 0) kind = write_box(L, k, n, e.mn, e.mx, v);
+    kind = __shfl_sync(FULL, kind, 0);
+    if (kind != K_INNER) {
+        tally.dense++;
+        return 0u;
+    }
+    float c[3];
+    PlainSum x;
+    x.init();
+    for (uint32_t j = lane; j < n; j += 32)
+        for (int a = 0; a < 3; a++) x.add(a, __fsub_rn(P[3 * (s0 + j) + a], e.mn[a]));
+    x.warp_merge();
+    for (int a = 0; a < 3; a++) {
+        const float acc = x.exact(a) ? x.sum[a] : warp_sum(P, s0, s0 + n, a, e.mn[a], 0.0f);
+        c[a] = centre_of(acc, n, e.mn[a], v[a]);
+        if (lane == 0) L.centre[3 * (size_t)k + a] = c[a];
+    }
+    for (uint32_t j = lane; j < n; j += 32) {
+        const float p[3] = {P[3 * (s0 + j)], P[3 * (s0 + j) + 1], P[3 * (s0 + j) + 2]};
+        w.buf[0][j] = (uint16_t)((octant(c, p) << 9) | j);
+    }
+    const uint32_t nw = (n + 31) / 32;
+    uint32_t cnt = 0, from = 0, cur = 0;
+    for (uint32_t o = 0; o < 8 && from < n; o++) {
+        const uint16_t *in = w.buf[cur];
+        uint16_t *out = w.buf[cur ^ 1];
+        __syncwarp();
+        uint32_t any = 0;
+        for (uint32_t i = from >> 5; i < nw; i++) {
+            const uint32_t t = (i << 5) + lane;
+            const bool range = t >= from && t < n, cl = range && (uint32_t)(in[t] >> 9) == o;
+            const uint32_t m = __ballot_sync(FULL, cl), u = __ballot_sync(FULL, range && !cl);
+            any |= m;
+            if (lane == 0) {
+                w.mask[i] = m;
+                w.before[i] = (uint32_t)__popc(m);
+                w.last[i] = u ? (i << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
+            }
+        }
+        if (!any) continue;
+        __syncwarp();
+        const uint32_t w0 = from >> 5;
+        uint32_t run = 0, prev = NO_POS;
+        scan_words<1>(w.before + w0, w.last + w0, nw - w0, run, prev);
+        if (lane == o) cnt = run;
+        __syncwarp();
+        const uint32_t rest = from + run;
+        auto claimed = [&](uint32_t s, uint32_t &before, uint32_t &last) {
+            const uint32_t i = s >> 5, b = s & 31, m = w.mask[i];
+            before = w.before[i] + (uint32_t)__popc(m & lanes_below(b));
+            last = last_in_word(i, b, m, from);
+            if (last == NO_POS) last = w.last[i];
+            return ((m >> b) & 1u) != 0u;
+        };
+        for (uint32_t t = from + lane; t < n; t += 32) {
+            uint32_t before, last;
+            if (claimed(t, before, last)) w.order[from + before] = in[t] & 511u;
+            if (t >= rest) out[t] = in[walk_back(t, from, SMALL, claimed, err)];
+        }
+        from = rest;
+        cur ^= 1;
+    }
+    __syncwarp();
+    for (uint32_t t = lane; t < n; t += 32) place(P, Pn, s0 + t, s0 + w.order[t]);
+    __syncwarp();
+    return tally.split(L, k, n, cnt, err);
+}
+
+// Nodes of VOX_MAX_DOTS+1..SMALL voxels, up to eight of them to a warp at a
+// time, as many as still leave every warp of the grid some; the warp then takes
+// their children's places in the next level with one atomic.
+constexpr int WARP_NODE_WARPS = 4, WARP_NODE_BLOCKS = 8;   // blocks per SM
+__global__ void __launch_bounds__(WARP_NODE_WARPS * 32, WARP_NODE_BLOCKS) k_nodes_warp(Level L, NodeLists lists, const float *P,
+                                                                     float *Pn, float vx, float vy, float vz,
+                                                                     Tally tally)
+{
+    __shared__ WarpNode shared[WARP_NODE_WARPS];
+    WarpNode &w = shared[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31, total = *lists.nsmall;
+    const uint32_t per = min(8u, max(1u, total / (gridDim.x * WARP_NODE_WARPS)));
+    const float v[3] = {vx, vy, vz};
+    WarpTally mine;
+    for (uint32_t b = (blockIdx.x * WARP_NODE_WARPS + (threadIdx.x >> 5)) * per; b < total;
+         b += gridDim.x * WARP_NODE_WARPS * per) {
+        uint32_t my = NONE, kids = 0;
+        for (uint32_t i = 0; i < per && b + i < total; i++) {
+            const uint32_t k = lists.small[b + i], n = L.n[k];
+            const uint32_t mask = n <= 32
+                ? node_in_lanes(L, k, n, P, Pn, v, reinterpret_cast<uint8_t *>(w.order), mine, tally.err)
+                : node_in_warp(L, k, n, P, Pn, v, w, mine, tally.err);
+            if (lane == i) { my = k; kids = (uint32_t)__popc(mask); }
+        }
+        const uint32_t incl = warp_incl_scan(kids);
+        uint32_t first = 0;
+        if (lane == 31 && incl) first = atomicAdd(tally.children, incl);
+        first = __shfl_sync(0xffffffffu, first, 31) + incl - kids;
+        if (kids) L.first_child[my] = first;
+    }
+    mine.flush(tally);
+}
+
+// Nodes of SMALL+1..MID voxels: a block each, as above, a voxel in 16 bits
+// {octant, place in the node}.
 constexpr int MID_THREADS = 512;
-__global__ void __launch_bounds__(MID_THREADS) k_partition_block(Level L, SplitLists lists, const uint8_t *oct,
-                                                                 const float *P, float *Pn, uint32_t *err)
+__global__ void __launch_bounds__(MID_THREADS) k_nodes_block(Level L, NodeLists lists, const float *P, float *Pn, float vx,
+                                                             float vy, float vz, Tally tally)
 {
     static_assert(MID == 8192 && MID / 32 == 256, "13 bits of place; 8 words a lane in scan_words");
+    constexpr int WARPS = MID_THREADS / 32;
     __shared__ uint16_t buf[2][MID];
-    __shared__ uint32_t mask[MID / 32], before[MID / 32], last[MID / 32], total;
+    __shared__ uint32_t mask[MID / 32], before[MID / 32], last[MID / 32], total, s_kind;
+    __shared__ Extremes epart[WARPS];
+    __shared__ PlainSum spart[WARPS];
+    __shared__ float centre[3];
     if (blockIdx.x >= *lists.nmid) return;
-    const uint32_t k = lists.mid[blockIdx.x], n = L.n[k], s0 = L.start[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t i = threadIdx.x; i < n; i += MID_THREADS) buf[0][i] = (uint16_t)(((uint32_t)oct[s0 + i] << 13) | i);
+    const uint32_t k = lists.mid[blockIdx.x], n = L.n[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t s0 = L.start[k];
+    const float v[3] = {vx, vy, vz};
+    {
+        Extremes e;
+        e.init();
+        for (uint32_t j = threadIdx.x; j < n; j += MID_THREADS) e.add(P + 3 * (s0 + j), j);
+        e.warp_merge();
+        if (lane == 0) epart[warp] = e;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int i = 1; i < WARPS; i++) e.merge(epart[i]);
+            s_kind = write_box(L, k, n, e.mn, e.mx, v);
+            epart[0] = e;
+            if (s_kind == K_DENSE) atomicAdd(&tally.stats[S_DENSE], 1ull);
+        }
+        __syncthreads();
+        if (s_kind != K_INNER) return;
+    }
+    const float mn[3] = {epart[0].mn[0], epart[0].mn[1], epart[0].mn[2]};
+    {
+        PlainSum x;
+        x.init();
+        for (uint32_t j = threadIdx.x; j < n; j += MID_THREADS)
+            for (int a = 0; a < 3; a++) x.add(a, __fsub_rn(P[3 * (s0 + j) + a], mn[a]));
+        x.warp_merge();
+        if (lane == 0) spart[warp] = x;
+        __syncthreads();
+        if (warp < 3) {             // an axis a warp
+            const int a = (int)warp;
+            float sum = lane < WARPS ? spart[lane].sum[a] : 0.0f;
+            for (int off = 16; off; off >>= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, off));
+            x.sum[a] = sum;
+            x.g[a] = __reduce_min_sync(0xffffffffu, lane < WARPS ? spart[lane].g[a] : 1000);
+            const float acc = x.exact(a) ? sum : warp_sum(P, s0, s0 + n, a, mn[a], 0.0f);
+            if (lane == 0) L.centre[3 * (size_t)k + a] = centre[a] = centre_of(acc, n, mn[a], v[a]);
+        }
+        __syncthreads();
+    }
+    for (uint32_t i = threadIdx.x; i < n; i += MID_THREADS) {
+        const float p[3] = {P[3 * (s0 + i)], P[3 * (s0 + i) + 1], P[3 * (s0 + i) + 2]};
+        buf[0][i] = (uint16_t)((octant(centre, p) << 13) | i);
+    }
     const uint32_t nw = (n + 31) / 32;
-    uint32_t from = 0;
-    for (uint32_t o = 0; o < 8; o++) {
+    uint32_t from = 0, cnt = 0;     // lane o of warp 0 holds octant o's count
+    for (uint32_t o = 0; o < 8 && from < n; o++) {
         const uint16_t *in = buf[o & 1];
         uint16_t *out = buf[(o & 1) ^ 1];
         __syncthreads();
-        for (uint32_t w = (from >> 5) + warp; w < nw; w += MID_THREADS / 32) {
+        for (uint32_t w = (from >> 5) + warp; w < nw; w += WARPS) {
             const uint32_t t = (w << 5) + lane;
             const bool range = t >= from && t < n;
-            const bool cl = range && (in[t] >> 13) == o;
+            const bool cl = range && (uint32_t)(in[t] >> 13) == o;
             const uint32_t m = __ballot_sync(0xffffffffu, cl), u = __ballot_sync(0xffffffffu, range && !cl);
             if (lane == 0) {
                 mask[w] = m;
@@ -1106,10 +1218,8 @@ __global__ void __launch_bounds__(MID_THREADS) k_partition_block(Level L, SplitL
             const uint32_t w0 = from >> 5;
             uint32_t run = 0, prev = NO_POS;
             scan_words<MID / 32 / 32>(before + w0, last + w0, nw - w0, run, prev);
-            if (lane == 0) {
-                total = run;
-                L.cnt[8 * k + o] = run;
-            }
+            if (lane == 0) total = run;
+            if (lane == o) cnt = run;
         }
         __syncthreads();
         const uint32_t rest = from + total;
@@ -1122,11 +1232,16 @@ __global__ void __launch_bounds__(MID_THREADS) k_partition_block(Level L, SplitL
         };
         for (uint32_t t = from + threadIdx.x; t < n; t += MID_THREADS) {
             uint32_t c, l;
-            if (claimed(t, c, l)) place(P, Pn, (uint64_t)s0 + from + c, (uint64_t)s0 + (in[t] & 8191u));
-            if (t >= rest) out[t] = in[walk_back(t, from, MID, claimed, err)];
+            if (claimed(t, c, l)) place(P, Pn, s0 + from + c, s0 + (in[t] & 8191u));
+            if (t >= rest) out[t] = in[walk_back(t, from, MID, claimed, tally.err)];
         }
         from = rest;
-        if (from >= n) break;
+    }
+    if (warp == 0) {
+        WarpTally mine;
+        const uint32_t m = mine.split(L, k, n, cnt, tally.err);
+        if (lane == 0 && m) L.first_child[k] = atomicAdd(tally.children, (uint32_t)__popc(m));
+        mine.flush(tally);
     }
 }
 
@@ -1167,36 +1282,32 @@ struct SubMarks {
     }
 };
 
-// The node of this block's tile: its slot, or NO_POS for a block without one.
-__device__ __forceinline__ uint32_t tile_slot(const SplitLists &lists, uint32_t tile)
-{
-    const unsigned long long n = *lists.ntiled;
-    if (tile >= (uint32_t)n) return NO_POS;
-    uint32_t lo = 0, hi = (uint32_t)(n >> 32);
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (lists.first_tile[mid] <= tile) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// Marks of octant 0 over the given order.
-__global__ void __launch_bounds__(PASS_THREADS) k_tile_marks(Level L, SplitLists lists, const uint8_t *oct, Marks out)
+// Octants, and the marks of octant 0 over the given order.
+__global__ void __launch_bounds__(PASS_THREADS) k_tile_marks(Level L, NodeLists lists, const float *P, uint8_t *oct,
+                                                             Marks out)
 {
     __shared__ SubMarks sub;
     const uint32_t slot = tile_slot(lists, blockIdx.x);
     if (slot == NO_POS) return;
     const uint32_t k = lists.tiled[slot], n = L.n[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (L.kind[k] != K_INNER) return;
     const uint64_t start = L.start[k];
     const uint32_t b = (blockIdx.x - lists.first_tile[slot]) * lists.tile, e = min(n, b + lists.tile);
+    const float centre[3] = {L.centre[3 * (size_t)k], L.centre[3 * (size_t)k + 1], L.centre[3 * (size_t)k + 2]};
+    if (b == 0 && threadIdx.x < 8) L.cnt[8 * (size_t)k + threadIdx.x] = 0;
     uint64_t word0 = (uint64_t)blockIdx.x * (lists.tile / 32);
     uint32_t run = 0, prev = NO_POS;
     for (uint32_t sb = b; sb < e; sb += SUB, word0 += SUB / 32) {
         const uint32_t nw = (min(e - sb, SUB) + 31) / 32;
         for (uint32_t w = warp; w < nw; w += PASS_THREADS / 32) {
             const uint32_t t = sb + (w << 5) + lane;
-            const bool in = t < e, cl = in && oct[start + t] == 0;
+            const bool in = t < e;
+            uint32_t q = 0xFF;
+            if (in) {
+                q = octant(centre, P + 3 * (start + t));
+                oct[start + t] = (uint8_t)q;
+            }
+            const bool cl = q == 0;
             const uint32_t m = __ballot_sync(0xffffffffu, cl), u = __ballot_sync(0xffffffffu, in && !cl);
             if (lane == 0) {
                 out.mask[word0 + w] = m;
@@ -1213,7 +1324,7 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_marks(Level L, SplitLists
 }
 
 // Pass o over every tiled node.
-__global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, SplitLists lists, uint32_t o, Marks in, Marks out,
+__global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists lists, uint32_t o, Marks in, Marks out,
                                                             const uint32_t *in_idx, const uint8_t *in_oct,
                                                             uint32_t *out_idx, uint8_t *out_oct, const float *P,
                                                             float *Pn, uint32_t *err)
@@ -1225,9 +1336,10 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, SplitLists 
     if (slot == NO_POS) return;
     const uint32_t tile = lists.tile, ft = lists.first_tile[slot], ti = blockIdx.x - ft;
     const uint32_t k = lists.tiled[slot], n = L.n[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (L.kind[k] != K_INNER) return;
     const uint64_t start = L.start[k];
     uint32_t from = 0;
-    for (uint32_t q = 0; q < o; q++) from += L.cnt[8 * k + q];
+    for (uint32_t q = 0; q < o; q++) from += L.cnt[8 * (size_t)k + q];
     const uint32_t b = ti * tile, e = min(n, b + tile);
     if (e <= from) return;                     // all of it placed by earlier passes
     const uint32_t t0 = from / tile, nt = (n + tile - 1) / tile - t0;   // the tiles still in play
@@ -1242,7 +1354,7 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, SplitLists 
             scan_words<4>(tbefore + i, tlast + i, min(nt - i, 128u), run, prev);
         if (lane == 0) {
             s_total = run;
-            if (e == n) L.cnt[8 * k + o] = run;   // read by later launches only
+            if (e == n) L.cnt[8 * (size_t)k + o] = run;   // read by later launches only
         }
     }
     __syncthreads();
@@ -1289,75 +1401,111 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, SplitLists 
     }
 }
 
-// The next level's order outside the nodes above SMALL, whose passes place
-// their voxels themselves.
-__global__ void k_gather(uint64_t N, Level L, const uint32_t *seg_of, const uint32_t *idx, const float *P, float *Pn)
+// Tiled nodes after their passes, a warp each.
+__global__ void k_finish_tiled(Level L, NodeLists lists, Tally tally)
 {
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= N) return;
-    const uint32_t k = seg_of[t];
-    if (k != NONE && L.kind[k] == K_INNER && L.n[k] > SMALL) return;
-    uint64_t i = idx[t];
-    Pn[3 * t] = P[3 * i];
-    Pn[3 * t + 1] = P[3 * i + 1];
-    Pn[3 * t + 2] = P[3 * i + 2];
+    const uint32_t slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (slot >= (uint32_t)(*lists.ntiled >> 32)) return;
+    const uint32_t k = lists.tiled[slot];
+    if (L.kind[k] != K_INNER) return;
+    WarpTally mine;
+    const uint32_t m = mine.split(L, k, L.n[k], lane < 8 ? L.cnt[8 * (size_t)k + lane] : 0u, tally.err);
+    if (lane == 0 && m) L.first_child[k] = atomicAdd(tally.children, (uint32_t)__popc(m));
+    mine.flush(tally);
 }
 
-// Overflowed leaves (one octant took the whole set, tree.c:281-305), child
-// masks, per-level counts (inner, leaves, dense leaves, leaf voxels) and the
-// largest child.
-__global__ void k_finish(Level L, unsigned long long *stats, uint32_t *largest, uint32_t *err)
+// A new node of n voxels from position s0 on (n 0: none; every thread of the
+// warp calls): made here when it has at most VOX_MAX_DOTS voxels (a leaf, or
+// dense), else put on the list of its class.
+__device__ __forceinline__ void new_node(const Level &L, uint32_t k, uint32_t s0, uint32_t n, const float *P, const float *v,
+                                         const NodeLists &lists, uint32_t &leaves, uint32_t &dense, uint32_t &dots)
 {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= L.m) return;
-    uint8_t kind = L.kind[k];
-    uint32_t mask = 0, top = 0;
-    if (kind == K_INNER) {
-        bool over = false;
-        for (int o = 0; o < 8; o++) {
-            uint32_t c = L.cnt[8 * k + o];
-            over |= c == L.n[k];
-            mask |= (c ? 1u : 0u) << o;
-            top = max(top, c);
-        }
-        if (over) {
-            kind = K_OVER;
-            mask = 0;
-            L.kind[k] = K_OVER;
+    constexpr uint32_t FULL = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31;
+    if (n) {
+        L.start[k] = s0;
+        L.n[k] = n;
+    }
+    if (n && n <= VOX_MAX_DOTS) {
+        const float *p = P + 3 * (uint64_t)s0;
+        float mn[3] = {p[0], p[1], p[2]}, mx[3] = {p[0], p[1], p[2]};
+        for (uint32_t i = 1; i < n; i++)
+            for (int a = 0; a < 3; a++) {
+                const float x = p[3 * i + a];
+                if (x < mn[a]) mn[a] = x;
+                else if (x > mx[a]) mx[a] = x;
+            }
+        if (write_box(L, k, n, mn, mx, v) == K_DENSE) {
+            dense++;
         } else {
-            atomicMax(largest, top);
+            leaves++;
+            dots += n;
         }
     }
-    L.mask[k] = (uint8_t)mask;
-    if (kind == K_INNER) {
-        atomicAdd(&stats[0], 1ull);
-    } else if (kind == K_DENSE) {
-        atomicAdd(&stats[2], 1ull);
-    } else {
-        atomicAdd(&stats[1], 1ull);
-        atomicAdd(&stats[3], (unsigned long long)L.n[k]);
-        if (L.n[k] >= (1u << 30)) atomicOr(err, ERR_BIG_LEAF);
+    if (n > SMALL) lists.add_large(k, n);
+    const bool small = n > VOX_MAX_DOTS && n <= SMALL;
+    const uint32_t m = __ballot_sync(FULL, small);
+    uint32_t at = 0;
+    if (lane == 0 && m) at = atomicAdd(lists.nsmall, (uint32_t)__popc(m));
+    at = __shfl_sync(FULL, at, 0) + (uint32_t)__popc(m & ((1u << lane) - 1u));
+    if (small) lists.small[at] = k;
+}
+
+// The next level's nodes: a thread per octant of every node of this one.
+constexpr int CHILD_THREADS = 256;
+__global__ void __launch_bounds__(CHILD_THREADS) k_children(Level L, Level Nx, NodeLists lists, const float *P, float vx,
+                                                            float vy, float vz, unsigned long long *stats)
+{
+    __shared__ uint32_t sums[3];
+    if (threadIdx.x < 3) sums[threadIdx.x] = 0;
+    __syncthreads();
+    const uint64_t t = (uint64_t)blockIdx.x * CHILD_THREADS + threadIdx.x;
+    const uint32_t o = threadIdx.x & 7;
+    const size_t k = t >> 3;
+    const uint32_t mask = k < L.m ? L.mask[k] : 0u;
+    const uint32_t n = mask ? L.cnt[8 * k + o] : 0u;
+    uint32_t incl = n;              // over the node's eight octants
+    for (int off = 1; off < 8; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off, 8);
+        if (o >= (uint32_t)off) incl += y;
+    }
+    const float v[3] = {vx, vy, vz};
+    uint32_t leaves = 0, dense = 0, dots = 0, child = 0, s0 = 0;
+    if (n) {
+        child = L.first_child[k] + (uint32_t)__popc(mask & ((1u << o) - 1u));
+        s0 = L.start[k] + incl - n;
+    }
+    new_node(Nx, child, s0, n, P, v, lists, leaves, dense, dots);
+    leaves = __reduce_add_sync(0xffffffffu, leaves);
+    dense = __reduce_add_sync(0xffffffffu, dense);
+    dots = __reduce_add_sync(0xffffffffu, dots);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&sums[0], leaves);
+        atomicAdd(&sums[1], dense);
+        atomicAdd(&sums[2], dots);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (sums[0]) atomicAdd(&stats[S_LEAF], (unsigned long long)sums[0]);
+        if (sums[1]) atomicAdd(&stats[S_DENSE], (unsigned long long)sums[1]);
+        if (sums[2]) atomicAdd(&stats[S_DOTS], (unsigned long long)sums[2]);
     }
 }
 
-struct ChildCount {
-    const uint8_t *mask;
-    __device__ uint32_t operator()(uint64_t k) const { return (uint32_t)__popc(mask[k]); }
-};
-
-__global__ void k_children(Level L, Level Nx)
+// The root (one warp).
+__global__ void k_root_node(Level L, uint32_t n, NodeLists lists, const float *P, float vx, float vy, float vz,
+                            unsigned long long *stats)
 {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= L.m || !L.mask[k]) return;
-    uint32_t f = L.first_child[k], s = L.start[k];
-    for (int o = 0; o < 8; o++) {
-        uint32_t c = L.cnt[8 * k + o];
-        if (c) {
-            Nx.start[f] = s;
-            Nx.n[f] = c;
-            f++;
-        }
-        s += c;
+    const float v[3] = {vx, vy, vz};
+    uint32_t leaves = 0, dense = 0, dots = 0;
+    new_node(L, 0, 0, threadIdx.x == 0 ? n : 0u, P, v, lists, leaves, dense, dots);
+    if (threadIdx.x == 0) {
+        stats[S_LEAF] = leaves;
+        stats[S_DENSE] = dense;
+        stats[S_DOTS] = dots;
+        L.id[0] = 0;
+        L.rec[0] = 0;
+        L.ustart[0] = VOXP_REC_UNITS;
     }
 }
 
@@ -1385,73 +1533,65 @@ __global__ void k_up(Level L, Level Nx, bool has_next)
     L.sub_units[k] = su;
 }
 
-__global__ void k_root(Level L)
-{
-    L.id[0] = 0;
-    L.rec[0] = 0;
-    L.ustart[0] = VOXP_REC_UNITS;
-}
-
-// Pre-order ids and image offsets of the children of every inner node.
-__global__ void k_down(Level L, Level Nx)
-{
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= L.m || L.kind[k] != K_INNER) return;
-    uint32_t nch = (uint32_t)__popc(L.mask[k]);
-    uint32_t f = L.first_child[k], us = L.ustart[k];
-    uint32_t cid = L.id[k] + 1, cu = us + VOXP_REC_UNITS * nch;
-    for (uint32_t j = 0; j < nch; j++) {
-        Nx.id[f + j] = cid;
-        Nx.ustart[f + j] = cu;
-        Nx.rec[f + j] = us + VOXP_REC_UNITS * j;
-        cid += Nx.sub_nodes[f + j];
-        cu += (uint32_t)Nx.sub_units[f + j];
-    }
-}
-
-// Node records (pool_layout.h) and the pre-order id map.
-__global__ void k_emit(Level L, uint4 *pool, uint32_t *rec_of_id, uint64_t units, uint64_t nodes, uint32_t *err,
-                       uint32_t *dots_of_id)
+// Node records (pool_layout.h), the pre-order id map, the voxel runs of leaves
+// of at most VOX_MAX_DOTS voxels; and pre-order ids and image offsets of the
+// children, for the next level's launch.
+__global__ void k_emit(Level L, Level Nx, const float *P, uint4 *pool, uint32_t *rec_of_id, uint64_t units, uint64_t nodes,
+                       uint32_t *err, uint32_t *dots_of_id)
 {
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= L.m) return;
     uint8_t kind = L.kind[k];
-    uint32_t id = L.id[k], rec = L.rec[k], meta, link;
+    uint32_t id = L.id[k], rec = L.rec[k], cnt = L.n[k], us = L.ustart[k], meta, link;
     if ((uint64_t)rec + VOXP_REC_UNITS > units || id >= nodes) {   // cannot happen for a consistent layout
         atomicOr(err, ERR_LAYOUT);
         return;
     }
-    if (dots_of_id) dots_of_id[id] = L.n[k];   // the node's dots_num (tree.c:262)
+    if (dots_of_id) dots_of_id[id] = cnt;   // the node's dots_num (tree.c:262)
     uint4 extra = make_uint4(0u, 0u, 0u, 0u);
     if (kind == K_DENSE) {
         meta = VOXP_KIND_DENSE;
         link = id;
     } else if (kind == K_INNER) {
-        meta = VOXP_KIND_INNER | ((uint32_t)L.mask[k] << 8);
-        link = L.ustart[k];
-        const float *c = L.centre + 3 * k;
+        const uint32_t mask = L.mask[k], nch = (uint32_t)__popc(mask), f = L.first_child[k];
+        meta = VOXP_KIND_INNER | (mask << 8);
+        link = us;
+        const float *c = L.centre + 3 * (size_t)k;
         extra = make_uint4(__float_as_uint(c[0]), __float_as_uint(c[1]), __float_as_uint(c[2]), 0u);
+        uint32_t cid = id + 1, cu = us + VOXP_REC_UNITS * nch;
+        for (uint32_t j = 0; j < nch; j++) {
+            Nx.id[f + j] = cid;
+            Nx.ustart[f + j] = cu;
+            Nx.rec[f + j] = us + VOXP_REC_UNITS * j;
+            cid += Nx.sub_nodes[f + j];
+            cu += (uint32_t)Nx.sub_units[f + j];
+        }
     } else {
-        uint32_t cnt = L.n[k];
         meta = VOXP_KIND_LEAF | (cnt << 2);
-        link = L.ustart[k];
+        link = us;
         extra = make_uint4(id, cnt, 0u, 0u);
+        if ((uint64_t)us + cnt > units) {
+            atomicOr(err, ERR_LAYOUT);
+        } else if (kind == K_LEAF) {
+            const float *p = P + 3 * (uint64_t)L.start[k];
+            for (uint32_t i = 0; i < cnt; i++)
+                pool[us + i] = make_uint4(__float_as_uint(p[3 * i]), __float_as_uint(p[3 * i + 1]),
+                                          __float_as_uint(p[3 * i + 2]), 0u);
+        }
     }
-    const float *b = L.box + 6 * k;
+    const float *b = L.box + 6 * (size_t)k;
     pool[rec] = make_uint4(__float_as_uint(b[0]), __float_as_uint(b[1]), __float_as_uint(b[2]), __float_as_uint(b[3]));
     pool[rec + 1] = make_uint4(__float_as_uint(b[4]), __float_as_uint(b[5]), meta, link);
     pool[rec + 2] = extra;
     rec_of_id[id] = rec;
 }
 
-// Voxel runs of the leaves, a warp per node.
-__global__ void k_emit_voxels(Level L, const float *P, uint4 *pool, uint64_t units, uint32_t *err)
+// Voxel runs of a level's overflowed leaves, a warp per node.
+__global__ void k_emit_over(Level L, const float *P, uint4 *pool, uint64_t units, uint32_t *err)
 {
     uint32_t k = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     int lane = threadIdx.x & 31;
-    if (k >= L.m) return;
-    uint8_t kind = L.kind[k];
-    if (kind != K_LEAF && kind != K_OVER) return;
+    if (k >= L.m || L.kind[k] != K_OVER) return;
     uint64_t s = L.start[k];
     uint32_t u = L.ustart[k], nk = L.n[k];
     if ((uint64_t)u + nk > units) {
@@ -1462,6 +1602,17 @@ __global__ void k_emit_voxels(Level L, const float *P, uint4 *pool, uint64_t uni
         const float *p = P + 3 * (s + i);
         pool[u + i] = make_uint4(__float_as_uint(p[0]), __float_as_uint(p[1]), __float_as_uint(p[2]), 0u);
     }
+}
+
+// The set's final order (tree.c sorts it in place): a level's leaves, a warp
+// per node.
+__global__ void k_final_order(Level L, const float *P, float *order)
+{
+    uint32_t k = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    int lane = threadIdx.x & 31;
+    if (k >= L.m || L.kind[k] == K_INNER) return;
+    const uint64_t b = 3 * (uint64_t)L.start[k], e = b + 3 * (uint64_t)L.n[k];
+    for (uint64_t i = b + lane; i < e; i += 32) order[i] = P[i];
 }
 
 // ------------------------------------------------------------ raw reader
@@ -1548,78 +1699,57 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     } level_free{levels, s};
 
     float *P[2];
-    uint32_t *idx[2], *seg_of, *tile, *scal, *cidx, *big;
-    uint8_t *oct[2], *cbase;
-    float *cv, *csum;
-    int *cgrid;
-    uint2 *maps, *starts;
+    uint32_t *scal, *cidx = nullptr, *idx[2] = {nullptr, nullptr};
+    uint8_t *oct[2] = {nullptr, nullptr}, *cbase = nullptr;
+    float *cv = nullptr, *csum = nullptr;
+    int *cgrid = nullptr;
+    uint2 *maps = nullptr, *starts = nullptr;
     unsigned long long *stats;
-    uint64_t max_chunks = N / CHUNK + N / BIG + 2;
-    uint64_t max_big = N / BIG + 1;
-    uint64_t max_tiles = N / SCAN_TILE + 2;
     TRY(d.get(&P[0], 3 * N));
     TRY(d.get(&P[1], 3 * N));
-    TRY(d.get(&idx[0], N));
-    TRY(d.get(&idx[1], N));
-    TRY(d.get(&oct[0], N));
-    TRY(d.get(&oct[1], N));
-    TRY(d.get(&seg_of, N));
-    TRY(d.get(&tile, max_tiles));
-    // scal: 0 chunks, 1 mid nodes, 2 children, 3 big nodes, 4 largest child, 6-7 tiled nodes and tiles,
-    // 8 error bits
+    TRY(d.get(&stats, NSTATS * (MAX_LEVELS + 1)));
+    // scal: 0 small nodes, 1 mid nodes, 2 children, 3 largest child, 6-7 tiled nodes and tiles, 8 error bits
     TRY(d.get(&scal, 12));
-    TRY(d.get(&big, max_big));
-    // past 2^24 additions a sum's roundings can add up to a sizeable part of it
-    const int window = N > (1u << 24) ? NBIN : 2;
-    if (N > BIG) {
-        TRY(d.get(&cv, 6 * max_chunks));
-        TRY(d.get(&cidx, 6 * max_chunks));
-        TRY(d.get(&maps, max_chunks * window * 3));
-        TRY(d.get(&starts, 3 * max_big));
-        TRY(d.get(&csum, 3 * max_chunks));
-        TRY(d.get(&cgrid, 3 * max_chunks));
-        TRY(d.get(&cbase, 3 * max_chunks));
-    } else {
-        cv = csum = nullptr;
-        cidx = nullptr;
-        maps = starts = nullptr;
-        cgrid = nullptr;
-        cbase = nullptr;
-    }
-    TRY(d.get(&stats, 4 * MAX_LEVELS));
     uint32_t *err = scal + 8;
-    TRY(cudaMemsetAsync(scal, 0, 12 * 4, s));
-    // nodes split by a block each and tile by tile, and the tiles' marks (two sets)
-    SplitLists lists{};
+    NodeLists lists{};
+    lists.nsmall = scal;
     lists.nmid = scal + 1;
     lists.ntiled = reinterpret_cast<unsigned long long *>(scal + 6);
     lists.tile = SUB * (uint32_t)((N + (uint64_t)SUB * MAX_TILES - 1) / ((uint64_t)SUB * MAX_TILES));
-    const uint64_t max_mid = N / SMALL, max_tiled = N / MID, max_pass_tiles = N / lists.tile + max_tiled;
+    const uint64_t max_mid = N / SMALL, max_tiled = N / MID, max_tiles = N / lists.tile + max_tiled,
+                   max_chunks = max_tiles * (lists.tile / CHUNK);
+    TRY(d.get(&lists.small, N / (VOX_MAX_DOTS + 1) + 1));
     TRY(d.get(&lists.mid, max_mid + 1));
+    // past 2^24 additions a sum's roundings can add up to a sizeable part of it
+    const int window = N > (1u << 24) ? NBIN : 2;
     Marks marks[2] = {};
     if (N > MID) {
+        for (int i = 0; i < 2; i++) {
+            TRY(d.get(&idx[i], N));
+            TRY(d.get(&oct[i], N));
+            TRY(d.get(&marks[i].mask, max_tiles * (lists.tile / 32)));
+            TRY(d.get(&marks[i].before, max_tiles * (lists.tile / 32)));
+            TRY(d.get(&marks[i].last, max_tiles * (lists.tile / 32)));
+            TRY(d.get(&marks[i].count, max_tiles));
+            TRY(d.get(&marks[i].tail, max_tiles));
+        }
         TRY(d.get(&lists.tiled, max_tiled));
         TRY(d.get(&lists.first_tile, max_tiled));
-        for (Marks &m : marks) {
-            TRY(d.get(&m.mask, max_pass_tiles * (lists.tile / 32)));
-            TRY(d.get(&m.before, max_pass_tiles * (lists.tile / 32)));
-            TRY(d.get(&m.last, max_pass_tiles * (lists.tile / 32)));
-            TRY(d.get(&m.count, max_pass_tiles));
-            TRY(d.get(&m.tail, max_pass_tiles));
-        }
+        TRY(d.get(&cv, 6 * max_chunks));
+        TRY(d.get(&cidx, 6 * max_chunks));
+        TRY(d.get(&csum, 3 * max_chunks));
+        TRY(d.get(&cgrid, 3 * max_chunks));
+        TRY(d.get(&cbase, 3 * max_chunks));
+        TRY(d.get(&maps, max_chunks * window * 3));
+        TRY(d.get(&starts, 3 * max_tiled));
     }
-    TRY(cudaMemsetAsync(stats, 0, 4 * MAX_LEVELS * sizeof(unsigned long long), s));
+    TRY(cudaMemsetAsync(scal, 0, 12 * 4, s));
+    TRY(cudaMemsetAsync(stats, 0, NSTATS * (MAX_LEVELS + 1) * sizeof(unsigned long long), s));
     TRY(cudaMemcpyAsync(P[0], d_set, 12 * N, cudaMemcpyDeviceToDevice, s));
 
-    Level root;
-    TRY(level_alloc(root, 1, s));
-    levels.push_back(root);
-    uint32_t root_sn[2] = {0u, (uint32_t)N};
-    TRY(cudaMemcpyAsync(levels[0].start, &root_sn[0], 4, cudaMemcpyHostToDevice, s));
-    TRY(cudaMemcpyAsync(levels[0].n, &root_sn[1], 4, cudaMemcpyHostToDevice, s));
-
-    const unsigned TB = 256;
-    int cur = 0;
+    int dev = 0, nsm = 0;
+    TRY(cudaGetDevice(&dev));
+    TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     uint32_t *h_next = nullptr;
     TRY(cudaMallocHost(&h_next, 64));
     struct HostFree {
@@ -1627,74 +1757,61 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         ~HostFree() { cudaFreeHost(p); }
     } host_free{h_next};
 
+    Level root;
+    TRY(level_alloc(root, 1, s));
+    levels.push_back(root);
+    k_root_node<<<1, 32, 0, s>>>(root, (uint32_t)N, lists, P[0], vx, vy, vz, stats);
+    count_launch();
+
     uint32_t largest = (uint32_t)N;   // the largest node of the level
     for (int lv = 0;; lv++) {
         if (lv >= MAX_LEVELS) return VOX_CUDA_EDEPTH;
         Level L = levels[lv];
-        uint32_t m = L.m;
-        TRY(cudaMemsetAsync(scal, 0, 8 * 4, s));
-        k_seg_of<<<grid_for(N, TB), TB, 0, s>>>(L.start, L.n, m, N, seg_of);
-        count_launch();
-        bool has_big = largest > BIG;
-        const unsigned nodes_big = (unsigned)max_big;
-        if (has_big) {   // boxes of big nodes from their chunks
-            scan(ChunkCount{L.n}, StoreChunks{L.chunk_base, big, scal + 3}, m, tile, scal + 0, s);
-            k_chunk_box<<<(unsigned)max_chunks, CHUNK_THREADS, 0, s>>>(P[cur], L, scal + 0, cv, cidx);
-            k_box_big<<<nodes_big, NODE_THREADS, 0, s>>>(L, big, scal + 3, cv, cidx, vx, vy, vz);
-            count_launch();
-            count_launch();
-        }
-        k_box_thread<<<grid_for(m, TB), TB, 0, s>>>(P[cur], L, vx, vy, vz);
-        count_launch();
-        if (largest > TINY) {
-            k_box_warp<<<grid_for((uint64_t)m * 32, TB), TB, 0, s>>>(P[cur], L, vx, vy, vz);
-            count_launch();
-        }
-        k_classify<<<grid_for((uint64_t)m * 32, TB), TB, 0, s>>>(P[cur], L, vx, vy, vz, lists);
-        count_launch();
-        if (has_big) {   // their centres
-            k_chunk_sums<<<(unsigned)max_chunks, CHUNK_THREADS, 0, s>>>(P[cur], L, scal + 0, csum, cgrid);
-            k_centre_plain<<<nodes_big, NODE_THREADS, 0, s>>>(L, big, scal + 3, csum, cgrid, cbase, window, starts, vx, vy, vz);
-            k_chunk_maps<<<(unsigned)max_chunks, CHUNK_THREADS, 0, s>>>(P[cur], L, scal + 0, cbase, window, maps,
-                                                                       max_chunks);
-            k_centre_big<<<grid_for(max_big * 3 * 32, CENTRE_WARPS * 32), CENTRE_WARPS * 32, 0, s>>>(
-                P[cur], L, big, scal + 3, maps, cbase, csum, window, starts, max_chunks, vx, vy, vz);
-            for (int i = 0; i < 4; i++) count_launch();
-        }
-        k_oct_init<<<grid_for(N, TB), TB, 0, s>>>(P[cur], L, seg_of, N, idx[0], oct[0]);
-        count_launch();
-        if (largest > MID) {   // the eight swapping passes of the largest nodes
-            k_tile_marks<<<(unsigned)max_pass_tiles, PASS_THREADS, 0, s>>>(L, lists, oct[0], marks[0]);
+        const uint32_t m = L.m;
+        const float *Pc = P[lv & 1];
+        float *Pn = P[(lv & 1) ^ 1];
+        const Tally tally{stats + NSTATS * lv, scal + 2, scal + 3, err};
+        if (largest > MID) {
+            // boxes, centres and the eight swapping passes of the largest nodes
+            const unsigned nt = (unsigned)max_tiled, nc = (unsigned)max_chunks, np = (unsigned)max_tiles;
+            k_chunk_box<<<nc, CHUNK_THREADS, 0, s>>>(Pc, L, lists, cv, cidx);
+            k_box_tiled<<<nt, NODE_THREADS, 0, s>>>(L, lists, cv, cidx, vx, vy, vz, tally);
+            k_chunk_sums<<<nc, CHUNK_THREADS, 0, s>>>(Pc, L, lists, csum, cgrid);
+            k_centre_plain<<<nt, NODE_THREADS, 0, s>>>(L, lists, csum, cgrid, cbase, window, starts, vx, vy, vz);
+            k_chunk_maps<<<nc, CHUNK_THREADS, 0, s>>>(Pc, L, lists, cbase, window, maps, max_chunks);
+            k_centre_big<<<grid_for(max_tiled * 3 * 32, CENTRE_WARPS * 32), CENTRE_WARPS * 32, 0, s>>>(
+                Pc, L, lists, maps, cbase, csum, window, starts, max_chunks, vx, vy, vz);
+            k_tile_marks<<<np, PASS_THREADS, 0, s>>>(L, lists, Pc, oct[0], marks[0]);
             for (uint32_t o = 0; o < 8; o++) {
                 const int in = o & 1, out = in ^ 1;
-                k_tile_pass<<<(unsigned)max_pass_tiles, PASS_THREADS, 0, s>>>(
-                    L, lists, o, marks[in], marks[out], idx[in], oct[in], idx[out], oct[out], P[cur], P[cur ^ 1], err);
+                k_tile_pass<<<np, PASS_THREADS, 0, s>>>(L, lists, o, marks[in], marks[out], idx[in], oct[in], idx[out],
+                                                        oct[out], Pc, Pn, err);
             }
-            for (int i = 0; i < 9; i++) count_launch();
+            k_finish_tiled<<<grid_for(max_tiled * 32, 256), 256, 0, s>>>(L, lists, tally);
+            for (int i = 0; i < 16; i++) count_launch();
         }
         if (largest > SMALL) {
-            k_partition_block<<<(unsigned)max_mid, MID_THREADS, 0, s>>>(L, lists, oct[0], P[cur], P[cur ^ 1], err);
+            k_nodes_block<<<(unsigned)max_mid, MID_THREADS, 0, s>>>(L, lists, Pc, Pn, vx, vy, vz, tally);
             count_launch();
         }
-        k_partition_warp<<<grid_for((uint64_t)m * 32, PART_WARPS * 32), PART_WARPS * 32, 0, s>>>(L, idx[0], oct[0],
-                                                                                              err);
-        k_gather<<<grid_for(N, TB), TB, 0, s>>>(N, L, seg_of, idx[0], P[cur], P[cur ^ 1]);
-        cur ^= 1;
-        k_finish<<<grid_for(m, TB), TB, 0, s>>>(L, stats + 4 * lv, scal + 4, err);
-        count_launch();
-        count_launch();
-        count_launch();
-        scan(ChildCount{L.mask}, StoreExcl{L.first_child}, m, tile, scal + 2, s);
+        if (largest > VOX_MAX_DOTS) {
+            const unsigned blocks = grid_for(std::min<uint64_t>(m, N / (VOX_MAX_DOTS + 1) + 1), WARP_NODE_WARPS);
+            k_nodes_warp<<<std::min(blocks, (unsigned)(nsm * WARP_NODE_BLOCKS)), WARP_NODE_WARPS * 32, 0, s>>>(
+                L, lists, Pc, Pn, vx, vy, vz, tally);
+            count_launch();
+        }
         TRY(cudaGetLastError());
-        TRY(cudaMemcpyAsync(h_next, scal + 2, 12, cudaMemcpyDeviceToHost, s));
+        TRY(cudaMemcpyAsync(h_next, scal + 2, 8, cudaMemcpyDeviceToHost, s));
         TRY(cudaStreamSynchronize(s));
-        uint32_t mn = h_next[0];
-        largest = h_next[2];
+        const uint32_t mn = h_next[0];
+        largest = h_next[1];
         if (mn == 0) break;
         Level Nx;
         TRY(level_alloc(Nx, mn, s));
         levels.push_back(Nx);
-        k_children<<<grid_for(m, TB), TB, 0, s>>>(L, Nx);
+        TRY(cudaMemsetAsync(scal, 0, 8 * 4, s));
+        k_children<<<grid_for((uint64_t)m * 8, CHILD_THREADS), CHILD_THREADS, 0, s>>>(L, Nx, lists, Pn, vx, vy, vz,
+                                                                                     stats + NSTATS * (lv + 1));
         count_launch();
     }
 
@@ -1706,12 +1823,12 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         k_up<<<grid_for(L.m, 256), 256, 0, s>>>(L, Nx, lv + 1 < nl);
         count_launch();
     }
-    std::vector<unsigned long long> h_stats(4 * MAX_LEVELS);
+    std::vector<unsigned long long> h_stats(NSTATS * MAX_LEVELS);
     uint32_t h_root[2];
     unsigned long long h_units = 0;
     float h_box[6];
-    TRY(cudaMemcpyAsync(h_stats.data(), stats, 4 * MAX_LEVELS * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                        s));
+    TRY(cudaMemcpyAsync(h_stats.data(), stats, NSTATS * MAX_LEVELS * sizeof(unsigned long long),
+                        cudaMemcpyDeviceToHost, s));
     TRY(cudaMemcpyAsync(&h_root[0], levels[0].sub_nodes, 4, cudaMemcpyDeviceToHost, s));
     TRY(cudaMemcpyAsync(&h_root[1], err, 4, cudaMemcpyDeviceToHost, s));
     TRY(cudaMemcpyAsync(&h_units, levels[0].sub_units, 8, cudaMemcpyDeviceToHost, s));
@@ -1723,28 +1840,31 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     if (units > VOXP_MAX_UNITS) return VOX_CUDA_ETOOBIG;
     uint64_t nodes = h_root[0];
 
-    // top down: ids and offsets
-    k_root<<<1, 1, 0, s>>>(levels[0]);
-    count_launch();
-    for (int lv = 0; lv + 1 < nl; lv++) {
-        k_down<<<grid_for(levels[lv].m, 256), 256, 0, s>>>(levels[lv], levels[lv + 1]);
-        count_launch();
-    }
     uint4 *pool = nullptr;
     uint32_t *map = nullptr, *dots = nullptr;
+    float *order = nullptr;
     size_t pool_bytes = units * 16, map_bytes = nodes * 4;
     if (x) TRY(d.get(&dots, nodes));
+    if (x && x->order) TRY(d.get(&order, 3 * N));
     TRY(cudaMalloc(&pool, pool_bytes));
     if (cudaMalloc(&map, map_bytes) != cudaSuccess) {
         cudaFree(pool);
         return VOX_CUDA_ENOMEM;
     }
+    // top down: ids, offsets and the image
     for (int lv = 0; lv < nl; lv++) {
-        Level L = levels[lv];
-        k_emit<<<grid_for(L.m, 256), 256, 0, s>>>(L, pool, map, units, nodes, err, dots);
-        k_emit_voxels<<<grid_for((uint64_t)L.m * 32, 256), 256, 0, s>>>(L, P[cur], pool, units, err);
+        const Level &L = levels[lv], &Nx = levels[std::min(lv + 1, nl - 1)];
+        const float *Pc = P[lv & 1];
+        k_emit<<<grid_for(L.m, 256), 256, 0, s>>>(L, Nx, Pc, pool, map, units, nodes, err, dots);
         count_launch();
-        count_launch();
+        if (h_stats[NSTATS * lv + S_OVER]) {
+            k_emit_over<<<grid_for((uint64_t)L.m * 32, 256), 256, 0, s>>>(L, Pc, pool, units, err);
+            count_launch();
+        }
+        if (order) {
+            k_final_order<<<grid_for((uint64_t)L.m * 32, 256), 256, 0, s>>>(L, Pc, order);
+            count_launch();
+        }
     }
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_root[1], err, 4, cudaMemcpyDeviceToHost, s);
@@ -1753,7 +1873,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     if (x) {
         x->dots_of_id.resize(nodes);
         if (e == cudaSuccess && x->order)
-            e = cudaMemcpyAsync(x->order, P[cur], 12 * N, cudaMemcpyDeviceToHost, s);
+            e = cudaMemcpyAsync(x->order, order, 12 * N, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(x->dots_of_id.data(), dots, nodes * 4, cudaMemcpyDeviceToHost, s);
     }
@@ -1766,11 +1886,12 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     st.nodes = nodes;
     st.units = units;
     for (int lv = 0; lv < nl; lv++) {
-        st.inner += h_stats[4 * lv];
-        st.leaf += h_stats[4 * lv + 1];
-        st.dense += h_stats[4 * lv + 2];
-        st.dots += h_stats[4 * lv + 3];
-        if (h_stats[4 * lv]) st.depth = (uint64_t)lv + 1;
+        const unsigned long long *h = &h_stats[NSTATS * lv];
+        st.inner += h[S_INNER];
+        st.leaf += h[S_LEAF];
+        st.dense += h[S_DENSE];
+        st.dots += h[S_DOTS];
+        if (h[S_INNER]) st.depth = (uint64_t)lv + 1;
     }
     for (int i = 0; i < 6; i++) st.bbox[i] = h_box[i];
     int rc = adopt_image(t, pool, pool_bytes, map, map_bytes, st);
