@@ -214,7 +214,7 @@ cudaError_t level_alloc(Level &L, uint32_t m, cudaStream_t s)
     auto add = [&](size_t b) { bytes += (b + 255) & ~size_t(255); };
     add(4 * mm); add(4 * mm); add(32 * mm); add(4 * mm); add(4 * mm); add(4 * mm); add(4 * mm);
     add(4 * mm); add(8 * mm); add(24 * mm); add(12 * mm); add(12 * mm); add(mm); add(mm);
-    cudaError_t e = cudaMallocAsync(&L.mem, bytes, s);
+    cudaError_t e = pool_alloc(&L.mem, bytes, s);
     if (e != cudaSuccess) { L.mem = nullptr; return e; }
     char *p = static_cast<char *>(L.mem);
     L.m = m;
@@ -1655,7 +1655,7 @@ struct Dev {
     cudaError_t get(T **p, size_t count)
     {
         void *q = nullptr;
-        cudaError_t e = cudaMallocAsync(&q, count * sizeof(T) + 16, s);
+        cudaError_t e = pool_alloc(&q, count * sizeof(T) + 16, s);
         if (e == cudaSuccess) owned.push_back(q);
         *p = static_cast<T *>(q);
         return e;
@@ -1663,7 +1663,7 @@ struct Dev {
     ~Dev()
     {
         for (void *p : owned) cudaFreeAsync(p, s);
-        cudaStreamSynchronize(s);
+        cudaStreamSynchronize(s);   // after an error, copies from the caller's memory may be in flight
     }
 };
 
@@ -1683,7 +1683,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     const float vx = vox_voxel[0], vy = vox_voxel[1], vz = vox_voxel[2];
     ImageStats st{};
     st.voxel[0] = vx; st.voxel[1] = vy; st.voxel[2] = vz;
-    if (N == 0) return adopt_image(t, nullptr, 0, nullptr, 0, st);
+    if (N == 0) return adopt_image(t, nullptr, 0, nullptr, 0, nullptr, st);
     if (N > MAX_VOXELS) return VOX_CUDA_ETOOBIG;
 
     Dev d(s);
@@ -1750,12 +1750,15 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     int dev = 0, nsm = 0;
     TRY(cudaGetDevice(&dev));
     TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    uint32_t *h_next = nullptr;
-    TRY(cudaMallocHost(&h_next, 64));
-    struct HostFree {
-        void *p;
-        ~HostFree() { cudaFreeHost(p); }
-    } host_free{h_next};
+    // what comes back to the host, in page-locked memory
+    struct Back {
+        uint32_t next[2], root_nodes, err, unshaped;
+        float box[6];
+        unsigned long long units, stats[NSTATS * MAX_LEVELS];
+    };
+    static_assert(sizeof(Back) <= THREAD_PAGE, "the counts of every level fit the thread's page");
+    Back *back = static_cast<Back *>(thread_page());
+    if (!back) return VOX_CUDA_ENOMEM;
 
     Level root;
     TRY(level_alloc(root, 1, s));
@@ -1801,10 +1804,10 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
             count_launch();
         }
         TRY(cudaGetLastError());
-        TRY(cudaMemcpyAsync(h_next, scal + 2, 8, cudaMemcpyDeviceToHost, s));
+        TRY(cudaMemcpyAsync(back->next, scal + 2, 8, cudaMemcpyDeviceToHost, s));
         TRY(cudaStreamSynchronize(s));
-        const uint32_t mn = h_next[0];
-        largest = h_next[1];
+        const uint32_t mn = back->next[0];
+        largest = back->next[1];
         if (mn == 0) break;
         Level Nx;
         TRY(level_alloc(Nx, mn, s));
@@ -1823,22 +1826,17 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         k_up<<<grid_for(L.m, 256), 256, 0, s>>>(L, Nx, lv + 1 < nl);
         count_launch();
     }
-    std::vector<unsigned long long> h_stats(NSTATS * MAX_LEVELS);
-    uint32_t h_root[2];
-    unsigned long long h_units = 0;
-    float h_box[6];
-    TRY(cudaMemcpyAsync(h_stats.data(), stats, NSTATS * MAX_LEVELS * sizeof(unsigned long long),
-                        cudaMemcpyDeviceToHost, s));
-    TRY(cudaMemcpyAsync(&h_root[0], levels[0].sub_nodes, 4, cudaMemcpyDeviceToHost, s));
-    TRY(cudaMemcpyAsync(&h_root[1], err, 4, cudaMemcpyDeviceToHost, s));
-    TRY(cudaMemcpyAsync(&h_units, levels[0].sub_units, 8, cudaMemcpyDeviceToHost, s));
-    TRY(cudaMemcpyAsync(h_box, levels[0].box, 24, cudaMemcpyDeviceToHost, s));
+    TRY(cudaMemcpyAsync(back->stats, stats, sizeof back->stats, cudaMemcpyDeviceToHost, s));
+    TRY(cudaMemcpyAsync(&back->root_nodes, levels[0].sub_nodes, 4, cudaMemcpyDeviceToHost, s));
+    TRY(cudaMemcpyAsync(&back->err, err, 4, cudaMemcpyDeviceToHost, s));
+    TRY(cudaMemcpyAsync(&back->units, levels[0].sub_units, 8, cudaMemcpyDeviceToHost, s));
+    TRY(cudaMemcpyAsync(back->box, levels[0].box, 24, cudaMemcpyDeviceToHost, s));
     TRY(cudaStreamSynchronize(s));
-    if (h_root[1] & ERR_WALK) return VOX_CUDA_ECUDA;
-    if (h_root[1] & ERR_BIG_LEAF) return VOX_CUDA_ETOOBIG;
-    uint64_t units = VOXP_REC_UNITS + h_units;
+    if (back->err & ERR_WALK) return VOX_CUDA_ECUDA;
+    if (back->err & ERR_BIG_LEAF) return VOX_CUDA_ETOOBIG;
+    uint64_t units = VOXP_REC_UNITS + back->units;
     if (units > VOXP_MAX_UNITS) return VOX_CUDA_ETOOBIG;
-    uint64_t nodes = h_root[0];
+    uint64_t nodes = back->root_nodes;
 
     uint4 *pool = nullptr;
     uint32_t *map = nullptr, *dots = nullptr;
@@ -1846,18 +1844,30 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     size_t pool_bytes = units * 16, map_bytes = nodes * 4;
     if (x) TRY(d.get(&dots, nodes));
     if (x && x->order) TRY(d.get(&order, 3 * N));
-    TRY(cudaMalloc(&pool, pool_bytes));
-    if (cudaMalloc(&map, map_bytes) != cudaSuccess) {
-        cudaFree(pool);
-        return VOX_CUDA_ENOMEM;
-    }
+    // the tree's own memory, given back unless the tree takes it
+    struct Image {
+        cudaStream_t s;
+        void *p[3] = {nullptr, nullptr, nullptr};
+        ~Image()
+        {
+            for (void *q : p)
+                if (q) cudaFreeAsync(q, s);
+        }
+    } image{s};
+    TRY(pool_alloc(&image.p[0], pool_bytes, s));
+    TRY(pool_alloc(&image.p[1], map_bytes, s));
+    TRY(pool_alloc(&image.p[2], 4, s));
+    pool = static_cast<uint4 *>(image.p[0]);
+    map = static_cast<uint32_t *>(image.p[1]);
+    uint32_t *status = static_cast<uint32_t *>(image.p[2]);
+    TRY(cudaMemsetAsync(status, 0, 4, s));
     // top down: ids, offsets and the image
     for (int lv = 0; lv < nl; lv++) {
         const Level &L = levels[lv], &Nx = levels[std::min(lv + 1, nl - 1)];
         const float *Pc = P[lv & 1];
         k_emit<<<grid_for(L.m, 256), 256, 0, s>>>(L, Nx, Pc, pool, map, units, nodes, err, dots);
         count_launch();
-        if (h_stats[NSTATS * lv + S_OVER]) {
+        if (back->stats[NSTATS * lv + S_OVER]) {
             k_emit_over<<<grid_for((uint64_t)L.m * 32, 256), 256, 0, s>>>(L, Pc, pool, units, err);
             count_launch();
         }
@@ -1867,9 +1877,9 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         }
     }
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&h_root[1], err, 4, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&back->err, err, 4, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = image_shape(pool, map, nodes, st.voxel, scal, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&st.unshaped, scal, 4, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&back->unshaped, scal, 4, cudaMemcpyDeviceToHost, s);
     if (x) {
         x->dots_of_id.resize(nodes);
         if (e == cudaSuccess && x->order)
@@ -1878,27 +1888,22 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
             e = cudaMemcpyAsync(x->dots_of_id.data(), dots, nodes * 4, cudaMemcpyDeviceToHost, s);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess || h_root[1]) {
-        cudaFree(pool);
-        cudaFree(map);
-        return e != cudaSuccess ? fail(e) : VOX_CUDA_ECUDA;
-    }
+    if (e != cudaSuccess || back->err) return e != cudaSuccess ? fail(e) : VOX_CUDA_ECUDA;
+    st.unshaped = back->unshaped;
     st.nodes = nodes;
     st.units = units;
     for (int lv = 0; lv < nl; lv++) {
-        const unsigned long long *h = &h_stats[NSTATS * lv];
+        const unsigned long long *h = &back->stats[NSTATS * lv];
         st.inner += h[S_INNER];
         st.leaf += h[S_LEAF];
         st.dense += h[S_DENSE];
         st.dots += h[S_DOTS];
         if (h[S_INNER]) st.depth = (uint64_t)lv + 1;
     }
-    for (int i = 0; i < 6; i++) st.bbox[i] = h_box[i];
-    int rc = adopt_image(t, pool, pool_bytes, map, map_bytes, st);
-    if (rc) {
-        cudaFree(pool);
-        cudaFree(map);
-    }
+    for (int i = 0; i < 6; i++) st.bbox[i] = back->box[i];
+    int rc = adopt_image(t, pool, pool_bytes, map, map_bytes, status, st);
+    if (rc == VOX_CUDA_OK)
+        for (void *&q : image.p) q = nullptr;
     return rc;
 }
 
@@ -1955,18 +1960,20 @@ int raw_build(vox_cuda_tree *t, const void *samples, const unsigned dim[3], unsi
         RawSolid solid{d_samples, d_mask, samplesize, test->lo, test->hi};
         // count the solid voxels first: the set is allocated to size
         uint32_t nt = (uint32_t)((V + SCAN_TILE - 1) / SCAN_TILE);
-        uint32_t h_total = 0;
+        uint32_t h_total = 0, *page = static_cast<uint32_t *>(thread_page());
+        if (!page) return VOX_CUDA_ENOMEM;
         if (nt) {
             k_tile_sums<<<nt, SCAN_THREADS, 0, s>>>(solid, V, tile);
             count_launch();
             k_scan_tiles<<<1, 1024, 0, s>>>(tile, nt, total);
             count_launch();
-            if (cudaMemcpyAsync(&h_total, total, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            if (cudaMemcpyAsync(page, total, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
                 cudaStreamSynchronize(s) != cudaSuccess)
                 return VOX_CUDA_ECUDA;
+            h_total = *page;
         }
         if (h_total) {
-            if (cudaMallocAsync(&P, 12ull * h_total, s) != cudaSuccess) return VOX_CUDA_ENOMEM;
+            if (pool_alloc(reinterpret_cast<void **>(&P), 12ull * h_total, s) != cudaSuccess) return VOX_CUDA_ENOMEM;
             RawPlace place{dim[1], dim[2], vox_voxel[0], vox_voxel[1], vox_voxel[2], P};
             k_tile_apply<<<nt, SCAN_THREADS, 0, s>>>(solid, place, V, tile);
             count_launch();
@@ -1997,7 +2004,7 @@ int build_for_host_tree(const float *set, size_t n, vox_cuda_tree **out, HostTre
     if (n == 0 || n > MAX_VOXELS || !set) return VOX_CUDA_EINVAL;
     return new_tree(out, [&](vox_cuda_tree *t, cudaStream_t s) {
         float *d = nullptr;
-        if (cudaMallocAsync(&d, 12ull * n, s) != cudaSuccess) return (int)VOX_CUDA_ENOMEM;
+        if (pool_alloc(reinterpret_cast<void **>(&d), 12ull * n, s) != cudaSuccess) return (int)VOX_CUDA_ENOMEM;
         int rc = VOX_CUDA_OK;
         if (cudaMemcpyAsync(d, set, 12ull * n, cudaMemcpyHostToDevice, s) != cudaSuccess) rc = VOX_CUDA_ECUDA;
         if (rc == VOX_CUDA_OK) rc = build_tree(t, d, n, s, x);
@@ -2019,7 +2026,7 @@ try {
     return new_tree(out, [&](vox_cuda_tree *t, cudaStream_t s) {
         if (n > MAX_VOXELS) return (int)VOX_CUDA_ETOOBIG;
         float *d = nullptr;
-        if (n && cudaMallocAsync(&d, 12ull * n, s) != cudaSuccess) return (int)VOX_CUDA_ENOMEM;
+        if (n && pool_alloc(reinterpret_cast<void **>(&d), 12ull * n, s) != cudaSuccess) return (int)VOX_CUDA_ENOMEM;
         int rc = VOX_CUDA_OK;
         if (n && cudaMemcpyAsync(d, set, 12ull * n, cudaMemcpyHostToDevice, s) != cudaSuccess) rc = VOX_CUDA_ECUDA;
         if (rc == VOX_CUDA_OK) rc = build_tree(t, d, n, s);

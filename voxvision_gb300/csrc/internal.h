@@ -7,6 +7,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <mutex>
 #include <utility>
@@ -21,6 +22,12 @@
 using vox::DevTree;
 
 struct vox_cuda_tree {
+    static std::atomic<int> live;          // trees there are
+    vox_cuda_tree() { live++; }
+    ~vox_cuda_tree() { live--; }
+    vox_cuda_tree(const vox_cuda_tree &) = delete;
+    vox_cuda_tree &operator=(const vox_cuda_tree &) = delete;
+    bool pooled = false;                   // the buffers below come from pool_alloc
     int device = 0;
     float bbox[6] = {0, 0, 0, 0, 0, 0};   // root bounding box (for scheduling only)
     uint4 *d_pool = nullptr;
@@ -53,12 +60,13 @@ cudaError_t image_shape(const uint4 *pool, const uint32_t *rec_of_id, uint64_t n
                         uint32_t *word, cudaStream_t s);
 
 /* Makes t serve a device image built in place: `pool` (st.units 16-byte
- * units) and `map` (st.nodes pre-order id -> record entries), both
- * cudaMalloc'ed and owned by t from then on; t's previous buffers are freed.
- * st.nodes == 0 (pool and map NULL) is the empty tree.  VOX_CUDA_EDEPTH when
+ * units) and `map` (st.nodes pre-order id -> record entries), both from
+ * pool_alloc and owned by t, a new handle, from then on, as `status`, a zeroed
+ * word for its status.
+ * st.nodes == 0 (all three NULL) is the empty tree.  VOX_CUDA_EDEPTH when
  * the tree is too deep for the traversal stack (the buffers stay the
  * caller's). */
-int adopt_image(vox_cuda_tree *t, uint4 *pool, size_t pool_bytes, uint32_t *map, size_t map_bytes,
+int adopt_image(vox_cuda_tree *t, uint4 *pool, size_t pool_bytes, uint32_t *map, size_t map_bytes, uint32_t *status,
                 const ImageStats &st);
 
 /* What a host tree (struct vox_node) needs beyond the device image when it
@@ -95,6 +103,23 @@ inline int cap_class_for_depth(uint64_t depth)
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
 inline int status_of(cudaError_t e) { return e == cudaSuccess ? VOX_CUDA_OK : VOX_CUDA_ECUDA; }
+
+/* Stream-ordered memory of the current device, freed with cudaFreeAsync (or
+ * cudaFree once nothing uses it): the library's scratch and the trees it builds.
+ * It comes from a pool of the library's own that keeps up to POOL_KEEP bytes
+ * across synchronisations, where the default pool gives everything back and
+ * maps it anew: five 16 MB buffers allocated, freed and synchronised cost 20 us
+ * against 240-390, a build's 37 MB image and its map and status 10 us against
+ * 190.  What it keeps goes back when the last tree is freed (pool_trim). */
+constexpr uint64_t POOL_KEEP = 512ull << 20;
+cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s);
+void pool_trim();
+
+/* A page-locked page of the calling thread for what a synchronous call reads
+ * back (THREAD_PAGE bytes; NULL when it cannot be had), kept until the thread
+ * ends: cudaMallocHost and cudaFreeHost take 260 us a call. */
+constexpr size_t THREAD_PAGE = 8192;
+void *thread_page();
 
 /* Adds one to the process-wide kernel launch count (vox_cuda_launch_count). */
 void count_launch();

@@ -507,7 +507,7 @@ cudaError_t launch_rays(const vox_cuda_tree *t, const float *o, const float *d, 
     void *scratch = nullptr;
     uint32_t *order = nullptr;
     if (!COUNT && n >= RAY_SORT_MIN && n <= 0xFFFFFFFFull) {
-        cudaError_t e = cudaMallocAsync(&scratch, ray_order_bytes(n), s);
+        cudaError_t e = pool_alloc(&scratch, ray_order_bytes(n), s);
         if (e != cudaSuccess) return e;
         e = ray_order(t, o, d, n, scratch, &order, s);
         if (e != cudaSuccess) {
@@ -545,7 +545,7 @@ cudaError_t launch_balls(const vox_cuda_tree *t, const float *c, const float *r,
     const bool nested = !COUNT && (t->dev.shape & SHAPE) == SHAPE;
     const bool sorted = nested ? n >= NESTED_SORT_MIN && t->n_units * 16 > NESTED_SORT_BYTES : n >= BALL_SORT_MIN;
     if (!COUNT && sorted && n <= 0xFFFFFFFFull) {
-        cudaError_t e = cudaMallocAsync(&scratch, ray_order_bytes(n), s);
+        cudaError_t e = pool_alloc(&scratch, ray_order_bytes(n), s);
         if (e != cudaSuccess) return e;
         e = ball_order(t, c, n, scratch, &order, s);
         if (e != cudaSuccess) {
@@ -705,7 +705,7 @@ struct Scratch {
     cudaStream_t s;
     void *p = nullptr;
     explicit Scratch(cudaStream_t st) : s(st) {}
-    cudaError_t get(size_t bytes) { return cudaMallocAsync(&p, bytes ? bytes : 16, s); }
+    cudaError_t get(size_t bytes) { return pool_alloc(&p, bytes ? bytes : 16, s); }
     ~Scratch() { if (p) cudaFreeAsync(p, s); }
 };
 
@@ -714,6 +714,65 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 }  // namespace
 
 void count_launch() { g_launches++; }
+
+std::atomic<int> vox_cuda_tree::live{0};
+
+namespace {
+constexpr int POOL_DEVICES = 64;
+std::mutex g_pool_mu;
+std::atomic<cudaMemPool_t> g_pool[POOL_DEVICES];
+}  // namespace
+
+cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s)
+{
+    *p = nullptr;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    cudaMemPool_t pool = dev < POOL_DEVICES ? g_pool[dev].load() : nullptr;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!pool && dev < POOL_DEVICES && cudaStreamIsCapturing(s, &cap) == cudaSuccess &&
+        cap == cudaStreamCaptureStatusNone) {   // (no pool is made inside a capture)
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        pool = g_pool[dev].load();
+        if (!pool) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            uint64_t keep = POOL_KEEP;
+            if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
+                cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+                g_pool[dev].store(pool);
+            } else {
+                pool = nullptr;
+                cudaGetLastError();
+            }
+        }
+    }
+    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+}
+
+void *thread_page()
+{
+    struct Page {
+        void *p = nullptr;
+        ~Page()                    // at thread exit, as ~HostCallState
+        {
+            if (p) cudaFreeHost(p);
+        }
+    };
+    thread_local Page page;
+    if (!page.p && cudaHostAlloc(&page.p, THREAD_PAGE, cudaHostAllocPortable) != cudaSuccess) page.p = nullptr;
+    return page.p;
+}
+
+void pool_trim()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= POOL_DEVICES) return;
+    if (cudaMemPool_t pool = g_pool[dev].load()) cudaMemPoolTrimTo(pool, 0);
+}
 
 
 
@@ -1093,36 +1152,33 @@ static int load_tree(vox_cuda_tree *t, const struct vox_node *root, int layout =
     return VOX_CUDA_OK;
 }
 
-int adopt_image(vox_cuda_tree *t, uint4 *pool, size_t pool_bytes, uint32_t *map, size_t map_bytes,
+int adopt_image(vox_cuda_tree *t, uint4 *pool, size_t pool_bytes, uint32_t *map, size_t map_bytes, uint32_t *status,
                 const ImageStats &st)
 {
     int cls = cap_class_for_depth(st.depth);
     if (cls < 0) return VOX_CUDA_EDEPTH;
     bool empty = st.nodes == 0;
-    uint4 *own_pool = nullptr;
-    uint32_t *own_map = nullptr;
     if (empty) {   // as the upload of a NULL tree: one record's worth of pool, a one-entry map
         pool_bytes = VOXP_REC_UNITS * 16;
         map_bytes = 4;
-        if (cudaMalloc(&own_pool, pool_bytes) != cudaSuccess) return VOX_CUDA_ENOMEM;
-        if (cudaMalloc(&own_map, map_bytes) != cudaSuccess) {
-            cudaFree(own_pool);
+        if (cudaMalloc(&pool, pool_bytes) != cudaSuccess) return VOX_CUDA_ENOMEM;
+        if (cudaMalloc(&map, map_bytes) != cudaSuccess) {
+            cudaFree(pool);
             return VOX_CUDA_ENOMEM;
         }
-        pool = own_pool;
-        map = own_map;
+        if (cudaMalloc(&status, 4) != cudaSuccess || cudaMemset(status, 0, 4) != cudaSuccess) {
+            cudaFree(pool);
+            cudaFree(map);
+            cudaFree(status);
+            return VOX_CUDA_ENOMEM;
+        }
     }
-    if ((!t->d_status && cudaMalloc(&t->d_status, 4) != cudaSuccess) || cudaMemset(t->d_status, 0, 4) != cudaSuccess) {
-        cudaFree(own_pool);
-        cudaFree(own_map);
-        return VOX_CUDA_ENOMEM;
-    }
-    if (t->d_pool) cudaFree(t->d_pool);
-    if (t->d_rec_of_id) cudaFree(t->d_rec_of_id);
+    t->pooled = !empty;
     t->d_pool = pool;
     t->pool_bytes = pool_bytes;
     t->d_rec_of_id = map;
     t->map_bytes = map_bytes;
+    t->d_status = status;
     t->cap_class = cls;
     for (int i = 0; i < 6; i++) t->bbox[i] = empty ? 0.0f : st.bbox[i];
     t->dev.pool = pool;
@@ -1248,13 +1304,17 @@ EXPORT int vox_cuda_tree_free(vox_cuda_tree *t)
 try {
     if (!t) return VOX_CUDA_EINVAL;
     int cur = 0;
+    const int dev = t->device;
     cudaGetDevice(&cur);
-    if (cur != t->device) cudaSetDevice(t->device);
+    if (cur != dev) cudaSetDevice(dev);
+    // (memory of a pool is freed without waiting for kernels that may read it)
+    if (t->pooled) cudaDeviceSynchronize();
     cudaFree(t->d_pool);
     cudaFree(t->d_rec_of_id);
     cudaFree(t->d_status);
-    if (cur != t->device) cudaSetDevice(cur);
     delete t;
+    if (vox_cuda_tree::live.load() == 0) pool_trim();
+    if (cur != dev) cudaSetDevice(cur);
     return VOX_CUDA_OK;
 } VOX_ABI_FAIL_INT
 
