@@ -74,9 +74,9 @@
 namespace {
 
 constexpr uint32_t NONE = 0xFFFFFFFFu;
-constexpr int SCAN_THREADS = 256;
-constexpr int SCAN_ITEMS = 8;
-constexpr uint32_t SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+constexpr int RAW_THREADS = 256;
+constexpr uint32_t RAW_ITEMS = 16;                       // consecutive samples a thread reads
+constexpr uint32_t RAW_TILE = RAW_THREADS * RAW_ITEMS;   // samples a block reads
 constexpr uint32_t SMALL = 512;      // nodes with at most this many voxels are made by one warp
 constexpr uint32_t MID = 8192;       // nodes with at most this many by one block, larger ones tile by tile
 constexpr uint32_t CHUNK = 1024;     // voxels per chunk
@@ -96,9 +96,7 @@ constexpr uint32_t ERR_LAYOUT = 4u;     // a record or voxel run fell outside th
 
 inline unsigned grid_for(uint64_t n, unsigned threads) { return (unsigned)((n + threads - 1) / threads); }
 
-// ------------------------------------------------------------------ scan
-// Exclusive scan of u32 values v(i), i in [0, m): per-tile sums, a one-block
-// scan of the tile sums, then each tile's own scan handed to w(i, excl, v(i)).
+// ------------------------------------------------------------------ scans
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x)
 {
@@ -110,26 +108,7 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x)
     return x;
 }
 
-template <class V>
-__global__ void __launch_bounds__(SCAN_THREADS) k_tile_sums(V v, uint64_t m, uint32_t *tile)
-{
-    __shared__ uint32_t ws[SCAN_THREADS / 32];
-    uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
-    uint32_t s = 0;
-    for (int j = 0; j < SCAN_ITEMS; j++) {
-        uint64_t i = base + (uint64_t)j * SCAN_THREADS + threadIdx.x;
-        if (i < m) s += v(i);
-    }
-    for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t t = 0;
-        for (int w = 0; w < SCAN_THREADS / 32; w++) t += ws[w];
-        tile[blockIdx.x] = t;
-    }
-}
-
+// Exclusive scan of n values in place, and their total (one block).
 __global__ void __launch_bounds__(1024) k_scan_tiles(uint32_t *a, uint32_t n, uint32_t *total)
 {
     __shared__ uint32_t ws[32];
@@ -155,31 +134,6 @@ __global__ void __launch_bounds__(1024) k_scan_tiles(uint32_t *a, uint32_t n, ui
         __syncthreads();
     }
     if (threadIdx.x == 0) *total = carry;
-}
-
-template <class V, class W>
-__global__ void __launch_bounds__(SCAN_THREADS) k_tile_apply(V v, W w, uint64_t m, const uint32_t *tile)
-{
-    __shared__ uint32_t ws[SCAN_THREADS / 32];
-    uint32_t run = tile[blockIdx.x];
-    uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int j = 0; j < SCAN_ITEMS; j++) {
-        uint64_t i = base + (uint64_t)j * SCAN_THREADS + threadIdx.x;
-        uint32_t x = i < m ? v(i) : 0;
-        uint32_t incl = warp_incl_scan(x);
-        if (lane == 31) ws[warp] = incl;
-        __syncthreads();
-        uint32_t before = 0, tot = 0;
-        for (int q = 0; q < SCAN_THREADS / 32; q++) {
-            uint32_t t = ws[q];
-            before += q < warp ? t : 0u;
-            tot += t;
-        }
-        if (i < m) w(i, run + before + incl - x, x);
-        run += tot;
-        __syncthreads();
-    }
 }
 
 // ------------------------------------------------------------ level arrays
@@ -1617,33 +1571,80 @@ __global__ void k_final_order(Level L, const float *P, float *order)
 
 // ------------------------------------------------------------ raw reader
 
-struct RawSolid {
+// Which samples are solid (datareader.c:51-77): 16 consecutive ones a thread,
+// read 16 bytes at a time (samples of SS little-endian bytes; the buffer starts
+// on a 256-byte boundary), as a bit mask.  Single-byte loads, 32 bytes a warp,
+// took 40 us to count and 107 to place a 256^3 volume of bytes; see raw_build.
+struct RawTest {
     const uint8_t *samples, *mask;
-    uint32_t ss, lo, hi;
-    __device__ uint32_t operator()(uint64_t v) const
-    {
-        uint32_t x = 0;
-        for (uint32_t l = 0; l < ss; l++) x |= (uint32_t)samples[v * ss + l] << (8 * l);   // datareader.c:61-72
-        if (mask) return (mask[x >> 3] >> (x & 7)) & 1u;
-        return x >= lo && x <= hi;
-    }
+    uint64_t V;
+    uint32_t lo, hi;
 };
 
-struct RawPlace {
-    uint32_t d1, d2;
-    float v0, v1, v2;
-    float *P;
-    __device__ void operator()(uint64_t v, uint32_t excl, uint32_t solid) const
-    {
-        if (!solid) return;
-        uint64_t jk = (uint64_t)d1 * d2;
-        uint32_t i = (uint32_t)(v / jk), j = (uint32_t)((v / d2) % d1), k = (uint32_t)(v % d2);
-        // array[counter][a] = index * vox_voxel[a] (datareader.c:73-77)
-        P[3 * (uint64_t)excl] = __fmul_rn(__uint2float_rn(i), v0);
-        P[3 * (uint64_t)excl + 1] = __fmul_rn(__uint2float_rn(j), v1);
-        P[3 * (uint64_t)excl + 2] = __fmul_rn(__uint2float_rn(k), v2);
+template <int SS>
+__device__ __forceinline__ uint32_t raw_solid(const RawTest &r, uint64_t v0)
+{
+    uint32_t w[4 * SS];
+    if (v0 + RAW_ITEMS <= r.V) {
+        const uint4 *p = reinterpret_cast<const uint4 *>(r.samples + v0 * SS);
+        for (int i = 0; i < SS; i++) {
+            const uint4 u = p[i];
+            w[4 * i] = u.x; w[4 * i + 1] = u.y; w[4 * i + 2] = u.z; w[4 * i + 3] = u.w;
+        }
+    } else {
+        for (int i = 0; i < 4 * SS; i++) {
+            w[i] = 0;
+            for (int b = 0; b < 4; b++)
+                if (v0 * SS + 4 * i + b < r.V * SS) w[i] |= (uint32_t)r.samples[v0 * SS + 4 * i + b] << (8 * b);
+        }
     }
-};
+    uint32_t m = 0;
+    for (int j = 0; j < (int)RAW_ITEMS; j++) {
+        uint32_t x = 0;
+        for (int l = 0; l < SS; l++) x |= ((w[(j * SS + l) / 4] >> (8 * ((j * SS + l) % 4))) & 0xFFu) << (8 * l);
+        const bool solid = r.mask ? ((r.mask[x >> 3] >> (x & 7)) & 1u) != 0u : x >= r.lo && x <= r.hi;
+        m |= (uint32_t)(solid && v0 + j < r.V) << j;
+    }
+    return m;
+}
+
+template <int SS>
+__global__ void __launch_bounds__(RAW_THREADS) k_raw_count(RawTest r, uint32_t *tile)
+{
+    __shared__ uint32_t ws[RAW_THREADS / 32];
+    const uint64_t v0 = ((uint64_t)blockIdx.x * RAW_THREADS + threadIdx.x) * RAW_ITEMS;
+    const uint32_t n = __reduce_add_sync(0xffffffffu, v0 < r.V ? (uint32_t)__popc(raw_solid<SS>(r, v0)) : 0u);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = n;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t t = 0;
+        for (int w = 0; w < RAW_THREADS / 32; w++) t += ws[w];
+        tile[blockIdx.x] = t;
+    }
+}
+
+// The solid samples' voxels in order, from the tiles' scanned counts:
+// array[counter][a] = index * vox_voxel[a] (datareader.c:73-77).
+template <int SS>
+__global__ void __launch_bounds__(RAW_THREADS) k_raw_place(RawTest r, const uint32_t *tile, uint32_t d1, uint32_t d2,
+                                                           float vx, float vy, float vz, float *P)
+{
+    __shared__ uint32_t ws[RAW_THREADS / 32];
+    const uint64_t v0 = ((uint64_t)blockIdx.x * RAW_THREADS + threadIdx.x) * RAW_ITEMS;
+    uint32_t m = v0 < r.V ? raw_solid<SS>(r, v0) : 0u;
+    const uint32_t n = (uint32_t)__popc(m), incl = warp_incl_scan(n);
+    if ((threadIdx.x & 31) == 31) ws[threadIdx.x >> 5] = incl;
+    __syncthreads();
+    uint64_t at = (uint64_t)tile[blockIdx.x] + incl - n;
+    for (uint32_t w = 0; w < (threadIdx.x >> 5); w++) at += ws[w];
+    for (; m; m &= m - 1, at++) {
+        const uint32_t v = (uint32_t)v0 + (uint32_t)__ffs((int)m) - 1u;   // below 2^32 (check_raw_args)
+        const uint32_t row = v / d2, k = v - row * d2, i = row / d1, j = row - i * d1;
+        P[3 * at] = __fmul_rn(__uint2float_rn(i), vx);
+        P[3 * at + 1] = __fmul_rn(__uint2float_rn(j), vy);
+        P[3 * at + 2] = __fmul_rn(__uint2float_rn(k), vz);
+    }
+}
 
 // ---------------------------------------------------------------- host side
 
@@ -1950,20 +1951,23 @@ int raw_build(vox_cuda_tree *t, const void *samples, const unsigned dim[3], unsi
     int rc = VOX_CUDA_OK;
     {
         Dev d(s);
-        if (d.get(&d_samples, bytes ? bytes : 1) != cudaSuccess || d.get(&tile, V / SCAN_TILE + 2) != cudaSuccess ||
+        if (d.get(&d_samples, bytes ? bytes : 1) != cudaSuccess || d.get(&tile, V / RAW_TILE + 2) != cudaSuccess ||
             d.get(&total, 1) != cudaSuccess || (mask_bytes && d.get(&d_mask, mask_bytes) != cudaSuccess))
             return VOX_CUDA_ENOMEM;
         if (bytes && cudaMemcpyAsync(d_samples, samples, bytes, cudaMemcpyHostToDevice, s) != cudaSuccess)
             return VOX_CUDA_ECUDA;
         if (mask_bytes && cudaMemcpyAsync(d_mask, test->mask, mask_bytes, cudaMemcpyHostToDevice, s) != cudaSuccess)
             return VOX_CUDA_ECUDA;
-        RawSolid solid{d_samples, d_mask, samplesize, test->lo, test->hi};
+        const RawTest raw{d_samples, d_mask, V, test->lo, test->hi};
+        void (*const count[])(RawTest, uint32_t *) = {k_raw_count<1>, k_raw_count<2>, k_raw_count<3>, k_raw_count<4>};
+        void (*const place[])(RawTest, const uint32_t *, uint32_t, uint32_t, float, float, float, float *) = {
+            k_raw_place<1>, k_raw_place<2>, k_raw_place<3>, k_raw_place<4>};
         // count the solid voxels first: the set is allocated to size
-        uint32_t nt = (uint32_t)((V + SCAN_TILE - 1) / SCAN_TILE);
+        uint32_t nt = (uint32_t)((V + RAW_TILE - 1) / RAW_TILE);
         uint32_t h_total = 0, *page = static_cast<uint32_t *>(thread_page());
         if (!page) return VOX_CUDA_ENOMEM;
         if (nt) {
-            k_tile_sums<<<nt, SCAN_THREADS, 0, s>>>(solid, V, tile);
+            count[samplesize - 1]<<<nt, RAW_THREADS, 0, s>>>(raw, tile);
             count_launch();
             k_scan_tiles<<<1, 1024, 0, s>>>(tile, nt, total);
             count_launch();
@@ -1974,8 +1978,8 @@ int raw_build(vox_cuda_tree *t, const void *samples, const unsigned dim[3], unsi
         }
         if (h_total) {
             if (pool_alloc(reinterpret_cast<void **>(&P), 12ull * h_total, s) != cudaSuccess) return VOX_CUDA_ENOMEM;
-            RawPlace place{dim[1], dim[2], vox_voxel[0], vox_voxel[1], vox_voxel[2], P};
-            k_tile_apply<<<nt, SCAN_THREADS, 0, s>>>(solid, place, V, tile);
+            place[samplesize - 1]<<<nt, RAW_THREADS, 0, s>>>(raw, tile, dim[1], dim[2], vox_voxel[0], vox_voxel[1],
+                                                             vox_voxel[2], P);
             count_launch();
             if (cudaGetLastError() != cudaSuccess) rc = VOX_CUDA_ECUDA;
         }
