@@ -77,8 +77,10 @@ constexpr uint32_t NONE = 0xFFFFFFFFu;
 constexpr int RAW_THREADS = 256;
 constexpr uint32_t RAW_ITEMS = 16;                       // consecutive samples a thread reads
 constexpr uint32_t RAW_TILE = RAW_THREADS * RAW_ITEMS;   // samples a block reads
-constexpr uint32_t SMALL = 512;      // nodes with at most this many voxels are made by one warp
-constexpr uint32_t MID = 8192;       // nodes with at most this many by one block, larger ones tile by tile
+constexpr uint32_t TINY = 32;        // nodes with at most this many voxels, and
+constexpr uint32_t SMALL = 128;      // with at most this many, are split by a lane each,
+constexpr uint32_t LOW = 1024;       // with at most this many by a block of 128 threads,
+constexpr uint32_t MID = 8192;       // with at most this many by a block of 512, larger ones tile by tile
 constexpr uint32_t CHUNK = 1024;     // voxels per chunk
 constexpr int CHUNK_THREADS = 128;   // 8 consecutive voxels per thread
 constexpr int NBIN = 16;             // binades with a precomputed map per chunk
@@ -192,12 +194,11 @@ cudaError_t level_alloc(Level &L, uint32_t m, cudaStream_t s)
 // -------------------------------------------------------- per-level kernels
 
 // The nodes of a level that take more than one thread, by size class, in no
-// particular order: above VOX_MAX_DOTS voxels a warp each, above SMALL a
-// block, above MID tile by tile.  A tiled node's slot and its first tile come
+// particular order (above VOX_MAX_DOTS, TINY, SMALL, LOW and MID voxels).  A tiled node's slot and its first tile come
 // from one counter, so that first tiles ascend with slots.
 struct NodeLists {
-    uint32_t *small, *mid, *tiled, *first_tile;
-    uint32_t *nsmall, *nmid;
+    uint32_t *tiny, *small, *low, *mid, *tiled, *first_tile;
+    uint32_t *ntiny, *nsmall, *nlow, *nmid;
     unsigned long long *ntiled;   // slots in the upper half, tiles in the lower
     uint32_t tile;                // positions per tile
     __device__ void add_large(uint32_t k, uint32_t n) const
@@ -206,8 +207,12 @@ struct NodeLists {
             const unsigned long long at = atomicAdd(ntiled, (1ull << 32) | ((n + tile - 1) / tile));
             tiled[at >> 32] = k;
             first_tile[at >> 32] = (uint32_t)at;
-        } else if (n > SMALL) {
+        } else if (n > LOW) {
             mid[atomicAdd(nmid, 1u)] = k;
+        } else if (n > SMALL) {
+            low[atomicAdd(nlow, 1u)] = k;
+        } else if (n > TINY) {
+            small[atomicAdd(nsmall, 1u)] = k;
         }
     }
 };
@@ -778,7 +783,7 @@ __device__ __forceinline__ uint32_t walk_back(uint32_t t, uint32_t from, uint32_
             return t;
         }
         const uint32_t a = last + 1;                       // start of the claimed run holding s
-        const uint32_t back = ((s - a) / u + 1) * u;
+        const uint32_t back = s - a < u ? u : ((s - a) / u + 1) * u;   // (mostly one step: no division)
         if (a > s || back > s - from) {
             atomicOr(err, ERR_WALK);
             return t;
@@ -900,220 +905,167 @@ __device__ __forceinline__ float unordered(uint32_t u)
     return __uint_as_float(u ^ ((u >> 31) ? 0x80000000u : 0xFFFFFFFFu));
 }
 
-// Nodes of VOX_MAX_DOTS+1..32 voxels in the lanes of a warp, a voxel a lane:
-// box, density, centre, octants and all eight passes in registers.  Returns
-// the child mask.
-__device__ uint32_t node_in_lanes(const Level &L, uint32_t k, uint32_t n, const float *P, float *Pn, const float *v,
-                                  uint8_t *order, WarpTally &tally, uint32_t *err)
+// Nodes of VOX_MAX_DOTS+1..MOST voxels, up to 32 of them to a warp at a time.
+// Each node's box, density, centre and octants are the warp's work, in
+// registers; then every lane makes the eight passes over one node of its own,
+// as the reference makes them (swap each claimed voxel to the front), in a
+// column of shared memory; then the warp moves each node's voxels and takes
+// the children's places in the next level, all with one atomic.
+//
+// What bounds the parallel form of a pass is instruction issue (945 of them a
+// voxel and level in the block kernel below); the serial one takes five steps
+// of ten instructions a voxel, and there are enough nodes for the lanes.  The
+// two levels of the 256^3 set where most nodes have 8 to 128 voxels took
+// 291 us with a warp on every pass, 160 like this.
+constexpr int LANE_WARPS = 4;
+template <uint32_t MOST>
+__global__ void __launch_bounds__(LANE_WARPS * 32) k_nodes_lanes(Level L, const uint32_t *list, const uint32_t *count,
+                                                                 const float *P, float *Pn, float vx, float vy, float vz,
+                                                                 Tally tally)
 {
-    constexpr uint32_t FULL = 0xffffffffu;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t s0 = L.start[k];
-    const bool in = lane < n;
-    float p[3] = {0.0f, 0.0f, 0.0f}, mn[3], mx[3];
-    if (in)
-        for (int a = 0; a < 3; a++) p[a] = P[3 * (s0 + lane) + a];
-    for (int a = 0; a < 3; a++) {   // the first of equal extremes (-0 equals +0), NaN never one
-        const float lo = in && p[a] < INFINITY ? p[a] + 0.0f : INFINITY, hi = in && p[a] > -INFINITY ? p[a] + 0.0f : -INFINITY;
-        mn[a] = unordered(__reduce_min_sync(FULL, ordered(lo)));
-        mx[a] = unordered(__reduce_max_sync(FULL, ordered(hi)));
-        const uint32_t il = __ballot_sync(FULL, in && p[a] == mn[a]), ih = __ballot_sync(FULL, in && p[a] == mx[a]);
-        const float fl = __shfl_sync(FULL, p[a], il ? __ffs((int)il) - 1 : 0), fh = __shfl_sync(FULL, p[a], ih ? __ffs((int)ih) - 1 : 0);
-        if (il) mn[a] = fl;
-        if (ih) mx[a] = fh;
-    }
-    uint32_t kind = 0;
-    if (lane == 0) kind = write_box(L, k, n, mn, mx, v);
-    kind = __shfl_sync(FULL, kind, 0);
-    if (kind != K_INNER) {
-        tally.dense++;              // above VOX_MAX_DOTS voxels it is no leaf
-        return 0u;
-    }
-    float c[3];
-    PlainSum x;
-    x.init();
-    if (in)
-        for (int a = 0; a < 3; a++) x.add(a, __fsub_rn(p[a], mn[a]));
-    for (int a = 0; a < 3; a++) {
-        x.g[a] = __reduce_min_sync(FULL, x.g[a]);
-        for (int off = 16; off; off >>= 1) x.sum[a] = __fadd_rn(x.sum[a], __shfl_xor_sync(FULL, x.sum[a], off));
-    }
-    for (int a = 0; a < 3; a++) {
-        const float acc = x.exact(a) ? x.sum[a] : warp_sum(P, s0, s0 + n, a, mn[a], 0.0f);
-        c[a] = centre_of(acc, n, mn[a], v[a]);
-        if (lane == 0) L.centre[3 * (size_t)k + a] = c[a];
-    }
-    uint32_t q = in ? octant(c, p) : 8u, src = lane, cnt = 0, from = 0;   // the voxel now at this lane, and where it was
-    for (uint32_t o = 0; o < 8; o++) {
-        const uint32_t m = __ballot_sync(FULL, q == o && lane >= from);
-        if (lane == o) cnt = (uint32_t)__popc(m);
-        if (!m) continue;           // nothing claimed: nothing moves
-        const uint32_t rest = from + (uint32_t)__popc(m);
-        if ((m >> lane) & 1u) order[from + __popc(m & lanes_below(lane))] = (uint8_t)src;
-        uint32_t s = lane;
-        if (in && lane >= rest) {
-            auto claimed = [&](uint32_t i, uint32_t &before, uint32_t &last) {
-                before = (uint32_t)__popc(m & lanes_below(i));
-                last = last_in_word(0, i, m, from);
-                return ((m >> i) & 1u) != 0u;
-            };
-            s = walk_back(lane, from, 32u, claimed, err);
-        }
-        const uint32_t q2 = __shfl_sync(FULL, q, s), src2 = __shfl_sync(FULL, src, s);
-        if (in && lane >= rest) { q = q2; src = src2; }
-        from = rest;
-    }
-    __syncwarp();
-    const uint32_t at = in ? order[lane] : lane;
-    for (int a = 0; a < 3; a++) {
-        const float y = __shfl_sync(FULL, p[a], at);
-        if (in) Pn[3 * (s0 + lane) + a] = y;
-    }
-    __syncwarp();
-    return tally.split(L, k, n, cnt, err);
-}
-
-// Nodes of 33..SMALL voxels by a warp: the same in shared memory, a voxel in
-// 16 bits {octant, place in the node}.
-struct WarpNode {
-    uint16_t buf[2][SMALL], order[SMALL];
-    uint32_t mask[SMALL / 32], before[SMALL / 32], last[SMALL / 32];
-};
-
-__device__ uint32_t node_in_warp(const Level &L, uint32_t k, uint32_t n, const float *P, float *Pn, const float *v,
-                                 WarpNode &w, WarpTally &tally, uint32_t *err)
-{
-    constexpr uint32_t FULL = 0xffffffffu;
-    static_assert(SMALL == 512, "9 bits of place; one word a lane in scan_words");
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t s0 = L.start[k];
-    Extremes e;
-    e.init();
-    for (uint32_t j = lane; j < n; j += 32) e.add(P + 3 * (s0 + j), j);
-    e.warp_merge();
-    uint32_t kind = 0;
-    if (lane == 0) kind = write_box(L, k, n, e.mn, e.mx, v);
-    kind = __shfl_sync(FULL, kind, 0);
-    if (kind != K_INNER) {
-        tally.dense++;
-        return 0u;
-    }
-    float c[3];
-    PlainSum x;
-    x.init();
-    for (uint32_t j = lane; j < n; j += 32)
-        for (int a = 0; a < 3; a++) x.add(a, __fsub_rn(P[3 * (s0 + j) + a], e.mn[a]));
-    x.warp_merge();
-    for (int a = 0; a < 3; a++) {
-        const float acc = x.exact(a) ? x.sum[a] : warp_sum(P, s0, s0 + n, a, e.mn[a], 0.0f);
-        c[a] = centre_of(acc, n, e.mn[a], v[a]);
-        if (lane == 0) L.centre[3 * (size_t)k + a] = c[a];
-    }
-    for (uint32_t j = lane; j < n; j += 32) {
-        const float p[3] = {P[3 * (s0 + j)], P[3 * (s0 + j) + 1], P[3 * (s0 + j) + 2]};
-        w.buf[0][j] = (uint16_t)((octant(c, p) << 9) | j);
-    }
-    const uint32_t nw = (n + 31) / 32;
-    uint32_t cnt = 0, from = 0, cur = 0;
-    for (uint32_t o = 0; o < 8 && from < n; o++) {
-        const uint16_t *in = w.buf[cur];
-        uint16_t *out = w.buf[cur ^ 1];
-        __syncwarp();
-        uint32_t any = 0;
-        for (uint32_t i = from >> 5; i < nw; i++) {
-            const uint32_t t = (i << 5) + lane;
-            const bool range = t >= from && t < n, cl = range && (uint32_t)(in[t] >> 9) == o;
-            const uint32_t m = __ballot_sync(FULL, cl), u = __ballot_sync(FULL, range && !cl);
-            any |= m;
-            if (lane == 0) {
-                w.mask[i] = m;
-                w.before[i] = (uint32_t)__popc(m);
-                w.last[i] = u ? (i << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
-            }
-        }
-        if (!any) continue;
-        __syncwarp();
-        const uint32_t w0 = from >> 5;
-        uint32_t run = 0, prev = NO_POS;
-        scan_words<1>(w.before + w0, w.last + w0, nw - w0, run, prev);
-        if (lane == o) cnt = run;
-        __syncwarp();
-        const uint32_t rest = from + run;
-        auto claimed = [&](uint32_t s, uint32_t &before, uint32_t &last) {
-            const uint32_t i = s >> 5, b = s & 31, m = w.mask[i];
-            before = w.before[i] + (uint32_t)__popc(m & lanes_below(b));
-            last = last_in_word(i, b, m, from);
-            if (last == NO_POS) last = w.last[i];
-            return ((m >> b) & 1u) != 0u;
-        };
-        for (uint32_t t = from + lane; t < n; t += 32) {
-            uint32_t before, last;
-            if (claimed(t, before, last)) w.order[from + before] = in[t] & 511u;
-            if (t >= rest) out[t] = in[walk_back(t, from, SMALL, claimed, err)];
-        }
-        from = rest;
-        cur ^= 1;
-    }
-    __syncwarp();
-    for (uint32_t t = lane; t < n; t += 32) place(P, Pn, s0 + t, s0 + w.order[t]);
-    __syncwarp();
-    return tally.split(L, k, n, cnt, err);
-}
-
-// Nodes of VOX_MAX_DOTS+1..SMALL voxels, up to eight of them to a warp at a
-// time, as many as still leave every warp of the grid some; the warp then takes
-// their children's places in the next level with one atomic.
-constexpr int WARP_NODE_WARPS = 4, WARP_NODE_BLOCKS = 8;   // blocks per SM
-__global__ void __launch_bounds__(WARP_NODE_WARPS * 32, WARP_NODE_BLOCKS) k_nodes_warp(Level L, NodeLists lists, const float *P,
-                                                                     float *Pn, float vx, float vy, float vz,
-                                                                     Tally tally)
-{
-    __shared__ WarpNode shared[WARP_NODE_WARPS];
-    WarpNode &w = shared[threadIdx.x >> 5];
-    const uint32_t lane = threadIdx.x & 31, total = *lists.nsmall;
-    const uint32_t per = min(8u, max(1u, total / (gridDim.x * WARP_NODE_WARPS)));
+    static_assert(MOST % 32 == 0 && MOST <= 128, "octants are counted in bytes");
+    constexpr uint32_t FULL = 0xffffffffu, J = MOST / 32;
+    __shared__ uint16_t columns[LANE_WARPS][MOST][32];   // per voxel of 32 nodes {octant, place in the node}
+    uint16_t (*col)[32] = columns[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31, total = *count;
+    const uint32_t warps = gridDim.x * LANE_WARPS, per = min(32u, max(1u, (total + warps - 1) / warps));
     const float v[3] = {vx, vy, vz};
     WarpTally mine;
-    for (uint32_t b = (blockIdx.x * WARP_NODE_WARPS + (threadIdx.x >> 5)) * per; b < total;
-         b += gridDim.x * WARP_NODE_WARPS * per) {
-        uint32_t my = NONE, kids = 0;
-        for (uint32_t i = 0; i < per && b + i < total; i++) {
-            const uint32_t k = lists.small[b + i], n = L.n[k];
-            const uint32_t mask = n <= 32
-                ? node_in_lanes(L, k, n, P, Pn, v, reinterpret_cast<uint8_t *>(w.order), mine, tally.err)
-                : node_in_warp(L, k, n, P, Pn, v, w, mine, tally.err);
-            if (lane == i) { my = k; kids = (uint32_t)__popc(mask); }
+    for (uint32_t b = (blockIdx.x * LANE_WARPS + (threadIdx.x >> 5)) * per; b < total; b += warps * per) {
+        const uint32_t here = min(per, total - b);
+        uint32_t my = NONE, my_n = 0, c03 = 0, c47 = 0;   // this lane's node, its octants' counts (a byte each)
+        uint64_t my_s = 0;
+        if (lane < here) {
+            my = list[b + lane];
+            my_n = L.n[my];
+            my_s = L.start[my];
+        }
+        bool split = false;
+        for (uint32_t q = 0; q < here; q++) {
+            const uint32_t k = __shfl_sync(FULL, my, q), n = __shfl_sync(FULL, my_n, q);
+            const uint64_t s0 = __shfl_sync(FULL, my_s, q);
+            float p[J][3], mn[3], mx[3];
+            for (uint32_t j = 0; j < J; j++)
+                for (int a = 0; a < 3; a++) p[j][a] = j * 32 + lane < n ? P[3 * (s0 + j * 32 + lane) + a] : 0.0f;
+            for (int a = 0; a < 3; a++) {
+                float lo = INFINITY, hi = -INFINITY;      // NaN is never an extreme
+                for (uint32_t j = 0; j < J; j++)
+                    if (j * 32 + lane < n) { lo = fminf(lo, p[j][a]); hi = fmaxf(hi, p[j][a]); }
+                mn[a] = unordered(__reduce_min_sync(FULL, ordered(lo)));
+                mx[a] = unordered(__reduce_max_sync(FULL, ordered(hi)));
+                if (mn[a] == 0.0f || mx[a] == 0.0f) {     // the first of equal extremes: -0 equals +0
+                    bool found = false;
+                    float zero = 0.0f;
+                    for (uint32_t j = 0; j < J; j++) {
+                        const uint32_t m = __ballot_sync(FULL, j * 32 + lane < n && p[j][a] == 0.0f);
+                        const float z = __shfl_sync(FULL, p[j][a], m ? __ffs((int)m) - 1 : 0);
+                        if (m && !found) { zero = z; found = true; }
+                    }
+                    if (mn[a] == 0.0f) mn[a] = zero;
+                    if (mx[a] == 0.0f) mx[a] = zero;
+                }
+            }
+            uint32_t kind = 0;
+            if (lane == 0) kind = write_box(L, k, n, mn, mx, v);
+            kind = __shfl_sync(FULL, kind, 0);
+            if (kind != K_INNER) {
+                mine.dense++;                             // above VOX_MAX_DOTS voxels it is no leaf
+                continue;
+            }
+            if (lane == q) split = true;
+            float c[3];
+            PlainSum x;
+            x.init();
+            for (uint32_t j = 0; j < J; j++)
+                if (j * 32 + lane < n)
+                    for (int a = 0; a < 3; a++) x.add(a, __fsub_rn(p[j][a], mn[a]));
+            for (int a = 0; a < 3; a++) {
+                x.g[a] = __reduce_min_sync(FULL, x.g[a]);
+                for (int off = 16; off; off >>= 1) x.sum[a] = __fadd_rn(x.sum[a], __shfl_xor_sync(FULL, x.sum[a], off));
+            }
+            for (int a = 0; a < 3; a++) {
+                const float acc = x.exact(a) ? x.sum[a] : warp_sum(P, s0, s0 + n, a, mn[a], 0.0f);
+                c[a] = centre_of(acc, n, mn[a], v[a]);
+                if (lane == 0) L.centre[3 * (size_t)k + a] = c[a];
+            }
+            uint32_t n03 = 0, n47 = 0;
+            for (uint32_t j = 0; j < J; j++)
+                if (j * 32 + lane < n) {
+                    const uint32_t o = octant(c, p[j]);
+                    col[j * 32 + lane][q] = (uint16_t)((o << 13) | (j * 32 + lane));
+                    if (o < 4) n03 += 1u << (8 * o);
+                    else n47 += 1u << (8 * (o - 4));
+                }
+            n03 = __reduce_add_sync(FULL, n03);
+            n47 = __reduce_add_sync(FULL, n47);
+            if (lane == q) { c03 = n03; c47 = n47; }
+        }
+        __syncwarp();
+        if (split) {                                      // sort_set, tree.c:166-183, on the lane's own node
+            uint32_t at = 0;
+            for (uint32_t o = 0; o < 8; o++) {
+                const uint32_t end = at + (((o < 4 ? c03 : c47) >> (8 * (o & 3))) & 0xFFu);
+                uint32_t i = at;
+                uint16_t x = at < end ? col[i][lane] : 0;
+                while (at < end) {                        // until the octant's last voxel is placed
+                    const uint16_t next = i + 1 < my_n ? col[i + 1][lane] : 0;
+                    if ((uint32_t)(x >> 13) == o) {
+                        col[i][lane] = col[at][lane];
+                        col[at][lane] = x;
+                        at++;
+                    }
+                    x = next;
+                    if (++i > my_n) {                     // impossible: the counts are of these voxels
+                        atomicOr(tally.err, ERR_WALK);
+                        break;
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        uint32_t kids = 0;
+        for (uint32_t q = 0; q < here; q++) {
+            if (!__shfl_sync(FULL, (int)split, q)) continue;
+            const uint32_t k = __shfl_sync(FULL, my, q), n = __shfl_sync(FULL, my_n, q), n03 = __shfl_sync(FULL, c03, q),
+                           n47 = __shfl_sync(FULL, c47, q);
+            const uint64_t s0 = __shfl_sync(FULL, my_s, q);
+            for (uint32_t t = lane; t < n; t += 32) place(P, Pn, s0 + t, s0 + (col[t][q] & 8191u));
+            const uint32_t mask = mine.split(L, k, n, ((lane < 4 ? n03 : n47) >> (8 * (lane & 3))) & 0xFFu, tally.err);
+            if (lane == q) kids = (uint32_t)__popc(mask);
         }
         const uint32_t incl = warp_incl_scan(kids);
         uint32_t first = 0;
         if (lane == 31 && incl) first = atomicAdd(tally.children, incl);
-        first = __shfl_sync(0xffffffffu, first, 31) + incl - kids;
+        first = __shfl_sync(FULL, first, 31) + incl - kids;
         if (kids) L.first_child[my] = first;
+        __syncwarp();
     }
     mine.flush(tally);
 }
 
-// Nodes of SMALL+1..MID voxels: a block each, as above, a voxel in 16 bits
-// {octant, place in the node}.
-constexpr int MID_THREADS = 512;
-__global__ void __launch_bounds__(MID_THREADS) k_nodes_block(Level L, NodeLists lists, const float *P, float *Pn, float vx,
-                                                             float vy, float vz, Tally tally)
+// Nodes of at most MOST voxels: a block of THREADS each, as above, a voxel in
+// 16 bits {octant, place in the node}.
+template <int THREADS, uint32_t MOST>
+__global__ void __launch_bounds__(THREADS) k_nodes_block(Level L, const uint32_t *list, const uint32_t *count,
+                                                         const float *P, float *Pn, float vx, float vy, float vz,
+                                                         Tally tally)
 {
-    static_assert(MID == 8192 && MID / 32 == 256, "13 bits of place; 8 words a lane in scan_words");
-    constexpr int WARPS = MID_THREADS / 32;
-    __shared__ uint16_t buf[2][MID];
-    __shared__ uint32_t mask[MID / 32], before[MID / 32], last[MID / 32], total, s_kind;
+    static_assert(MOST <= 8192 && MOST % 1024 == 0, "13 bits of place; whole words a lane in scan_words");
+    constexpr int WARPS = THREADS / 32;
+    static_assert(WARPS >= 3 && WARPS <= 32, "an axis a warp");
+    __shared__ uint16_t buf[2][MOST];
+    __shared__ uint32_t mask[MOST / 32], before[MOST / 32], last[MOST / 32], total, s_kind;
     __shared__ Extremes epart[WARPS];
     __shared__ PlainSum spart[WARPS];
     __shared__ float centre[3];
-    if (blockIdx.x >= *lists.nmid) return;
-    const uint32_t k = lists.mid[blockIdx.x], n = L.n[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (blockIdx.x >= *count) return;
+    const uint32_t k = list[blockIdx.x], n = L.n[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t s0 = L.start[k];
     const float v[3] = {vx, vy, vz};
     {
         Extremes e;
         e.init();
-        for (uint32_t j = threadIdx.x; j < n; j += MID_THREADS) e.add(P + 3 * (s0 + j), j);
+        for (uint32_t j = threadIdx.x; j < n; j += THREADS) e.add(P + 3 * (s0 + j), j);
         e.warp_merge();
         if (lane == 0) epart[warp] = e;
         __syncthreads();
@@ -1130,7 +1082,7 @@ __global__ void __launch_bounds__(MID_THREADS) k_nodes_block(Level L, NodeLists 
     {
         PlainSum x;
         x.init();
-        for (uint32_t j = threadIdx.x; j < n; j += MID_THREADS)
+        for (uint32_t j = threadIdx.x; j < n; j += THREADS)
             for (int a = 0; a < 3; a++) x.add(a, __fsub_rn(P[3 * (s0 + j) + a], mn[a]));
         x.warp_merge();
         if (lane == 0) spart[warp] = x;
@@ -1146,7 +1098,7 @@ __global__ void __launch_bounds__(MID_THREADS) k_nodes_block(Level L, NodeLists 
         }
         __syncthreads();
     }
-    for (uint32_t i = threadIdx.x; i < n; i += MID_THREADS) {
+    for (uint32_t i = threadIdx.x; i < n; i += THREADS) {
         const float p[3] = {P[3 * (s0 + i)], P[3 * (s0 + i) + 1], P[3 * (s0 + i) + 2]};
         buf[0][i] = (uint16_t)((octant(centre, p) << 13) | i);
     }
@@ -1171,7 +1123,7 @@ __global__ void __launch_bounds__(MID_THREADS) k_nodes_block(Level L, NodeLists 
         if (warp == 0) {
             const uint32_t w0 = from >> 5;
             uint32_t run = 0, prev = NO_POS;
-            scan_words<MID / 32 / 32>(before + w0, last + w0, nw - w0, run, prev);
+            scan_words<MOST / 32 / 32>(before + w0, last + w0, nw - w0, run, prev);
             if (lane == 0) total = run;
             if (lane == o) cnt = run;
         }
@@ -1184,10 +1136,10 @@ __global__ void __launch_bounds__(MID_THREADS) k_nodes_block(Level L, NodeLists 
             if (l == NO_POS) l = last[w];
             return ((m >> i) & 1u) != 0u;
         };
-        for (uint32_t t = from + threadIdx.x; t < n; t += MID_THREADS) {
+        for (uint32_t t = from + threadIdx.x; t < n; t += THREADS) {
             uint32_t c, l;
             if (claimed(t, c, l)) place(P, Pn, s0 + from + c, s0 + (in[t] & 8191u));
-            if (t >= rest) out[t] = in[walk_back(t, from, MID, claimed, tally.err)];
+            if (t >= rest) out[t] = in[walk_back(t, from, MOST, claimed, tally.err)];
         }
         from = rest;
     }
@@ -1216,21 +1168,22 @@ constexpr uint32_t SUB = 1024;          // positions marked at a time; a tile is
 constexpr uint32_t MAX_TILES = 2048;    // tiles of one node
 
 struct Marks {
-    uint32_t *mask, *before, *last;     // per word of a tile
-    uint32_t *count, *tail;             // per tile
+    uint4 *word;                        // per word of a tile: claimed bits, count before, last before
+    uint2 *tile;                        // per tile: claimed count, last unclaimed position + 1 (0: none)
 };
 
-// Marks of one SUB of positions from their claimed flags, word by word.
+// Marks of one SUB of positions from their claimed flags, word by word.  (run
+// and prev, what comes before, are warp 0's.)
 struct SubMarks {
-    uint32_t before[SUB / 32], last[SUB / 32];
+    uint32_t mask[SUB / 32], before[SUB / 32], last[SUB / 32];
     __device__ void flush(const Marks &m, uint64_t word0, uint32_t nw, uint32_t &run, uint32_t &prev)
     {
         __syncthreads();
-        if (threadIdx.x < 32) scan_words<SUB / 32 / 32>(before, last, nw, run, prev);
-        __syncthreads();
-        for (uint32_t w = threadIdx.x; w < nw; w += PASS_THREADS) {
-            m.before[word0 + w] = before[w];
-            m.last[word0 + w] = last[w];
+        if (threadIdx.x < 32) {
+            scan_words<SUB / 32 / 32>(before, last, nw, run, prev);
+            __syncwarp();
+            for (uint32_t w = threadIdx.x; w < nw; w += 32)
+                m.word[word0 + w] = make_uint4(mask[w], before[w], last[w], 0u);
         }
         __syncthreads();
     }
@@ -1264,17 +1217,14 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_marks(Level L, NodeLists 
             const bool cl = q == 0;
             const uint32_t m = __ballot_sync(0xffffffffu, cl), u = __ballot_sync(0xffffffffu, in && !cl);
             if (lane == 0) {
-                out.mask[word0 + w] = m;
+                sub.mask[w] = m;
                 sub.before[w] = (uint32_t)__popc(m);
                 sub.last[w] = u ? sb + (w << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
             }
         }
         sub.flush(out, word0, nw, run, prev);
     }
-    if (threadIdx.x == 0) {
-        out.count[blockIdx.x] = run;
-        out.tail[blockIdx.x] = prev;
-    }
+    if (threadIdx.x == 0) out.tile[blockIdx.x] = make_uint2(run, prev + 1u);
 }
 
 // Pass o over every tiled node.
@@ -1285,7 +1235,7 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
 {
     __shared__ SubMarks sub;
     __shared__ uint32_t tbefore[MAX_TILES], tlast[MAX_TILES];
-    __shared__ uint32_t s_total;
+    __shared__ uint32_t wsum[PASS_THREADS / 32], wtop[PASS_THREADS / 32];
     const uint32_t slot = tile_slot(lists, blockIdx.x);
     if (slot == NO_POS) return;
     const uint32_t tile = lists.tile, ft = lists.first_tile[slot], ti = blockIdx.x - ft;
@@ -1297,28 +1247,45 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
     const uint32_t b = ti * tile, e = min(n, b + tile);
     if (e <= from) return;                     // all of it placed by earlier passes
     const uint32_t t0 = from / tile, nt = (n + tile - 1) / tile - t0;   // the tiles still in play
-    for (uint32_t i = threadIdx.x; i < nt; i += PASS_THREADS) {
-        tbefore[i] = in.count[ft + t0 + i];
-        tlast[i] = in.tail[ft + t0 + i];
+    // what comes before each of them: a run of tiles a thread, scanned over the block
+    constexpr uint32_t PER = MAX_TILES / PASS_THREADS;
+    const uint32_t i0 = threadIdx.x * PER;
+    uint2 t[PER];
+    uint32_t sum = 0, top = 0;
+    for (uint32_t j = 0; j < PER; j++) {
+        t[j] = i0 + j < nt ? in.tile[ft + t0 + i0 + j] : make_uint2(0u, 0u);
+        sum += t[j].x;
+        top = max(top, t[j].y);
     }
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t run = 0, prev = NO_POS;
-        for (uint32_t i = 0; i < nt; i += 128)
-            scan_words<4>(tbefore + i, tlast + i, min(nt - i, 128u), run, prev);
-        if (lane == 0) {
-            s_total = run;
-            if (e == n) L.cnt[8 * (size_t)k + o] = run;   // read by later launches only
-        }
+    uint32_t ps = sum, pt = top;
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, ps, off), y = __shfl_up_sync(0xffffffffu, pt, off);
+        if (lane >= (uint32_t)off) { ps += x; pt = max(pt, y); }
     }
+    if (lane == 31) { wsum[warp] = ps; wtop[warp] = pt; }
     __syncthreads();
-    const uint32_t rest = from + s_total;
+    uint32_t total = 0, before = ps - sum, above = __shfl_up_sync(0xffffffffu, pt, 1);
+    if (lane == 0) above = 0;
+    for (uint32_t w = 0; w < PASS_THREADS / 32; w++) {
+        if (w < warp) { before += wsum[w]; above = max(above, wtop[w]); }
+        total += wsum[w];
+    }
+    for (uint32_t j = 0; j < PER; j++) {
+        if (i0 + j < nt) { tbefore[i0 + j] = before; tlast[i0 + j] = above - 1u; }
+        before += t[j].x;
+        above = max(above, t[j].y);
+    }
+    if (e == n && threadIdx.x == 0) L.cnt[8 * (size_t)k + o] = total;   // read by later launches only
+    __syncthreads();
+    const uint32_t rest = from + total;
     const uint64_t words = (uint64_t)ft * (tile / 32);   // the node's first word: tiles hold whole words
     auto claimed = [&](uint32_t s, uint32_t &c, uint32_t &l) {
-        const uint32_t w = s >> 5, i = s & 31, m = in.mask[words + w], ts = s / tile - t0;
-        c = tbefore[ts] + in.before[words + w] + (uint32_t)__popc(m & lanes_below(i));
+        const uint32_t w = s >> 5, i = s & 31, ts = s / tile - t0;
+        const uint4 word = in.word[words + w];
+        const uint32_t m = word.x;
+        c = tbefore[ts] + word.y + (uint32_t)__popc(m & lanes_below(i));
         l = last_in_word(w, i, m, from);
-        if (l == NO_POS) l = in.last[words + w];
+        if (l == NO_POS) l = word.z;
         if (l == NO_POS) l = tlast[ts];
         return ((m >> i) & 1u) != 0u;
     };
@@ -1342,17 +1309,14 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
             const bool left = t >= rest && t < e, cl = left && q == o + 1;
             const uint32_t m = __ballot_sync(0xffffffffu, cl), u = __ballot_sync(0xffffffffu, left && !cl);
             if (lane == 0) {
-                out.mask[words + (sb >> 5) + w] = m;
+                sub.mask[w] = m;
                 sub.before[w] = (uint32_t)__popc(m);
                 sub.last[w] = u ? sb + (w << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
             }
         }
         sub.flush(out, words + (sb >> 5), nw, run, prev);
     }
-    if (threadIdx.x == 0) {
-        out.count[blockIdx.x] = run;
-        out.tail[blockIdx.x] = prev;
-    }
+    if (threadIdx.x == 0) out.tile[blockIdx.x] = make_uint2(run, prev + 1u);
 }
 
 // Tiled nodes after their passes, a warp each.
@@ -1396,13 +1360,13 @@ __device__ __forceinline__ void new_node(const Level &L, uint32_t k, uint32_t s0
             dots += n;
         }
     }
-    if (n > SMALL) lists.add_large(k, n);
-    const bool small = n > VOX_MAX_DOTS && n <= SMALL;
-    const uint32_t m = __ballot_sync(FULL, small);
+    if (n > TINY) lists.add_large(k, n);
+    const bool tiny = n > VOX_MAX_DOTS && n <= TINY;
+    const uint32_t m = __ballot_sync(FULL, tiny);
     uint32_t at = 0;
-    if (lane == 0 && m) at = atomicAdd(lists.nsmall, (uint32_t)__popc(m));
+    if (lane == 0 && m) at = atomicAdd(lists.ntiny, (uint32_t)__popc(m));
     at = __shfl_sync(FULL, at, 0) + (uint32_t)__popc(m & ((1u << lane) - 1u));
-    if (small) lists.small[at] = k;
+    if (tiny) lists.tiny[at] = k;
 }
 
 // The next level's nodes: a thread per octant of every node of this one.
@@ -1574,7 +1538,7 @@ __global__ void k_final_order(Level L, const float *P, float *order)
 // Which samples are solid (datareader.c:51-77): 16 consecutive ones a thread,
 // read 16 bytes at a time (samples of SS little-endian bytes; the buffer starts
 // on a 256-byte boundary), as a bit mask.  Single-byte loads, 32 bytes a warp,
-// took 40 us to count and 107 to place a 256^3 volume of bytes; see raw_build.
+// took 40 us to count and 107 to place a 256^3 volume of bytes, these 13 and 25.
 struct RawTest {
     const uint8_t *samples, *mask;
     uint64_t V;
@@ -1709,17 +1673,22 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     TRY(d.get(&P[0], 3 * N));
     TRY(d.get(&P[1], 3 * N));
     TRY(d.get(&stats, NSTATS * (MAX_LEVELS + 1)));
-    // scal: 0 small nodes, 1 mid nodes, 2 children, 3 largest child, 6-7 tiled nodes and tiles, 8 error bits
+    // scal: 0 tiny nodes, 1 mid nodes, 2 children, 3 largest child, 4 low, 5 small, 6-7 tiled nodes and tiles,
+    // 8 error bits
     TRY(d.get(&scal, 12));
     uint32_t *err = scal + 8;
     NodeLists lists{};
-    lists.nsmall = scal;
+    lists.ntiny = scal;
+    lists.nsmall = scal + 5;
     lists.nmid = scal + 1;
+    lists.nlow = scal + 4;
     lists.ntiled = reinterpret_cast<unsigned long long *>(scal + 6);
     lists.tile = SUB * (uint32_t)((N + (uint64_t)SUB * MAX_TILES - 1) / ((uint64_t)SUB * MAX_TILES));
-    const uint64_t max_mid = N / SMALL, max_tiled = N / MID, max_tiles = N / lists.tile + max_tiled,
+    const uint64_t max_low = N / SMALL, max_mid = N / LOW, max_tiled = N / MID, max_tiles = N / lists.tile + max_tiled,
                    max_chunks = max_tiles * (lists.tile / CHUNK);
-    TRY(d.get(&lists.small, N / (VOX_MAX_DOTS + 1) + 1));
+    TRY(d.get(&lists.tiny, N / (VOX_MAX_DOTS + 1) + 1));
+    TRY(d.get(&lists.small, N / (TINY + 1) + 1));
+    TRY(d.get(&lists.low, max_low + 1));
     TRY(d.get(&lists.mid, max_mid + 1));
     // past 2^24 additions a sum's roundings can add up to a sizeable part of it
     const int window = N > (1u << 24) ? NBIN : 2;
@@ -1728,11 +1697,8 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         for (int i = 0; i < 2; i++) {
             TRY(d.get(&idx[i], N));
             TRY(d.get(&oct[i], N));
-            TRY(d.get(&marks[i].mask, max_tiles * (lists.tile / 32)));
-            TRY(d.get(&marks[i].before, max_tiles * (lists.tile / 32)));
-            TRY(d.get(&marks[i].last, max_tiles * (lists.tile / 32)));
-            TRY(d.get(&marks[i].count, max_tiles));
-            TRY(d.get(&marks[i].tail, max_tiles));
+            TRY(d.get(&marks[i].word, max_tiles * (lists.tile / 32)));
+            TRY(d.get(&marks[i].tile, max_tiles));
         }
         TRY(d.get(&lists.tiled, max_tiled));
         TRY(d.get(&lists.first_tile, max_tiled));
@@ -1794,14 +1760,26 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
             k_finish_tiled<<<grid_for(max_tiled * 32, 256), 256, 0, s>>>(L, lists, tally);
             for (int i = 0; i < 16; i++) count_launch();
         }
+        if (largest > LOW) {
+            k_nodes_block<512, MID><<<(unsigned)std::min<uint64_t>(m, max_mid), 512, 0, s>>>(L, lists.mid, lists.nmid, Pc, Pn,
+                                                                                           vx, vy, vz, tally);
+            count_launch();
+        }
         if (largest > SMALL) {
-            k_nodes_block<<<(unsigned)max_mid, MID_THREADS, 0, s>>>(L, lists, Pc, Pn, vx, vy, vz, tally);
+            k_nodes_block<128, LOW><<<(unsigned)std::min<uint64_t>(m, max_low), 128, 0, s>>>(L, lists.low, lists.nlow, Pc, Pn,
+                                                                                           vx, vy, vz, tally);
+            count_launch();
+        }
+        if (largest > TINY) {
+            const unsigned blocks = grid_for(std::min<uint64_t>(m, N / (TINY + 1) + 1), LANE_WARPS);
+            k_nodes_lanes<SMALL><<<std::min(blocks, (unsigned)(nsm * 5)), LANE_WARPS * 32, 0, s>>>(
+                L, lists.small, lists.nsmall, Pc, Pn, vx, vy, vz, tally);
             count_launch();
         }
         if (largest > VOX_MAX_DOTS) {
-            const unsigned blocks = grid_for(std::min<uint64_t>(m, N / (VOX_MAX_DOTS + 1) + 1), WARP_NODE_WARPS);
-            k_nodes_warp<<<std::min(blocks, (unsigned)(nsm * WARP_NODE_BLOCKS)), WARP_NODE_WARPS * 32, 0, s>>>(
-                L, lists, Pc, Pn, vx, vy, vz, tally);
+            const unsigned blocks = grid_for(std::min<uint64_t>(m, N / (VOX_MAX_DOTS + 1) + 1), LANE_WARPS);
+            k_nodes_lanes<TINY><<<std::min(blocks, (unsigned)(nsm * 8)), LANE_WARPS * 32, 0, s>>>(
+                L, lists.tiny, lists.ntiny, Pc, Pn, vx, vy, vz, tally);
             count_launch();
         }
         TRY(cudaGetLastError());
