@@ -150,3 +150,21 @@ def test_both_forms_of_the_ball_search_match_the_oracle(kind, voxel, shift, off_
     finally:
         vg.set_voxel_size((1, 1, 1))
         orc.set_voxel((1, 1, 1))
+
+
+@pytest.mark.parametrize("n", [1, 2432, 2433, 4865, 9728, 38913, 38912, 77825])
+def test_batches_of_every_lane_count(n):
+    """Batches that fill one, two, ... all of a warp's lanes."""
+    import voxvision_gb300 as vg
+    vox = _voxels(5, (1, 1, 1), (0, 0, 0))
+    ht = vg.HostTree.from_voxels(vox)
+    dt = vg.DeviceTree(ht.ptr)
+    box = vox.min(0).astype(np.float64), vox.max(0).astype(np.float64) + 1
+    o, d = (np.resize(x, (n, 3)) for x in _family("plain", 9, box, np.ones(3)))
+    c, rad = _balls("plain", 11, box, np.ones(3))
+    c, rad = np.resize(c, (n, 3)), np.resize(rad, n)
+    leaf, slot, pts = dt.rays(o, d)
+    oleaf, oslot, opts, _ = orc.ray_batch(ht.ptr, o, d)
+    assert np.array_equal(leaf, oleaf) and np.array_equal(slot, oslot)
+    assert same_points(pts, opts, leaf != MISS)[0]
+    assert np.array_equal(dt.balls(c, rad), orc.ball_batch(ht.ptr, c, rad)[0])
