@@ -464,6 +464,12 @@ __device__ __forceinline__ f32x2 quot2(f32x2 a, f32x2 nd, f32x2 y)   // nd = -d
     return fma2(fma2(nd, q, a), y, q);
 }
 
+// -0 twice, where ptxas does not see what it holds: as an operand in constant
+// memory it costs the batch kernel no registers (32 frames 1,324 -> 1,314 us, the mixed
+// batch 815 -> 809); the other kernels do better with one computed per ray (near 4K FAST frame 1,056 against
+// 1,063 us).
+static __constant__ f32x2 c_mzero = 0x8000000080000000ull;
+
 // Whether the mirrored search may make this search.
 __device__ __forceinline__ bool mirror_ok(const DevTree &t, float ox, float oy, float oz, float dx, float dy, float dz)
 {
@@ -475,7 +481,7 @@ __device__ __forceinline__ bool mirror_ok(const DevTree &t, float ox, float oy, 
 }
 
 
-template <int CAP>
+template <int CAP, bool MZERO_CONST>
 __device__ __forceinline__ int trace_mirrored(const DevTree &t, uint32_t start, float ox, float oy, float oz,
                                               float dx, float dy, float dz, uint4 (&stack)[CAP], RayHit &hit)
 {
@@ -485,8 +491,8 @@ __device__ __forceinline__ int trace_mirrored(const DevTree &t, uint32_t start, 
     ox = nx ? -ox : ox; oy = ny ? -oy : oy; oz = nz ? -oz : oz;
     dx = fabsf(dx); dy = fabsf(dy); dz = fabsf(dz);
     const float yz = __frcp_rn(dz);
-    const float mz = __fmul_rn(-dx, 0.0f);   // -0
-    const f32x2 mzero = pair(mz, mz), ndxy = pair(-dx, -dy), yxy = pair(__frcp_rn(dx), __frcp_rn(dy));
+    const float mz = MZERO_CONST ? 0.0f : __fmul_rn(-dx, 0.0f);   // -0
+    const f32x2 mzero = MZERO_CONST ? c_mzero : pair(mz, mz), ndxy = pair(-dx, -dy), yxy = pair(__frcp_rn(dx), __frcp_rn(dy));
     int sp = 0;
     uint32_t cur = start;      // a record, or while scanning a leaf the voxel to test
     uint32_t vend = 0;         // one past the leaf's last voxel; 0: cur is a record
@@ -607,7 +613,7 @@ __device__ __forceinline__ int trace_mirrored(const DevTree &t, uint32_t start, 
                 const bool w0 = v0 && ((mask >> s0) & 1u), w1 = v1 && ((mask >> s1) & 1u),
                            w2 = v2 && ((mask >> s2) & 1u);
                 const int n = (int)w0 + (int)w1 + (int)w2;
-                if (sp + n > CAP) return STEP_ERROR;
+                if (sp > CAP - 3) return STEP_ERROR;   // (never in a tree whose depth the class holds)
                 // each child above those visited after it
                 if (w0)
                     stack[sp + (int)(w1 && !o10) + (int)(w2 && !o20)] =
@@ -688,7 +694,7 @@ __device__ __noinline__ GeneralResult trace_general_call(const uint4 *pool, uint
 /* The whole search from the node whose record is at `start`.  Returns true
  * on a hit; `overflow` is set (and the search ends as a miss) on STEP_ERROR.
  * Counting searches count the reference's work: the general search. */
-template <int CAP, bool COUNT>
+template <int CAP, bool COUNT, bool MZERO_CONST = false>
 __device__ __forceinline__ bool trace_ray(const DevTree &t, uint32_t start,
                                           float ox0, float oy0, float oz0,
                                           float dx, float dy, float dz,
@@ -698,7 +704,7 @@ __device__ __forceinline__ bool trace_ray(const DevTree &t, uint32_t start,
     if (COUNT) return trace_general<CAP, COUNT>(t, start, ox0, oy0, oz0, dx, dy, dz, stack, hit, cnt, overflow);
     int r = STEP_AGAIN;
     if (mirror_ok(t, ox0, oy0, oz0, dx, dy, dz))
-        r = trace_mirrored<CAP>(t, start, ox0, oy0, oz0, dx, dy, dz, stack, hit);
+        r = trace_mirrored<CAP, MZERO_CONST>(t, start, ox0, oy0, oz0, dx, dy, dz, stack, hit);
     if (r == STEP_AGAIN) {
         GeneralResult g = trace_general_call<CAP>(t.pool, start, ox0, oy0, oz0, dx, dy, dz, t.vx, t.vy, t.vz,
                                                   t.max_steps, t.n_units, t.fault, stack);
