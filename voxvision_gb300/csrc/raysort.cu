@@ -110,25 +110,25 @@ __global__ void __launch_bounds__(SORT_THREADS) k_keys(const float *__restrict__
     for (uint32_t k = threadIdx.x; k < NKEYS; k += SORT_THREADS) hist[(size_t)blockIdx.x * NKEYS + k] = h[k];
 }
 
-// For every key: its count before each block (in place) and its total; a warp
-// a key, 32 blocks at a time.
-__global__ void __launch_bounds__(256) k_key_blocks(uint32_t *hist, uint32_t nblocks, uint32_t *total)
+// For every key: its count before each block (in place) and its total; a block
+// takes 32 keys, a lane each, and its warps a run of the blocks each.
+__global__ void __launch_bounds__(1024) k_key_blocks(uint32_t *hist, uint32_t nblocks, uint32_t *total)
 {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t k = blockIdx.x * 8 + (threadIdx.x >> 5);
+    __shared__ uint32_t part[32][32];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
+    const uint32_t per = (nblocks + 31) / 32, b0 = min(warp * per, nblocks), b1 = min(b0 + per, nblocks);
+    uint32_t sum = 0;
+    for (uint32_t b = b0; b < b1; b++) sum += hist[(size_t)b * NKEYS + k];
+    part[warp][lane] = sum;
+    __syncthreads();
     uint32_t run = 0;
-    for (uint32_t b0 = 0; b0 < nblocks; b0 += 32) {
-        const uint32_t b = b0 + lane;
-        const uint32_t c = b < nblocks ? hist[(size_t)b * NKEYS + k] : 0u;
-        uint32_t x = c;
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
-            if (lane >= (uint32_t)off) x += y;
-        }
-        if (b < nblocks) hist[(size_t)b * NKEYS + k] = run + x - c;
-        run += __shfl_sync(0xFFFFFFFFu, x, 31);
+    for (uint32_t w = 0; w < warp; w++) run += part[w][lane];
+    if (warp == 31) total[k] = run + sum;
+    for (uint32_t b = b0; b < b1; b++) {
+        const uint32_t c = hist[(size_t)b * NKEYS + k];
+        hist[(size_t)b * NKEYS + k] = run;
+        run += c;
     }
-    if (lane == 0) total[k] = run;
 }
 
 // Each item's slot in the traced order: the keys' starts (an exclusive scan of
@@ -204,7 +204,7 @@ static cudaError_t sort_order(const vox_cuda_tree *t, const float *o, const floa
         f.inv[a] = cells / fmaxf(t->bbox[3 + a] - t->bbox[a], 1e-30f);
     }
     k_keys<<<(unsigned)nb, SORT_THREADS, 0, s>>>(o, d, n, per, f, keys, hist);
-    k_key_blocks<<<NKEYS / 8, 256, 0, s>>>(hist, (uint32_t)nb, total);
+    k_key_blocks<<<NKEYS / 32, 1024, 0, s>>>(hist, (uint32_t)nb, total);
     k_place<<<(unsigned)nb, SORT_THREADS, 0, s>>>(keys, n, per, hist, total, *order);
     for (int i = 0; i < 3; i++) count_launch();
     return cudaGetLastError();
