@@ -120,7 +120,8 @@ __device__ __forceinline__ void run_tile(const BatchJobDev &J, uint32_t local, u
 }
 
 // The `c`-th clearing item of frame J: CLEAR_ROWS rows, the parts outside
-// the traced rectangle.
+// the traced rectangle, stored past the trees in L2 (streaming stores; 32 frames
+// 1,314 -> 1,306 us; of the traced pixels as well, 1,322).
 __device__ __forceinline__ void run_clear(const BatchJobDev &J, uint32_t c, uint32_t lane)
 {
     const uint32_t w = J.w, y0r = c * CLEAR_ROWS;
@@ -132,8 +133,8 @@ __device__ __forceinline__ void run_clear(const BatchJobDev &J, uint32_t c, uint
         if (y >= J.y0 && y < J.y1) { b0 = J.x0; a1 = J.x1; b1 = w; }
         if (vec) {
             uint4 *r4 = reinterpret_cast<uint4 *>(row);
-            for (uint32_t i = a0 / 4 + lane; i < b0 / 4; i += 32) r4[i] = make_uint4(0u, 0u, 0u, 0u);
-            for (uint32_t i = a1 / 4 + lane; i < b1 / 4; i += 32) r4[i] = make_uint4(0u, 0u, 0u, 0u);
+            for (uint32_t i = a0 / 4 + lane; i < b0 / 4; i += 32) __stcs(r4 + i, make_uint4(0u, 0u, 0u, 0u));
+            for (uint32_t i = a1 / 4 + lane; i < b1 / 4; i += 32) __stcs(r4 + i, make_uint4(0u, 0u, 0u, 0u));
         } else {
             for (uint32_t i = a0 + lane; i < b0; i += 32) row[i] = 0u;
             for (uint32_t i = a1 + lane; i < b1; i += 32) row[i] = 0u;

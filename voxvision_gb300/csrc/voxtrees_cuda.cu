@@ -202,7 +202,8 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // clearing rectangle of the plan outside the traced one, rows dealt to the
 // block's warps; a warp's lanes store 16 bytes each when the frame is 16-byte
 // aligned (row starts and every bound then are: w is a multiple of 16, the
-// rectangles' x bounds of 8 or w).
+// rectangles' x bounds of 8 or w), past the tree in L2 (streaming stores: a 1080p
+// orbit frame 61.5 -> 59.7 us back to back, 89 -> 86 alone).
 __device__ __forceinline__ void clear_outside(const FramePlan &p, uint32_t w, uint32_t h, uint32_t *argb,
                                               uint32_t warp, uint32_t lane)
 {
@@ -218,8 +219,8 @@ __device__ __forceinline__ void clear_outside(const FramePlan &p, uint32_t w, ui
         }
         if (vec) {
             uint4 *r4 = reinterpret_cast<uint4 *>(row);
-            for (uint32_t i = a0 / 4 + lane; i < b0 / 4; i += 32) r4[i] = make_uint4(0u, 0u, 0u, 0u);
-            for (uint32_t i = a1 / 4 + lane; i < b1 / 4; i += 32) r4[i] = make_uint4(0u, 0u, 0u, 0u);
+            for (uint32_t i = a0 / 4 + lane; i < b0 / 4; i += 32) __stcs(r4 + i, make_uint4(0u, 0u, 0u, 0u));
+            for (uint32_t i = a1 / 4 + lane; i < b1 / 4; i += 32) __stcs(r4 + i, make_uint4(0u, 0u, 0u, 0u));
         } else {
             for (uint32_t i = a0 + lane; i < b0; i += 32) row[i] = 0u;
             for (uint32_t i = a1 + lane; i < b1; i += 32) row[i] = 0u;
