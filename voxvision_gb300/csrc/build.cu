@@ -109,6 +109,20 @@ __device__ __forceinline__ void after_previous()
     asm volatile("griddepcontrol.launch_dependents;");
 }
 
+// The kernels of a level's size classes need nothing of one another: only the
+// first waits before its work, the others after theirs (so that none is
+// complete before its predecessors), and each level's few large nodes run
+// beside its many small ones.
+__device__ __forceinline__ void class_begin(bool first)
+{
+    if (first) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+__device__ __forceinline__ void class_end(bool first)
+{
+    if (!first) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 template <class... K, class... A>
 void launch_after(void (*kern)(K...), unsigned grid, unsigned block, cudaStream_t s, A... args)
 {
@@ -559,7 +573,7 @@ __global__ void __launch_bounds__(NODE_THREADS) k_centre_plain(Level L, NodeList
 {
     after_previous();
     __shared__ PlainSum part[NODE_THREADS / 32];
-    __shared__ double wsum[NODE_THREADS / 32], carry;
+    __shared__ float wsum[NODE_THREADS / 32], carry;
     if (blockIdx.x >= (uint32_t)(*lists.ntiled >> 32)) return;
     const uint32_t k = lists.tiled[blockIdx.x], nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK,
                    c0 = lists.first_tile[blockIdx.x] * (lists.tile / CHUNK);
@@ -582,27 +596,29 @@ __global__ void __launch_bounds__(NODE_THREADS) k_centre_plain(Level L, NodeList
             continue;
         }
         const int top = max(1, min(254, L.ehi[3 * k + a] + 150 - (window - 1)));
-        const double limit = ldexp(1.0, x.g[a] + 24);
+        const float limit = ldexpf(1.0f, x.g[a] + 24);   // (below it float sums are exact)
         if (threadIdx.x == 0) starts[3 * blockIdx.x + a] = make_uint2(0u, 0u);
         __syncthreads();   // the axis before may still set it
-        if (threadIdx.x == 0) carry = 0.0;
+        if (threadIdx.x == 0) carry = 0.0f;
         for (uint32_t j0 = 0; j0 < nch; j0 += NODE_THREADS) {
             const uint32_t j = j0 + threadIdx.x;
-            const double d = j < nch ? (double)csum[3 * (c0 + j) + a] : 0.0;
-            double s = d;
+            const float d = j < nch ? csum[3 * (c0 + j) + a] : 0.0f;
+            float s = d;
             for (int off = 1; off < 32; off <<= 1) {
-                const double y = __shfl_up_sync(0xffffffffu, s, off);
+                const float y = __shfl_up_sync(0xffffffffu, s, off);
                 if (lane >= (uint32_t)off) s += y;
             }
             if (lane == 31) wsum[warp] = s;
             __syncthreads();
-            double before = carry + s - d;
+            float before = __shfl_up_sync(0xffffffffu, s, 1);
+            before = lane ? before : 0.0f;
             for (uint32_t w = 0; w < warp; w++) before += wsum[w];
+            before += carry;
             if (j < nch) {
-                const uint32_t e = __float_as_uint((float)(before * (63.0 / 64.0))) >> 23;
+                const uint32_t e = __float_as_uint(before * (63.0f / 64.0f)) >> 23;
                 cbase[3 * (c0 + j) + a] = (uint8_t)(window > 2 ? (uint32_t)top : max(1u, min(e, 253u)));
                 if (before < limit && before + d >= limit)
-                    starts[3 * blockIdx.x + a] = make_uint2(j, __float_as_uint((float)before));
+                    starts[3 * blockIdx.x + a] = make_uint2(j, __float_as_uint(before));
             }
             __syncthreads();
             if (threadIdx.x == NODE_THREADS - 1) carry = before + d;
@@ -954,11 +970,9 @@ __device__ __forceinline__ float unordered(uint32_t u)
 // 291 us with a warp on every pass, 160 like this.
 constexpr int LANE_WARPS = 4;
 template <uint32_t MOST>
-__global__ void __launch_bounds__(LANE_WARPS * 32) k_nodes_lanes(Level L, const uint32_t *list, const uint32_t *count,
-                                                                 const float *P, float *Pn, float vx, float vy, float vz,
-                                                                 Tally tally)
+__device__ __forceinline__ void nodes_lanes(const Level &L, const uint32_t *list, const uint32_t *count, const float *P,
+                                            float *Pn, float vx, float vy, float vz, const Tally &tally)
 {
-    after_previous();
     static_assert(MOST % 32 == 0 && MOST <= 128, "octants are counted in bytes");
     constexpr uint32_t FULL = 0xffffffffu, J = MOST / 32;
     __shared__ uint16_t columns[LANE_WARPS][MOST][32];   // per voxel of 32 nodes {octant, place in the node}
@@ -1079,14 +1093,22 @@ __global__ void __launch_bounds__(LANE_WARPS * 32) k_nodes_lanes(Level L, const 
     mine.flush(tally);
 }
 
+template <uint32_t MOST>
+__global__ void __launch_bounds__(LANE_WARPS * 32) k_nodes_lanes(Level L, const uint32_t *list, const uint32_t *count,
+                                                                 const float *P, float *Pn, float vx, float vy, float vz,
+                                                                 Tally tally, bool first)
+{
+    class_begin(first);
+    nodes_lanes<MOST>(L, list, count, P, Pn, vx, vy, vz, tally);
+    class_end(first);
+}
+
 // Nodes of at most MOST voxels: a block of THREADS each, as above, a voxel in
 // 16 bits {octant, place in the node}.
 template <int THREADS, uint32_t MOST>
-__global__ void __launch_bounds__(THREADS) k_nodes_block(Level L, const uint32_t *list, const uint32_t *count,
-                                                         const float *P, float *Pn, float vx, float vy, float vz,
-                                                         Tally tally)
+__device__ __forceinline__ void nodes_block(const Level &L, const uint32_t *list, const uint32_t *count, const float *P,
+                                            float *Pn, float vx, float vy, float vz, const Tally &tally)
 {
-    after_previous();
     static_assert(MOST <= 8192 && MOST % 1024 == 0, "13 bits of place; whole words a lane in scan_words");
     constexpr int WARPS = THREADS / 32;
     static_assert(WARPS >= 3 && WARPS <= 32, "an axis a warp");
@@ -1186,6 +1208,16 @@ __global__ void __launch_bounds__(THREADS) k_nodes_block(Level L, const uint32_t
         if (lane == 0 && m) L.first_child[k] = atomicAdd(tally.children, (uint32_t)__popc(m));
         mine.flush(tally);
     }
+}
+
+template <int THREADS, uint32_t MOST>
+__global__ void __launch_bounds__(THREADS) k_nodes_block(Level L, const uint32_t *list, const uint32_t *count,
+                                                         const float *P, float *Pn, float vx, float vy, float vz,
+                                                         Tally tally, bool first)
+{
+    class_begin(first);
+    nodes_block<THREADS, MOST>(L, list, count, P, Pn, vx, vy, vz, tally);
+    class_end(first);
 }
 
 // Larger nodes, tile by tile: a launch a pass, a block a tile of one node.
@@ -1803,19 +1835,27 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
             }
             launch_after(k_finish_tiled, grid_for(max_tiled * 32, 256), 256, s, L, lists, tally);
         }
+        bool first = true;   // of the size classes that are made whole
         if (largest > LOW) {
-            launch_after(k_nodes_block<512, MID>, (unsigned)std::min<uint64_t>(m, max_mid), 512, s, L, lists.mid, lists.nmid, Pc, Pn, vx, vy, vz, tally);
+            launch_after(k_nodes_block<512, MID>, (unsigned)std::min<uint64_t>(m, max_mid), 512, s, L, lists.mid, lists.nmid,
+                         Pc, Pn, vx, vy, vz, tally, first);
+            first = false;
         }
         if (largest > SMALL) {
-            launch_after(k_nodes_block<128, LOW>, (unsigned)std::min<uint64_t>(m, max_low), 128, s, L, lists.low, lists.nlow, Pc, Pn, vx, vy, vz, tally);
+            launch_after(k_nodes_block<128, LOW>, (unsigned)std::min<uint64_t>(m, max_low), 128, s, L, lists.low, lists.nlow,
+                         Pc, Pn, vx, vy, vz, tally, first);
+            first = false;
         }
         if (largest > TINY) {
             const unsigned blocks = grid_for(std::min<uint64_t>(m, N / (TINY + 1) + 1), LANE_WARPS);
-            launch_after(k_nodes_lanes<SMALL>, std::min(blocks, (unsigned)(nsm * 5)), LANE_WARPS * 32, s, L, lists.small, lists.nsmall, Pc, Pn, vx, vy, vz, tally);
+            launch_after(k_nodes_lanes<SMALL>, std::min(blocks, (unsigned)(nsm * 5)), LANE_WARPS * 32, s, L, lists.small,
+                         lists.nsmall, Pc, Pn, vx, vy, vz, tally, first);
+            first = false;
         }
         if (largest > VOX_MAX_DOTS) {
             const unsigned blocks = grid_for(std::min<uint64_t>(m, N / (VOX_MAX_DOTS + 1) + 1), LANE_WARPS);
-            launch_after(k_nodes_lanes<TINY>, std::min(blocks, (unsigned)(nsm * 8)), LANE_WARPS * 32, s, L, lists.tiny, lists.ntiny, Pc, Pn, vx, vy, vz, tally);
+            launch_after(k_nodes_lanes<TINY>, std::min(blocks, (unsigned)(nsm * 8)), LANE_WARPS * 32, s, L, lists.tiny,
+                         lists.ntiny, Pc, Pn, vx, vy, vz, tally, first);
         }
         TRY(cudaGetLastError());
         TRY(cudaMemcpyAsync(back->next, scal + 2, 8, cudaMemcpyDeviceToHost, s));
