@@ -1405,6 +1405,29 @@ __global__ void k_finish_tiled(Level L, NodeLists lists, Tally tally)
     mine.flush(tally);
 }
 
+// The set into the first level's order; *odd is set when a coordinate is not
+// finite or above LIMIT in magnitude.
+constexpr float LIMIT = 1.4411518807585587e17f;   // 2^57
+__global__ void __launch_bounds__(256) k_copy_set(const float *__restrict__ set, float *__restrict__ P, uint64_t n,
+                                                  uint32_t *odd)
+{
+    after_previous();
+    const uint64_t i0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    bool fine = true;
+    if (i0 + 4 <= n && (reinterpret_cast<uintptr_t>(set) & 15u) == 0) {
+        const float4 v = *reinterpret_cast<const float4 *>(set + i0);
+        fine = fabsf(v.x) <= LIMIT && fabsf(v.y) <= LIMIT && fabsf(v.z) <= LIMIT && fabsf(v.w) <= LIMIT;
+        *reinterpret_cast<float4 *>(P + i0) = v;
+    } else {
+        for (uint64_t i = i0; i < n && i < i0 + 4; i++) {
+            const float v = set[i];
+            fine = fine && fabsf(v) <= LIMIT;
+            P[i] = v;
+        }
+    }
+    if (__any_sync(0xffffffffu, !fine) && (threadIdx.x & 31) == 0) *odd = 1u;
+}
+
 // A new node of n voxels from position s0 on (n 0: none; every thread of the
 // warp calls): made here when it has at most VOX_MAX_DOTS voxels (a leaf, or
 // dense), else put on the list of its class.
@@ -1753,7 +1776,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     TRY(d.get(&P[1], 3 * N));
     TRY(d.get(&stats, NSTATS * (MAX_LEVELS + 1)));
     // scal: 0 tiny nodes, 1 mid nodes, 2 children, 3 largest child, 4 low, 5 small, 6-7 tiled nodes and tiles,
-    // 8 error bits
+    // 8 error bits, 9 whether a coordinate is out of the ordinary
     TRY(d.get(&scal, 12));
     uint32_t *err = scal + 8;
     NodeLists lists{};
@@ -1791,14 +1814,14 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     }
     TRY(cudaMemsetAsync(scal, 0, 12 * 4, s));
     TRY(cudaMemsetAsync(stats, 0, NSTATS * (MAX_LEVELS + 1) * sizeof(unsigned long long), s));
-    TRY(cudaMemcpyAsync(P[0], d_set, 12 * N, cudaMemcpyDeviceToDevice, s));
+    launch_after(k_copy_set, grid_for(3 * N, 1024), 256, s, d_set, P[0], 3 * N, scal + 9);
 
     int dev = 0, nsm = 0;
     TRY(cudaGetDevice(&dev));
     TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     // what comes back to the host, in page-locked memory
     struct Back {
-        uint32_t next[2], root_nodes, err, unshaped;
+        uint32_t next[2], root_nodes, err, odd, unshaped;
         float box[6];
         unsigned long long units, stats[NSTATS * MAX_LEVELS];
     };
@@ -1879,7 +1902,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     }
     TRY(cudaMemcpyAsync(back->stats, stats, sizeof back->stats, cudaMemcpyDeviceToHost, s));
     TRY(cudaMemcpyAsync(&back->root_nodes, levels[0].sub_nodes, 4, cudaMemcpyDeviceToHost, s));
-    TRY(cudaMemcpyAsync(&back->err, err, 4, cudaMemcpyDeviceToHost, s));
+    TRY(cudaMemcpyAsync(&back->err, err, 8, cudaMemcpyDeviceToHost, s));
     TRY(cudaMemcpyAsync(&back->units, levels[0].sub_units, 8, cudaMemcpyDeviceToHost, s));
     TRY(cudaMemcpyAsync(back->box, levels[0].box, 24, cudaMemcpyDeviceToHost, s));
     TRY(cudaStreamSynchronize(s));
@@ -1926,8 +1949,16 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     }
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(&back->err, err, 4, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = image_shape(pool, map, nodes, st.voxel, scal, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&back->unshaped, scal, 4, cudaMemcpyDeviceToHost, s);
+    // A tree made here of ordinary voxels has every property the searches may
+    // rely on: boxes are least boxes of their voxels (min <= max as the voxel
+    // size is positive), children's voxels lie on their side of the dividing
+    // planes, and no centre passes 2^60.  Any other is looked over.
+    const auto ordinary = [](float v) { return v >= 8.67e-19f && v <= LIMIT; };   // 2^-60
+    back->unshaped = 0;
+    if (back->odd || !ordinary(vx) || !ordinary(vy) || !ordinary(vz)) {
+        if (e == cudaSuccess) e = image_shape(pool, map, nodes, st.voxel, scal, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&back->unshaped, scal, 4, cudaMemcpyDeviceToHost, s);
+    }
     if (x) {
         x->dots_of_id.resize(nodes);
         if (e == cudaSuccess && x->order)
