@@ -51,7 +51,7 @@ def _set(kind, n, seed):
 
 @pytest.mark.parametrize("kind", ["scattered", "raster", "rounding", "duplicates"])
 @pytest.mark.parametrize("n", [1, 7, 8, 31, 32, 33, 64, 65, 511, 512, 513, 1024, 1025, 1056, 8191, 8192, 8193, 9216,
-                               17409, 60000])
+                               17409, 32768, 32769, 60000])
 def test_sizes_at_class_edges(vg, kind, n):
     vox = _set(kind, n, n)
     _same(vg, vox, vg.DeviceTree.build(vox))

@@ -80,7 +80,8 @@ constexpr uint32_t RAW_TILE = RAW_THREADS * RAW_ITEMS;   // samples a block read
 constexpr uint32_t TINY = 32;        // nodes with at most this many voxels, and
 constexpr uint32_t SMALL = 128;      // with at most this many, are split by a lane each,
 constexpr uint32_t LOW = 1024;       // with at most this many by a block of 128 threads,
-constexpr uint32_t MID = 8192;       // with at most this many by a block of 512, larger ones tile by tile
+constexpr uint32_t MID = 8192;       // with at most this many by a block of 512, and
+constexpr uint32_t HIGH = 32768;     // with at most this many by a block of 1024, larger ones tile by tile
 constexpr uint32_t CHUNK = 1024;     // voxels per chunk
 constexpr int CHUNK_THREADS = 128;   // 8 consecutive voxels per thread
 constexpr int NBIN = 16;             // binades with a precomputed map per chunk
@@ -124,11 +125,12 @@ __device__ __forceinline__ void class_end(bool first)
 }
 
 template <class... K, class... A>
-void launch_after(void (*kern)(K...), unsigned grid, unsigned block, cudaStream_t s, A... args)
+void launch_after_with(size_t shared, void (*kern)(K...), unsigned grid, unsigned block, cudaStream_t s, A... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = shared;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -137,6 +139,12 @@ void launch_after(void (*kern)(K...), unsigned grid, unsigned block, cudaStream_
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kern, K(args)...);   // errors: cudaGetLastError
     count_launch();
+}
+
+template <class... K, class... A>
+void launch_after(void (*kern)(K...), unsigned grid, unsigned block, cudaStream_t s, A... args)
+{
+    launch_after_with(0, kern, grid, block, s, args...);
 }
 
 inline unsigned grid_for(uint64_t n, unsigned threads) { return (unsigned)((n + threads - 1) / threads); }
@@ -237,19 +245,21 @@ cudaError_t level_alloc(Level &L, uint32_t m, cudaStream_t s)
 // -------------------------------------------------------- per-level kernels
 
 // The nodes of a level that take more than one thread, by size class, in no
-// particular order (above VOX_MAX_DOTS, TINY, SMALL, LOW and MID voxels).  A tiled node's slot and its first tile come
+// particular order (above VOX_MAX_DOTS, TINY, SMALL, LOW, MID and HIGH voxels).  A tiled node's slot and its first tile come
 // from one counter, so that first tiles ascend with slots.
 struct NodeLists {
-    uint32_t *tiny, *small, *low, *mid, *tiled, *first_tile;
-    uint32_t *ntiny, *nsmall, *nlow, *nmid;
+    uint32_t *tiny, *small, *low, *mid, *high, *tiled, *first_tile;
+    uint32_t *ntiny, *nsmall, *nlow, *nmid, *nhigh;
     unsigned long long *ntiled;   // slots in the upper half, tiles in the lower
     uint32_t tile;                // positions per tile
     __device__ void add_large(uint32_t k, uint32_t n) const
     {
-        if (n > MID) {
+        if (n > HIGH) {
             const unsigned long long at = atomicAdd(ntiled, (1ull << 32) | ((n + tile - 1) / tile));
             tiled[at >> 32] = k;
             first_tile[at >> 32] = (uint32_t)at;
+        } else if (n > MID) {
+            high[atomicAdd(nhigh, 1u)] = k;
         } else if (n > LOW) {
             mid[atomicAdd(nmid, 1u)] = k;
         } else if (n > SMALL) {
@@ -1104,16 +1114,43 @@ __global__ void __launch_bounds__(LANE_WARPS * 32) k_nodes_lanes(Level L, const 
 }
 
 // Nodes of at most MOST voxels: a block of THREADS each, as above, a voxel in
-// 16 bits {octant, place in the node}.
+// 16 bits {octant, place in the node}, or above 8,192 voxels in 24.  (A level
+// of 64 nodes of 21,000 tile by tile is eighteen launches, 210 us; by a block
+// each the raw volume's 1,600 us become 1,566, a build of 13.8 M voxels 13.0 ms
+// 11.5.)
+template <uint32_t MOST, bool WIDE = (MOST > 8192)>
+struct NodeBuffer {                      // two orders of a node's voxels
+    uint16_t v[2][MOST];
+    __device__ void set(uint32_t i, uint32_t o) { v[0][i] = (uint16_t)((o << 13) | i); }
+    __device__ uint32_t oct(uint32_t b, uint32_t t) const { return v[b][t] >> 13; }
+    __device__ uint32_t place(uint32_t b, uint32_t t) const { return v[b][t] & 8191u; }
+    __device__ void move(uint32_t b, uint32_t t, uint32_t s) { v[b ^ 1][t] = v[b][s]; }
+};
+template <uint32_t MOST>
+struct NodeBuffer<MOST, true> {
+    uint16_t v[2][MOST];
+    uint8_t q[2][MOST];
+    __device__ void set(uint32_t i, uint32_t o) { v[0][i] = (uint16_t)i; q[0][i] = (uint8_t)o; }
+    __device__ uint32_t oct(uint32_t b, uint32_t t) const { return q[b][t]; }
+    __device__ uint32_t place(uint32_t b, uint32_t t) const { return v[b][t]; }
+    __device__ void move(uint32_t b, uint32_t t, uint32_t s) { v[b ^ 1][t] = v[b][s]; q[b ^ 1][t] = q[b][s]; }
+};
+template <uint32_t MOST>
+struct NodeShared {
+    NodeBuffer<MOST> buf;
+    uint32_t mask[MOST / 32], before[MOST / 32], last[MOST / 32];
+};
 template <int THREADS, uint32_t MOST>
 __device__ __forceinline__ void nodes_block(const Level &L, const uint32_t *list, const uint32_t *count, const float *P,
                                             float *Pn, float vx, float vy, float vz, const Tally &tally)
 {
-    static_assert(MOST <= 8192 && MOST % 1024 == 0, "13 bits of place; whole words a lane in scan_words");
+    static_assert(MOST <= 65536 && MOST % 1024 == 0, "16 bits of place; whole words a lane in scan_words");
     constexpr int WARPS = THREADS / 32;
     static_assert(WARPS >= 3 && WARPS <= 32, "an axis a warp");
-    __shared__ uint16_t buf[2][MOST];
-    __shared__ uint32_t mask[MOST / 32], before[MOST / 32], last[MOST / 32], total, s_kind;
+    extern __shared__ __align__(16) unsigned char dynamic[];
+    NodeShared<MOST> &w = *reinterpret_cast<NodeShared<MOST> *>(dynamic);
+    uint32_t *const mask = w.mask, *const before = w.before, *const last = w.last;
+    __shared__ uint32_t total, s_kind;
     __shared__ Extremes epart[WARPS];
     __shared__ PlainSum spart[WARPS];
     __shared__ float centre[3];
@@ -1159,46 +1196,46 @@ __device__ __forceinline__ void nodes_block(const Level &L, const uint32_t *list
     }
     for (uint32_t i = threadIdx.x; i < n; i += THREADS) {
         const float p[3] = {P[3 * (s0 + i)], P[3 * (s0 + i) + 1], P[3 * (s0 + i) + 2]};
-        buf[0][i] = (uint16_t)((octant(centre, p) << 13) | i);
+        w.buf.set(i, octant(centre, p));
     }
     const uint32_t nw = (n + 31) / 32;
     uint32_t from = 0, cnt = 0;     // lane o of warp 0 holds octant o's count
     for (uint32_t o = 0; o < 8 && from < n; o++) {
-        const uint16_t *in = buf[o & 1];
-        uint16_t *out = buf[(o & 1) ^ 1];
+        const uint32_t in = o & 1;
         __syncthreads();
-        for (uint32_t w = (from >> 5) + warp; w < nw; w += WARPS) {
-            const uint32_t t = (w << 5) + lane;
+        for (uint32_t i = (from >> 5) + warp; i < nw; i += WARPS) {
+            const uint32_t t = (i << 5) + lane;
             const bool range = t >= from && t < n;
-            const bool cl = range && (uint32_t)(in[t] >> 13) == o;
+            const bool cl = range && w.buf.oct(in, t) == o;
             const uint32_t m = __ballot_sync(0xffffffffu, cl), u = __ballot_sync(0xffffffffu, range && !cl);
             if (lane == 0) {
-                mask[w] = m;
-                before[w] = (uint32_t)__popc(m);
-                last[w] = u ? (w << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
+                mask[i] = m;
+                before[i] = (uint32_t)__popc(m);
+                last[i] = u ? (i << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
             }
         }
         __syncthreads();
         if (warp == 0) {
-            const uint32_t w0 = from >> 5;
+            constexpr uint32_t PER = MOST / 1024 < 8 ? MOST / 1024 : 8;
             uint32_t run = 0, prev = NO_POS;
-            scan_words<MOST / 32 / 32>(before + w0, last + w0, nw - w0, run, prev);
+            for (uint32_t i = from >> 5; i < nw; i += 32 * PER)
+                scan_words<PER>(before + i, last + i, min(nw - i, 32 * PER), run, prev);
             if (lane == 0) total = run;
             if (lane == o) cnt = run;
         }
         __syncthreads();
         const uint32_t rest = from + total;
         auto claimed = [&](uint32_t s, uint32_t &c, uint32_t &l) {
-            const uint32_t w = s >> 5, i = s & 31, m = mask[w];
-            c = before[w] + (uint32_t)__popc(m & lanes_below(i));
-            l = last_in_word(w, i, m, from);
-            if (l == NO_POS) l = last[w];
-            return ((m >> i) & 1u) != 0u;
+            const uint32_t i = s >> 5, b = s & 31, m = mask[i];
+            c = before[i] + (uint32_t)__popc(m & lanes_below(b));
+            l = last_in_word(i, b, m, from);
+            if (l == NO_POS) l = last[i];
+            return ((m >> b) & 1u) != 0u;
         };
         for (uint32_t t = from + threadIdx.x; t < n; t += THREADS) {
             uint32_t c, l;
-            if (claimed(t, c, l)) place(P, Pn, s0 + from + c, s0 + (in[t] & 8191u));
-            if (t >= rest) out[t] = in[walk_back(t, from, MOST, claimed, tally.err)];
+            if (claimed(t, c, l)) place(P, Pn, s0 + from + c, s0 + w.buf.place(in, t));
+            if (t >= rest) w.buf.move(in, t, walk_back(t, from, MOST, claimed, tally.err));
         }
         from = rest;
     }
@@ -1775,27 +1812,29 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     TRY(d.get(&P[0], 3 * N));
     TRY(d.get(&P[1], 3 * N));
     TRY(d.get(&stats, NSTATS * (MAX_LEVELS + 1)));
-    // scal: 0 tiny nodes, 1 mid nodes, 2 children, 3 largest child, 4 low, 5 small, 6-7 tiled nodes and tiles,
-    // 8 error bits, 9 whether a coordinate is out of the ordinary
+    // scal: the level's tiny, small, children, largest child, low, mid, tiled nodes and tiles (6-7), high (8);
+    // 10 error bits, 11 whether a coordinate is out of the ordinary
     TRY(d.get(&scal, 12));
-    uint32_t *err = scal + 8;
+    uint32_t *err = scal + 10;
     NodeLists lists{};
     lists.ntiny = scal;
-    lists.nsmall = scal + 5;
-    lists.nmid = scal + 1;
+    lists.nsmall = scal + 1;
     lists.nlow = scal + 4;
+    lists.nmid = scal + 5;
+    lists.nhigh = scal + 8;
     lists.ntiled = reinterpret_cast<unsigned long long *>(scal + 6);
     lists.tile = SUB * (uint32_t)((N + (uint64_t)SUB * MAX_TILES - 1) / ((uint64_t)SUB * MAX_TILES));
-    const uint64_t max_low = N / SMALL, max_mid = N / LOW, max_tiled = N / MID, max_tiles = N / lists.tile + max_tiled,
+    const uint64_t max_low = N / SMALL, max_mid = N / LOW, max_high = N / MID, max_tiled = N / HIGH, max_tiles = N / lists.tile + max_tiled,
                    max_chunks = max_tiles * (lists.tile / CHUNK);
     TRY(d.get(&lists.tiny, N / (VOX_MAX_DOTS + 1) + 1));
     TRY(d.get(&lists.small, N / (TINY + 1) + 1));
     TRY(d.get(&lists.low, max_low + 1));
     TRY(d.get(&lists.mid, max_mid + 1));
+    TRY(d.get(&lists.high, max_high + 1));
     // past 2^24 additions a sum's roundings can add up to a sizeable part of it
     const int window = N > (1u << 24) ? NBIN : 2;
     Marks marks[2] = {};
-    if (N > MID) {
+    if (N > HIGH) {
         for (int i = 0; i < 2; i++) {
             TRY(d.get(&idx[i], N));
             TRY(d.get(&oct[i], N));
@@ -1814,7 +1853,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     }
     TRY(cudaMemsetAsync(scal, 0, 12 * 4, s));
     TRY(cudaMemsetAsync(stats, 0, NSTATS * (MAX_LEVELS + 1) * sizeof(unsigned long long), s));
-    launch_after(k_copy_set, grid_for(3 * N, 1024), 256, s, d_set, P[0], 3 * N, scal + 9);
+    launch_after(k_copy_set, grid_for(3 * N, 1024), 256, s, d_set, P[0], 3 * N, scal + 11);
 
     int dev = 0, nsm = 0;
     TRY(cudaGetDevice(&dev));
@@ -1842,7 +1881,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         const float *Pc = P[lv & 1];
         float *Pn = P[(lv & 1) ^ 1];
         const Tally tally{stats + NSTATS * lv, scal + 2, scal + 3, err};
-        if (largest > MID) {
+        if (largest > HIGH) {
             // boxes, centres and the eight swapping passes of the largest nodes
             const unsigned nt = (unsigned)max_tiled, nc = (unsigned)max_chunks, np = (unsigned)max_tiles;
             launch_after(k_chunk_box, nc, CHUNK_THREADS, s, Pc, L, lists, cv, cidx);
@@ -1859,14 +1898,21 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
             launch_after(k_finish_tiled, grid_for(max_tiled * 32, 256), 256, s, L, lists, tally);
         }
         bool first = true;   // of the size classes that are made whole
+        if (largest > MID) {
+            TRY(cudaFuncSetAttribute(k_nodes_block<1024, HIGH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(NodeShared<HIGH>)));
+            launch_after_with(sizeof(NodeShared<HIGH>), k_nodes_block<1024, HIGH>, (unsigned)std::min<uint64_t>(m, max_high),
+                              1024, s, L, lists.high, lists.nhigh, Pc, Pn, vx, vy, vz, tally, first);
+            first = false;
+        }
         if (largest > LOW) {
-            launch_after(k_nodes_block<512, MID>, (unsigned)std::min<uint64_t>(m, max_mid), 512, s, L, lists.mid, lists.nmid,
-                         Pc, Pn, vx, vy, vz, tally, first);
+            launch_after_with(sizeof(NodeShared<MID>), k_nodes_block<512, MID>, (unsigned)std::min<uint64_t>(m, max_mid), 512, s,
+                              L, lists.mid, lists.nmid, Pc, Pn, vx, vy, vz, tally, first);
             first = false;
         }
         if (largest > SMALL) {
-            launch_after(k_nodes_block<128, LOW>, (unsigned)std::min<uint64_t>(m, max_low), 128, s, L, lists.low, lists.nlow,
-                         Pc, Pn, vx, vy, vz, tally, first);
+            launch_after_with(sizeof(NodeShared<LOW>), k_nodes_block<128, LOW>, (unsigned)std::min<uint64_t>(m, max_low), 128, s,
+                              L, lists.low, lists.nlow, Pc, Pn, vx, vy, vz, tally, first);
             first = false;
         }
         if (largest > TINY) {
@@ -1889,7 +1935,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         Level Nx;
         TRY(level_alloc(Nx, mn, s));
         levels.push_back(Nx);
-        TRY(cudaMemsetAsync(scal, 0, 8 * 4, s));
+        TRY(cudaMemsetAsync(scal, 0, 9 * 4, s));
         launch_after(k_children, grid_for((uint64_t)m * 8, CHILD_THREADS), CHILD_THREADS, s, L, Nx, lists, Pn, vx, vy, vz, stats + NSTATS * (lv + 1));
     }
 
