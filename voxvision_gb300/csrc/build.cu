@@ -1672,6 +1672,62 @@ __global__ void k_final_order(Level L, const float *P, float *order)
     for (uint64_t i = b + lane; i < e; i += 32) order[i] = P[i];
 }
 
+// --------------------------------------------------------- host's page
+
+// What comes back to the host while it builds, in page-locked memory: kernels
+// write it there, and `step` last.
+struct Back {
+    uint32_t next[2], root_nodes, err, odd, unshaped, step;
+    float box[6];
+    unsigned long long units, stats[NSTATS * MAX_LEVELS];
+};
+static_assert(sizeof(Back) <= THREAD_PAGE, "the counts of every level fit the thread's page");
+
+// A level is split: the next one's nodes and the largest of them, and the
+// level's counters zeroed.  The host sees them as soon as they are stored; with
+// a copy, a wait for the stream and a memset a level the 256^3 raw volume with
+// a first frame took 1,570 us, with this 1,496.
+__global__ void k_level_done(uint32_t *scal, Back *back, uint32_t step)
+{
+    after_previous();
+    back->next[0] = scal[2];
+    back->next[1] = scal[3];
+    for (int i = 0; i < 9; i++) scal[i] = 0;
+    __threadfence_system();
+    *static_cast<volatile uint32_t *>(&back->step) = step;
+}
+
+// The tree is split: every level's counts, and the image's size.
+__global__ void __launch_bounds__(128) k_all_done(Level root, const unsigned long long *stats, const uint32_t *err, Back *back, uint32_t step)
+{
+    after_previous();
+    for (int i = threadIdx.x; i < NSTATS * MAX_LEVELS; i += 128) back->stats[i] = stats[i];
+    if (threadIdx.x < 6) back->box[threadIdx.x] = root.box[threadIdx.x];
+    if (threadIdx.x == 0) {
+        back->root_nodes = root.sub_nodes[0];
+        back->units = root.sub_units[0];
+        back->err = err[0];
+        back->odd = err[1];
+    }
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) *static_cast<volatile uint32_t *>(&back->step) = step;
+}
+
+// Waits for `step` from the stream's kernels; an error when they end without it.
+cudaError_t wait_step(const Back *back, uint32_t step, cudaStream_t s)
+{
+    for (uint32_t spin = 1;; spin++) {
+        if (__atomic_load_n(&back->step, __ATOMIC_ACQUIRE) == step) return cudaSuccess;
+        if (spin % 1024 == 0) {
+            const cudaError_t e = cudaStreamQuery(s);
+            if (e == cudaErrorNotReady) continue;
+            if (e != cudaSuccess) return e;
+            return __atomic_load_n(&back->step, __ATOMIC_ACQUIRE) == step ? cudaSuccess : cudaErrorUnknown;
+        }
+    }
+}
+
 // ------------------------------------------------------------ raw reader
 
 // Which samples are solid (datareader.c:51-77): 16 consecutive ones a thread,
@@ -1858,15 +1914,13 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     int dev = 0, nsm = 0;
     TRY(cudaGetDevice(&dev));
     TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    // what comes back to the host, in page-locked memory
-    struct Back {
-        uint32_t next[2], root_nodes, err, odd, unshaped;
-        float box[6];
-        unsigned long long units, stats[NSTATS * MAX_LEVELS];
-    };
-    static_assert(sizeof(Back) <= THREAD_PAGE, "the counts of every level fit the thread's page");
     Back *back = static_cast<Back *>(thread_page());
     if (!back) return VOX_CUDA_ENOMEM;
+    void *back_dev = nullptr;
+    TRY(cudaHostGetDevicePointer(&back_dev, back, 0));
+    Back *back_d = static_cast<Back *>(back_dev);
+    back->step = 0;
+    uint32_t step = 0;
 
     Level root;
     TRY(level_alloc(root, 1, s));
@@ -1926,16 +1980,15 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
             launch_after(k_nodes_lanes<TINY>, std::min(blocks, (unsigned)(nsm * 8)), LANE_WARPS * 32, s, L, lists.tiny,
                          lists.ntiny, Pc, Pn, vx, vy, vz, tally, first);
         }
+        launch_after(k_level_done, 1, 1, s, scal, back_d, ++step);
         TRY(cudaGetLastError());
-        TRY(cudaMemcpyAsync(back->next, scal + 2, 8, cudaMemcpyDeviceToHost, s));
-        TRY(cudaStreamSynchronize(s));
+        TRY(wait_step(back, step, s));
         const uint32_t mn = back->next[0];
         largest = back->next[1];
         if (mn == 0) break;
         Level Nx;
         TRY(level_alloc(Nx, mn, s));
         levels.push_back(Nx);
-        TRY(cudaMemsetAsync(scal, 0, 9 * 4, s));
         launch_after(k_children, grid_for((uint64_t)m * 8, CHILD_THREADS), CHILD_THREADS, s, L, Nx, lists, Pn, vx, vy, vz, stats + NSTATS * (lv + 1));
     }
 
@@ -1946,12 +1999,9 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         Level Nx = lv + 1 < nl ? levels[lv + 1] : L;
         launch_after(k_up, grid_for(L.m, 256), 256, s, L, Nx, lv + 1 < nl);
     }
-    TRY(cudaMemcpyAsync(back->stats, stats, sizeof back->stats, cudaMemcpyDeviceToHost, s));
-    TRY(cudaMemcpyAsync(&back->root_nodes, levels[0].sub_nodes, 4, cudaMemcpyDeviceToHost, s));
-    TRY(cudaMemcpyAsync(&back->err, err, 8, cudaMemcpyDeviceToHost, s));
-    TRY(cudaMemcpyAsync(&back->units, levels[0].sub_units, 8, cudaMemcpyDeviceToHost, s));
-    TRY(cudaMemcpyAsync(back->box, levels[0].box, 24, cudaMemcpyDeviceToHost, s));
-    TRY(cudaStreamSynchronize(s));
+    launch_after(k_all_done, 1, 128, s, levels[0], stats, err, back_d, ++step);
+    TRY(cudaGetLastError());
+    TRY(wait_step(back, step, s));
     if (back->err & ERR_WALK) return VOX_CUDA_ECUDA;
     if (back->err & ERR_BIG_LEAF) return VOX_CUDA_ETOOBIG;
     uint64_t units = VOXP_REC_UNITS + back->units;

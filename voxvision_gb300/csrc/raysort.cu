@@ -19,10 +19,11 @@
  * kernel reads the j-th item of the order from where it was given and writes
  * its result there.  Items of one (key, block) pair land in any order among
  * themselves; that, too, changes no result.
- * (Copying the rays into order instead makes a 16M-ray batch slower: each
- * ray's six floats become scattered partial-sector stores.  Finer keys are
- * slower too: the entry point's cell on a 16^3 grid, 2.84-2.87 ms, and the
- * direction's dominant axis added to the key, 2.99 ms, against 2.77-2.78.)
+ * (Copying the rays into order instead makes a batch slower: each ray's six
+ * floats become scattered partial-sector stores.  Finer keys are slower too:
+ * of the entry point's cell on a 16^3 grid 2.84-2.87 ms, of the direction's
+ * dominant axis as well 2.99, against 2.77-2.78, for 16M rays with the general
+ * search.)
  */
 #include <cuda_runtime.h>
 
@@ -72,7 +73,7 @@ __device__ __forceinline__ uint32_t morton_cell(const float *pt, size_t i, const
 // where the ray enters that box (rays that miss it: the last key).  Rays of
 // one key start their searches at the same part of the tree and walk it the
 // same way; keyed on the origin's cell instead, a warp's rays of one octant
-// still entered the box anywhere (16M rays: 3.94 ms against 2.80).
+// still entered the box anywhere (16M rays, general search: 3.94 ms against 2.80).
 __device__ __forceinline__ uint32_t ray_key(const float *o, const float *d, size_t i, const KeyFrame &f)
 {
     uint32_t oct = (d[3 * i] < 0.0f) | ((d[3 * i + 1] < 0.0f) << 1) | ((d[3 * i + 2] < 0.0f) << 2);

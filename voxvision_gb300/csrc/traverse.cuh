@@ -9,7 +9,10 @@
  * result is the reference's leaf, voxel and intersection point, bit for bit.
  *
  * Recursion becomes an explicit per-thread stack of pending tasks {record
- * offset, ray origin} (see trace_ray).
+ * offset, ray origin} (see trace_ray).  Over images of the SHAPE_* kinds below
+ * rays and balls take cheaper searches with the same results (trace_mirrored,
+ * trace_ball_nested); over any other image, and for the rays and boxes those
+ * leave, the general ones run.
  *
  * Checked build (-DVOX_CUDA_CHECKED, libvoxtrees_cuda_checked.so): every
  * load from the tree image and the light tree first proves its index inside

@@ -4,11 +4,16 @@
  *
  * Kernels (one thread per query, traversal in traverse.cuh):
  *   ray_kernel     batched vox_ray_tree_intersection, optional per-ray roots
- *   ball_kernel    batched vox_tree_ball_collidep
+ *   nested_ball_kernel, ball_kernel
+ *                  batched vox_tree_ball_collidep: over images whose boxes
+ *                  nest, and over any other
  *   render_kernel  vox_render BEST: camera ray, search and colour fused; a
  *                  warp covers an 8x4 pixel tile, a block 16x8 pixels, so the
  *                  rays of a warp are neighbours and walk the same nodes.
- * Each has a counting twin (COUNT=true) that only tallies the work.
+ *   render_squares_kernel  the other qualities: a 4x4 square per half-warp.
+ *   image_shape_kernel     what the searches may rely on in a tree's image.
+ * The ray, ball and BEST kernels have a counting twin (COUNT=true) that only
+ * tallies the work.
  *
  * The stack capacity is a template parameter picked from the tree depth at
  * upload time, so a kernel never needs more stack than it has.
