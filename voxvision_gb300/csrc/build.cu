@@ -251,7 +251,7 @@ struct NodeLists {
     uint32_t *tiny, *small, *low, *mid, *high, *tiled, *first_tile;
     uint32_t *ntiny, *nsmall, *nlow, *nmid, *nhigh;
     unsigned long long *ntiled;   // slots in the upper half, tiles in the lower
-    uint32_t tile;                // positions per tile
+    uint32_t tile, shift;         // positions per tile: 1 << shift
     __device__ void add_large(uint32_t k, uint32_t n) const
     {
         if (n > HIGH) {
@@ -829,15 +829,17 @@ __global__ void __launch_bounds__(CENTRE_WARPS * 32) k_centre_big(const float *P
 // position so far (Marks).  Claimed voxels leave for good, straight to their
 // place in the next level's order; only the others move on to the next pass.
 
-// The source of position t (local to the node) in a pass whose range starts
-// at `from`: the walk back described at the top of the file.  claimed(s, c, u)
-// says whether position s is claimed and gives the claimed count before it
-// and the last unclaimed position before it.
+// The source of position t (local to the node), which is claimed, in a pass
+// whose range starts at `from`: the walk back described at the top of the
+// file.  c and last are the claimed count and the last unclaimed position
+// before t; claimed(s, c, last) says whether position s is claimed and gives
+// both for it.
 template <class F>
-__device__ __forceinline__ uint32_t walk_back(uint32_t t, uint32_t from, uint32_t limit, F claimed, uint32_t *err)
+__device__ __forceinline__ uint32_t walk_back(uint32_t t, uint32_t from, uint32_t limit, uint32_t c, uint32_t last,
+                                              F claimed, uint32_t *err)
 {
-    uint32_t s = t, c, last;
-    for (uint32_t steps = 0; claimed(s, c, last); steps++) {
+    uint32_t s = t;
+    for (uint32_t steps = 0;; steps++) {
         const uint32_t u = (s - from) - c;                 // unclaimed positions before s
         if (u == 0 || last == NO_POS || steps > limit) {   // impossible for a consistent pass
             atomicOr(err, ERR_WALK);
@@ -850,8 +852,8 @@ __device__ __forceinline__ uint32_t walk_back(uint32_t t, uint32_t from, uint32_
             return t;
         }
         s -= back;
+        if (!claimed(s, c, last)) return s;
     }
-    return s;
 }
 
 // Scan of up to 32 * PER words' claimed counts and last unclaimed positions
@@ -898,7 +900,18 @@ __device__ __forceinline__ uint32_t last_in_word(uint32_t w, uint32_t i, uint32_
     return u ? (w << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
 }
 
-// The gathered voxels of a claimed position's place in the next order.
+// Octants are listed by pass: a pass leaves the places of its octant's voxels,
+// in their order, in the buffer that it writes.  The seventh has the eighth's
+// there too: nothing but octant 7 is left, and its own pass would move nothing.
+// So the octant of a position, given where each octant ends, tells the buffer.
+__device__ __forceinline__ uint32_t final_buffer(const uint32_t *ends, uint32_t t)
+{
+    uint32_t o = 0;
+    for (int j = 0; j < 7; j++) o += t >= ends[j];
+    return o == 7 ? 1u : (o & 1u) ^ 1u;
+}
+
+// Voxel i of one order to place `to` of the next.
 __device__ __forceinline__ void place(const float *P, float *Pn, uint64_t to, uint64_t i)
 {
     Pn[3 * to] = P[3 * i];
@@ -968,7 +981,7 @@ __device__ __forceinline__ float unordered(uint32_t u)
 
 // Nodes of VOX_MAX_DOTS+1..MOST voxels, up to 32 of them to a warp at a time.
 // Each node's box, density, centre and octants are the warp's work, in
-// registers; then every lane makes the eight passes over one node of its own,
+// registers; then every lane makes the passes over one node of its own,
 // as the reference makes them (swap each claimed voxel to the front), in a
 // column of shared memory; then the warp moves each node's voxels and takes
 // the children's places in the next level, all with one atomic.
@@ -1063,7 +1076,7 @@ __device__ __forceinline__ void nodes_lanes(const Level &L, const uint32_t *list
         __syncwarp();
         if (split) {                                      // sort_set, tree.c:166-183, on the lane's own node
             uint32_t at = 0;
-            for (uint32_t o = 0; o < 8; o++) {
+            for (uint32_t o = 0; o < 7; o++) {            // (the last has nothing to move)
                 const uint32_t end = at + (((o < 4 ? c03 : c47) >> (8 * (o & 3))) & 0xFFu);
                 uint32_t i = at;
                 uint16_t x = at < end ? col[i][lane] : 0;
@@ -1138,7 +1151,7 @@ struct NodeBuffer<MOST, true> {
 template <uint32_t MOST>
 struct NodeShared {
     NodeBuffer<MOST> buf;
-    uint32_t mask[MOST / 32], before[MOST / 32], last[MOST / 32];
+    uint32_t mask[2][MOST / 32], before[2][MOST / 32], last[2][MOST / 32];   // the marks of a pass and of the next
 };
 template <int THREADS, uint32_t MOST>
 __device__ __forceinline__ void nodes_block(const Level &L, const uint32_t *list, const uint32_t *count, const float *P,
@@ -1149,8 +1162,7 @@ __device__ __forceinline__ void nodes_block(const Level &L, const uint32_t *list
     static_assert(WARPS >= 3 && WARPS <= 32, "an axis a warp");
     extern __shared__ __align__(16) unsigned char dynamic[];
     NodeShared<MOST> &w = *reinterpret_cast<NodeShared<MOST> *>(dynamic);
-    uint32_t *const mask = w.mask, *const before = w.before, *const last = w.last;
-    __shared__ uint32_t total, s_kind;
+    __shared__ uint32_t total, s_kind, ends[8];
     __shared__ Extremes epart[WARPS];
     __shared__ PlainSum spart[WARPS];
     __shared__ float centre[3];
@@ -1194,33 +1206,39 @@ __device__ __forceinline__ void nodes_block(const Level &L, const uint32_t *list
         }
         __syncthreads();
     }
-    for (uint32_t i = threadIdx.x; i < n; i += THREADS) {
-        const float p[3] = {P[3 * (s0 + i)], P[3 * (s0 + i) + 1], P[3 * (s0 + i) + 2]};
-        w.buf.set(i, octant(centre, p));
-    }
     const uint32_t nw = (n + 31) / 32;
-    uint32_t from = 0, cnt = 0;     // lane o of warp 0 holds octant o's count
-    for (uint32_t o = 0; o < 8 && from < n; o++) {
-        const uint32_t in = o & 1;
-        __syncthreads();
-        for (uint32_t i = (from >> 5) + warp; i < nw; i += WARPS) {
-            const uint32_t t = (i << 5) + lane;
-            const bool range = t >= from && t < n;
-            const bool cl = range && w.buf.oct(in, t) == o;
-            const uint32_t m = __ballot_sync(0xffffffffu, cl), u = __ballot_sync(0xffffffffu, range && !cl);
-            if (lane == 0) {
-                mask[i] = m;
-                before[i] = (uint32_t)__popc(m);
-                last[i] = u ? (i << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
-            }
+    auto mark = [&](uint32_t b, uint32_t i, bool cl, bool un) {   // word i's claimed and unclaimed flags
+        const uint32_t m = __ballot_sync(0xffffffffu, cl), u = __ballot_sync(0xffffffffu, un);
+        if (lane == 0) {
+            w.mask[b][i] = m;
+            w.before[b][i] = (uint32_t)__popc(m);
+            w.last[b][i] = u ? (i << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
         }
+    };
+    for (uint32_t i = warp; i < nw; i += WARPS) {
+        const uint32_t t = (i << 5) + lane;
+        uint32_t q = 8;
+        if (t < n) {
+            const float p[3] = {P[3 * (s0 + t)], P[3 * (s0 + t) + 1], P[3 * (s0 + t) + 2]};
+            q = octant(centre, p);
+            w.buf.set(t, q);
+        }
+        mark(0, i, q == 0, t < n && q != 0);
+    }
+    if (threadIdx.x < 8) ends[threadIdx.x] = n;
+    uint32_t from = 0, cnt = 0;     // lane o of warp 0 holds octant o's count
+    for (uint32_t o = 0; o < 7 && from < n; o++) {
+        const uint32_t in = o & 1, *const mask = w.mask[in], *const before = w.before[in], *const last = w.last[in];
         __syncthreads();
         if (warp == 0) {
             constexpr uint32_t PER = MOST / 1024 < 8 ? MOST / 1024 : 8;
             uint32_t run = 0, prev = NO_POS;
             for (uint32_t i = from >> 5; i < nw; i += 32 * PER)
-                scan_words<PER>(before + i, last + i, min(nw - i, 32 * PER), run, prev);
-            if (lane == 0) total = run;
+                scan_words<PER>(w.before[in] + i, w.last[in] + i, min(nw - i, 32 * PER), run, prev);
+            if (lane == 0) {
+                total = run;
+                ends[o] = from + run;
+            }
             if (lane == o) cnt = run;
         }
         __syncthreads();
@@ -1232,12 +1250,45 @@ __device__ __forceinline__ void nodes_block(const Level &L, const uint32_t *list
             if (l == NO_POS) l = last[i];
             return ((m >> b) & 1u) != 0u;
         };
-        for (uint32_t t = from + threadIdx.x; t < n; t += THREADS) {
-            uint32_t c, l;
-            if (claimed(t, c, l)) place(P, Pn, s0 + from + c, s0 + w.buf.place(in, t));
-            if (t >= rest) w.buf.move(in, t, walk_back(t, from, MOST, claimed, tally.err));
+        for (uint32_t i = (from >> 5) + warp; i < nw; i += WARPS) {
+            const uint32_t t = (i << 5) + lane;
+            const bool left = t >= rest && t < n;
+            uint32_t q = 8;
+            if (t >= from && t < n) {
+                uint32_t c, l, s = t;
+                if (claimed(t, c, l)) {
+                    w.buf.move(in, from + c, t);
+                    if (left) s = walk_back(t, from, MOST, c, l, claimed, tally.err);
+                }
+                if (left) {
+                    w.buf.move(in, t, s);
+                    q = w.buf.oct(in, s);
+                }
+            }
+            if (o < 6) mark(in ^ 1, i, q == o + 1, left && q != o + 1);
         }
         from = rest;
+    }
+    if (warp == 0 && lane == 7) cnt = n - from;
+    __syncthreads();
+    // the voxels, all at once (a pass at a time, an eighth of the lanes had a
+    // load to wait for; here and tile by tile together, with the eighth pass
+    // gone and marks made as voxels move, a 256^3 raw volume 1,496 -> 1,402 us)
+    for (uint32_t t0 = threadIdx.x; t0 < n; t0 += 4 * THREADS) {
+        float p[4][3];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++) {
+            const uint32_t t = t0 + j * THREADS;
+            if (t >= n) break;
+            const uint64_t i = s0 + w.buf.place(final_buffer(ends, t), t);
+            for (int a = 0; a < 3; a++) p[j][a] = P[3 * i + a];
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++) {
+            const uint32_t t = t0 + j * THREADS;
+            if (t >= n) break;
+            for (int a = 0; a < 3; a++) Pn[3 * (s0 + t) + a] = p[j][a];
+        }
     }
     if (warp == 0) {
         WarpTally mine;
@@ -1337,8 +1388,7 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_marks(Level L, NodeLists 
 // Pass o over every tiled node.
 __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists lists, uint32_t o, Marks in, Marks out,
                                                             const uint32_t *in_idx, const uint8_t *in_oct,
-                                                            uint32_t *out_idx, uint8_t *out_oct, const float *P,
-                                                            float *Pn, uint32_t *err)
+                                                            uint32_t *out_idx, uint8_t *out_oct, uint32_t *err)
 {
     __shared__ SubMarks sub;
     __shared__ uint32_t tbefore[MAX_TILES], tlast[MAX_TILES];
@@ -1384,12 +1434,15 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
         before += t[j].x;
         above = max(above, t[j].y);
     }
-    if (e == n && threadIdx.x == 0) L.cnt[8 * (size_t)k + o] = total;   // read by later launches only
-    __syncthreads();
     const uint32_t rest = from + total;
+    if (e == n && threadIdx.x == 0) {          // read by later launches only
+        L.cnt[8 * (size_t)k + o] = total;
+        if (o == 6) L.cnt[8 * (size_t)k + 7] = n - rest;
+    }
+    __syncthreads();
     const uint64_t words = (uint64_t)ft * (tile / 32);   // the node's first word: tiles hold whole words
     auto claimed = [&](uint32_t s, uint32_t &c, uint32_t &l) {
-        const uint32_t w = s >> 5, i = s & 31, ts = s / tile - t0;
+        const uint32_t w = s >> 5, i = s & 31, ts = (s >> lists.shift) - t0;
         const uint4 word = in.word[words + w];
         const uint32_t m = word.x;
         c = tbefore[ts] + word.y + (uint32_t)__popc(m & lanes_below(i));
@@ -1403,19 +1456,25 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
         const uint32_t nw = (min(e - sb, SUB) + 31) / 32;
         for (uint32_t w = warp; w < nw; w += PASS_THREADS / 32) {
             const uint32_t t = sb + (w << 5) + lane;
+            const bool left = t >= rest && t < e;
             uint8_t q = 0xFF;
             if (t >= from && t < e) {
-                uint32_t c, l;
-                if (claimed(t, c, l))
-                    place(P, Pn, start + from + c, o == 0 ? start + t : (uint64_t)in_idx[start + t]);
-                if (t >= rest) {
-                    const uint32_t s = walk_back(t, from, 1u << 22, claimed, err);
+                q = in_oct[start + t];
+                const uint32_t own = o == 0 ? (uint32_t)start + t : in_idx[start + t];
+                uint32_t c, l, src = own;
+                const bool taken = claimed(t, c, l);
+                if (taken && left) {
+                    const uint32_t s = walk_back(t, from, 1u << 22, c, l, claimed, err);
                     q = in_oct[start + s];
-                    out_idx[start + t] = o == 0 ? (uint32_t)start + s : in_idx[start + s];
+                    src = o == 0 ? (uint32_t)start + s : in_idx[start + s];
+                }
+                if (taken) out_idx[start + from + c] = own;
+                if (left) {
+                    out_idx[start + t] = src;
                     out_oct[start + t] = q;
                 }
             }
-            const bool left = t >= rest && t < e, cl = left && q == o + 1;
+            const bool cl = left && q == o + 1;
             const uint32_t m = __ballot_sync(0xffffffffu, cl), u = __ballot_sync(0xffffffffu, left && !cl);
             if (lane == 0) {
                 sub.mask[w] = m;
@@ -1426,6 +1485,40 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
         sub.flush(out, words + (sb >> 5), nw, run, prev);
     }
     if (threadIdx.x == 0) out.tile[blockIdx.x] = make_uint2(run, prev + 1u);
+}
+
+// The voxels of tiled nodes in their order after the passes, a block a tile.
+__global__ void __launch_bounds__(PASS_THREADS) k_tile_gather(Level L, NodeLists lists, const uint32_t *idx0,
+                                                              const uint32_t *idx1, const float *P, float *Pn)
+{
+    after_previous();
+    const uint32_t slot = tile_slot(lists, blockIdx.x);
+    if (slot == NO_POS) return;
+    const uint32_t k = lists.tiled[slot], n = L.n[k];
+    if (L.kind[k] != K_INNER) return;
+    const uint64_t start = L.start[k];
+    const uint32_t b = (blockIdx.x - lists.first_tile[slot]) * lists.tile, e = min(n, b + lists.tile);
+    uint32_t ends[7], sum = 0;
+    for (int o = 0; o < 7; o++) ends[o] = sum += L.cnt[8 * (size_t)k + o];
+    constexpr uint32_t PER = SUB / PASS_THREADS;
+    for (uint32_t t0 = b + threadIdx.x; t0 < e; t0 += SUB) {
+        uint32_t i[PER];
+        float p[PER][3];
+#pragma unroll
+        for (uint32_t j = 0; j < PER; j++) {
+            const uint32_t t = min(t0 + j * PASS_THREADS, e - 1);
+            i[j] = (final_buffer(ends, t) ? idx1 : idx0)[start + t];
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < PER; j++)
+            for (int a = 0; a < 3; a++) p[j][a] = P[3 * (uint64_t)i[j] + a];
+#pragma unroll
+        for (uint32_t j = 0; j < PER; j++) {
+            const uint32_t t = t0 + j * PASS_THREADS;
+            if (t < e)
+                for (int a = 0; a < 3; a++) Pn[3 * (start + t) + a] = p[j][a];
+        }
+    }
 }
 
 // Tiled nodes after their passes, a warp each.
@@ -1879,7 +1972,8 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     lists.nmid = scal + 5;
     lists.nhigh = scal + 8;
     lists.ntiled = reinterpret_cast<unsigned long long *>(scal + 6);
-    lists.tile = SUB * (uint32_t)((N + (uint64_t)SUB * MAX_TILES - 1) / ((uint64_t)SUB * MAX_TILES));
+    while ((uint64_t)MAX_TILES << lists.shift < N || (1u << lists.shift) < SUB) lists.shift++;
+    lists.tile = 1u << lists.shift;
     const uint64_t max_low = N / SMALL, max_mid = N / LOW, max_high = N / MID, max_tiled = N / HIGH, max_tiles = N / lists.tile + max_tiled,
                    max_chunks = max_tiles * (lists.tile / CHUNK);
     TRY(d.get(&lists.tiny, N / (VOX_MAX_DOTS + 1) + 1));
@@ -1936,7 +2030,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         float *Pn = P[(lv & 1) ^ 1];
         const Tally tally{stats + NSTATS * lv, scal + 2, scal + 3, err};
         if (largest > HIGH) {
-            // boxes, centres and the eight swapping passes of the largest nodes
+            // boxes, centres and the swapping passes of the largest nodes
             const unsigned nt = (unsigned)max_tiled, nc = (unsigned)max_chunks, np = (unsigned)max_tiles;
             launch_after(k_chunk_box, nc, CHUNK_THREADS, s, Pc, L, lists, cv, cidx);
             launch_after(k_box_tiled, nt, NODE_THREADS, s, L, lists, cv, cidx, vx, vy, vz, tally);
@@ -1945,10 +2039,11 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
             launch_after(k_chunk_maps, nc, CHUNK_THREADS, s, Pc, L, lists, cbase, window, maps, max_chunks);
             launch_after(k_centre_big, grid_for(max_tiled * 3 * 32, CENTRE_WARPS * 32), CENTRE_WARPS * 32, s, Pc, L, lists, maps, cbase, csum, window, starts, max_chunks, vx, vy, vz);
             launch_after(k_tile_marks, np, PASS_THREADS, s, L, lists, Pc, oct[0], marks[0]);
-            for (uint32_t o = 0; o < 8; o++) {
+            for (uint32_t o = 0; o < 7; o++) {
                 const int in = o & 1, out = in ^ 1;
-                launch_after(k_tile_pass, np, PASS_THREADS, s, L, lists, o, marks[in], marks[out], idx[in], oct[in], idx[out], oct[out], Pc, Pn, err);
+                launch_after(k_tile_pass, np, PASS_THREADS, s, L, lists, o, marks[in], marks[out], idx[in], oct[in], idx[out], oct[out], err);
             }
+            launch_after(k_tile_gather, np, PASS_THREADS, s, L, lists, idx[0], idx[1], Pc, Pn);
             launch_after(k_finish_tiled, grid_for(max_tiled * 32, 256), 256, s, L, lists, tally);
         }
         bool first = true;   // of the size classes that are made whole
