@@ -829,44 +829,47 @@ __global__ void __launch_bounds__(CENTRE_WARPS * 32) k_centre_big(const float *P
 // position so far (Marks).  Claimed voxels leave for good, straight to their
 // place in the next level's order; only the others move on to the next pass.
 
-// The source of position t (local to the node), which is claimed, in a pass
-// whose range starts at `from`: the walk back described at the top of the
-// file.  c and last are the claimed count and the last unclaimed position
-// before t; claimed(s, c, last) says whether position s is claimed and gives
-// both for it.
-template <class F>
-__device__ __forceinline__ uint32_t walk_back(uint32_t t, uint32_t from, uint32_t limit, uint32_t c, uint32_t last,
-                                              F claimed, uint32_t *err)
+// The source of position t (local to the node), which is claimed with c
+// claimed positions before it, in a pass whose range starts at `from`: the
+// walk back described at the top of the file.  claimed(s, c) says whether
+// position s is claimed and gives that count; unclaimed_before(s) gives the
+// last unclaimed position before s.  Few walks have more than a step or two
+// inside one run, so the first are made one at a time, without looking for
+// the run's start (256^3 raw volume with a first frame 1,402 -> 1,376 us).
+constexpr uint32_t PLAIN_STEPS = 6;
+template <class F, class G>
+__device__ __forceinline__ uint32_t walk_back(uint32_t t, uint32_t from, uint32_t limit, uint32_t c, F claimed,
+                                              G unclaimed_before, uint32_t *err)
 {
     uint32_t s = t;
     for (uint32_t steps = 0;; steps++) {
-        const uint32_t u = (s - from) - c;                 // unclaimed positions before s
-        if (u == 0 || last == NO_POS || steps > limit) {   // impossible for a consistent pass
+        uint32_t to = from + c;                            // one step: unclaimed positions before s back
+        if (steps >= PLAIN_STEPS && to < s) {              // to before the run's start
+            const uint32_t u = s - to, last = unclaimed_before(s);
+            if (last < s) to = s - ((s - last - 1) / u + 1) * u;
+            else to = s;
+        }
+        if (to >= s || to < from || steps > limit) {       // impossible for a consistent pass
             atomicOr(err, ERR_WALK);
             return t;
         }
-        const uint32_t a = last + 1;                       // start of the claimed run holding s
-        const uint32_t back = s - a < u ? u : ((s - a) / u + 1) * u;   // (mostly one step: no division)
-        if (a > s || back > s - from) {
-            atomicOr(err, ERR_WALK);
-            return t;
-        }
-        s -= back;
-        if (!claimed(s, c, last)) return s;
+        s = to;
+        if (!claimed(s, c)) return s;
     }
 }
 
 // Scan of up to 32 * PER words' claimed counts and last unclaimed positions
 // by one warp, in place: before[w] and last[w] become those of the words
 // before w (from `run` and `prev` on, which advance).
-template <int PER>
+// (Word w's count is before[STRIDE * w].)
+template <int PER, int STRIDE>
 __device__ __forceinline__ void scan_words(uint32_t *before, uint32_t *last, uint32_t nw, uint32_t &run, uint32_t &prev)
 {
     const uint32_t lane = threadIdx.x & 31;
     uint32_t c[PER], l[PER], sum = 0, top = 0;   // top: last position + 1, 0 for none
     for (int j = 0; j < PER; j++) {
         const uint32_t w = lane * PER + j;
-        c[j] = w < nw ? before[w] : 0u;
+        c[j] = w < nw ? before[STRIDE * w] : 0u;
         l[j] = w < nw ? last[w] + 1u : 0u;
         sum += c[j];
         top = max(top, l[j]);
@@ -881,7 +884,7 @@ __device__ __forceinline__ void scan_words(uint32_t *before, uint32_t *last, uin
     t = max(lane ? t : 0u, prev + 1u);
     for (int j = 0; j < PER; j++) {
         const uint32_t w = lane * PER + j;
-        if (w < nw) { before[w] = r; last[w] = t - 1u; }
+        if (w < nw) { before[STRIDE * w] = r; last[w] = t - 1u; }
         r += c[j];
         t = max(t, l[j]);
     }
@@ -1151,7 +1154,8 @@ struct NodeBuffer<MOST, true> {
 template <uint32_t MOST>
 struct NodeShared {
     NodeBuffer<MOST> buf;
-    uint32_t mask[2][MOST / 32], before[2][MOST / 32], last[2][MOST / 32];   // the marks of a pass and of the next
+    uint2 word[2][MOST / 32];            // the marks of a pass and of the next: claimed bits, claimed count before
+    uint32_t last[2][MOST / 32];         // and the last unclaimed position before
 };
 template <int THREADS, uint32_t MOST>
 __device__ __forceinline__ void nodes_block(const Level &L, const uint32_t *list, const uint32_t *count, const float *P,
@@ -1210,8 +1214,7 @@ __device__ __forceinline__ void nodes_block(const Level &L, const uint32_t *list
     auto mark = [&](uint32_t b, uint32_t i, bool cl, bool un) {   // word i's claimed and unclaimed flags
         const uint32_t m = __ballot_sync(0xffffffffu, cl), u = __ballot_sync(0xffffffffu, un);
         if (lane == 0) {
-            w.mask[b][i] = m;
-            w.before[b][i] = (uint32_t)__popc(m);
+            w.word[b][i] = make_uint2(m, (uint32_t)__popc(m));
             w.last[b][i] = u ? (i << 5) + 31u - (uint32_t)__clz((int)u) : NO_POS;
         }
     };
@@ -1228,13 +1231,14 @@ __device__ __forceinline__ void nodes_block(const Level &L, const uint32_t *list
     if (threadIdx.x < 8) ends[threadIdx.x] = n;
     uint32_t from = 0, cnt = 0;     // lane o of warp 0 holds octant o's count
     for (uint32_t o = 0; o < 7 && from < n; o++) {
-        const uint32_t in = o & 1, *const mask = w.mask[in], *const before = w.before[in], *const last = w.last[in];
+        const uint32_t in = o & 1, *const last = w.last[in];
+        const uint2 *const word = w.word[in];
         __syncthreads();
         if (warp == 0) {
             constexpr uint32_t PER = MOST / 1024 < 8 ? MOST / 1024 : 8;
             uint32_t run = 0, prev = NO_POS;
             for (uint32_t i = from >> 5; i < nw; i += 32 * PER)
-                scan_words<PER>(w.before[in] + i, w.last[in] + i, min(nw - i, 32 * PER), run, prev);
+                scan_words<PER, 2>(&w.word[in][i].y, w.last[in] + i, min(nw - i, 32 * PER), run, prev);
             if (lane == 0) {
                 total = run;
                 ends[o] = from + run;
@@ -1243,22 +1247,24 @@ __device__ __forceinline__ void nodes_block(const Level &L, const uint32_t *list
         }
         __syncthreads();
         const uint32_t rest = from + total;
-        auto claimed = [&](uint32_t s, uint32_t &c, uint32_t &l) {
-            const uint32_t i = s >> 5, b = s & 31, m = mask[i];
-            c = before[i] + (uint32_t)__popc(m & lanes_below(b));
-            l = last_in_word(i, b, m, from);
-            if (l == NO_POS) l = last[i];
-            return ((m >> b) & 1u) != 0u;
+        auto claimed = [&](uint32_t s, uint32_t &c) {
+            const uint2 m = word[s >> 5];
+            c = m.y + (uint32_t)__popc(m.x & lanes_below(s & 31));
+            return ((m.x >> (s & 31)) & 1u) != 0u;
+        };
+        auto unclaimed_before = [&](uint32_t s) {
+            const uint32_t l = last_in_word(s >> 5, s & 31, word[s >> 5].x, from);
+            return l != NO_POS ? l : last[s >> 5];
         };
         for (uint32_t i = (from >> 5) + warp; i < nw; i += WARPS) {
             const uint32_t t = (i << 5) + lane;
             const bool left = t >= rest && t < n;
             uint32_t q = 8;
             if (t >= from && t < n) {
-                uint32_t c, l, s = t;
-                if (claimed(t, c, l)) {
+                uint32_t c, s = t;
+                if (claimed(t, c)) {
                     w.buf.move(in, from + c, t);
-                    if (left) s = walk_back(t, from, MOST, c, l, claimed, tally.err);
+                    if (left) s = walk_back(t, from, MOST, c, claimed, unclaimed_before, tally.err);
                 }
                 if (left) {
                     w.buf.move(in, t, s);
@@ -1337,7 +1343,7 @@ struct SubMarks {
     {
         __syncthreads();
         if (threadIdx.x < 32) {
-            scan_words<SUB / 32 / 32>(before, last, nw, run, prev);
+            scan_words<SUB / 32 / 32, 1>(before, last, nw, run, prev);
             __syncwarp();
             for (uint32_t w = threadIdx.x; w < nw; w += 32)
                 m.word[word0 + w] = make_uint4(mask[w], before[w], last[w], 0u);
@@ -1441,15 +1447,16 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
     }
     __syncthreads();
     const uint64_t words = (uint64_t)ft * (tile / 32);   // the node's first word: tiles hold whole words
-    auto claimed = [&](uint32_t s, uint32_t &c, uint32_t &l) {
-        const uint32_t w = s >> 5, i = s & 31, ts = (s >> lists.shift) - t0;
-        const uint4 word = in.word[words + w];
-        const uint32_t m = word.x;
-        c = tbefore[ts] + word.y + (uint32_t)__popc(m & lanes_below(i));
-        l = last_in_word(w, i, m, from);
+    auto claimed = [&](uint32_t s, uint32_t &c) {
+        const uint4 word = in.word[words + (s >> 5)];
+        c = tbefore[(s >> lists.shift) - t0] + word.y + (uint32_t)__popc(word.x & lanes_below(s & 31));
+        return ((word.x >> (s & 31)) & 1u) != 0u;
+    };
+    auto unclaimed_before = [&](uint32_t s) {
+        const uint4 word = in.word[words + (s >> 5)];
+        uint32_t l = last_in_word(s >> 5, s & 31, word.x, from);
         if (l == NO_POS) l = word.z;
-        if (l == NO_POS) l = tlast[ts];
-        return ((m >> i) & 1u) != 0u;
+        return l != NO_POS ? l : tlast[(s >> lists.shift) - t0];
     };
     uint32_t run = 0, prev = NO_POS;
     for (uint32_t sb = b; sb < e; sb += SUB) {
@@ -1461,10 +1468,10 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
             if (t >= from && t < e) {
                 q = in_oct[start + t];
                 const uint32_t own = o == 0 ? (uint32_t)start + t : in_idx[start + t];
-                uint32_t c, l, src = own;
-                const bool taken = claimed(t, c, l);
+                uint32_t c, src = own;
+                const bool taken = claimed(t, c);
                 if (taken && left) {
-                    const uint32_t s = walk_back(t, from, 1u << 22, c, l, claimed, err);
+                    const uint32_t s = walk_back(t, from, 1u << 22, c, claimed, unclaimed_before, err);
                     q = in_oct[start + s];
                     src = o == 0 ? (uint32_t)start + s : in_idx[start + s];
                 }
