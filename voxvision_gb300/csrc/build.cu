@@ -79,7 +79,7 @@ constexpr uint32_t RAW_ITEMS = 16;                       // consecutive samples 
 constexpr uint32_t RAW_TILE = RAW_THREADS * RAW_ITEMS;   // samples a block reads
 constexpr uint32_t TINY = 32;        // nodes with at most this many voxels, and
 constexpr uint32_t SMALL = 128;      // with at most this many, are split by a lane each,
-constexpr uint32_t LOW = 1024;       // with at most this many by a block of 128 threads,
+constexpr uint32_t LOW = 1024;       // with at most this many by a block of 96 threads,
 constexpr uint32_t MID = 8192;       // with at most this many by a block of 512, and
 constexpr uint32_t HIGH = 32768;     // with at most this many by a block of 1024, larger ones tile by tile
 constexpr uint32_t CHUNK = 1024;     // voxels per chunk
@@ -835,8 +835,9 @@ __global__ void __launch_bounds__(CENTRE_WARPS * 32) k_centre_big(const float *P
 // position s is claimed and gives that count; unclaimed_before(s) gives the
 // last unclaimed position before s.  Few walks have more than a step or two
 // inside one run, so the first are made one at a time, without looking for
-// the run's start (256^3 raw volume with a first frame 1,402 -> 1,376 us).
-constexpr uint32_t PLAIN_STEPS = 6;
+// the run's start (256^3 raw volume with a first frame 1,402 -> 1,376 us with
+// 6 of them; 1,397 with 2, 1,357 with 12 or 24, 1,366 with 64).
+constexpr uint32_t PLAIN_STEPS = 12;
 template <class F, class G>
 __device__ __forceinline__ uint32_t walk_back(uint32_t t, uint32_t from, uint32_t limit, uint32_t c, F claimed,
                                               G unclaimed_before, uint32_t *err)
@@ -1321,13 +1322,12 @@ __global__ void __launch_bounds__(THREADS) k_nodes_block(Level L, const uint32_t
 // its node's tiles for itself (at most MAX_TILES).
 //
 // What bounds a pass is the chain of dependent loads of each word's walk, so
-// a warp has few words to go through: the 256^3 set's raw build takes 4,790 us
-// with 4 words a warp (256 threads on 1,024 positions, or 512 on 2,048), 5,190
-// with 16, and 4,930 with 2 in blocks of 1,024 threads.  With the four kernels
-// a pass (count, scan, place, walk) over every position of the level that
-// this replaces it took 6,080.
-constexpr int PASS_THREADS = 256;
-constexpr uint32_t SUB = 1024;          // positions marked at a time; a tile is a multiple of it
+// a warp has few words to go through, and enough for a block's scan to be worth
+// it: the 256^3 set's raw build takes 1,349 us with 4 words a warp and 512
+// threads, 1,363 with 256 threads, 1,390 with 1,024; with 8 words a warp 1,380
+// (256 threads), with 2 1,405 (1,024 threads).
+constexpr int PASS_THREADS = 512;
+constexpr uint32_t SUB = 2048;          // positions marked at a time; a tile is a multiple of it
 constexpr uint32_t MAX_TILES = 2048;    // tiles of one node
 
 struct Marks {
@@ -2067,7 +2067,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
             first = false;
         }
         if (largest > SMALL) {
-            launch_after_with(sizeof(NodeShared<LOW>), k_nodes_block<128, LOW>, (unsigned)std::min<uint64_t>(m, max_low), 128, s,
+            launch_after_with(sizeof(NodeShared<LOW>), k_nodes_block<96, LOW>, (unsigned)std::min<uint64_t>(m, max_low), 96, s,
                               L, lists.low, lists.nlow, Pc, Pn, vx, vy, vz, tally, first);
             first = false;
         }
