@@ -373,7 +373,7 @@ __device__ __forceinline__ int ray_step(const DevTree &t, RaySearch &s, uint4 (&
  * limit), and most of the instructions were the IEEE divisions of the box
  * test and the plane crossings, the two-sided comparisons and the sort of the
  * crossings.  For a ray whose direction has no component near zero and whose
- * numbers are of ordinary size (mirror_begin), in a tree whose boxes are
+ * numbers are of ordinary size (mirror_ok), in a tree whose boxes are
  * ordered (SHAPE_ORDERED), the same results come from fewer operations:
  *
  *  - Every axis on which the ray goes backwards is negated, in the ray and in
@@ -402,11 +402,12 @@ __device__ __forceinline__ int ray_step(const DevTree &t, RaySearch &s, uint4 (&
  * coordinate of a negated axis (whose sign of zero the mirror cannot tell),
  * reports STEP_AGAIN and is made again by the general search below.
  *
- * Measured against the general search alone (start -> now, 256^3 noise tree):
+ * Measured against the general search alone (256^3 noise tree; in brackets
+ * with the packed arithmetic and the smaller changes since):
  * a 1080p orbit frame 80.6 -> 51.5 us back to back, ADAPTIVE 112 -> 74 us;
- * 32 such frames in the batch kernel 1,995 -> 1,366 us; 24 mixed frames over
- * four trees 1,203 -> 850 us; a near 4K FAST frame of the 512^3 tree 1,496 ->
- * 1,145 us; 4M incoherent rays 710 -> 569 us. */
+ * 32 such frames in the batch kernel 1,995 -> 1,366 us (1,304); 24 mixed frames
+ * over four trees 1,203 -> 850 us (782); a near 4K FAST frame of the 512^3 tree
+ * 1,496 -> 1,145 us (994); 4M incoherent rays 710 -> 569 us (477). */
 constexpr int STEP_AGAIN = 4;
 constexpr float DIR_MIN = 9.313225746154785e-10f, DIR_MAX = 1048576.0f;   // 2^-30, 2^20
 // Quotients and crossing distances in use are at least this.  A quotient a/d
