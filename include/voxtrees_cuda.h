@@ -116,7 +116,8 @@ int vox_cuda_tree_get_info(const vox_cuda_tree *tree, vox_cuda_tree_info *info);
 /* `set`: n voxels (a vox_dot array, 3n floats) in host memory, left
  * unmodified (vox_make_tree reorders its set). */
 int vox_cuda_tree_build(const float *set, size_t n, vox_cuda_tree **out);
-/* `d_set`: n voxels (3n floats) in device memory of the current device. */
+/* `d_set`: n voxels (3n floats) in device memory of the current device; work
+ * enqueued before the call, in any stream, is waited for. */
 int vox_cuda_tree_build_device(const float *d_set, size_t n, vox_cuda_tree **out);
 
 /* vox_make_tree builds sets of at least this many voxels on the GPU (when a

@@ -84,3 +84,17 @@ def test_raw_volumes_at_tile_edges(vg, dim, size):
             _same(vg, np.ascontiguousarray(vox), made)
         else:
             assert made.info()["nodes"] == 0
+
+
+@pytest.mark.parametrize("side_stream", [False, True])
+def test_voxels_still_on_their_way(vg, side_stream):
+    # the set is written by work that is not done when the build is called
+    vox = _set("scattered", 40000, 11)
+    src, dst = torch.from_numpy(vox).cuda(), torch.zeros(vox.shape, device="cuda")
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream() if side_stream else torch.cuda.current_stream()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(20_000_000)   # some 10 ms
+        dst.copy_(src)
+        made = vg.DeviceTree.build_device(dst)
+    _same(vg, vox, made)

@@ -2297,7 +2297,12 @@ int build_for_host_tree(const float *set, size_t n, vox_cuda_tree **out, HostTre
 EXPORT int vox_cuda_tree_build_device(const float *d_set, size_t n, vox_cuda_tree **out)
 try {
     if (n && !d_set) return VOX_CUDA_EINVAL;
-    return new_tree(out, [&](vox_cuda_tree *t, cudaStream_t s) { return build_tree(t, d_set, n, s); });
+    return new_tree(out, [&](vox_cuda_tree *t, cudaStream_t s) {
+        // the set may still be on its way, in any stream of the caller's: the
+        // build's own stream waits for none of them
+        if (n && cudaDeviceSynchronize() != cudaSuccess) return (int)VOX_CUDA_ECUDA;
+        return build_tree(t, d_set, n, s);
+    });
 } VOX_ABI_FAIL_INT
 
 EXPORT int vox_cuda_tree_build(const float *set, size_t n, vox_cuda_tree **out)
