@@ -614,26 +614,30 @@ __device__ __forceinline__ int trace_mirrored(const DevTree &t, uint32_t start, 
                 const uint32_t s0 = sub ^ 1u ^ (o10 ? 2u : 0u) ^ (o20 ? 4u : 0u);
                 const uint32_t s1 = sub ^ 2u ^ (o10 ? 0u : 1u) ^ (o21 ? 4u : 0u);
                 const uint32_t s2 = sub ^ 4u ^ (o20 ? 0u : 1u) ^ (o21 ? 0u : 2u);
-                const bool w0 = v0 && ((mask >> s0) & 1u), w1 = v1 && ((mask >> s1) & 1u),
-                           w2 = v2 && ((mask >> s2) & 1u);
+                // the children's bits, at the bottom, and above them the siblings that follow: one shift gives
+                // both whether a child is there and, counted back from the block's end, its record (32 orbit
+                // frames in the batch kernel 1,305 -> 1,277 us, against the siblings before it masked and counted)
+                const uint32_t r0 = mask >> s0, r1 = mask >> s1, r2 = mask >> s2, r3 = mask >> sub;
+                const uint32_t end = link + VOXP_REC_UNITS * (uint32_t)__popc(mask);
+                const bool w0 = v0 && (r0 & 1u), w1 = v1 && (r1 & 1u), w2 = v2 && (r2 & 1u);
                 const int n = (int)w0 + (int)w1 + (int)w2;
                 if (sp > CAP - 3) return STEP_ERROR;   // (never in a tree whose depth the class holds)
                 // each child above those visited after it
                 if (w0)
                     stack[sp + (int)(w1 && !o10) + (int)(w2 && !o20)] =
-                        make_uint4(link + VOXP_REC_UNITS * (uint32_t)__popc(mask & ((1u << s0) - 1u)),
+                        make_uint4(end - VOXP_REC_UNITS * (uint32_t)__popc(r0),
                                    __float_as_uint(x0), __float_as_uint(y0), __float_as_uint(z0));
                 if (w1)
                     stack[sp + (int)(w0 && o10) + (int)(w2 && !o21)] =
-                        make_uint4(link + VOXP_REC_UNITS * (uint32_t)__popc(mask & ((1u << s1) - 1u)),
+                        make_uint4(end - VOXP_REC_UNITS * (uint32_t)__popc(r1),
                                    __float_as_uint(x1), __float_as_uint(y1), __float_as_uint(z1));
                 if (w2)
                     stack[sp + (int)(w0 && o20) + (int)(w1 && o21)] =
-                        make_uint4(link + VOXP_REC_UNITS * (uint32_t)__popc(mask & ((1u << s2) - 1u)),
+                        make_uint4(end - VOXP_REC_UNITS * (uint32_t)__popc(r2),
                                    __float_as_uint(x2), __float_as_uint(y2), __float_as_uint(z2));
                 sp += n;
-                if ((mask >> sub) & 1u) {                       // search.c:92-93
-                    cur = link + VOXP_REC_UNITS * (uint32_t)__popc(mask & ((1u << sub) - 1u));
+                if (r3 & 1u) {                                  // search.c:92-93
+                    cur = end - VOXP_REC_UNITS * (uint32_t)__popc(r3);
                     ox = ex; oy = ey; oz = ez;
                 } else {
                     resume = true;
