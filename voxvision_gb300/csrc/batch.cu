@@ -143,11 +143,11 @@ __device__ __forceinline__ void run_clear(const BatchJobDev &J, uint32_t c, uint
 }
 
 // Register bounds of the persistent kernels, in resident blocks of 128 threads
-// per SM.  32 frames of the 1080p orbit in the batch kernel take 1,298 us with
-// 7 blocks (72 registers), 1,310 with 8 (64) and 1,360 with 6; 24 host frames
-// in the frames kernel take 1,188 us with 6 blocks (its item count keeps more
-// values live), 1,200 with 7 and 1,270 with 8.
-constexpr int BATCH_MIN_BLOCKS = 7, FRAMES_MIN_BLOCKS = 6;
+// per SM.  32 frames of the 1080p orbit in the batch kernel take 1,253 us with
+// 8 blocks (64 registers), 1,277 with 7 (72), 1,326 with 9 and 1,337 with 6; 24
+// host frames in the frames kernel take 1,185 us with 6 blocks (its item count
+// keeps more values live), 1,193 with 7 and 1,195 with 5.
+constexpr int BATCH_MIN_BLOCKS = 8, FRAMES_MIN_BLOCKS = 6;
 
 // Queue index -> frame: the last job whose tile (or clearing) base is <=
 // item (frames with no item of that kind share their base with the next
