@@ -399,8 +399,8 @@ __device__ __forceinline__ int ray_step(const DevTree &t, RaySearch &s, uint4 (&
  *    included), each child stored at its own place on the stack.
  *
  * A search that meets a quotient too small for the bounds, or ends on a zero
- * coordinate of a negated axis (whose sign of zero the mirror cannot tell),
- * reports STEP_AGAIN and is made again by the general search below.
+ * whose sign the mirror cannot tell (zero_sign_open), reports STEP_AGAIN and is
+ * made again by the general search below.
  *
  * Measured against the general search alone (256^3 noise tree; in brackets
  * with the packed arithmetic and the smaller changes since):
@@ -484,6 +484,21 @@ __device__ __forceinline__ bool mirror_ok(const DevTree &t, float ox, float oy, 
            fabsf(dx + dy + dz) < 4e6f && fabsf(ox + oy + oz) < 4e18f;
 }
 
+// Whether a hit has a coordinate whose sign of zero the mirror leaves open: a
+// sum that cancels is +0 with the axis negated or not, so a -0 on a negated
+// axis is either such a sum (+0 to the reference) or a face or origin at -0.
+// A +0 there can only be a face or origin at +0: floors and walls that end at
+// zero, whose +0 face every ray down the axis ends on, are not searched again
+// (a 1080p frame of a floor with its top at z = 0: 257 us with every zero
+// searched again, 134 without; with its top at z = 1, 142).
+// (The form is the one of several that leaves the loop's code as it was: 32
+// orbit frames in the batch kernel take 1,254 us; 1,262 with `||` throughout,
+// 1,297 with `&` throughout, 1,285 with the test made after the search.)
+__device__ __forceinline__ bool zero_sign_open(const RayHit &h, bool nx, bool ny, bool nz)
+{
+    return (__float_as_uint(h.x) == 0x80000000u && nx) | (__float_as_uint(h.y) == 0x80000000u && ny) |
+           (__float_as_uint(h.z) == 0x80000000u && nz);
+}
 
 template <int CAP, bool MZERO_CONST>
 __device__ __forceinline__ int trace_mirrored(const DevTree &t, uint32_t start, float ox, float oy, float oz,
@@ -554,7 +569,7 @@ __device__ __forceinline__ int trace_mirrored(const DevTree &t, uint32_t start, 
                     hit.x = nx ? -bx : bx; hit.y = ny ? -by : by; hit.z = nz ? -bz : bz;
                     const uint4 r1 = ld16(pool + vrec + 1), r2 = ld16(pool + vrec + 2);
                     hit.leaf = r2.x; hit.slot = win - r1.w; hit.rec = vrec;
-                    return (nx && bx == 0.0f) || (ny && by == 0.0f) || (nz && bz == 0.0f) ? STEP_AGAIN : STEP_HIT;
+                    return zero_sign_open(hit, nx, ny, nz) ? STEP_AGAIN : STEP_HIT;
                 }
                 vend = 0;
                 resume = true;
@@ -564,7 +579,7 @@ __device__ __forceinline__ int trace_mirrored(const DevTree &t, uint32_t start, 
             if (kind == VOXP_KIND_DENSE) {                      // search.c:31-37
                 hit.x = nx ? -ex : ex; hit.y = ny ? -ey : ey; hit.z = nz ? -ez : ez;
                 hit.leaf = link; hit.slot = 0xFFu; hit.rec = cur;
-                return (nx && ex == 0.0f) || (ny && ey == 0.0f) || (nz && ez == 0.0f) ? STEP_AGAIN : STEP_HIT;
+                return zero_sign_open(hit, nx, ny, nz) ? STEP_AGAIN : STEP_HIT;
             }
             if (kind == VOXP_KIND_LEAF) {                       // search.c:39-50
                 const uint32_t vn = meta >> 2;
