@@ -1543,8 +1543,13 @@ __global__ void k_finish_tiled(Level L, NodeLists lists, Tally tally)
 }
 
 // The set into the first level's order; *odd is set when a coordinate is not
-// finite or above LIMIT in magnitude.
-constexpr float LIMIT = 1.4411518807585587e17f;   // 2^57
+// finite, above LIMIT in magnitude or below LEAST and not zero.
+constexpr float LIMIT = 1.4411518807585587e17f;    // 2^57
+constexpr float LEAST = 2.7755575615628914e-17f;   // 2^-55
+__device__ __forceinline__ bool ordinary_coordinate(float v)
+{
+    return v == 0.0f || (fabsf(v) >= LEAST && fabsf(v) <= LIMIT);
+}
 __global__ void __launch_bounds__(256) k_copy_set(const float *__restrict__ set, float *__restrict__ P, uint64_t n,
                                                   uint32_t *odd)
 {
@@ -1553,12 +1558,12 @@ __global__ void __launch_bounds__(256) k_copy_set(const float *__restrict__ set,
     bool fine = true;
     if (i0 + 4 <= n && (reinterpret_cast<uintptr_t>(set) & 15u) == 0) {
         const float4 v = *reinterpret_cast<const float4 *>(set + i0);
-        fine = fabsf(v.x) <= LIMIT && fabsf(v.y) <= LIMIT && fabsf(v.z) <= LIMIT && fabsf(v.w) <= LIMIT;
+        fine = ordinary_coordinate(v.x) && ordinary_coordinate(v.y) && ordinary_coordinate(v.z) && ordinary_coordinate(v.w);
         *reinterpret_cast<float4 *>(P + i0) = v;
     } else {
         for (uint64_t i = i0; i < n && i < i0 + 4; i++) {
             const float v = set[i];
-            fine = fine && fabsf(v) <= LIMIT;
+            fine = fine && ordinary_coordinate(v);
             P[i] = v;
         }
     }
@@ -2150,8 +2155,10 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     // A tree made here of ordinary voxels has every property the searches may
     // rely on: boxes are least boxes of their voxels (min <= max as the voxel
     // size is positive), children's voxels lie on their side of the dividing
-    // planes, and no centre passes 2^60.  Any other is looked over.
-    const auto ordinary = [](float v) { return v >= 8.67e-19f && v <= LIMIT; };   // 2^-60
+    // planes, no centre passes 2^60, and every number is a multiple of 2^-78
+    // (sums of the voxels' own, which are of LEAST's ulp, and of the voxel
+    // size's).  Any other is looked over.
+    const auto ordinary = [](float v) { return v >= vox::SHAPE_VOXEL && v <= LIMIT; };
     back->unshaped = 0;
     if (back->odd || !ordinary(vx) || !ordinary(vy) || !ordinary(vz)) {
         if (e == cudaSuccess) e = image_shape(pool, map, nodes, st.voxel, scal, s);

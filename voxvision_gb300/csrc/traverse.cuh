@@ -44,17 +44,19 @@ struct DevTree {
     uint32_t *fault;             // the tree's status word (checked build only)
 };
 
-// What is known of every box of a tree's image.  SHAPE_ORDERED: every node's
-// box, every centre and voxel and the voxel size are finite, at most
-// SHAPE_LIMIT in magnitude, and min <= max on every axis (the voxel size
-// positive).  Trees that vox_make_tree or the GPU build make from ordinary
+// What is known of every box of a tree's image.  SHAPE_ORDERED: every number of
+// a node's box, a centre or a voxel is zero or SHAPE_LEAST to SHAPE_LIMIT in
+// magnitude, min <= max on every axis, and the voxel size SHAPE_VOXEL to
+// SHAPE_LIMIT.  Trees that vox_make_tree or the GPU build make from ordinary
 // voxels have it; a caller's own tree need not.
 //
 // SHAPE_NESTED: every child's box and every leaf's voxel lie inside their
 // node's box, and a child on the lower side of a dividing plane reaches at
 // most one voxel past it, one on the upper side not below it.
 constexpr uint32_t SHAPE_ORDERED = 1u, SHAPE_NESTED = 2u;
-constexpr float SHAPE_LIMIT = 1.152921504606847e18f;   // 2^60
+constexpr float SHAPE_LIMIT = 1.152921504606847e18f;     // 2^60
+constexpr float SHAPE_LEAST = 1.6543612251060553e-24f;   // 2^-79
+constexpr float SHAPE_VOXEL = 1.4901161193847656e-8f;    // 2^-26
 
 struct Counts {
     uint32_t nodes, inner, voxels;
@@ -393,7 +395,7 @@ __device__ __forceinline__ int ray_step(const DevTree &t, RaySearch &s, uint4 (&
  *    RN(1/d), q0 = RN(a*y), r = fma(-d, q0, a) (exact), the quotient is
  *    RN(q0 + r*y) -- the correctly rounded a/d for every pair of significands
  *    (checked exhaustively against __fdiv_rn) while nothing leaves the normal
- *    range, which the bounds below ensure for every quotient that is used.
+ *    range, which the bounds below ensure for every quotient.
  *  - Crossings that are not there count as infinitely far, and the order the
  *    reference's selection sort gives is read off three comparisons (ties
  *    included), each child stored at its own place on the stack.
@@ -409,13 +411,19 @@ __device__ __forceinline__ int ray_step(const DevTree &t, RaySearch &s, uint4 (&
  * over four trees 1,203 -> 850 us (782); a near 4K FAST frame of the 512^3 tree
  * 1,496 -> 1,145 us (994); 4M incoherent rays 710 -> 569 us (477). */
 constexpr int STEP_AGAIN = 4;
-constexpr float DIR_MIN = 9.313225746154785e-10f, DIR_MAX = 1048576.0f;   // 2^-30, 2^20
-// Quotients and crossing distances in use are at least this.  A quotient a/d
-// with d >= 2^-30 that is at least 2^-68 has a >= 2^-98, for which r above is
-// exact (its last bit is at least 2^(-98-47)); a numerator below 2^-98 gives a
-// quotient below 2^-68, and a crossing at most 3 * 2^(-68+21) = 2^-45.4 away.
-constexpr float QUOT_MIN = 3.3881317890172014e-21f;    // 2^-68
-constexpr float DIST_MIN = 5.684341886080802e-14f;     // 2^-44
+constexpr float DIR_MIN = 2.384185791015625e-7f, DIR_MAX = 262144.0f;   // 2^-22, 2^18
+// Every coordinate of such a search is a multiple of 2^-102: the image's numbers
+// and the ray's origin are zero or at least SHAPE_LEAST = 2^-79, and so is every
+// q*d that is added to one, as a search goes on only from quotients q of at
+// least QUOT_MIN = 2^-57 (of a crossing that is known by its distance: a smaller
+// q takes a point no more than 3 * 2 * q * DIR_MAX < DIST_MIN away, roundings
+// included).  So a numerator a is zero or at least 2^-102, the quotient a/d at
+// least 2^-120 and r above, a multiple of 2^(-102-47), exact: every quotient is
+// right, those that lose a comparison too.  (With numerators unbounded below,
+// searches over voxels of 2^-145 lost crossings by a wrong last bit.)  A smaller
+// voxel than SHAPE_VOXEL would have many of its searches made again.
+constexpr float QUOT_MIN = 6.938893903907228e-18f;     // 2^-57
+constexpr float DIST_MIN = 1.4551915228366852e-11f;    // 2^-36
 
 __device__ __forceinline__ float quot(float a, float d, float y)
 {
@@ -479,9 +487,11 @@ __device__ __forceinline__ bool mirror_ok(const DevTree &t, float ox, float oy, 
 {
     const float lo = fminf(fminf(fabsf(dx), fabsf(dy)), fabsf(dz)), hi = fmaxf(fmaxf(fabsf(dx), fabsf(dy)), fabsf(dz));
     const float o = fmaxf(fmaxf(fabsf(ox), fabsf(oy)), fabsf(oz));
+    const auto bits = [](float v) { return 2u * __float_as_uint(v) - 1u; };   // of the magnitude; zero's are the largest
+    const uint32_t least = min(min(bits(ox), bits(oy)), bits(oz));
     // (the sum is not finite where a NaN hid from the extremes)
     return (t.shape & SHAPE_ORDERED) && lo >= DIR_MIN && hi <= DIR_MAX && o <= SHAPE_LIMIT &&
-           fabsf(dx + dy + dz) < 4e6f && fabsf(ox + oy + oz) < 4e18f;
+           fabsf(dx + dy + dz) < 4e6f && fabsf(ox + oy + oz) < 4e18f && least >= 2u * __float_as_uint(SHAPE_LEAST) - 1u;
 }
 
 // Whether a hit has a coordinate whose sign of zero the mirror leaves open: a

@@ -490,8 +490,9 @@ __global__ void __launch_bounds__(256) image_shape_kernel(const uint4 *__restric
                                                           float vx, float vy, float vz, uint32_t *__restrict__ bad)
 {
     using vox::ubf;
-    auto fine = [](float v) { return fabsf(v) <= vox::SHAPE_LIMIT; };   // false for NaN
-    bool ok = fine(vx) && fine(vy) && fine(vz) && vx > 0.0f && vy > 0.0f && vz > 0.0f, nested = true;
+    auto fine = [](float v) { return v == 0.0f || (fabsf(v) >= vox::SHAPE_LEAST && fabsf(v) <= vox::SHAPE_LIMIT); };
+    bool ok = fine(vx) && fine(vy) && fine(vz) && vx >= vox::SHAPE_VOXEL && vy >= vox::SHAPE_VOXEL && vz >= vox::SHAPE_VOXEL,
+         nested = true;
     const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id < n_nodes) {
         const uint32_t rec = rec_of_id[id];
