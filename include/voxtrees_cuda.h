@@ -407,7 +407,8 @@ int vox_cuda_batch_create(const vox_cuda_frame_job *jobs, uint32_t njobs,
 /* Change one frame's camera; takes effect at the next launch. */
 int vox_cuda_batch_set_camera(vox_cuda_batch *batch, uint32_t job, const vox_cuda_camera *camera);
 /* Replay the graph on `stream` (asynchronous).  Waits for the batch's
- * previous replay first, so cameras set in between are the ones drawn. */
+ * previous replay first, so cameras set in between are the ones drawn; after a
+ * refresh of one of its trees the graph is made anew first. */
 int vox_cuda_batch_launch(vox_cuda_batch *batch, void *stream);
 int vox_cuda_batch_get_config(const vox_cuda_batch *batch, vox_cuda_batch_config *config);
 int vox_cuda_batch_set_config(vox_cuda_batch *batch, const vox_cuda_batch_config *config);

@@ -315,6 +315,7 @@ struct vox_cuda_batch {
     int cap_class = 0;
     std::vector<vox_cuda_frame_job> jobs;     // caller's jobs, in caller order
     std::vector<uint32_t> order;              // queue position -> caller index
+    std::vector<uint32_t> loads;              // of each job's tree, when the table was made for it
     BatchHead head{};                         // queue totals of the current cameras
     std::vector<BatchJobDev> table;           // host copy, in queue order
     unsigned char *h_stage = nullptr;         // pinned copy of head + table that the graph reads
@@ -331,6 +332,39 @@ struct vox_cuda_batch {
 namespace {
 
 size_t table_bytes(uint32_t njobs) { return sizeof(BatchHead) + (size_t)njobs * sizeof(BatchJobDev); }
+
+// What follows from the jobs' trees as they are now: the stack class and the
+// queue order.
+void follow_trees(vox_cuda_batch *b)
+{
+    const std::vector<vox_cuda_frame_job> &jobs = b->jobs;
+    b->cap_class = 0;
+    b->loads.clear();
+    for (const vox_cuda_frame_job &j : jobs) {
+        b->cap_class = std::max(b->cap_class, j.tree->cap_class);
+        b->loads.push_back(j.tree->loads);
+    }
+    b->order.resize(jobs.size());
+    std::iota(b->order.begin(), b->order.end(), 0u);
+    // frames of the largest tree first (their tiles run longest), each tree's
+    // largest frames first: one tree's frames at a time keep its nodes in L2
+    // (the mixed set: 2.79 ms against 2.81 with the largest frames of all
+    // trees first)
+    std::stable_sort(b->order.begin(), b->order.end(), [&](uint32_t x, uint32_t y) {
+        if (jobs[x].tree->dev.n_units != jobs[y].tree->dev.n_units)
+            return jobs[x].tree->dev.n_units > jobs[y].tree->dev.n_units;
+        if (jobs[x].tree != jobs[y].tree) return jobs[x].tree < jobs[y].tree;
+        return (uint64_t)jobs[x].w * jobs[x].h > (uint64_t)jobs[y].w * jobs[y].h;
+    });
+}
+
+// Whether a job's tree was refreshed since.
+bool trees_changed(const vox_cuda_batch *b)
+{
+    for (size_t i = 0; i < b->jobs.size(); i++)
+        if (b->jobs[i].tree->loads != b->loads[i]) return true;
+    return false;
+}
 
 void fill_table(vox_cuda_batch *b)
 {
@@ -422,19 +456,7 @@ try {
         return VOX_CUDA_ENODEV;
     }
     b->jobs.assign(jobs, jobs + njobs);
-    for (uint32_t i = 0; i < njobs; i++) b->cap_class = std::max(b->cap_class, jobs[i].tree->cap_class);
-    b->order.resize(njobs);
-    std::iota(b->order.begin(), b->order.end(), 0u);
-    // frames of the largest tree first (their tiles run longest), each tree's
-    // largest frames first: one tree's frames at a time keep its nodes in L2
-    // (the mixed set: 2.79 ms against 2.81 with the largest frames of all
-    // trees first)
-    std::stable_sort(b->order.begin(), b->order.end(), [&](uint32_t x, uint32_t y) {
-        if (jobs[x].tree->dev.n_units != jobs[y].tree->dev.n_units)
-            return jobs[x].tree->dev.n_units > jobs[y].tree->dev.n_units;
-        if (jobs[x].tree != jobs[y].tree) return jobs[x].tree < jobs[y].tree;
-        return (uint64_t)jobs[x].w * jobs[x].h > (uint64_t)jobs[y].w * jobs[y].h;
-    });
+    follow_trees(b);
     if (config) b->cfg = *config;
     size_t tb = table_bytes(njobs);
     if (cudaMallocHost(&b->h_stage, tb) != cudaSuccess || cudaMalloc(&b->d_table, tb) != cudaSuccess ||
@@ -472,6 +494,10 @@ try {
     // The graph reads h_stage when it runs: wait for the previous replay before
     // refreshing it with the current cameras.
     if (b->launched && cudaEventSynchronize(b->done) != cudaSuccess) return VOX_CUDA_ECUDA;
+    if (trees_changed(b)) {   // other buffers, boxes, depth and search than the table and the graph have
+        follow_trees(b);
+        if (int rc = build_graph(b)) return rc;
+    }
     stage_table(b);
     cudaStream_t s = as_stream(stream);
     if (cudaGraphLaunch(b->exec, s) != cudaSuccess) return VOX_CUDA_ECUDA;

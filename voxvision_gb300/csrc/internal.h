@@ -34,6 +34,7 @@ struct vox_cuda_tree {
     uint32_t *d_rec_of_id = nullptr;
     uint32_t *d_status = nullptr;          // bit 0: a traversal stack overflowed
     DevTree dev{};
+    uint32_t loads = 0;                    // times an image was loaded: what was made for an earlier one is stale
     int cap_class = 0;                     // 0: 28 stack entries, 1: 64, 2: 256
     FlatTree flat;                         // host copy: pre-order table and maps
     size_t pool_bytes = 0;                 // device pool allocation

@@ -1163,6 +1163,7 @@ static int load_tree(vox_cuda_tree *t, const struct vox_node *root, int layout =
         t->d_rec_of_id = map;
         t->map_bytes = map_bytes;
     }
+    t->loads++;
     t->cap_class = cls;
     if (root) {   // the root record: {min.xyz, max.x}, {max.yz, ...}
         const uint4_host &a = flat.units[0], &b = flat.units[1];
