@@ -68,26 +68,22 @@
 
 #include "internal.h"
 #include "abi_guard.h"
+#include "build_sizes.h"
 
 #define EXPORT extern "C" __attribute__((visibility("default")))
 
 namespace {
 
+using namespace build_sizes;
+
 constexpr uint32_t NONE = 0xFFFFFFFFu;
 constexpr int RAW_THREADS = 256;
 constexpr uint32_t RAW_ITEMS = 16;                       // consecutive samples a thread reads
 constexpr uint32_t RAW_TILE = RAW_THREADS * RAW_ITEMS;   // samples a block reads
-constexpr uint32_t TINY = 32;        // nodes with at most this many voxels, and
-constexpr uint32_t SMALL = 128;      // with at most this many, are split by a lane each,
-constexpr uint32_t LOW = 1024;       // with at most this many by a block of 96 threads,
-constexpr uint32_t MID = 8192;       // with at most this many by a block of 512, and
-constexpr uint32_t HIGH = 32768;     // with at most this many by a block of 1024, larger ones tile by tile
-constexpr uint32_t CHUNK = 1024;     // voxels per chunk
 constexpr int CHUNK_THREADS = 128;   // 8 consecutive voxels per thread
-constexpr int NBIN = 16;             // binades with a precomputed map per chunk
 constexpr uint32_t SAT = 1u << 25;   // map increments saturate here (any >= 2^24 is unusable)
 constexpr int MAX_LEVELS = 90;       // deeper trees exceed the traversal stack anyway
-constexpr uint64_t MAX_VOXELS = 0x7FFFFFFFull;
+static_assert(LEAF == VOX_MAX_DOTS, "leaves");
 
 enum : uint8_t { K_INNER = 0, K_LEAF = 1, K_DENSE = 2, K_OVER = 3 };
 enum : int { S_INNER = 0, S_LEAF = 1, S_DENSE = 2, S_DOTS = 3, S_OVER = 4, NSTATS = 5 };   // a level's counts
@@ -245,19 +241,21 @@ cudaError_t level_alloc(Level &L, uint32_t m, cudaStream_t s)
 // -------------------------------------------------------- per-level kernels
 
 // The nodes of a level that take more than one thread, by size class, in no
-// particular order (above VOX_MAX_DOTS, TINY, SMALL, LOW, MID and HIGH voxels).  A tiled node's slot and its first tile come
-// from one counter, so that first tiles ascend with slots.
+// particular order (above VOX_MAX_DOTS, TINY, SMALL, LOW, MID and HIGH voxels).
+// A tiled node's slot, its first tile and its first sub come from one counter,
+// so that first tiles and subs ascend with slots.
 struct NodeLists {
-    uint32_t *tiny, *small, *low, *mid, *high, *tiled, *first_tile;
+    uint32_t *tiny, *small, *low, *mid, *high, *tiled, *first_tile, *first_sub;
     uint32_t *ntiny, *nsmall, *nlow, *nmid, *nhigh;
-    unsigned long long *ntiled;   // slots in the upper half, tiles in the lower
-    uint32_t tile, shift;         // positions per tile: 1 << shift
+    unsigned long long *ntiled;   // slots from bit 48 on, tiles from bit 24, subs (all below 2^24: N < 2^31)
     __device__ void add_large(uint32_t k, uint32_t n) const
     {
         if (n > HIGH) {
-            const unsigned long long at = atomicAdd(ntiled, (1ull << 32) | ((n + tile - 1) / tile));
-            tiled[at >> 32] = k;
-            first_tile[at >> 32] = (uint32_t)at;
+            const unsigned long long at = atomicAdd(ntiled, (1ull << 48) | ((unsigned long long)parts(n, tile_shift(n)) << 24) |
+                                                                parts(n, SUB_SHIFT));
+            tiled[at >> 48] = k;
+            first_tile[at >> 48] = (uint32_t)(at >> 24) & 0xFFFFFFu;
+            first_sub[at >> 48] = (uint32_t)at & 0xFFFFFFu;
         } else if (n > MID) {
             high[atomicAdd(nhigh, 1u)] = k;
         } else if (n > LOW) {
@@ -268,6 +266,7 @@ struct NodeLists {
             small[atomicAdd(nsmall, 1u)] = k;
         }
     }
+    __device__ uint32_t slots() const { return (uint32_t)(*ntiled >> 48); }
 };
 
 // What a level counts: kinds (S_*), the next level's nodes and the largest.
@@ -276,33 +275,40 @@ struct Tally {
     uint32_t *children, *largest, *err;
 };
 
-// The node of a tile: its slot, or NO_POS for a block without one.
-constexpr uint32_t NO_POS = 0xFFFFFFFFu;
-__device__ __forceinline__ uint32_t tile_slot(const NodeLists &lists, uint32_t tile)
+// The slot whose part (tile or sub) this is, from the slots' first ones: the
+// last that starts at or before it.
+__device__ __forceinline__ uint32_t slot_of(const uint32_t *first, uint32_t slots, uint32_t part)
 {
-    const unsigned long long n = *lists.ntiled;
-    if (tile >= (uint32_t)n) return NO_POS;
-    uint32_t lo = 0, hi = (uint32_t)(n >> 32);
+    uint32_t lo = 0, hi = slots;
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (lists.first_tile[mid] <= tile) lo = mid;
+        if (first[mid] <= part) lo = mid;
         else hi = mid;
     }
     return lo;
 }
 
-// Tiled nodes are summed by chunks of CHUNK voxels, counted through the tiles
-// (a tile is a multiple of CHUNK): the range of chunk c; false for a chunk
-// past its node's end.
+// The node of a tile: its slot, or NO_POS for a block without one.
+constexpr uint32_t NO_POS = 0xFFFFFFFFu;
+__device__ __forceinline__ uint32_t tile_slot(const NodeLists &lists, uint32_t tile)
+{
+    const unsigned long long n = *lists.ntiled;
+    return tile < ((uint32_t)(n >> 24) & 0xFFFFFFu) ? slot_of(lists.first_tile, (uint32_t)(n >> 48), tile) : NO_POS;
+}
+
+// Tiled nodes are summed by chunks of CHUNK voxels, counted through the subs:
+// the range of chunk c; false for a chunk past its node's end.
+constexpr uint32_t SUB_CHUNKS = SUB / CHUNK;
 struct ChunkRange {
     uint32_t k;
     uint64_t b, e;
     __device__ bool find(const NodeLists &lists, const Level &L, uint32_t c)
     {
-        const uint32_t per = lists.tile / CHUNK, slot = tile_slot(lists, c / per);
-        if (slot == NO_POS) return false;
+        const unsigned long long count = *lists.ntiled;
+        if (c / SUB_CHUNKS >= ((uint32_t)count & 0xFFFFFFu)) return false;
+        const uint32_t slot = slot_of(lists.first_sub, (uint32_t)(count >> 48), c / SUB_CHUNKS);
         k = lists.tiled[slot];
-        const uint32_t at = (c - lists.first_tile[slot] * per) * CHUNK, n = L.n[k];
+        const uint32_t at = (c - lists.first_sub[slot] * SUB_CHUNKS) * CHUNK, n = L.n[k];
         if (at >= n) return false;
         b = (uint64_t)L.start[k] + at;
         e = min(b + CHUNK, (uint64_t)L.start[k] + n);
@@ -411,9 +417,9 @@ __global__ void __launch_bounds__(NODE_THREADS) k_box_tiled(Level L, NodeLists l
 {
     after_previous();
     __shared__ Extremes part[NODE_THREADS / 32];
-    if (blockIdx.x >= (uint32_t)(*lists.ntiled >> 32)) return;
+    if (blockIdx.x >= lists.slots()) return;
     const uint32_t k = lists.tiled[blockIdx.x], nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK,
-                   c0 = lists.first_tile[blockIdx.x] * (lists.tile / CHUNK);
+                   c0 = lists.first_sub[blockIdx.x] * SUB_CHUNKS;
     Extremes x;
     x.init();
     for (uint32_t j = threadIdx.x; j < nch; j += NODE_THREADS) {
@@ -584,9 +590,9 @@ __global__ void __launch_bounds__(NODE_THREADS) k_centre_plain(Level L, NodeList
     after_previous();
     __shared__ PlainSum part[NODE_THREADS / 32];
     __shared__ float wsum[NODE_THREADS / 32], carry;
-    if (blockIdx.x >= (uint32_t)(*lists.ntiled >> 32)) return;
+    if (blockIdx.x >= lists.slots()) return;
     const uint32_t k = lists.tiled[blockIdx.x], nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK,
-                   c0 = lists.first_tile[blockIdx.x] * (lists.tile / CHUNK);
+                   c0 = lists.first_sub[blockIdx.x] * SUB_CHUNKS;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     PlainSum x;
     x.init();
@@ -769,8 +775,8 @@ __global__ void __launch_bounds__(CENTRE_WARPS * 32) k_centre_big(const float *P
     const uint32_t lane = threadIdx.x & 31;
     uint32_t j = w / 3;
     int a = (int)(w % 3);
-    if (j >= (uint32_t)(*lists.ntiled >> 32)) return;
-    uint32_t k = lists.tiled[j], c0 = lists.first_tile[j] * (lists.tile / CHUNK);
+    if (j >= lists.slots()) return;
+    uint32_t k = lists.tiled[j], c0 = lists.first_sub[j] * SUB_CHUNKS;
     if (L.kind[k] != K_INNER || !cbase[3 * c0 + a]) return;
     uint32_t nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK;
     uint64_t s = L.start[k], end = s + nk;
@@ -1327,11 +1333,9 @@ __global__ void __launch_bounds__(THREADS) k_nodes_block(Level L, const uint32_t
 // threads, 1,363 with 256 threads, 1,390 with 1,024; with 8 words a warp 1,380
 // (256 threads), with 2 1,405 (1,024 threads).
 constexpr int PASS_THREADS = 512;
-constexpr uint32_t SUB = 2048;          // positions marked at a time; a tile is a multiple of it
-constexpr uint32_t MAX_TILES = 2048;    // tiles of one node
 
 struct Marks {
-    uint4 *word;                        // per word of a tile: claimed bits, count before, last before
+    uint4 *word;                        // per word of a node (from its first sub on): claimed bits, count before, last before
     uint2 *tile;                        // per tile: claimed count, last unclaimed position + 1 (0: none)
 };
 
@@ -1363,10 +1367,10 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_marks(Level L, NodeLists 
     const uint32_t k = lists.tiled[slot], n = L.n[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (L.kind[k] != K_INNER) return;
     const uint64_t start = L.start[k];
-    const uint32_t b = (blockIdx.x - lists.first_tile[slot]) * lists.tile, e = min(n, b + lists.tile);
+    const uint32_t tile = 1u << tile_shift(n), b = (blockIdx.x - lists.first_tile[slot]) * tile, e = min(n, b + tile);
     const float centre[3] = {L.centre[3 * (size_t)k], L.centre[3 * (size_t)k + 1], L.centre[3 * (size_t)k + 2]};
     if (b == 0 && threadIdx.x < 8) L.cnt[8 * (size_t)k + threadIdx.x] = 0;
-    uint64_t word0 = (uint64_t)blockIdx.x * (lists.tile / 32);
+    uint64_t word0 = (uint64_t)lists.first_sub[slot] * (SUB / 32) + b / 32;
     uint32_t run = 0, prev = NO_POS;
     for (uint32_t sb = b; sb < e; sb += SUB, word0 += SUB / 32) {
         const uint32_t nw = (min(e - sb, SUB) + 31) / 32;
@@ -1401,8 +1405,9 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
     __shared__ uint32_t wsum[PASS_THREADS / 32], wtop[PASS_THREADS / 32];
     const uint32_t slot = tile_slot(lists, blockIdx.x);
     if (slot == NO_POS) return;
-    const uint32_t tile = lists.tile, ft = lists.first_tile[slot], ti = blockIdx.x - ft;
+    const uint32_t ft = lists.first_tile[slot], ti = blockIdx.x - ft;
     const uint32_t k = lists.tiled[slot], n = L.n[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t shift = tile_shift(n), tile = 1u << shift;
     const uint64_t start = L.start[k];
     const bool inner = L.kind[k] == K_INNER;
     after_previous();                          // the marks and counts of the pass before
@@ -1411,7 +1416,7 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
     for (uint32_t q = 0; q < o; q++) from += L.cnt[8 * (size_t)k + q];
     const uint32_t b = ti * tile, e = min(n, b + tile);
     if (e <= from) return;                     // all of it placed by earlier passes
-    const uint32_t t0 = from / tile, nt = (n + tile - 1) / tile - t0;   // the tiles still in play
+    const uint32_t t0 = from >> shift, nt = parts(n, shift) - t0;   // the tiles still in play
     // what comes before each of them: a run of tiles a thread, scanned over the block
     constexpr uint32_t PER = MAX_TILES / PASS_THREADS;
     const uint32_t i0 = threadIdx.x * PER;
@@ -1446,17 +1451,17 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
         if (o == 6) L.cnt[8 * (size_t)k + 7] = n - rest;
     }
     __syncthreads();
-    const uint64_t words = (uint64_t)ft * (tile / 32);   // the node's first word: tiles hold whole words
+    const uint64_t words = (uint64_t)lists.first_sub[slot] * (SUB / 32);   // the node's first word
     auto claimed = [&](uint32_t s, uint32_t &c) {
         const uint4 word = in.word[words + (s >> 5)];
-        c = tbefore[(s >> lists.shift) - t0] + word.y + (uint32_t)__popc(word.x & lanes_below(s & 31));
+        c = tbefore[(s >> shift) - t0] + word.y + (uint32_t)__popc(word.x & lanes_below(s & 31));
         return ((word.x >> (s & 31)) & 1u) != 0u;
     };
     auto unclaimed_before = [&](uint32_t s) {
         const uint4 word = in.word[words + (s >> 5)];
         uint32_t l = last_in_word(s >> 5, s & 31, word.x, from);
         if (l == NO_POS) l = word.z;
-        return l != NO_POS ? l : tlast[(s >> lists.shift) - t0];
+        return l != NO_POS ? l : tlast[(s >> shift) - t0];
     };
     uint32_t run = 0, prev = NO_POS;
     for (uint32_t sb = b; sb < e; sb += SUB) {
@@ -1504,7 +1509,7 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_gather(Level L, NodeLists
     const uint32_t k = lists.tiled[slot], n = L.n[k];
     if (L.kind[k] != K_INNER) return;
     const uint64_t start = L.start[k];
-    const uint32_t b = (blockIdx.x - lists.first_tile[slot]) * lists.tile, e = min(n, b + lists.tile);
+    const uint32_t tile = 1u << tile_shift(n), b = (blockIdx.x - lists.first_tile[slot]) * tile, e = min(n, b + tile);
     uint32_t ends[7], sum = 0;
     for (int o = 0; o < 7; o++) ends[o] = sum += L.cnt[8 * (size_t)k + o];
     constexpr uint32_t PER = SUB / PASS_THREADS;
@@ -1533,7 +1538,7 @@ __global__ void k_finish_tiled(Level L, NodeLists lists, Tally tally)
 {
     after_previous();
     const uint32_t slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (slot >= (uint32_t)(*lists.ntiled >> 32)) return;
+    if (slot >= lists.slots()) return;
     const uint32_t k = lists.tiled[slot];
     if (L.kind[k] != K_INNER) return;
     WarpTally mine;
@@ -1984,34 +1989,31 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     lists.nmid = scal + 5;
     lists.nhigh = scal + 8;
     lists.ntiled = reinterpret_cast<unsigned long long *>(scal + 6);
-    while ((uint64_t)MAX_TILES << lists.shift < N || (1u << lists.shift) < SUB) lists.shift++;
-    lists.tile = 1u << lists.shift;
-    const uint64_t max_low = N / SMALL, max_mid = N / LOW, max_high = N / MID, max_tiled = N / HIGH, max_tiles = N / lists.tile + max_tiled,
-                   max_chunks = max_tiles * (lists.tile / CHUNK);
-    TRY(d.get(&lists.tiny, N / (VOX_MAX_DOTS + 1) + 1));
-    TRY(d.get(&lists.small, N / (TINY + 1) + 1));
-    TRY(d.get(&lists.low, max_low + 1));
-    TRY(d.get(&lists.mid, max_mid + 1));
-    TRY(d.get(&lists.high, max_high + 1));
-    // past 2^24 additions a sum's roundings can add up to a sizeable part of it
-    const int window = N > (1u << 24) ? NBIN : 2;
+    const Sizes sz(N);
+    const int window = (int)sz.window;
+    TRY(d.get(&lists.tiny, sz.tiny));
+    TRY(d.get(&lists.small, sz.small));
+    TRY(d.get(&lists.low, sz.low));
+    TRY(d.get(&lists.mid, sz.mid));
+    TRY(d.get(&lists.high, sz.high));
     Marks marks[2] = {};
-    if (N > HIGH) {
+    if (sz.tiled) {
         for (int i = 0; i < 2; i++) {
             TRY(d.get(&idx[i], N));
             TRY(d.get(&oct[i], N));
-            TRY(d.get(&marks[i].word, max_tiles * (lists.tile / 32)));
-            TRY(d.get(&marks[i].tile, max_tiles));
+            TRY(d.get(&marks[i].word, sz.subs * (SUB / 32)));
+            TRY(d.get(&marks[i].tile, sz.tiles));
         }
-        TRY(d.get(&lists.tiled, max_tiled));
-        TRY(d.get(&lists.first_tile, max_tiled));
-        TRY(d.get(&cv, 6 * max_chunks));
-        TRY(d.get(&cidx, 6 * max_chunks));
-        TRY(d.get(&csum, 3 * max_chunks));
-        TRY(d.get(&cgrid, 3 * max_chunks));
-        TRY(d.get(&cbase, 3 * max_chunks));
-        TRY(d.get(&maps, max_chunks * window * 3));
-        TRY(d.get(&starts, 3 * max_tiled));
+        TRY(d.get(&lists.tiled, sz.tiled));
+        TRY(d.get(&lists.first_tile, sz.tiled));
+        TRY(d.get(&lists.first_sub, sz.tiled));
+        TRY(d.get(&cv, 6 * sz.chunks));
+        TRY(d.get(&cidx, 6 * sz.chunks));
+        TRY(d.get(&csum, 3 * sz.chunks));
+        TRY(d.get(&cgrid, 3 * sz.chunks));
+        TRY(d.get(&cbase, 3 * sz.chunks));
+        TRY(d.get(&maps, sz.chunks * window * 3));
+        TRY(d.get(&starts, 3 * sz.tiled));
     }
     TRY(cudaMemsetAsync(scal, 0, 12 * 4, s));
     TRY(cudaMemsetAsync(stats, 0, NSTATS * (MAX_LEVELS + 1) * sizeof(unsigned long long), s));
@@ -2043,47 +2045,48 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         const Tally tally{stats + NSTATS * lv, scal + 2, scal + 3, err};
         if (largest > HIGH) {
             // boxes, centres and the swapping passes of the largest nodes
-            const unsigned nt = (unsigned)max_tiled, nc = (unsigned)max_chunks, np = (unsigned)max_tiles;
+            const uint64_t most = std::min<uint64_t>(m, sz.tiled);   // of the level's nodes
+            const unsigned nt = (unsigned)most, nc = (unsigned)sz.subs_of(most) * SUB_CHUNKS, np = (unsigned)sz.tiles_of(most);
             launch_after(k_chunk_box, nc, CHUNK_THREADS, s, Pc, L, lists, cv, cidx);
             launch_after(k_box_tiled, nt, NODE_THREADS, s, L, lists, cv, cidx, vx, vy, vz, tally);
             launch_after(k_chunk_sums, nc, CHUNK_THREADS, s, Pc, L, lists, csum, cgrid);
             launch_after(k_centre_plain, nt, NODE_THREADS, s, L, lists, csum, cgrid, cbase, window, starts, vx, vy, vz);
-            launch_after(k_chunk_maps, nc, CHUNK_THREADS, s, Pc, L, lists, cbase, window, maps, max_chunks);
-            launch_after(k_centre_big, grid_for(max_tiled * 3 * 32, CENTRE_WARPS * 32), CENTRE_WARPS * 32, s, Pc, L, lists, maps, cbase, csum, window, starts, max_chunks, vx, vy, vz);
+            launch_after(k_chunk_maps, nc, CHUNK_THREADS, s, Pc, L, lists, cbase, window, maps, sz.chunks);
+            launch_after(k_centre_big, grid_for(most * 3 * 32, CENTRE_WARPS * 32), CENTRE_WARPS * 32, s, Pc, L, lists, maps, cbase, csum, window, starts, sz.chunks, vx, vy, vz);
             launch_after(k_tile_marks, np, PASS_THREADS, s, L, lists, Pc, oct[0], marks[0]);
             for (uint32_t o = 0; o < 7; o++) {
                 const int in = o & 1, out = in ^ 1;
                 launch_after(k_tile_pass, np, PASS_THREADS, s, L, lists, o, marks[in], marks[out], idx[in], oct[in], idx[out], oct[out], err);
             }
             launch_after(k_tile_gather, np, PASS_THREADS, s, L, lists, idx[0], idx[1], Pc, Pn);
-            launch_after(k_finish_tiled, grid_for(max_tiled * 32, 256), 256, s, L, lists, tally);
+            launch_after(k_finish_tiled, grid_for(most * 32, 256), 256, s, L, lists, tally);
         }
         bool first = true;   // of the size classes that are made whole
         if (largest > MID) {
             TRY(cudaFuncSetAttribute(k_nodes_block<1024, HIGH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(NodeShared<HIGH>)));
-            launch_after_with(sizeof(NodeShared<HIGH>), k_nodes_block<1024, HIGH>, (unsigned)std::min<uint64_t>(m, max_high),
+            launch_after_with(sizeof(NodeShared<HIGH>), k_nodes_block<1024, HIGH>, (unsigned)std::min<uint64_t>(m, sz.high),
                               1024, s, L, lists.high, lists.nhigh, Pc, Pn, vx, vy, vz, tally, first);
             first = false;
         }
         if (largest > LOW) {
-            launch_after_with(sizeof(NodeShared<MID>), k_nodes_block<512, MID>, (unsigned)std::min<uint64_t>(m, max_mid), 512, s,
+            launch_after_with(sizeof(NodeShared<MID>), k_nodes_block<512, MID>, (unsigned)std::min<uint64_t>(m, sz.mid), 512, s,
                               L, lists.mid, lists.nmid, Pc, Pn, vx, vy, vz, tally, first);
             first = false;
         }
         if (largest > SMALL) {
-            launch_after_with(sizeof(NodeShared<LOW>), k_nodes_block<96, LOW>, (unsigned)std::min<uint64_t>(m, max_low), 96, s,
+            launch_after_with(sizeof(NodeShared<LOW>), k_nodes_block<96, LOW>, (unsigned)std::min<uint64_t>(m, sz.low), 96, s,
                               L, lists.low, lists.nlow, Pc, Pn, vx, vy, vz, tally, first);
             first = false;
         }
         if (largest > TINY) {
-            const unsigned blocks = grid_for(std::min<uint64_t>(m, N / (TINY + 1) + 1), LANE_WARPS);
+            const unsigned blocks = grid_for(std::min<uint64_t>(m, sz.small), LANE_WARPS);
             launch_after(k_nodes_lanes<SMALL>, std::min(blocks, (unsigned)(nsm * 5)), LANE_WARPS * 32, s, L, lists.small,
                          lists.nsmall, Pc, Pn, vx, vy, vz, tally, first);
             first = false;
         }
         if (largest > VOX_MAX_DOTS) {
-            const unsigned blocks = grid_for(std::min<uint64_t>(m, N / (VOX_MAX_DOTS + 1) + 1), LANE_WARPS);
+            const unsigned blocks = grid_for(std::min<uint64_t>(m, sz.tiny), LANE_WARPS);
             launch_after(k_nodes_lanes<TINY>, std::min(blocks, (unsigned)(nsm * 8)), LANE_WARPS * 32, s, L, lists.tiny,
                          lists.ntiny, Pc, Pn, vx, vy, vz, tally, first);
         }
