@@ -484,46 +484,65 @@ render_squares_kernel(DevTree t, vox_cuda_camera cam, uint32_t w, uint32_t h,
 }
 
 // What the searches may rely on in the image (SHAPE_* of traverse.cuh),
-// checked record by record: *bad gets the bits that do not hold.
-__global__ void __launch_bounds__(256) image_shape_kernel(const uint4 *__restrict__ pool,
-                                                          const uint32_t *__restrict__ rec_of_id, uint32_t n_nodes,
-                                                          float vx, float vy, float vz, uint32_t *__restrict__ bad)
+// checked record by record, a thread each: *bad gets the bits that do not hold.
+// The voxels of an overflowed leaf, of which there may be any number, are the
+// block's: 1M equal voxels took one thread 192 ms, an upload of 2.5 ms without.
+constexpr int SHAPE_THREADS = 1024;
+__global__ void __launch_bounds__(SHAPE_THREADS) image_shape_kernel(const uint4 *__restrict__ pool,
+                                                                    const uint32_t *__restrict__ rec_of_id,
+                                                                    uint32_t n_nodes, float vx, float vy, float vz,
+                                                                    uint32_t *__restrict__ bad)
 {
     using vox::ubf;
+    __shared__ uint32_t big[SHAPE_THREADS], n_big;   // the block's records of overflowed leaves
+    if (threadIdx.x == 0) n_big = 0;
+    __syncthreads();
     auto fine = [](float v) { return v == 0.0f || (fabsf(v) >= vox::SHAPE_LEAST && fabsf(v) <= vox::SHAPE_LIMIT); };
     bool ok = fine(vx) && fine(vy) && fine(vz) && vx >= vox::SHAPE_VOXEL && vy >= vox::SHAPE_VOXEL && vz >= vox::SHAPE_VOXEL,
          nested = true;
+    const float vox[3] = {vx, vy, vz};
+    auto voxel = [&](const uint4 v, const float *lo, const float *hi) {   // of a leaf whose box is [lo, hi]
+        const float p[3] = {ubf(v.x), ubf(v.y), ubf(v.z)};
+        for (int k = 0; k < 3; k++) {
+            ok = ok && fine(p[k]);
+            nested = nested && p[k] >= lo[k] && __fadd_rn(p[k], vox[k]) <= hi[k];
+        }
+    };
     const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id < n_nodes) {
         const uint32_t rec = rec_of_id[id];
         const uint4 a = pool[rec], b = pool[rec + 1], c = pool[rec + 2];
-        ok = ok && fine(ubf(a.x)) && fine(ubf(a.y)) && fine(ubf(a.z)) && fine(ubf(a.w)) && fine(ubf(b.x)) &&
-             fine(ubf(b.y)) && ubf(a.x) <= ubf(a.w) && ubf(a.y) <= ubf(b.x) && ubf(a.z) <= ubf(b.y);
+        const float lo[3] = {ubf(a.x), ubf(a.y), ubf(a.z)}, hi[3] = {ubf(a.w), ubf(b.x), ubf(b.y)};
+        for (int k = 0; k < 3; k++) ok = ok && fine(lo[k]) && fine(hi[k]) && lo[k] <= hi[k];
         const uint32_t kind = b.z & 3u;
-        if (kind != VOXP_KIND_DENSE) {
-            const bool inner = kind == VOXP_KIND_INNER;
-            if (inner) ok = ok && fine(ubf(c.x)) && fine(ubf(c.y)) && fine(ubf(c.z));
-            const float lo[3] = {ubf(a.x), ubf(a.y), ubf(a.z)}, hi[3] = {ubf(a.w), ubf(b.x), ubf(b.y)};
-            const float plane[3] = {ubf(c.x), ubf(c.y), ubf(c.z)}, vox[3] = {vx, vy, vz};
-            const uint32_t mask = (b.z >> 8) & 0xFFu, n = inner ? (uint32_t)__popc(mask) : b.z >> 2;
+        if (kind == VOXP_KIND_INNER) {
+            const float plane[3] = {ubf(c.x), ubf(c.y), ubf(c.z)};
+            const uint32_t mask = (b.z >> 8) & 0xFFu, n = (uint32_t)__popc(mask);
             uint32_t oct = 0;   // of the i-th child
             for (uint32_t i = 0; i < n; i++, oct++) {
-                const uint4 v = pool[b.w + (inner ? VOXP_REC_UNITS * i : i)];
-                const float p[3] = {ubf(v.x), ubf(v.y), ubf(v.z)};
-                float q[3] = {__fadd_rn(p[0], vx), __fadd_rn(p[1], vy), __fadd_rn(p[2], vz)};
-                if (inner) {
-                    const uint4 u = pool[b.w + VOXP_REC_UNITS * i + 1];
-                    q[0] = ubf(v.w); q[1] = ubf(u.x); q[2] = ubf(u.y);
-                    while (!((mask >> oct) & 1u)) oct++;
-                }
-                for (int k = 0; k < 3; k++) {
-                    if (!inner) ok = ok && fine(p[k]);
-                    nested = nested && p[k] >= lo[k] && q[k] <= hi[k];
-                    if (inner)
-                        nested = nested && ((oct >> k) & 1u ? q[k] <= __fadd_rn(plane[k], vox[k]) : p[k] >= plane[k]);
-                }
+                const uint4 v = pool[b.w + VOXP_REC_UNITS * i], u = pool[b.w + VOXP_REC_UNITS * i + 1];
+                const float p[3] = {ubf(v.x), ubf(v.y), ubf(v.z)}, q[3] = {ubf(v.w), ubf(u.x), ubf(u.y)};
+                while (!((mask >> oct) & 1u)) oct++;
+                for (int k = 0; k < 3; k++)
+                    nested = nested && p[k] >= lo[k] && q[k] <= hi[k] &&
+                             ((oct >> k) & 1u ? q[k] <= __fadd_rn(plane[k], vox[k]) : p[k] >= plane[k]);
             }
+            for (int k = 0; k < 3; k++) ok = ok && fine(plane[k]);
+        } else if (kind == VOXP_KIND_LEAF) {
+            const uint32_t n = b.z >> 2;
+            if (n > VOX_MAX_DOTS) big[atomicAdd(&n_big, 1u)] = rec;
+            else
+                for (uint32_t i = 0; i < n; i++) voxel(pool[b.w + i], lo, hi);
         }
+    }
+    __syncthreads();
+    for (uint32_t i = 0; i < n_big; i++) {
+        const uint32_t rec = big[i];
+        const uint4 a = pool[rec], b = pool[rec + 1];
+        const float lo[3] = {ubf(a.x), ubf(a.y), ubf(a.z)}, hi[3] = {ubf(a.w), ubf(b.x), ubf(b.y)};
+        const uint32_t n = b.z >> 2;
+#pragma unroll 4
+        for (uint32_t j = threadIdx.x; j < n; j += SHAPE_THREADS) voxel(pool[b.w + j], lo, hi);
     }
     const uint32_t missing = __reduce_or_sync(0xFFFFFFFFu, (ok ? 0u : vox::SHAPE_ORDERED) | (nested ? 0u : vox::SHAPE_NESTED));
     if (missing && (threadIdx.x & 31) == 0) atomicOr(bad, missing);
@@ -1092,7 +1111,7 @@ cudaError_t image_shape(const uint4 *pool, const uint32_t *rec_of_id, uint64_t n
 {
     cudaError_t e = cudaMemsetAsync(word, 0, 4, s);
     if (e != cudaSuccess || nodes == 0) return e;
-    image_shape_kernel<<<(unsigned)((nodes + 255) / 256), 256, 0, s>>>(pool, rec_of_id, (uint32_t)nodes, voxel[0],
+    image_shape_kernel<<<(unsigned)((nodes + SHAPE_THREADS - 1) / SHAPE_THREADS), SHAPE_THREADS, 0, s>>>(pool, rec_of_id, (uint32_t)nodes, voxel[0],
                                                                        voxel[1], voxel[2], word);
     count_launch();
     return cudaGetLastError();
