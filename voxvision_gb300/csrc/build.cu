@@ -1958,6 +1958,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
 
     Dev d(s);
     std::vector<Level> levels;
+    levels.reserve(MAX_LEVELS + 1);   // throws here or not at all
     struct LevelFree {
         std::vector<Level> &v;
         cudaStream_t s;
@@ -2213,15 +2214,14 @@ int new_tree(vox_cuda_tree **out, F f)
     if (cudaGetDevice(&dev) != cudaSuccess) return VOX_CUDA_ENODEV;
     Stream st;
     if (!st.s) return VOX_CUDA_ECUDA;
-    vox_cuda_tree *t = new (std::nothrow) vox_cuda_tree();
-    if (!t) return VOX_CUDA_ENOMEM;
-    t->device = dev;
-    int rc = f(t, st.s);
-    if (rc) {
-        vox_cuda_tree_free(t);
-        return rc;
-    }
-    *out = t;
+    struct Owned {
+        vox_cuda_tree *t;
+        ~Owned() { if (t) vox_cuda_tree_free(t); }   // on an error, also one that f throws
+    } own{new (std::nothrow) vox_cuda_tree(dev)};
+    if (!own.t) return VOX_CUDA_ENOMEM;
+    if (int rc = f(own.t, st.s)) return rc;
+    *out = own.t;
+    own.t = nullptr;
     return VOX_CUDA_OK;
 }
 

@@ -7,7 +7,6 @@
 
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <cstdint>
 #include <mutex>
 #include <utility>
@@ -15,6 +14,7 @@
 
 #include "flatten.h"
 #include "frame_memo.h"
+#include "pool.h"
 #include "pool_layout.h"
 #include "traverse.cuh"
 #include "../../include/voxtrees_cuda.h"
@@ -22,13 +22,12 @@
 using vox::DevTree;
 
 struct vox_cuda_tree {
-    static std::atomic<int> live;          // trees there are
-    vox_cuda_tree() { live++; }
-    ~vox_cuda_tree() { live--; }
+    explicit vox_cuda_tree(int dev) : device(dev) { tree_made(dev); }
+    ~vox_cuda_tree() { tree_gone(device); }   // after its buffers are freed
     vox_cuda_tree(const vox_cuda_tree &) = delete;
     vox_cuda_tree &operator=(const vox_cuda_tree &) = delete;
     bool pooled = false;                   // the buffers below come from pool_alloc
-    int device = 0;
+    const int device;
     float bbox[6] = {0, 0, 0, 0, 0, 0};   // root bounding box (for scheduling only)
     uint4 *d_pool = nullptr;
     uint32_t *d_rec_of_id = nullptr;
@@ -104,17 +103,6 @@ inline int cap_class_for_depth(uint64_t depth)
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
 inline int status_of(cudaError_t e) { return e == cudaSuccess ? VOX_CUDA_OK : VOX_CUDA_ECUDA; }
-
-/* Stream-ordered memory of the current device, freed with cudaFreeAsync (or
- * cudaFree once nothing uses it): the library's scratch and the trees it builds.
- * It comes from a pool of the library's own that keeps up to POOL_KEEP bytes
- * across synchronisations, where the default pool gives everything back and
- * maps it anew: five 16 MB buffers allocated, freed and synchronised cost 20 us
- * against 240-390, a build's 37 MB image and its map and status 10 us against
- * 190.  What it keeps goes back when the last tree is freed (pool_trim). */
-constexpr uint64_t POOL_KEEP = 512ull << 20;
-cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s);
-void pool_trim();
 
 /* A page-locked page of the calling thread for what a synchronous call reads
  * back (THREAD_PAGE bytes; NULL when it cannot be had), kept until the thread

@@ -776,44 +776,6 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 void count_launch() { g_launches++; }
 
-std::atomic<int> vox_cuda_tree::live{0};
-
-namespace {
-constexpr int POOL_DEVICES = 64;
-std::mutex g_pool_mu;
-std::atomic<cudaMemPool_t> g_pool[POOL_DEVICES];
-}  // namespace
-
-cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s)
-{
-    *p = nullptr;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    cudaMemPool_t pool = dev < POOL_DEVICES ? g_pool[dev].load() : nullptr;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (!pool && dev < POOL_DEVICES && cudaStreamIsCapturing(s, &cap) == cudaSuccess &&
-        cap == cudaStreamCaptureStatusNone) {   // (no pool is made inside a capture)
-        std::lock_guard<std::mutex> lock(g_pool_mu);
-        pool = g_pool[dev].load();
-        if (!pool) {
-            cudaMemPoolProps props = {};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
-            uint64_t keep = POOL_KEEP;
-            if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
-                cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-                g_pool[dev].store(pool);
-            } else {
-                pool = nullptr;
-                cudaGetLastError();
-            }
-        }
-    }
-    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
-}
-
 void *thread_page()
 {
     struct Page {
@@ -827,15 +789,6 @@ void *thread_page()
     if (!page.p && cudaHostAlloc(&page.p, THREAD_PAGE, cudaHostAllocPortable) != cudaSuccess) page.p = nullptr;
     return page.p;
 }
-
-void pool_trim()
-{
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev >= POOL_DEVICES) return;
-    if (cudaMemPool_t pool = g_pool[dev].load()) cudaMemPoolTrimTo(pool, 0);
-}
-
-
 
 // Linear map of screen2world: direction = M * (mul*sx - xsub, 1, ysub' - mul*sy)
 // with ysub' = ysub for the simple camera (quaternion rotation, every term of
@@ -1299,9 +1252,8 @@ static int upload_as(const struct vox_node *root, int layout, const float *voxel
     *out = nullptr;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return VOX_CUDA_ENODEV;
-    vox_cuda_tree *t = new (std::nothrow) vox_cuda_tree();
+    vox_cuda_tree *t = new (std::nothrow) vox_cuda_tree(dev);
     if (!t) return VOX_CUDA_ENOMEM;
-    t->device = dev;
     int rc = load_tree(t, root, layout, voxel);
     if (rc) {
         cudaFree(t->d_pool);
@@ -1375,7 +1327,6 @@ try {
     cudaFree(t->d_rec_of_id);
     cudaFree(t->d_status);
     delete t;
-    if (vox_cuda_tree::live.load() == 0) pool_trim();
     if (cur != dev) cudaSetDevice(cur);
     return VOX_CUDA_OK;
 } VOX_ABI_FAIL_INT
