@@ -75,7 +75,7 @@ def pool(tmp_path):
     inc = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
     src, so = tmp_path / "fake.cpp", tmp_path / "pool.so"
     src.write_text(FAKE)
-    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, "-I", inc, str(src),
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", CSRC, "-I", inc, str(src),
                     os.path.join(CSRC, "pool.cpp"), "-o", str(so), "-lpthread"], check=True)
     m = C.CDLL(str(so))
     m.alloc.argtypes, m.keeps.restype = [C.c_size_t], C.c_uint64
