@@ -35,7 +35,7 @@ CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-ffp-contract
 
 CUDA_SOURCES = ["voxtrees_cuda.cu", "batch.cu", "server.cu", "build.cu", "raysort.cu", "make_tree.cu"]
 C_SOURCES = ["host_tree.c", "cameras.c", "lights.c", "modules.c"]
-CXX_SOURCES = ["flatten.cpp", "dropin_search.cpp", "renderer.cpp", "pool.cpp"]
+CXX_SOURCES = ["flatten.cpp", "dropin_search.cpp", "renderer.cpp", "pool.cpp", "host_wait.cpp"]
 
 
 def _nvcc() -> str:

@@ -69,6 +69,7 @@
 #include "internal.h"
 #include "abi_guard.h"
 #include "build_sizes.h"
+#include "host_wait.h"
 
 #define EXPORT extern "C" __attribute__((visibility("default")))
 
@@ -1824,20 +1825,6 @@ __global__ void __launch_bounds__(128) k_all_done(Level root, const unsigned lon
     if (threadIdx.x == 0) *static_cast<volatile uint32_t *>(&back->step) = step;
 }
 
-// Waits for `step` from the stream's kernels; an error when they end without it.
-cudaError_t wait_step(const Back *back, uint32_t step, cudaStream_t s)
-{
-    for (uint32_t spin = 1;; spin++) {
-        if (__atomic_load_n(&back->step, __ATOMIC_ACQUIRE) == step) return cudaSuccess;
-        if (spin % 1024 == 0) {
-            const cudaError_t e = cudaStreamQuery(s);
-            if (e == cudaErrorNotReady) continue;
-            if (e != cudaSuccess) return e;
-            return __atomic_load_n(&back->step, __ATOMIC_ACQUIRE) == step ? cudaSuccess : cudaErrorUnknown;
-        }
-    }
-}
-
 // ------------------------------------------------------------ raw reader
 
 // Which samples are solid (datareader.c:51-77): 16 consecutive ones a thread,
@@ -2030,6 +2017,8 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     Back *back_d = static_cast<Back *>(back_dev);
     back->step = 0;
     uint32_t step = 0;
+    unsigned schedule = 0;
+    TRY(wait_schedule(&schedule));
 
     Level root;
     TRY(level_alloc(root, 1, s));
@@ -2093,7 +2082,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
         }
         launch_after(k_level_done, 1, 1, s, scal, back_d, ++step);
         TRY(cudaGetLastError());
-        TRY(wait_step(back, step, s));
+        TRY(wait_for_word(&back->step, step, schedule, s));
         const uint32_t mn = back->next[0];
         largest = back->next[1];
         if (mn == 0) break;
@@ -2112,7 +2101,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     }
     launch_after(k_all_done, 1, 128, s, levels[0], stats, err, back_d, ++step);
     TRY(cudaGetLastError());
-    TRY(wait_step(back, step, s));
+    TRY(wait_for_word(&back->step, step, schedule, s));
     if (back->err & ERR_WALK) return VOX_CUDA_ECUDA;
     if (back->err & ERR_BIG_LEAF) return VOX_CUDA_ETOOBIG;
     uint64_t units = VOXP_REC_UNITS + back->units;
