@@ -246,7 +246,8 @@ cudaError_t level_alloc(Level &L, uint32_t m, cudaStream_t s)
 // A tiled node's slot, its first tile and its first sub come from one counter,
 // so that first tiles and subs ascend with slots.
 struct NodeLists {
-    uint32_t *tiny, *small, *low, *mid, *high, *tiled, *first_tile, *first_sub;
+    uint32_t *tiny, *small, *low, *mid, *high;
+    uint4 *tiled;                 // a slot: its node, first tile, first sub and voxels, in one load
     uint32_t *ntiny, *nsmall, *nlow, *nmid, *nhigh;
     unsigned long long *ntiled;   // slots from bit 48 on, tiles from bit 24, subs (all below 2^24: N < 2^31)
     __device__ void add_large(uint32_t k, uint32_t n) const
@@ -254,9 +255,7 @@ struct NodeLists {
         if (n > HIGH) {
             const unsigned long long at = atomicAdd(ntiled, (1ull << 48) | ((unsigned long long)parts(n, tile_shift(n)) << 24) |
                                                                 parts(n, SUB_SHIFT));
-            tiled[at >> 48] = k;
-            first_tile[at >> 48] = (uint32_t)(at >> 24) & 0xFFFFFFu;
-            first_sub[at >> 48] = (uint32_t)at & 0xFFFFFFu;
+            tiled[at >> 48] = make_uint4(k, (uint32_t)(at >> 24) & 0xFFFFFFu, (uint32_t)at & 0xFFFFFFu, n);
         } else if (n > MID) {
             high[atomicAdd(nhigh, 1u)] = k;
         } else if (n > LOW) {
@@ -276,26 +275,41 @@ struct Tally {
     uint32_t *children, *largest, *err;
 };
 
-// The slot whose part (tile or sub) this is, from the slots' first ones: the
-// last that starts at or before it.
-__device__ __forceinline__ uint32_t slot_of(const uint32_t *first, uint32_t slots, uint32_t part)
+constexpr uint32_t NO_POS = 0xFFFFFFFFu;
+
+// The slot whose part (tile or sub, by `first`) this is: the last that starts at
+// or before it.
+template <class F>
+__device__ __forceinline__ uint32_t slot_of(const uint4 *tiled, uint32_t slots, uint32_t part, F first)
 {
     uint32_t lo = 0, hi = slots;
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (first[mid] <= part) lo = mid;
+        if (first(tiled[mid]) <= part) lo = mid;
         else hi = mid;
     }
     return lo;
 }
 
-// The node of a tile: its slot, or NO_POS for a block without one.
-constexpr uint32_t NO_POS = 0xFFFFFFFFu;
-__device__ __forceinline__ uint32_t tile_slot(const NodeLists &lists, uint32_t tile)
-{
-    const unsigned long long n = *lists.ntiled;
-    return tile < ((uint32_t)(n >> 24) & 0xFFFFFFu) ? slot_of(lists.first_tile, (uint32_t)(n >> 48), tile) : NO_POS;
-}
+// A block's tile of a tiled node: the node, its voxels, first tile and first
+// sub, the tile's size and its positions in the node; false for a block
+// without one.  (From the slot alone: with loads by node and by slot on the way
+// the 256^3 raw volume took 1,352 us, 1,345 with this.)
+struct TileRange {
+    uint32_t k, n, ft, fs, shift, b, e;
+    __device__ __forceinline__ bool find(const NodeLists &lists)
+    {
+        const unsigned long long count = *lists.ntiled;
+        if (blockIdx.x >= ((uint32_t)(count >> 24) & 0xFFFFFFu)) return false;
+        const uint4 s = lists.tiled[slot_of(lists.tiled, (uint32_t)(count >> 48), blockIdx.x, [](const uint4 &x) { return x.y; })];
+        k = s.x; ft = s.y; fs = s.z; n = s.w;
+        shift = tile_shift(n);
+        b = (blockIdx.x - ft) << shift;
+        e = min(n, b + (1u << shift));
+        return true;
+    }
+    __device__ __forceinline__ uint64_t words() const { return (uint64_t)fs * (SUB / 32); }   // the node's first word
+};
 
 // Tiled nodes are summed by chunks of CHUNK voxels, counted through the subs:
 // the range of chunk c; false for a chunk past its node's end.
@@ -307,9 +321,9 @@ struct ChunkRange {
     {
         const unsigned long long count = *lists.ntiled;
         if (c / SUB_CHUNKS >= ((uint32_t)count & 0xFFFFFFu)) return false;
-        const uint32_t slot = slot_of(lists.first_sub, (uint32_t)(count >> 48), c / SUB_CHUNKS);
-        k = lists.tiled[slot];
-        const uint32_t at = (c - lists.first_sub[slot] * SUB_CHUNKS) * CHUNK, n = L.n[k];
+        const uint4 s = lists.tiled[slot_of(lists.tiled, (uint32_t)(count >> 48), c / SUB_CHUNKS, [](const uint4 &x) { return x.z; })];
+        k = s.x;
+        const uint32_t at = (c - s.z * SUB_CHUNKS) * CHUNK, n = s.w;
         if (at >= n) return false;
         b = (uint64_t)L.start[k] + at;
         e = min(b + CHUNK, (uint64_t)L.start[k] + n);
@@ -419,8 +433,8 @@ __global__ void __launch_bounds__(NODE_THREADS) k_box_tiled(Level L, NodeLists l
     after_previous();
     __shared__ Extremes part[NODE_THREADS / 32];
     if (blockIdx.x >= lists.slots()) return;
-    const uint32_t k = lists.tiled[blockIdx.x], nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK,
-                   c0 = lists.first_sub[blockIdx.x] * SUB_CHUNKS;
+    const uint4 slot = lists.tiled[blockIdx.x];
+    const uint32_t k = slot.x, nk = slot.w, nch = (nk + CHUNK - 1) / CHUNK, c0 = slot.z * SUB_CHUNKS;
     Extremes x;
     x.init();
     for (uint32_t j = threadIdx.x; j < nch; j += NODE_THREADS) {
@@ -592,8 +606,8 @@ __global__ void __launch_bounds__(NODE_THREADS) k_centre_plain(Level L, NodeList
     __shared__ PlainSum part[NODE_THREADS / 32];
     __shared__ float wsum[NODE_THREADS / 32], carry;
     if (blockIdx.x >= lists.slots()) return;
-    const uint32_t k = lists.tiled[blockIdx.x], nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK,
-                   c0 = lists.first_sub[blockIdx.x] * SUB_CHUNKS;
+    const uint4 slot = lists.tiled[blockIdx.x];
+    const uint32_t k = slot.x, nk = slot.w, nch = (nk + CHUNK - 1) / CHUNK, c0 = slot.z * SUB_CHUNKS;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     PlainSum x;
     x.init();
@@ -777,10 +791,11 @@ __global__ void __launch_bounds__(CENTRE_WARPS * 32) k_centre_big(const float *P
     uint32_t j = w / 3;
     int a = (int)(w % 3);
     if (j >= lists.slots()) return;
-    uint32_t k = lists.tiled[j], c0 = lists.first_sub[j] * SUB_CHUNKS;
+    const uint4 slot = lists.tiled[j];
+    const uint32_t k = slot.x, c0 = slot.z * SUB_CHUNKS;
     if (L.kind[k] != K_INNER || !cbase[3 * c0 + a]) return;
-    uint32_t nk = L.n[k], nch = (nk + CHUNK - 1) / CHUNK;
-    uint64_t s = L.start[k], end = s + nk;
+    const uint32_t nk = slot.w, nch = (nk + CHUNK - 1) / CHUNK;
+    const uint64_t s = L.start[k], end = s + nk;
     const uint2 first = starts[3 * j + a];
     float mn = L.box[6 * k + a], acc = __uint_as_float(first.y);
     uint32_t g = first.x;
@@ -1363,15 +1378,14 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_marks(Level L, NodeLists 
 {
     after_previous();
     __shared__ SubMarks sub;
-    const uint32_t slot = tile_slot(lists, blockIdx.x);
-    if (slot == NO_POS) return;
-    const uint32_t k = lists.tiled[slot], n = L.n[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    TileRange range;
+    if (!range.find(lists)) return;
+    const uint32_t k = range.k, b = range.b, e = range.e, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (L.kind[k] != K_INNER) return;
     const uint64_t start = L.start[k];
-    const uint32_t tile = 1u << tile_shift(n), b = (blockIdx.x - lists.first_tile[slot]) * tile, e = min(n, b + tile);
     const float centre[3] = {L.centre[3 * (size_t)k], L.centre[3 * (size_t)k + 1], L.centre[3 * (size_t)k + 2]};
     if (b == 0 && threadIdx.x < 8) L.cnt[8 * (size_t)k + threadIdx.x] = 0;
-    uint64_t word0 = (uint64_t)lists.first_sub[slot] * (SUB / 32) + b / 32;
+    uint64_t word0 = range.words() + b / 32;
     uint32_t run = 0, prev = NO_POS;
     for (uint32_t sb = b; sb < e; sb += SUB, word0 += SUB / 32) {
         const uint32_t nw = (min(e - sb, SUB) + 31) / 32;
@@ -1404,18 +1418,17 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
     __shared__ SubMarks sub;
     __shared__ uint32_t tbefore[MAX_TILES], tlast[MAX_TILES];
     __shared__ uint32_t wsum[PASS_THREADS / 32], wtop[PASS_THREADS / 32];
-    const uint32_t slot = tile_slot(lists, blockIdx.x);
-    if (slot == NO_POS) return;
-    const uint32_t ft = lists.first_tile[slot], ti = blockIdx.x - ft;
-    const uint32_t k = lists.tiled[slot], n = L.n[k], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t shift = tile_shift(n), tile = 1u << shift;
+    TileRange range;
+    if (!range.find(lists)) return;
+    const uint32_t k = range.k, n = range.n, ft = range.ft, shift = range.shift, b = range.b, e = range.e,
+                   lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t words = range.words();
     const uint64_t start = L.start[k];
     const bool inner = L.kind[k] == K_INNER;
     after_previous();                          // the marks and counts of the pass before
     if (!inner) return;
     uint32_t from = 0;
     for (uint32_t q = 0; q < o; q++) from += L.cnt[8 * (size_t)k + q];
-    const uint32_t b = ti * tile, e = min(n, b + tile);
     if (e <= from) return;                     // all of it placed by earlier passes
     const uint32_t t0 = from >> shift, nt = parts(n, shift) - t0;   // the tiles still in play
     // what comes before each of them: a run of tiles a thread, scanned over the block
@@ -1452,7 +1465,6 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_pass(Level L, NodeLists l
         if (o == 6) L.cnt[8 * (size_t)k + 7] = n - rest;
     }
     __syncthreads();
-    const uint64_t words = (uint64_t)lists.first_sub[slot] * (SUB / 32);   // the node's first word
     auto claimed = [&](uint32_t s, uint32_t &c) {
         const uint4 word = in.word[words + (s >> 5)];
         c = tbefore[(s >> shift) - t0] + word.y + (uint32_t)__popc(word.x & lanes_below(s & 31));
@@ -1505,12 +1517,11 @@ __global__ void __launch_bounds__(PASS_THREADS) k_tile_gather(Level L, NodeLists
                                                               const uint32_t *idx1, const float *P, float *Pn)
 {
     after_previous();
-    const uint32_t slot = tile_slot(lists, blockIdx.x);
-    if (slot == NO_POS) return;
-    const uint32_t k = lists.tiled[slot], n = L.n[k];
+    TileRange range;
+    if (!range.find(lists)) return;
+    const uint32_t k = range.k, b = range.b, e = range.e;
     if (L.kind[k] != K_INNER) return;
     const uint64_t start = L.start[k];
-    const uint32_t tile = 1u << tile_shift(n), b = (blockIdx.x - lists.first_tile[slot]) * tile, e = min(n, b + tile);
     uint32_t ends[7], sum = 0;
     for (int o = 0; o < 7; o++) ends[o] = sum += L.cnt[8 * (size_t)k + o];
     constexpr uint32_t PER = SUB / PASS_THREADS;
@@ -1540,10 +1551,10 @@ __global__ void k_finish_tiled(Level L, NodeLists lists, Tally tally)
     after_previous();
     const uint32_t slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (slot >= lists.slots()) return;
-    const uint32_t k = lists.tiled[slot];
+    const uint32_t k = lists.tiled[slot].x;
     if (L.kind[k] != K_INNER) return;
     WarpTally mine;
-    const uint32_t m = mine.split(L, k, L.n[k], lane < 8 ? L.cnt[8 * (size_t)k + lane] : 0u, tally.err);
+    const uint32_t m = mine.split(L, k, lists.tiled[slot].w, lane < 8 ? L.cnt[8 * (size_t)k + lane] : 0u, tally.err);
     if (lane == 0 && m) L.first_child[k] = atomicAdd(tally.children, (uint32_t)__popc(m));
     mine.flush(tally);
 }
@@ -1993,8 +2004,6 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
             TRY(d.get(&marks[i].tile, sz.tiles));
         }
         TRY(d.get(&lists.tiled, sz.tiled));
-        TRY(d.get(&lists.first_tile, sz.tiled));
-        TRY(d.get(&lists.first_sub, sz.tiled));
         TRY(d.get(&cv, 6 * sz.chunks));
         TRY(d.get(&cidx, 6 * sz.chunks));
         TRY(d.get(&csum, 3 * sz.chunks));

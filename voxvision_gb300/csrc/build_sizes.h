@@ -60,7 +60,7 @@ struct Sizes {
     uint64_t lists() const { return 4 * (tiny + small + low + mid + high); }
     uint64_t orders() const { return tiled ? 2 * N * (4 + 1) : 0; }                 // places and octants, twice
     uint64_t marks() const { return 2 * (subs * (SUB / 32) * 16 + tiles * 8); }
-    uint64_t sums() const { return chunks * (24 + 24 + 12 + 12 + 3 + (uint64_t)window * 3 * 8) + tiled * (12 + 3 * 8); }
+    uint64_t sums() const { return chunks * (24 + 24 + 12 + 12 + 3 + (uint64_t)window * 3 * 8) + tiled * (16 + 3 * 8); }
     // beside the two orders of the voxels themselves (24 bytes a voxel)
     uint64_t scratch() const { return lists() + orders() + marks() + sums(); }
 };
