@@ -726,15 +726,16 @@ __device__ __noinline__ GeneralResult trace_general_call(const uint4 *pool, uint
 
 /* The whole search from the node whose record is at `start`.  Returns true
  * on a hit; `overflow` is set (and the search ends as a miss) on STEP_ERROR.
- * Counting searches count the reference's work: the general search. */
-template <int CAP, bool COUNT, bool MZERO_CONST = false>
+ * Counting searches count the reference's work: the general search, as those
+ * of a kernel built for images that the mirrored one leaves (GENERAL). */
+template <int CAP, bool COUNT, bool MZERO_CONST = false, bool GENERAL = false>
 __device__ __forceinline__ bool trace_ray(const DevTree &t, uint32_t start,
                                           float ox0, float oy0, float oz0,
                                           float dx, float dy, float dz,
                                           RayHit &hit, Counts &cnt, bool &overflow)
 {
     uint4 stack[CAP];
-    if (COUNT) return trace_general<CAP, COUNT>(t, start, ox0, oy0, oz0, dx, dy, dz, stack, hit, cnt, overflow);
+    if (COUNT || GENERAL) return trace_general<CAP, COUNT>(t, start, ox0, oy0, oz0, dx, dy, dz, stack, hit, cnt, overflow);
     int r = STEP_AGAIN;
     if (mirror_ok(t, ox0, oy0, oz0, dx, dy, dz))
         r = trace_mirrored<CAP, MZERO_CONST>(t, start, ox0, oy0, oz0, dx, dy, dz, stack, hit);

@@ -240,7 +240,10 @@ __device__ __forceinline__ void clear_outside(const FramePlan &p, uint32_t w, ui
 // its frames take 98 us against 88.
 constexpr int RENDER_MIN_BLOCKS = 8;
 
-template <int CAP, bool COUNT, bool LIT>
+// A build for images without SHAPE_ORDERED (GENERAL) has the general search in
+// line: a 1080p frame of such an image takes 89 us, 93 through the call that
+// searches left over by the mirrored one take.
+template <int CAP, bool COUNT, bool LIT, bool GENERAL>
 __global__ void __launch_bounds__(128, RENDER_MIN_BLOCKS) render_kernel(DevTree t, vox_cuda_camera cam, uint32_t w, uint32_t h,
                                                      FramePlan p, const uint8_t *__restrict__ tex,
                                                      uint32_t *__restrict__ argb,
@@ -265,7 +268,7 @@ __global__ void __launch_bounds__(128, RENDER_MIN_BLOCKS) render_kernel(DevTree 
         float dx, dy, dz;
         vox::screen2world(cam, (int)px, (int)py, dx, dy, dz);
         if (t.root != VOXP_EMPTY)
-            hit = vox::trace_ray<CAP, COUNT>(t, t.root, cam.position[0], cam.position[1], cam.position[2],
+            hit = vox::trace_ray<CAP, COUNT, false, GENERAL>(t, t.root, cam.position[0], cam.position[1], cam.position[2],
                                              dx, dy, dz, hh, c, overflow);
     }
     pdl_wait();
@@ -309,7 +312,9 @@ __device__ __forceinline__ void pixel_dir(const vox_cuda_camera &cam, const floa
 // Register bound of render_squares_kernel: 7 blocks of 128 threads per SM (72
 // registers).  Unbounded it takes 80 (6 blocks): the 1080p orbit's ADAPTIVE
 // frames take 77.6 us with the bound and 79.2 without, the near 4K FAST frame
-// 1,040 and 1,070 us; 8 blocks give 78.5 and 1,033 us.
+// 1,040 and 1,070 us; 8 blocks give 78.5 and 1,033 us.  The build for images
+// without SHAPE_ORDERED (GENERAL, as for BEST frames): a 1080p ADAPTIVE frame of
+// one 110 us (119 through the call), 115 unbounded, 113 with 8 blocks.
 constexpr int SQUARES_MIN_BLOCKS = 7;
 
 // FAST and ADAPTIVE frames, and with a ray buffer frames of every quality,
@@ -330,7 +335,7 @@ constexpr int SQUARES_MIN_BLOCKS = 7;
 // results are the reference's by construction: the same searches of the
 // same rays, the same choices between them; searches made for pixels the
 // walk then reaches another way are dropped.
-template <int CAP, bool RAYS>
+template <int CAP, bool RAYS, bool GENERAL>
 __global__ void __launch_bounds__(128, SQUARES_MIN_BLOCKS)
 render_squares_kernel(DevTree t, vox_cuda_camera cam, uint32_t w, uint32_t h,
                                                      FramePlan fp, unsigned int quality,
@@ -370,7 +375,7 @@ render_squares_kernel(DevTree t, vox_cuda_camera cam, uint32_t w, uint32_t h,
     if (valid) {
         pixel_dir<RAYS>(cam, rays, w, px, py, dx, dy, dz);
         RayHit hh;
-        if (t.root != VOXP_EMPTY && vox::trace_ray<CAP, false>(t, t.root, ox, oy, oz, dx, dy, dz, hh, c, overflow)) {
+        if (t.root != VOXP_EMPTY && vox::trace_ray<CAP, false, false, GENERAL>(t, t.root, ox, oy, oz, dx, dy, dz, hh, c, overflow)) {
             rrec = hh.rec;
             rx = hh.x; ry = hh.y; rz = hh.z;
         }
@@ -431,7 +436,7 @@ render_squares_kernel(DevTree t, vox_cuda_camera cam, uint32_t w, uint32_t h,
         float sx = 0.f, sy = 0.f, sz = 0.f;
         if (pending && searched && ip >= pos && ip < iend && !(bmerge && (ip & 1))) {
             RayHit hh;
-            if (vox::trace_ray<CAP, false>(t, leaf, ox, oy, oz, dx, dy, dz, hh, c, overflow)) {
+            if (vox::trace_ray<CAP, false, false, GENERAL>(t, leaf, ox, oy, oz, dx, dy, dz, hh, c, overflow)) {
                 shit = true;
                 sx = hh.x; sy = hh.y; sz = hh.z;
             }
@@ -644,6 +649,15 @@ cudaError_t launch_balls(const vox_cuda_tree *t, const float *c, const float *r,
 // Process-wide settings of the BEST frame kernel (vox_cuda_render_set_config).
 std::atomic<uint32_t> g_render_cull{1}, g_render_overlap{1};
 
+using FrameKernel = void (*)(DevTree, vox_cuda_camera, uint32_t, uint32_t, FramePlan, const uint8_t *, uint32_t *,
+                             unsigned long long *, uint32_t *, vox::DevLights);
+template <bool COUNT, bool LIT, bool GENERAL>
+FrameKernel frame_kernel(int cap)
+{
+    return cap == 0 ? render_kernel<CAP0, COUNT, LIT, GENERAL>
+         : cap == 1 ? render_kernel<CAP1, COUNT, LIT, GENERAL> : render_kernel<CAP2, COUNT, LIT, GENERAL>;
+}
+
 template <bool COUNT>
 cudaError_t launch_render(const vox_cuda_tree *t, const vox_cuda_camera &cam, uint32_t w, uint32_t h,
                           const uint8_t *tex, uint32_t *argb, unsigned long long *counts, cudaStream_t s,
@@ -653,18 +667,14 @@ cudaError_t launch_render(const vox_cuda_tree *t, const vox_cuda_camera &cam, ui
     FramePlan p;
     plan_frame(t, cam, w, h, !COUNT && g_render_cull.load(), p);
     if (memo) plan_clearing(p, memo);
-    void (*kern)(DevTree, vox_cuda_camera, uint32_t, uint32_t, FramePlan, const uint8_t *, uint32_t *,
-                 unsigned long long *, uint32_t *, vox::DevLights);
+    FrameKernel kern;
     vox::DevLights L{};
     if (lights) L = *lights;
     const bool lit = !COUNT && L.on;
     const int cap = t->cap_class;
-    if (lit)
-        kern = cap == 0 ? render_kernel<CAP0, COUNT, true>
-             : cap == 1 ? render_kernel<CAP1, COUNT, true> : render_kernel<CAP2, COUNT, true>;
-    else
-        kern = cap == 0 ? render_kernel<CAP0, COUNT, false>
-             : cap == 1 ? render_kernel<CAP1, COUNT, false> : render_kernel<CAP2, COUNT, false>;
+    const bool general = !COUNT && !(t->dev.shape & vox::SHAPE_ORDERED);
+    kern = general ? (lit ? frame_kernel<COUNT, true, !COUNT>(cap) : frame_kernel<COUNT, false, !COUNT>(cap))
+                   : (lit ? frame_kernel<COUNT, true, false>(cap) : frame_kernel<COUNT, false, false>(cap));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.ntiles + p.nclear);
     cfg.blockDim = dim3(128);
@@ -680,6 +690,15 @@ cudaError_t launch_render(const vox_cuda_tree *t, const vox_cuda_camera &cam, ui
     if (e == cudaSuccess) e = cudaGetLastError();
     if (memo) *memo = FrameMemo{e == cudaSuccess, p.x0, p.y0, p.x1, p.y1};
     return e;
+}
+
+using SquaresKernel = void (*)(DevTree, vox_cuda_camera, uint32_t, uint32_t, FramePlan, unsigned int, const uint8_t *,
+                               uint32_t *, uint32_t *, vox::DevLights, const float *);
+template <bool RAYS, bool GENERAL>
+SquaresKernel squares_kernel(int cap)
+{
+    return cap == 0 ? render_squares_kernel<CAP0, RAYS, GENERAL>
+         : cap == 1 ? render_squares_kernel<CAP1, RAYS, GENERAL> : render_squares_kernel<CAP2, RAYS, GENERAL>;
 }
 
 // FAST / ADAPTIVE frames, and with a ray buffer frames of every quality: one
@@ -714,14 +733,9 @@ cudaError_t launch_render_squares(const vox_cuda_tree *t, const vox_cuda_camera 
     }
     if (memo) plan_clearing(p, memo);
     const int cap = t->cap_class;
-    void (*squares)(DevTree, vox_cuda_camera, uint32_t, uint32_t, FramePlan, unsigned int, const uint8_t *,
-                    uint32_t *, uint32_t *, vox::DevLights, const float *);
-    if (rays)
-        squares = cap == 0 ? render_squares_kernel<CAP0, true>
-                : cap == 1 ? render_squares_kernel<CAP1, true> : render_squares_kernel<CAP2, true>;
-    else
-        squares = cap == 0 ? render_squares_kernel<CAP0, false>
-                : cap == 1 ? render_squares_kernel<CAP1, false> : render_squares_kernel<CAP2, false>;
+    const bool general = !(t->dev.shape & vox::SHAPE_ORDERED);
+    const SquaresKernel squares = general ? (rays ? squares_kernel<true, true>(cap) : squares_kernel<false, true>(cap))
+                                          : (rays ? squares_kernel<true, false>(cap) : squares_kernel<false, false>(cap));
     // overlapping the previous kernel of the stream, as the BEST frames do
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.ntiles + p.nclear);
