@@ -216,7 +216,7 @@ int vox_cuda_tree_node_id(const vox_cuda_tree *tree, const struct vox_node *node
  * ray at the tree's root, else n pre-order indices of the node each search
  * starts from (vox_ray_tree_intersection accepts any node as its root;
  * renderer.c:297).  slot and points may be NULL.  Batches of 393,216 rays or
- * more are traced grouped by direction and origin (results are the same for
+ * more (262,144 over a tree whose boxes are not ordered) are traced grouped by direction and origin (results are the same for
  * any order), with a stream-ordered scratch allocation of about 6 bytes per
  * ray for that order.
  * Replaces vox_ray_tree_intersection (src/voxtrees/search.h:24-26). */

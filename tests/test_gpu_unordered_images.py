@@ -85,3 +85,24 @@ def test_lit_frames(scene, quality):
         o.insert(c, rad, col)
     ref = orc.render_lit(s.ht.ptr, s.cam.state(), W, H, quality, s.tex, o)
     assert np.array_equal(s.dt.render_lit(s.cam.gpu_struct(), W, H, quality, s.tex, m.upload()), ref)
+
+
+@pytest.mark.parametrize("n,launches", [(262143, 1), (262144, 4), (300000, 4), (393216, 4)])
+def test_ray_batches_are_sorted_where_it_pays(scene, n, launches):
+    """From 262,144 rays on these batches are traced grouped (three kernels more), and answer the same."""
+    s = scene
+    r = np.random.RandomState(n)
+    o = r.uniform(-40, 104, (n, 3)).astype(np.float32)
+    d = r.standard_normal((n, 3)).astype(np.float32)
+    do, dd = torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda()
+    leaf = torch.zeros(n, dtype=torch.int32, device="cuda")
+    slot, pts = torch.zeros(n, dtype=torch.uint8, device="cuda"), torch.zeros((n, 3), device="cuda")
+    before = s.vg.lib().vox_cuda_launch_count()
+    s.dt.rays_device(do, dd, leaf, slot, pts)
+    torch.cuda.synchronize()
+    assert s.vg.lib().vox_cuda_launch_count() - before == launches
+    oleaf, oslot, opts, _ = orc.ray_batch(s.ht.ptr, o, d)
+    got = leaf.cpu().numpy().view(np.uint32)
+    assert np.array_equal(got, oleaf) and np.array_equal(slot.cpu().numpy(), oslot)
+    ok, bad = same_points(pts.cpu().numpy(), opts, got != MISS)
+    assert ok, f"{bad} points differ"

@@ -560,7 +560,12 @@ __global__ void __launch_bounds__(SHAPE_THREADS) image_shape_kernel(const uint4 
 // 256^3 / 512^3 trees take 52 / 74 / 86 us as given and 69 / 85 / 103 sorted,
 // 393,216 take 65 / 101 / 125 and 77 / 101 / 126, 524,288 84 / 123 / 144 and
 // 83 / 110 / 136.
-constexpr size_t RAY_SORT_MIN = 3 << 17;
+// Over an image without SHAPE_ORDERED, whose searches are longer, the order pays
+// earlier: 200,000 / 262,144 / 393,215 rays over the 256^3 tree 98 / 112 / 149 us
+// as given and 108 / 111 / 125 sorted.  (Axis-parallel rays, which take the
+// same search over any image: 85 / 110 / 180 / 248 us for 65,536 / 131,072 /
+// 262,144 / 393,215 as given; 260 sorted for 393,216.)
+constexpr size_t RAY_SORT_MIN = 3 << 17, GENERAL_SORT_MIN = 1 << 18;
 
 template <bool COUNT>
 cudaError_t launch_rays(const vox_cuda_tree *t, const float *o, const float *d, const uint32_t *roots,
@@ -570,7 +575,8 @@ cudaError_t launch_rays(const vox_cuda_tree *t, const float *o, const float *d, 
     if (n == 0) return cudaSuccess;
     void *scratch = nullptr;
     uint32_t *order = nullptr;
-    if (!COUNT && n >= RAY_SORT_MIN && n <= 0xFFFFFFFFull) {
+    const size_t least = t->dev.shape & vox::SHAPE_ORDERED ? RAY_SORT_MIN : GENERAL_SORT_MIN;
+    if (!COUNT && n >= least && n <= 0xFFFFFFFFull) {
         cudaError_t e = pool_alloc(&scratch, ray_order_bytes(n), s);
         if (e != cudaSuccess) return e;
         e = ray_order(t, o, d, n, scratch, &order, s);
