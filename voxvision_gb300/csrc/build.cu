@@ -405,6 +405,14 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_chunk_box(const float *P, Lev
     }
 }
 
+// The scan of tree.c:138-155 starts with the first voxel's coordinate, and
+// nothing is less or greater than a NaN: one there is the node's bound on both
+// sides.  (A later NaN is no extreme.)
+__device__ __forceinline__ void first_nan(float first, float &mn, float &mx)
+{
+    if (first != first) mn = mx = first;
+}
+
 // The box of node k (calc_bounding_box, tree.c:138-155) and what it is by its
 // density (geom.c:157-167) and size, before it is split (tree.c:249-275).
 __device__ uint8_t write_box(const Level &L, uint32_t k, uint32_t nk, const float *mn, const float *mx, const float *v)
@@ -427,7 +435,7 @@ __device__ uint8_t write_box(const Level &L, uint32_t k, uint32_t nk, const floa
 // Tiled nodes: a block per node over its chunks' partial extremes; and the top
 // binade its coordinate sums can reach.
 constexpr int NODE_THREADS = 256;
-__global__ void __launch_bounds__(NODE_THREADS) k_box_tiled(Level L, NodeLists lists, const float *cv,
+__global__ void __launch_bounds__(NODE_THREADS) k_box_tiled(const float *P, Level L, NodeLists lists, const float *cv,
                                                             const uint32_t *ci, float vx, float vy, float vz, Tally tally)
 {
     after_previous();
@@ -451,6 +459,7 @@ __global__ void __launch_bounds__(NODE_THREADS) k_box_tiled(Level L, NodeLists l
     __syncthreads();
     if (threadIdx.x) return;
     for (int w = 1; w < NODE_THREADS / 32; w++) x.merge(part[w]);
+    for (int a = 0; a < 3; a++) first_nan(P[3 * (uint64_t)L.start[k] + a], x.mn[a], x.mx[a]);
     const float v[3] = {vx, vy, vz};
     if (write_box(L, k, nk, x.mn, x.mx, v) == K_DENSE) atomicAdd(&tally.stats[S_DENSE], 1ull);
     for (int a = 0; a < 3; a++) {
@@ -1063,6 +1072,7 @@ __device__ __forceinline__ void nodes_lanes(const Level &L, const uint32_t *list
                     if (mn[a] == 0.0f) mn[a] = zero;
                     if (mx[a] == 0.0f) mx[a] = zero;
                 }
+                first_nan(__shfl_sync(FULL, p[0][a], 0), mn[a], mx[a]);
             }
             uint32_t kind = 0;
             if (lane == 0) kind = write_box(L, k, n, mn, mx, v);
@@ -1206,6 +1216,7 @@ __device__ __forceinline__ void nodes_block(const Level &L, const uint32_t *list
         __syncthreads();
         if (threadIdx.x == 0) {
             for (int i = 1; i < WARPS; i++) e.merge(epart[i]);
+            for (int a = 0; a < 3; a++) first_nan(P[3 * s0 + a], e.mn[a], e.mx[a]);
             s_kind = write_box(L, k, n, e.mn, e.mx, v);
             epart[0] = e;
             if (s_kind == K_DENSE) atomicAdd(&tally.stats[S_DENSE], 1ull);
@@ -2047,7 +2058,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
             const uint64_t most = std::min<uint64_t>(m, sz.tiled);   // of the level's nodes
             const unsigned nt = (unsigned)most, nc = (unsigned)sz.subs_of(most) * SUB_CHUNKS, np = (unsigned)sz.tiles_of(most);
             launch_after(k_chunk_box, nc, CHUNK_THREADS, s, Pc, L, lists, cv, cidx);
-            launch_after(k_box_tiled, nt, NODE_THREADS, s, L, lists, cv, cidx, vx, vy, vz, tally);
+            launch_after(k_box_tiled, nt, NODE_THREADS, s, Pc, L, lists, cv, cidx, vx, vy, vz, tally);
             launch_after(k_chunk_sums, nc, CHUNK_THREADS, s, Pc, L, lists, csum, cgrid);
             launch_after(k_centre_plain, nt, NODE_THREADS, s, L, lists, csum, cgrid, cbase, window, starts, vx, vy, vz);
             launch_after(k_chunk_maps, nc, CHUNK_THREADS, s, Pc, L, lists, cbase, window, maps, sz.chunks);
