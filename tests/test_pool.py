@@ -13,6 +13,9 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 FAKE = r'''
 #include "pool.h"
 #include <cstdlib>
+#include <map>
+static int blocks[4], waits, broken;
+static std::map<void *, int> owner;
 static int current = 0, refuse = 0, capturing = 0;
 static long made[4], trimmed[4], kept[4], from_pool[4], from_default;
 static uint64_t threshold[4];
@@ -53,6 +56,30 @@ cudaError_t cudaMemPoolTrimTo(cudaMemPool_t pool, size_t least)
     if (least == 0) kept[d] = 0;
     return cudaSuccess;
 }
+cudaError_t cudaMalloc(void **p, size_t)
+{
+    if (broken) return (cudaError_t)broken;
+    *p = std::malloc(1);
+    blocks[current]++;
+    owner[*p] = current;
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void *p)
+{
+    if (p) { blocks[owner[p]]--; waits++; std::free(p); }
+    return (cudaError_t)broken;
+}
+cudaError_t cudaDeviceSynchronize() { return cudaErrorStreamCaptureUnsupported; }   // as while any thread captures
+int wait_device(int error)
+{
+    broken = error;
+    waits = 0;
+    const int e = (int)wait_for_device();
+    broken = 0;
+    return e;
+}
+int n_waits() { return waits; }
+int n_blocks(int d) { return blocks[d]; }
 void set_device(int d) { current = d; }
 void set_refuse(int r) { refuse = r; }
 void set_capturing(int c) { capturing = c; }
@@ -118,3 +145,19 @@ def test_no_pool_is_made_in_a_capture_or_where_none_can_be(pool):
     assert pool.alloc(10) == 0 and pool.pools(0) == 1 and pool.pooled(0) == 1
     pool.set_capturing(1)        # a pool there is serves captures too
     assert pool.alloc(10) == 0 and pool.pooled(0) == 2
+
+
+def test_waiting_for_a_device_in_spite_of_captures(pool):
+    pool.set_device(1)
+    pool.made_tree(1)
+    for _ in range(3):
+        assert pool.wait_device(0) == 0 and pool.n_waits() == 1   # a block made and freed
+        assert pool.n_blocks(1) == 1                              # beside the one that is kept
+    assert pool.wait_device(700) == 700
+    pool.set_device(0)
+    pool.gone_tree(1)
+    assert pool.n_blocks(1) == 0 and pool.n_blocks(0) == 0
+    pool.made_tree(0)
+    assert pool.wait_device(0) == 0 and (pool.n_blocks(0), pool.n_blocks(1)) == (1, 0)
+    pool.gone_tree(0)
+    assert pool.n_blocks(0) == 0

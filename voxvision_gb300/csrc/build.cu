@@ -2319,7 +2319,7 @@ try {
     return new_tree(out, [&](vox_cuda_tree *t, cudaStream_t s) {
         // the set may still be on its way, in any stream of the caller's: the
         // build's own stream waits for none of them
-        if (n && cudaDeviceSynchronize() != cudaSuccess) return (int)VOX_CUDA_ECUDA;
+        if (n && wait_for_device() != cudaSuccess) return (int)VOX_CUDA_ECUDA;
         return build_tree(t, d_set, n, s);
     });
 } VOX_ABI_FAIL_INT

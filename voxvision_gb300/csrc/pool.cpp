@@ -10,6 +10,7 @@ constexpr int POOL_DEVICES = 64;
 std::mutex g_pool_mu;
 std::atomic<cudaMemPool_t> g_pool[POOL_DEVICES];
 std::atomic<int> g_trees[POOL_DEVICES];
+std::atomic<void *> g_anchor[POOL_DEVICES];   // of wait_for_device
 
 }  // namespace
 
@@ -43,6 +44,21 @@ cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s)
     return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
 }
 
+cudaError_t wait_for_device()
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < POOL_DEVICES && !g_anchor[dev].load()) {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        void *a = nullptr;
+        if (!g_anchor[dev].load() && cudaMalloc(&a, 4) == cudaSuccess) g_anchor[dev].store(a);
+    }
+    void *p = nullptr;
+    e = cudaMalloc(&p, 4);
+    return e != cudaSuccess ? e : cudaFree(p);
+}
+
 void tree_made(int device)
 {
     if (device >= 0 && device < POOL_DEVICES) g_trees[device]++;
@@ -52,4 +68,6 @@ void tree_gone(int device)
 {
     if (device < 0 || device >= POOL_DEVICES || --g_trees[device] != 0) return;
     if (cudaMemPool_t pool = g_pool[device].load()) cudaMemPoolTrimTo(pool, 0);
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    if (void *a = g_anchor[device].exchange(nullptr)) cudaFree(a);
 }

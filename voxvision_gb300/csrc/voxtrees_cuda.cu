@@ -1341,11 +1341,14 @@ try {
     const int dev = t->device;
     cudaGetDevice(&cur);
     if (cur != dev) cudaSetDevice(dev);
-    // (memory of a pool is freed without waiting for kernels that may read it)
-    if (t->pooled) cudaDeviceSynchronize();
-    cudaFree(t->d_pool);
-    cudaFree(t->d_rec_of_id);
-    cudaFree(t->d_status);
+    // Memory of a pool is freed without waiting for kernels that may read it.
+    // Where there is no waiting for them (a capture in cudaStreamCaptureModeGlobal)
+    // it stays, as cudaFree of other memory fails there.
+    if (!t->pooled || wait_for_device() == cudaSuccess) {
+        cudaFree(t->d_pool);
+        cudaFree(t->d_rec_of_id);
+        cudaFree(t->d_status);
+    }
     delete t;
     if (cur != dev) cudaSetDevice(cur);
     return VOX_CUDA_OK;
