@@ -190,3 +190,32 @@ def test_builds_with_a_coordinate_out_of_the_ordinary(vg, n, value, ordinary):
         assert np.array_equal(leaf, oleaf) and np.array_equal(slot, oslot)
         ok, bad = same_points(pts, opts, leaf != MISS)
         assert ok, f"{bad} points differ"
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("what", ["nothing", "child past its parent", "upper child below the plane", "voxel past its leaf",
+                                  "box turned round", "tiny voxel", "not a number"])
+def test_one_thing_broken_in_a_small_tree(vg, what, axis):
+    """Small images are checked on the host: the routes are the same."""
+    r = np.random.RandomState(axis)
+    cells = np.argwhere(r.random_sample((8, 8, 8)) < 0.3).astype(np.float32)
+    ht = vg.HostTree(vg.lib().vox_make_tree_host(np.ascontiguousarray(cells).ctypes.data_as(C.c_void_p), len(cells)))
+    lost = _break(what, ht.ptr, axis, r)
+    before = vg.lib().vox_cuda_launch_count()
+    dt = vg.DeviceTree(ht.ptr)
+    assert vg.lib().vox_cuda_launch_count() == before   # no kernel to check it
+    n = 1 << 18
+    c, rad = r.uniform(-4, 12, (n, 3)).astype(np.float32), r.uniform(0.1, 3, n).astype(np.float32)
+    before = vg.lib().vox_cuda_launch_count()
+    hit = dt.balls(c, rad)
+    assert vg.lib().vox_cuda_launch_count() - before == (1 if lost == "" else 4)
+    assert np.array_equal(hit, orc.ball_batch(ht.ptr, c, rad)[0])
+    o = r.uniform(-20, 28, (n, 3)).astype(np.float32)
+    d = (r.uniform(0, 8, (n, 3)) - o).astype(np.float32)
+    before = vg.lib().vox_cuda_launch_count()
+    leaf, slot, pts = dt.rays(o, d)
+    assert vg.lib().vox_cuda_launch_count() - before == (4 if lost.startswith("ordered") else 1)
+    oleaf, oslot, opts, _ = orc.ray_batch(ht.ptr, o, d)
+    assert np.array_equal(leaf, oleaf) and np.array_equal(slot, oslot)
+    ok, bad = same_points(pts, opts, leaf != MISS)
+    assert ok, f"{bad} points differ"

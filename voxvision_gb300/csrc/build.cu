@@ -2174,8 +2174,7 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     const auto ordinary = [](float v) { return v >= vox::SHAPE_VOXEL && v <= LIMIT; };
     back->unshaped = 0;
     if (back->odd || !ordinary(vx) || !ordinary(vy) || !ordinary(vz)) {
-        if (e == cudaSuccess) e = image_shape(pool, map, nodes, st.voxel, scal, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&back->unshaped, scal, 4, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = image_shape(pool, map, nodes, st.voxel, &back_d->unshaped, s);
     }
     if (x) {
         x->dots_of_id.resize(nodes);

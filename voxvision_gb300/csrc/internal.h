@@ -54,8 +54,9 @@ struct ImageStats {
     uint32_t unshaped;   // SHAPE_* bits the image does not have (image_shape)
 };
 
-/* The SHAPE_* bits (traverse.cuh) an image on the device does not have, into
- * the device word `word`; enqueued on s (voxtrees_cuda.cu). */
+/* The SHAPE_* bits (image_shape.h) an image on the device does not have, into
+ * `word`, which is zero and which the device can write; enqueued on s
+ * (voxtrees_cuda.cu). */
 cudaError_t image_shape(const uint4 *pool, const uint32_t *rec_of_id, uint64_t nodes, const float voxel[3],
                         uint32_t *word, cudaStream_t s);
 

@@ -27,6 +27,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "image_shape.h"
 #include "pool_layout.h"
 #include "../../include/voxtrees_cuda.h"
 
@@ -43,20 +44,6 @@ struct DevTree {
     uint32_t shape;              // SHAPE_* bits of the image (image_shape in voxtrees_cuda.cu)
     uint32_t *fault;             // the tree's status word (checked build only)
 };
-
-// What is known of every box of a tree's image.  SHAPE_ORDERED: every number of
-// a node's box, a centre or a voxel is zero or SHAPE_LEAST to SHAPE_LIMIT in
-// magnitude, min <= max on every axis, and the voxel size SHAPE_VOXEL to
-// SHAPE_LIMIT.  Trees that vox_make_tree or the GPU build make from ordinary
-// voxels have it; a caller's own tree need not.
-//
-// SHAPE_NESTED: every child's box and every leaf's voxel lie inside their
-// node's box, and a child on the lower side of a dividing plane reaches at
-// most one voxel past it, one on the upper side not below it.
-constexpr uint32_t SHAPE_ORDERED = 1u, SHAPE_NESTED = 2u;
-constexpr float SHAPE_LIMIT = 1.152921504606847e18f;     // 2^60
-constexpr float SHAPE_LEAST = 1.6543612251060553e-24f;   // 2^-79
-constexpr float SHAPE_VOXEL = 1.4901161193847656e-8f;    // 2^-26
 
 struct Counts {
     uint32_t nodes, inner, voxels;

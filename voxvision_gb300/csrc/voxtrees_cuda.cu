@@ -488,10 +488,10 @@ render_squares_kernel(DevTree t, vox_cuda_camera cam, uint32_t w, uint32_t h,
     if (overflow) atomicOr(status, 1u);
 }
 
-// What the searches may rely on in the image (SHAPE_* of traverse.cuh),
-// checked record by record, a thread each: *bad gets the bits that do not hold.
-// The voxels of an overflowed leaf, of which there may be any number, are the
-// block's: 1M equal voxels took one thread 192 ms, an upload of 2.5 ms without.
+// What the searches may rely on in the image (image_shape.h), checked record by
+// record, a thread each: *bad gets the bits that do not hold.  The voxels of an
+// overflowed leaf, of which there may be any number, are the block's: 1M equal
+// voxels took one thread 192 ms, an upload of 2.5 ms without.
 constexpr int SHAPE_THREADS = 1024;
 __global__ void __launch_bounds__(SHAPE_THREADS) image_shape_kernel(const uint4 *__restrict__ pool,
                                                                     const uint32_t *__restrict__ rec_of_id,
@@ -502,43 +502,11 @@ __global__ void __launch_bounds__(SHAPE_THREADS) image_shape_kernel(const uint4 
     __shared__ uint32_t big[SHAPE_THREADS], n_big;   // the block's records of overflowed leaves
     if (threadIdx.x == 0) n_big = 0;
     __syncthreads();
-    auto fine = [](float v) { return v == 0.0f || (fabsf(v) >= vox::SHAPE_LEAST && fabsf(v) <= vox::SHAPE_LIMIT); };
-    bool ok = fine(vx) && fine(vy) && fine(vz) && vx >= vox::SHAPE_VOXEL && vy >= vox::SHAPE_VOXEL && vz >= vox::SHAPE_VOXEL,
-         nested = true;
-    const float vox[3] = {vx, vy, vz};
-    auto voxel = [&](const uint4 v, const float *lo, const float *hi) {   // of a leaf whose box is [lo, hi]
-        const float p[3] = {ubf(v.x), ubf(v.y), ubf(v.z)};
-        for (int k = 0; k < 3; k++) {
-            ok = ok && fine(p[k]);
-            nested = nested && p[k] >= lo[k] && __fadd_rn(p[k], vox[k]) <= hi[k];
-        }
-    };
+    vox::ImageShape shape(vx, vy, vz);
     const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id < n_nodes) {
         const uint32_t rec = rec_of_id[id];
-        const uint4 a = pool[rec], b = pool[rec + 1], c = pool[rec + 2];
-        const float lo[3] = {ubf(a.x), ubf(a.y), ubf(a.z)}, hi[3] = {ubf(a.w), ubf(b.x), ubf(b.y)};
-        for (int k = 0; k < 3; k++) ok = ok && fine(lo[k]) && fine(hi[k]) && lo[k] <= hi[k];
-        const uint32_t kind = b.z & 3u;
-        if (kind == VOXP_KIND_INNER) {
-            const float plane[3] = {ubf(c.x), ubf(c.y), ubf(c.z)};
-            const uint32_t mask = (b.z >> 8) & 0xFFu, n = (uint32_t)__popc(mask);
-            uint32_t oct = 0;   // of the i-th child
-            for (uint32_t i = 0; i < n; i++, oct++) {
-                const uint4 v = pool[b.w + VOXP_REC_UNITS * i], u = pool[b.w + VOXP_REC_UNITS * i + 1];
-                const float p[3] = {ubf(v.x), ubf(v.y), ubf(v.z)}, q[3] = {ubf(v.w), ubf(u.x), ubf(u.y)};
-                while (!((mask >> oct) & 1u)) oct++;
-                for (int k = 0; k < 3; k++)
-                    nested = nested && p[k] >= lo[k] && q[k] <= hi[k] &&
-                             ((oct >> k) & 1u ? q[k] <= __fadd_rn(plane[k], vox[k]) : p[k] >= plane[k]);
-            }
-            for (int k = 0; k < 3; k++) ok = ok && fine(plane[k]);
-        } else if (kind == VOXP_KIND_LEAF) {
-            const uint32_t n = b.z >> 2;
-            if (n > VOX_MAX_DOTS) big[atomicAdd(&n_big, 1u)] = rec;
-            else
-                for (uint32_t i = 0; i < n; i++) voxel(pool[b.w + i], lo, hi);
-        }
+        if (shape.record(pool, rec, VOX_MAX_DOTS)) big[atomicAdd(&n_big, 1u)] = rec;
     }
     __syncthreads();
     for (uint32_t i = 0; i < n_big; i++) {
@@ -547,10 +515,10 @@ __global__ void __launch_bounds__(SHAPE_THREADS) image_shape_kernel(const uint4 
         const float lo[3] = {ubf(a.x), ubf(a.y), ubf(a.z)}, hi[3] = {ubf(a.w), ubf(b.x), ubf(b.y)};
         const uint32_t n = b.z >> 2;
 #pragma unroll 4
-        for (uint32_t j = threadIdx.x; j < n; j += SHAPE_THREADS) voxel(pool[b.w + j], lo, hi);
+        for (uint32_t j = threadIdx.x; j < n; j += SHAPE_THREADS) shape.voxel(pool[b.w + j], lo, hi);
     }
-    const uint32_t missing = __reduce_or_sync(0xFFFFFFFFu, (ok ? 0u : vox::SHAPE_ORDERED) | (nested ? 0u : vox::SHAPE_NESTED));
-    if (missing && (threadIdx.x & 31) == 0) atomicOr(bad, missing);
+    const uint32_t missing = __reduce_or_sync(0xFFFFFFFFu, shape.missing());
+    if (missing && (threadIdx.x & 31) == 0) atomicOr_system(bad, missing);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -1077,17 +1045,24 @@ EXPORT int vox_cuda_build_checked(void) { return vox::CHECKED ? 1 : 0; }
 
 EXPORT uint64_t vox_cuda_launch_count(void) { return g_launches.load(); }
 
-// The SHAPE_* bits of an image on the device, enqueued on s: `word` (device)
-// holds the bits that do not hold once s has run.
+// The SHAPE_* bits of an image on the device, enqueued on s: `word`, zero, has
+// the bits that do not hold once s has run.
 cudaError_t image_shape(const uint4 *pool, const uint32_t *rec_of_id, uint64_t nodes, const float voxel[3],
                         uint32_t *word, cudaStream_t s)
 {
-    cudaError_t e = cudaMemsetAsync(word, 0, 4, s);
-    if (e != cudaSuccess || nodes == 0) return e;
-    image_shape_kernel<<<(unsigned)((nodes + SHAPE_THREADS - 1) / SHAPE_THREADS), SHAPE_THREADS, 0, s>>>(pool, rec_of_id, (uint32_t)nodes, voxel[0],
-                                                                       voxel[1], voxel[2], word);
+    if (nodes == 0) return cudaSuccess;
+    image_shape_kernel<<<(unsigned)((nodes + SHAPE_THREADS - 1) / SHAPE_THREADS), SHAPE_THREADS, 0, s>>>(
+        pool, rec_of_id, (uint32_t)nodes, voxel[0], voxel[1], voxel[2], word);
     count_launch();
     return cudaGetLastError();
+}
+
+// The same of a small image on the host.
+static uint32_t image_shape_host(const FlatTree &flat)
+{
+    vox::ImageShape shape(flat.voxel[0], flat.voxel[1], flat.voxel[2]);
+    for (uint32_t rec : flat.rec_of_id) shape.record(flat.units.data(), rec, 0xFFFFFFFFu);
+    return shape.missing();
 }
 
 // Flattens `root` into t (host maps) and copies the image to the device,
@@ -1127,19 +1102,32 @@ static int load_tree(vox_cuda_tree *t, const struct vox_node *root, int layout =
         if (new_map) cudaFree(map);
         return VOX_CUDA_ENOMEM;
     }
-    uint32_t unshaped = 0;
-    cudaError_t e = cudaSuccess;
-    if (flat.units.size())
+    // Images of up to SHAPE_HOST_UNITS are checked here, 7 ns a unit, larger ones
+    // by a kernel that stores into the thread's page, some 10 us.  A tree of 100
+    // voxels is refreshed in 37 us, 35 without a check, 50 with the kernel and
+    // its word copied back.
+    constexpr size_t SHAPE_HOST_UNITS = 1024;
+    uint32_t *page = nullptr, *page_dev = nullptr;
+    uint32_t unshaped = vox::SHAPE_ORDERED | vox::SHAPE_NESTED;   // (also where there is no page)
+    if (flat.units.size() <= SHAPE_HOST_UNITS) {
+        unshaped = image_shape_host(flat);
+    } else if ((page = static_cast<uint32_t *>(thread_page())) != nullptr) {
+        void *dev = nullptr;
+        if (cudaHostGetDevicePointer(&dev, page, 0) == cudaSuccess) page_dev = static_cast<uint32_t *>(dev);
+    }
+    cudaError_t e = cudaMemset(t->d_status, 0, 4);
+    if (e == cudaSuccess && flat.units.size())
         e = cudaMemcpy(pool, flat.units.data(), flat.units.size() * 16, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && nodes) e = cudaMemcpy(map, flat.rec_of_id.data(), nodes * 4, cudaMemcpyHostToDevice);
-    // (the status word is the check's output first, then cleared)
-    if (e == cudaSuccess) e = image_shape(pool, map, nodes, flat.voxel, t->d_status, cudaStreamLegacy);
-    if (e == cudaSuccess) e = cudaMemcpy(&unshaped, t->d_status, 4, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemset(t->d_status, 0, 4);
+    if (page_dev) {
+        *page = 0;
+        if (e == cudaSuccess) e = image_shape(pool, map, nodes, flat.voxel, page_dev, cudaStreamLegacy);
+    }
     // A copy from pageable memory may still be in flight when cudaMemcpy
     // returns; the pool must be complete before any kernel on any stream
     // reads it (the frame kernel reads it ahead of its stream dependency).
     if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    if (page_dev) unshaped = *static_cast<volatile uint32_t *>(page);
     if (e != cudaSuccess) {
         if (new_pool) cudaFree(pool);
         if (new_map) cudaFree(map);
