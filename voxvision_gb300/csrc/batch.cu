@@ -108,7 +108,7 @@ __device__ __forceinline__ void run_tile(const BatchJobDev &J, uint32_t local, u
                 vox::Counts c{0, 0, 0};
                 bool overflow = false, hit = false;
                 if (t.root != VOXP_EMPTY)
-                    hit = vox::trace_ray<CAP, false>(t, t.root, cam.position[0], cam.position[1], cam.position[2],
+                    hit = vox::trace_ray<CAP, false, false, false, true>(t, t.root, cam.position[0], cam.position[1], cam.position[2],
                                                      dx, dy, dz, hh, c, overflow);
                 v = hit ? vox::texel_color(J.tex, t, hh.x, hh.y, hh.z) : 0u;
                 if (overflow) atomicOr(J.status, 1u);

@@ -2,8 +2,8 @@
  * of one record of it, for the host (small images) and the device.
  *
  * SHAPE_ORDERED: every number of a node's box, a centre or a voxel is zero or
- * SHAPE_LEAST to SHAPE_LIMIT in magnitude, min <= max on every axis, and the
- * voxel size SHAPE_VOXEL to SHAPE_LIMIT.  Trees that vox_make_tree or the GPU
+ * SHAPE_LEAST to SHAPE_LIMIT in magnitude, min <= max on every axis and no max
+ * is -0, and the voxel size is SHAPE_VOXEL to SHAPE_LIMIT.  Trees that vox_make_tree or the GPU
  * build make from ordinary voxels have it; a caller's own tree need not.
  *
  * SHAPE_NESTED: every child's box and every leaf's voxel lie inside their
@@ -75,6 +75,7 @@ struct ImageShape {
         const float lo[3] = {shape_float(a.x), shape_float(a.y), shape_float(a.z)},
                     hi[3] = {shape_float(a.w), shape_float(b.x), shape_float(b.y)};
         for (int k = 0; k < 3; k++) ok = ok && shape_fine(lo[k]) && shape_fine(hi[k]) && lo[k] <= hi[k];
+        ok = ok && a.w != 0x80000000u && b.x != 0x80000000u && b.y != 0x80000000u;
         const uint32_t kind = b.z & 3u;
         if (kind == VOXP_KIND_INNER) {
             const float plane[3] = {shape_float(c.x), shape_float(c.y), shape_float(c.z)};

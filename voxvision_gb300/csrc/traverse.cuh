@@ -387,9 +387,12 @@ __device__ __forceinline__ int ray_step(const DevTree &t, RaySearch &s, uint4 (&
  *    reference's selection sort gives is read off three comparisons (ties
  *    included), each child stored at its own place on the stack.
  *
- * A search that meets a quotient too small for the bounds, or ends on a zero
- * whose sign the mirror cannot tell (zero_sign_open), reports STEP_AGAIN and is
- * made again by the general search below.
+ *  - A zero on a negated axis is +0 once turned back (turned_back): a sum that
+ *    cancels is +0 with the axis negated or not, and the other zeros there are
+ *    faces and origins, of which none is -0 (image_shape.h, mirror_ok).
+ *
+ * A search that meets a quotient too small for the bounds reports STEP_AGAIN and
+ * is made again by the general search below.
  *
  * Measured against the general search alone (256^3 noise tree; in brackets
  * with the packed arithmetic and the smaller changes since):
@@ -477,27 +480,32 @@ __device__ __forceinline__ bool mirror_ok(const DevTree &t, float ox, float oy, 
     const auto bits = [](float v) { return 2u * __float_as_uint(v) - 1u; };   // of the magnitude; zero's are the largest
     const uint32_t least = min(min(bits(ox), bits(oy)), bits(oz));
     // (the sum is not finite where a NaN hid from the extremes)
+    const uint32_t mzero = 0x80000000u;
     return (t.shape & SHAPE_ORDERED) && lo >= DIR_MIN && hi <= DIR_MAX && o <= SHAPE_LIMIT &&
-           fabsf(dx + dy + dz) < 4e6f && fabsf(ox + oy + oz) < 4e18f && least >= 2u * __float_as_uint(SHAPE_LEAST) - 1u;
+           fabsf(dx + dy + dz) < 4e6f && fabsf(ox + oy + oz) < 4e18f && least >= 2u * __float_as_uint(SHAPE_LEAST) - 1u &&
+           __float_as_uint(ox) != mzero && __float_as_uint(oy) != mzero && __float_as_uint(oz) != mzero;
 }
 
-// Whether a hit has a coordinate whose sign of zero the mirror leaves open: a
-// sum that cancels is +0 with the axis negated or not, so a -0 on a negated
-// axis is either such a sum (+0 to the reference) or a face or origin at -0.
-// A +0 there can only be a face or origin at +0: floors and walls that end at
-// zero, whose +0 face every ray down the axis ends on, are not searched again
-// (a 1080p frame of a floor with its top at z = 0: 257 us with every zero
-// searched again, 134 without; with its top at z = 1, 142).
-// (The form is the one of several that leaves the loop's code as it was: 32
-// orbit frames in the batch kernel take 1,254 us; 1,262 with `||` throughout,
-// 1,297 with `&` throughout, 1,285 with the test made after the search.)
-__device__ __forceinline__ bool zero_sign_open(const RayHit &h, bool nx, bool ny, bool nz)
+// A coordinate of a hit turned back; a zero becomes +0 on a negated axis, here
+// or, in the batch kernels (LATE), by late_zero after the search.  (There this
+// form, as any other in the loop, takes 32 orbit frames from 1,255 to 1,287 us;
+// after the search they take 1,257, but a 1080p frame of its own 58.9 instead
+// of 58.0.  Searching again every ray that ended on such a zero made a frame
+// from inside a tree about the origin, where crossings of the planes at zero
+// cancel, 27.6 us instead of 9.4, a floor with its top at zero 257 instead of 134.)
+template <bool LATE>
+__device__ __forceinline__ float turned_back(bool negated, float v)
 {
-    return (__float_as_uint(h.x) == 0x80000000u && nx) | (__float_as_uint(h.y) == 0x80000000u && ny) |
-           (__float_as_uint(h.z) == 0x80000000u && nz);
+    if (LATE) return negated ? -v : v;
+    return __fsub_rn(negated ? 0.0f : v, negated ? v : 0.0f);
+}
+// -0 to +0 where the direction is negative: adding +0 does, adding -0 changes nothing.
+__device__ __forceinline__ float late_zero(float v, float d)
+{
+    return __fadd_rn(v, __uint_as_float(~__float_as_uint(d) & 0x80000000u));
 }
 
-template <int CAP, bool MZERO_CONST>
+template <int CAP, bool MZERO_CONST, bool LATE>
 __device__ __forceinline__ int trace_mirrored(const DevTree &t, uint32_t start, float ox, float oy, float oz,
                                               float dx, float dy, float dz, uint4 (&stack)[CAP], RayHit &hit)
 {
@@ -563,10 +571,10 @@ __device__ __forceinline__ int trace_mirrored(const DevTree &t, uint32_t start, 
             resume = false;
             if (stop || cur == vend) {
                 if (win) {
-                    hit.x = nx ? -bx : bx; hit.y = ny ? -by : by; hit.z = nz ? -bz : bz;
+                    hit.x = turned_back<LATE>(nx, bx); hit.y = turned_back<LATE>(ny, by); hit.z = turned_back<LATE>(nz, bz);
                     const uint4 r1 = ld16(pool + vrec + 1), r2 = ld16(pool + vrec + 2);
                     hit.leaf = r2.x; hit.slot = win - r1.w; hit.rec = vrec;
-                    return zero_sign_open(hit, nx, ny, nz) ? STEP_AGAIN : STEP_HIT;
+                    return STEP_HIT;
                 }
                 vend = 0;
                 resume = true;
@@ -574,9 +582,9 @@ __device__ __forceinline__ int trace_mirrored(const DevTree &t, uint32_t start, 
         } else if (in) {
             const uint32_t meta = u1.z, link = u1.w, kind = meta & 3u;
             if (kind == VOXP_KIND_DENSE) {                      // search.c:31-37
-                hit.x = nx ? -ex : ex; hit.y = ny ? -ey : ey; hit.z = nz ? -ez : ez;
+                hit.x = turned_back<LATE>(nx, ex); hit.y = turned_back<LATE>(ny, ey); hit.z = turned_back<LATE>(nz, ez);
                 hit.leaf = link; hit.slot = 0xFFu; hit.rec = cur;
-                return zero_sign_open(hit, nx, ny, nz) ? STEP_AGAIN : STEP_HIT;
+                return STEP_HIT;
             }
             if (kind == VOXP_KIND_LEAF) {                       // search.c:39-50
                 const uint32_t vn = meta >> 2;
@@ -715,7 +723,7 @@ __device__ __noinline__ GeneralResult trace_general_call(const uint4 *pool, uint
  * on a hit; `overflow` is set (and the search ends as a miss) on STEP_ERROR.
  * Counting searches count the reference's work: the general search, as those
  * of a kernel built for images that the mirrored one leaves (GENERAL). */
-template <int CAP, bool COUNT, bool MZERO_CONST = false, bool GENERAL = false>
+template <int CAP, bool COUNT, bool MZERO_CONST = false, bool GENERAL = false, bool LATE = MZERO_CONST>
 __device__ __forceinline__ bool trace_ray(const DevTree &t, uint32_t start,
                                           float ox0, float oy0, float oz0,
                                           float dx, float dy, float dz,
@@ -725,7 +733,7 @@ __device__ __forceinline__ bool trace_ray(const DevTree &t, uint32_t start,
     if (COUNT || GENERAL) return trace_general<CAP, COUNT>(t, start, ox0, oy0, oz0, dx, dy, dz, stack, hit, cnt, overflow);
     int r = STEP_AGAIN;
     if (mirror_ok(t, ox0, oy0, oz0, dx, dy, dz))
-        r = trace_mirrored<CAP, MZERO_CONST>(t, start, ox0, oy0, oz0, dx, dy, dz, stack, hit);
+        r = trace_mirrored<CAP, MZERO_CONST, LATE>(t, start, ox0, oy0, oz0, dx, dy, dz, stack, hit);
     if (r == STEP_AGAIN) {
         GeneralResult g = trace_general_call<CAP>(t.pool, start, ox0, oy0, oz0, dx, dy, dz, t.vx, t.vy, t.vz,
                                                   t.max_steps, t.n_units, t.fault, stack);
@@ -734,6 +742,9 @@ __device__ __forceinline__ bool trace_ray(const DevTree &t, uint32_t start,
         return g.found;
     }
     if (r == STEP_ERROR) overflow = true;
+    if (LATE) {
+        hit.x = late_zero(hit.x, dx); hit.y = late_zero(hit.y, dy); hit.z = late_zero(hit.z, dz);
+    }
     return r == STEP_HIT;
 }
 
