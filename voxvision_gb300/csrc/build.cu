@@ -42,7 +42,7 @@
  *  only where the sum leaves its binade inside the chunk (a dozen times per
  *  node) or no map was made for it.  The root of the 256^3 set: 423 us walking
  *  its 1,332 chunks one by one, and 147 for maps of 16 binades, became 70 and
- *  26 (raw volume with a first frame 4,790 -> 3,920 us).
+ *  26 (raw volume with a first frame 4,790 -> 3,830 us).
  *
  * The rest (bounding boxes, the density test, leaf decisions, children) is
  * per node or per voxel.  The tree is built a level at a time.  Then subtree
@@ -1362,7 +1362,7 @@ __global__ void __launch_bounds__(THREADS) k_nodes_block(Level L, const uint32_t
 constexpr int PASS_THREADS = 512;
 
 struct Marks {
-    uint4 *word;                        // per word of a node (from its first sub on): claimed bits, count before, last before
+    uint4 *word;                        // per word of a node, from its first sub on: claimed bits, count before, last before
     uint2 *tile;                        // per tile: claimed count, last unclaimed position + 1 (0: none)
 };
 
@@ -1988,8 +1988,9 @@ int build_tree(vox_cuda_tree *t, const float *d_set, uint64_t N, cudaStream_t s,
     TRY(d.get(&P[0], 3 * N));
     TRY(d.get(&P[1], 3 * N));
     TRY(d.get(&stats, NSTATS * (MAX_LEVELS + 1)));
-    // scal: the level's tiny, small, children, largest child, low, mid, tiled nodes and tiles (6-7), high (8);
-    // 10 error bits, 11 whether a coordinate is out of the ordinary
+    // scal: the level's tiny, small, children, largest child, low, mid, tiled nodes
+    // with their tiles and subs (6-7), high (8); 10 error bits, 11 whether a
+    // coordinate is out of the ordinary
     TRY(d.get(&scal, 12));
     uint32_t *err = scal + 10;
     NodeLists lists{};

@@ -79,7 +79,7 @@ __device__ __forceinline__ uint32_t ray_key(const float *o, const float *d, size
     uint32_t oct = (d[3 * i] < 0.0f) | ((d[3 * i + 1] < 0.0f) << 1) | ((d[3 * i + 2] < 0.0f) << 2);
     float t0 = 0.0f, t1 = 3.0e38f;
     for (int a = 0; a < 3; a++) {
-                const float inv = 1.0f / d[3 * i + a];
+        const float inv = 1.0f / d[3 * i + a];
         float ta = (f.blo[a] - o[3 * i + a]) * inv, tb = (f.bhi[a] - o[3 * i + a]) * inv;
         if (ta > tb) { float x = ta; ta = tb; tb = x; }
         t0 = fmaxf(t0, ta);      // NaN (a zero direction inside the slab) keeps the bound

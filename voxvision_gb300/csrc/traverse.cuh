@@ -396,10 +396,11 @@ __device__ __forceinline__ int ray_step(const DevTree &t, RaySearch &s, uint4 (&
  *
  * Measured against the general search alone (256^3 noise tree; in brackets
  * with the packed arithmetic and the smaller changes since):
- * a 1080p orbit frame 80.6 -> 51.5 us back to back, ADAPTIVE 112 -> 74 us;
- * 32 such frames in the batch kernel 1,995 -> 1,366 us (1,304); 24 mixed frames
- * over four trees 1,203 -> 850 us (782); a near 4K FAST frame of the 512^3 tree
- * 1,496 -> 1,145 us (994); 4M incoherent rays 710 -> 569 us (477). */
+ * a 1080p orbit frame 80.6 -> 51.5 us back to back (52.4), ADAPTIVE 112 -> 74
+ * us (75); 32 such frames in the batch kernel 1,995 -> 1,366 us (1,260); 24
+ * mixed frames over four trees 1,203 -> 850 us (762); a near 4K FAST frame of
+ * the 512^3 tree 1,496 -> 1,145 us (1,030); 4M incoherent rays 710 -> 569 us
+ * (474). */
 constexpr int STEP_AGAIN = 4;
 constexpr float DIR_MIN = 2.384185791015625e-7f, DIR_MAX = 262144.0f;   // 2^-22, 2^18
 // Every coordinate of such a search is a multiple of 2^-102: the image's numbers
@@ -428,9 +429,9 @@ __device__ __forceinline__ float quot(float a, float d, float y)
 // quotient wants -d.  A packed product that a packed sum takes is written as an
 // fma with -0, which rounds alike: ptxas 13.0 joins mul.rn.f32x2 and
 // sub.rn.f32x2 into one fma and rounds once (seen in results), and the -0 is
-// computed so that it cannot see through it.  Measured beside the scalar form: 32 frames in the batch
-// kernel 1,363 -> 1,309 us, the near 4K FAST frame 1,097 -> 1,067 us, ADAPTIVE
-// 80.8 -> 79.0 us.
+// computed so that it cannot see through it.  Measured beside the scalar form:
+// 32 frames in the batch kernel 1,363 -> 1,309 us, the near 4K FAST frame 1,097
+// -> 1,067 us, ADAPTIVE 80.8 -> 79.0 us.
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pair(float a, float b)
 {
@@ -467,9 +468,9 @@ __device__ __forceinline__ f32x2 quot2(f32x2 a, f32x2 nd, f32x2 y)   // nd = -d
 }
 
 // -0 twice, where ptxas does not see what it holds: as an operand in constant
-// memory it costs the batch kernel no registers (32 frames 1,324 -> 1,314 us, the mixed
-// batch 815 -> 809); the other kernels do better with one computed per ray (near 4K FAST frame 1,056 against
-// 1,063 us).
+// memory it costs the batch kernel no registers (32 frames 1,324 -> 1,314 us, the
+// mixed batch 815 -> 809); the other kernels do better with one computed per ray
+// (near 4K FAST frame 1,056 against 1,063 us).
 static __constant__ f32x2 c_mzero = 0x8000000080000000ull;
 
 // Whether the mirrored search may make this search.
@@ -627,16 +628,18 @@ __device__ __forceinline__ int trace_mirrored(const DevTree &t, uint32_t start, 
                 d2 = __fadd_rn(__fadd_rn(d2, t2), __fsub_rn(z2, ez));
                 d0 = v0 ? d0 : inf; d1 = v1 ? d1 : inf; d2 = v2 ? d2 : inf;
                 if (fminf(fminf(d0, d1), d2) < DIST_MIN) return STEP_AGAIN;
-                // oij: crossing i comes before crossing j.  The selection sort with immediate swaps keeps
-                // equal distances in axis order, except that crossing 2 before an equal pair 0, 1 turns it round
+                // oij: crossing i comes before crossing j.  The selection sort with immediate
+                // swaps keeps equal distances in axis order, except that crossing 2 before an
+                // equal pair 0, 1 turns it round
                 const bool o20 = d2 < d0, o21 = d2 < d1, o10 = d1 < d0 || (d1 == d0 && o20);
                 // the octant behind each crossing (:137): the bits of the crossings up to it flipped
                 const uint32_t s0 = sub ^ 1u ^ (o10 ? 2u : 0u) ^ (o20 ? 4u : 0u);
                 const uint32_t s1 = sub ^ 2u ^ (o10 ? 0u : 1u) ^ (o21 ? 4u : 0u);
                 const uint32_t s2 = sub ^ 4u ^ (o20 ? 0u : 1u) ^ (o21 ? 0u : 2u);
-                // the children's bits, at the bottom, and above them the siblings that follow: one shift gives
-                // both whether a child is there and, counted back from the block's end, its record (32 orbit
-                // frames in the batch kernel 1,305 -> 1,277 us, against the siblings before it masked and counted)
+                // the children's bits, at the bottom, and above them the siblings that follow:
+                // one shift gives both whether a child is there and, counted back from the
+                // block's end, its record (32 orbit frames in the batch kernel 1,305 -> 1,277
+                // us, against the siblings before it masked and counted)
                 const uint32_t r0 = mask >> s0, r1 = mask >> s1, r2 = mask >> s2, r3 = mask >> sub;
                 const uint32_t end = link + VOXP_REC_UNITS * (uint32_t)__popc(mask);
                 const bool w0 = v0 && (r0 & 1u), w1 = v1 && (r1 & 1u), w2 = v2 && (r2 & 1u);
@@ -825,7 +828,8 @@ __device__ __forceinline__ bool trace_ball(const DevTree &t, float cx, float cy,
  * child's own distance there is at least the radius, its square at least the
  * radius's square (ball_side).
  *
- * What bounds the search is instruction issue at few active lanes.  A ball
+ * What bounds the search is instruction issue at few active lanes (7 of 32 in
+ * 73% of the slots for 1M balls) and the loads waited for beside it.  A ball
  * small beside the upper nodes can meet one or two of their eight children,
  * so leaving the others out takes a search from 45 box tests to 13 on
  * average (balls of radius 0.5-8 in the 256^3 tree), and the child where the

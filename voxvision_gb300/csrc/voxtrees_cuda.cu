@@ -127,8 +127,9 @@ __global__ void __launch_bounds__(RAY_THREADS) ray_kernel(DevTree t, const float
         RayHit h;
         bool hit = false;
         if (start != VOXP_EMPTY)
-            // a ray is read once: streaming loads leave the caches to the tree (4M incoherent rays of the 256^3
-            // tree, gathered in their order, 528 -> 488 us; copied into order as 32-byte records first, 486)
+            // a ray is read once: streaming loads leave the caches to the tree (4M
+            // incoherent rays of the 256^3 tree, gathered in their order, 528 -> 488 us;
+            // copied into order as 32-byte records first, 486)
             hit = vox::trace_ray<CAP, COUNT>(t, start, __ldcs(o + 3 * i), __ldcs(o + 3 * i + 1), __ldcs(o + 3 * i + 2),
                                              __ldcs(d + 3 * i), __ldcs(d + 3 * i + 1), __ldcs(d + 3 * i + 2), h, c,
                                              overflow);
@@ -593,8 +594,9 @@ cudaError_t launch_balls(const vox_cuda_tree *t, const float *c, const float *r,
         }
     }
     // A tree of ordered, nested boxes: the search that may choose its own order
-    // (1M balls of radius 0.5-8 over the 256^3 tree: 185 us against 341).  Counting calls count the reference's work, and other
-    // trees (image_shape) take its own order.
+    // (1M balls of radius 0.5-8 over the 256^3 tree: 182 us against 341).  Counting
+    // calls count the reference's work, and other trees (image_shape) take its own
+    // order.
     if (nested) {
         const uint32_t lanes = query_lanes(n);
         const dim3 block(BALL_THREADS), grid(query_blocks(n, lanes, BALL_THREADS));
@@ -1866,10 +1868,10 @@ static uint32_t *host_call_frame(HostCallState *hc, size_t bytes)
 // traced rectangle m, into the host buffer argb: the zeros outside the
 // rectangle from the copy stream, which starts at once and runs beside the
 // kernel, then the rectangle once the kernel is done (on s, which also waits
-// for the zeros).  A 1080p orbit frame, BEST / ADAPTIVE: 140 / 167 us into a
-// page-locked frame against 148 / 176 drawn in place over the host link,
-// 147 / 175 us into a pageable one against 183 / 211 with the whole frame
-// copied after the kernel.
+// for the zeros).  With the general search a 1080p orbit frame, BEST / ADAPTIVE,
+// took 140 / 167 us into a page-locked frame (BEST 93 since the mirrored one)
+// against 148 / 176 drawn in place over the host link, 147 / 175 us into a
+// pageable one against 183 / 211 with the whole frame copied after the kernel.
 static cudaError_t host_frame_out(HostCallState *hc, uint32_t *argb, const uint32_t *d_argb, uint32_t w, uint32_t h,
                                   const FrameMemo &m, cudaStream_t s)
 {
